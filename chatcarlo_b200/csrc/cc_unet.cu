@@ -105,6 +105,20 @@ __device__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     }
 }
 
+// One lane of a converged warp.  The tensor-core instructions take their
+// descriptors from uniform registers: issued under elect.sync by a warp
+// whose control flow and operands are uniform they cost one instruction
+// each, while a thread picked by `lane == 0` makes the compiler serialise
+// every one of them over the lanes that might be active.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+// The warp's index as a value the compiler knows to be warp-uniform.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // One arrival on an mbarrier (release semantics, CTA scope).
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar))
@@ -124,6 +138,12 @@ __device__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity, volatile int* 
             return false;
         }
     }
+}
+
+// mbar_wait_or_fail by a whole converged warp: true where every lane saw
+// the phase complete, the same for all lanes.
+__device__ __forceinline__ bool warp_wait_or_fail(uint64_t* bar, uint32_t parity, volatile int* fail) {
+    return __all_sync(0xffffffffu, mbar_wait_or_fail(bar, parity, fail)) != 0;
 }
 
 // The mbarrier receives one arrival when all of this thread's earlier
@@ -409,7 +429,7 @@ __global__ void __launch_bounds__(THREADS) conv_kernel(const ConvP P) {
     __shared__ uint64_t bar[NS];
     __shared__ uint32_t s_tmem;
     __shared__ int s_off[27];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const Src& S = P.src;
     const int cin = S.ca + S.cb;
     const int n_stages = (27 * cin + KS - 1) / KS;
@@ -451,7 +471,7 @@ __global__ void __launch_bounds__(THREADS) conv_kernel(const ConvP P) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     const uint32_t sbase = smem_u32(smem);
     constexpr uint32_t IDESC = idesc_bf16(TILE_M, N, 0, 0);
 
@@ -491,7 +511,7 @@ __global__ void __launch_bounds__(THREADS) conv_kernel(const ConvP P) {
         cp_async_wait<NS - 2>();                     // this thread's copies of stage it landed
         fence_proxy_async();                         // ... and are visible to the tensor core
         if (!__syncthreads_and(ok)) { ok = false; break; }
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             tc_fence_after();
             const uint32_t a0 = sbase + (uint32_t)(it % NS) * STAGE, b0 = a0 + A_BYTES;
 #pragma unroll
@@ -1113,7 +1133,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
     __shared__ uint64_t full[WS_RING_MAX], empty[WS_RING_MAX], rfull[PS_REGIONS_MAX], rfree[PS_REGIONS_MAX];
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const Src& S = P.src;
     const int c8n = (S.ca + S.cb) / 8, c8p = Q.c8_hi - Q.c8_lo;
     const int tiles_x = (S.W + 7) / 8, tiles_y = (S.H + 15) / 16;
@@ -1150,7 +1170,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
     if (warp >= 1 && warp <= 3) {
         // ---- loaders: planes zs - 1 .. ze of each segment, channel groups of the pass ----
@@ -1187,7 +1207,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
             }
         }
         cp_async_wait<0>();
-    } else if (warp == 0 && lane == 0) {
+    } else if (warp == 0) {
         // ---- MMA issuer: per input plane one chain of 9 x c8p / 2 MMAs; the chains of a
         // group of planes are issued tap by tap in turn ----
         const uint64_t a0 = smem_desc(sbase, RING_V * 16, HALO_X * 16);
@@ -1202,7 +1222,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
         // plane L's ring slot and region with their phases, advanced without divisions
         uint32_t L = 0, fs = 0, fph = 0, rs = 0, rph = 0;
         bool ok = true;
-        while (L < n_planes && ok && !*fail) {
+        while (L < n_planes && ok) {
             const uint32_t gn = min((uint32_t)G, n_planes - L);      // G but for the CTA's last group
             uint32_t d[G], so[G], fsk[G], rsk[G];
             {
@@ -1214,8 +1234,8 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
                     d[k] = tmem + r * RC;
                     so[k] = f * slot16;
                     if (G == 1 || (uint32_t)k < gn) {
-                        if (ok) ok = mbar_wait_or_fail(&full[f], fp, fail);
-                        if (ok && L + k >= NQ) ok = mbar_wait_or_fail(&rfree[r], rp ^ 1u, fail);
+                        if (ok) ok = warp_wait_or_fail(&full[f], fp, fail);
+                        if (ok && L + k >= NQ) ok = warp_wait_or_fail(&rfree[r], rp ^ 1u, fail);
                     }
                     ring_next(f, fp, R);
                     ring_next(r, rp, NQ);
@@ -1224,24 +1244,27 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
             if (!ok) break;
             fence_proxy_async();              // the loaders' copies, seen through the barrier, to the tensor core
             tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
-            for (int t9 = 0; t9 < 9; ++t9) {
-                const uint32_t ta = (uint32_t)((t9 / 3) * HALO_X + t9 % 3);
-                for (int j = 0; j < c8p / 2; ++j) {
-                    const uint64_t bd = b0 + (uint32_t)((t9 * c8p + 2 * j) * NP);
-                    const uint32_t acc = (t9 > 0 || j > 0) ? 1u : 0u;
+                for (int t9 = 0; t9 < 9; ++t9) {
+                    const uint32_t ta = (uint32_t)((t9 / 3) * HALO_X + t9 % 3);
+                    for (int j = 0; j < c8p / 2; ++j) {
+                        const uint64_t bd = b0 + (uint32_t)((t9 * c8p + 2 * j) * NP);
+                        const uint32_t acc = (t9 > 0 || j > 0) ? 1u : 0u;
 #pragma unroll
-                    for (int k = 0; k < G; ++k)
-                        if (G == 1 || (uint32_t)k < gn)
-                            mma_bf16(d[k], a0 + so[k] + ta + (uint32_t)(2 * j * RING_V), bd, IDESC, acc);
+                        for (int k = 0; k < G; ++k)
+                            if (G == 1 || (uint32_t)k < gn)
+                                mma_bf16(d[k], a0 + so[k] + ta + (uint32_t)(2 * j * RING_V), bd, IDESC, acc);
+                    }
                 }
+#pragma unroll
+                for (int k = 0; k < G; ++k)
+                    if (G == 1 || (uint32_t)k < gn) {
+                        mma_commit(&rfull[rsk[k]]);
+                        mma_commit(&empty[fsk[k]]);
+                    }
             }
-#pragma unroll
-            for (int k = 0; k < G; ++k)
-                if (G == 1 || (uint32_t)k < gn) {
-                    mma_commit(&rfull[rsk[k]]);
-                    mma_commit(&empty[fsk[k]]);
-                }
+            __syncwarp();
             for (uint32_t k = 0; k < gn; ++k) {
                 ring_next(fs, fph, R);
                 ring_next(rs, rph, NQ);
@@ -1542,7 +1565,7 @@ __global__ void __launch_bounds__(THREADS) wgrad_tma_kernel(const __grid_constan
     __shared__ uint64_t full[NS], empty[NS], done;
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int r0 = blockIdx.x * TILE_M;
     const long long s_begin = P.stages * blockIdx.y / gridDim.y;
     const int n_st = (int)(P.stages * (blockIdx.y + 1) / gridDim.y - s_begin);
@@ -1561,7 +1584,7 @@ __global__ void __launch_bounds__(THREADS) wgrad_tma_kernel(const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     const uint32_t sbase = (smem_u32(smem) + 1023u) & ~1023u;     // the launch adds 1 KB of slack
 
     if (warp == 0) {
@@ -1610,23 +1633,28 @@ __global__ void __launch_bounds__(THREADS) wgrad_tma_kernel(const __grid_constan
         // after a failure, the copies still in flight land before the CTA ends
         if (lane == 0 && *fail)
             for (int s = max(0, issued - NS); s < issued; ++s) mbar_wait(&full[s % NS], (uint32_t)(s / NS) & 1u);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // ---- MMAs: four of K = 16 voxels per stage ----
         constexpr uint32_t IDESC = idesc_bf16(TILE_M, N, 1, 1);
         const uint32_t ar = 2u * (uint32_t)P.a_ch, al = swizzle_layout((int)ar);      // A row bytes, layout
         constexpr uint32_t BR = 2u * B_CH, BL = swizzle_layout(2 * B_CH);
         for (int s = 0; s < n_st; ++s) {
             const int slot = s % NS;
-            if (!mbar_wait_or_fail(&full[slot], (uint32_t)(s / NS) & 1u, fail)) break;
+            if (!warp_wait_or_fail(&full[slot], (uint32_t)(s / NS) & 1u, fail)) break;
             tc_fence_after();
             const uint32_t a0 = sbase + (uint32_t)slot * STAGE, b0 = a0 + A_BYTES;
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < KSTAGE / 16; ++k)
-                mma_bf16(tmem, smem_desc_sw(a0 + k * 16 * ar, KSTAGE * ar, 8 * ar, al),
-                         smem_desc_sw(b0 + k * 16 * BR, KSTAGE * BR, 8 * BR, BL), IDESC, (s > 0 || k > 0) ? 1u : 0u);
-            mma_commit(&empty[slot]);
+                for (int k = 0; k < KSTAGE / 16; ++k)
+                    mma_bf16(tmem, smem_desc_sw(a0 + k * 16 * ar, KSTAGE * ar, 8 * ar, al),
+                             smem_desc_sw(b0 + k * 16 * BR, KSTAGE * BR, 8 * BR, BL), IDESC,
+                             (s > 0 || k > 0) ? 1u : 0u);
+                mma_commit(&empty[slot]);
+            }
+            __syncwarp();
         }
-        mma_commit(&done);          // arrives once every MMA issued above has finished
+        if (elect_one()) mma_commit(&done);          // arrives once every MMA issued above has finished
+        __syncwarp();
     }
     // ---- epilogue: the accumulator into dw ----
     if (lane == 0) mbar_wait_or_fail(&done, 0u, fail);
