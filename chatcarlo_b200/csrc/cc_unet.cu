@@ -246,6 +246,14 @@ __device__ __forceinline__ void tmem_ld8_nw(uint32_t taddr, uint32_t r[8]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr));
 }
+// the same for 16 columns
+__device__ __forceinline__ void tmem_ld16_nw(uint32_t taddr, uint32_t r[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                 "%14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ uint4 pack_bf16x8(const float f[8]) {
@@ -1092,6 +1100,7 @@ __global__ void __launch_bounds__(THREADS, 4) conv_ws_kernel(const ConvP P, int 
 // a layer with more (64 output channels: two slices of 32).
 constexpr int PS_REGIONS_MAX = 8;
 constexpr int PS_GROUP_MAX = 3;
+constexpr int PS_LV = (RING_V + WS_LOADERS / 2 - 1) / (WS_LOADERS / 2);     // halo voxels of a loader thread
 
 // tensor-memory columns of one region: 3 x cout
 __host__ __device__ constexpr uint32_t ps_region_cols(int n) { return 3u * (uint32_t)n; }
@@ -1151,7 +1160,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
         }
         for (uint32_t r = 0; r < NQ; ++r) {
             mbar_init(&rfull[r], 1);
-            mbar_init(&rfree[r], 128);
+            mbar_init(&rfree[r], 4);                // one arrival per epilogue warp
         }
         s_fail = 0;
         mbar_init_fence();
@@ -1177,31 +1186,46 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
         // Each thread's copies of a plane arrive on the slot's "full" barrier
         // when they land, so the loaders never wait for their own copies:
         // as many planes are in flight as the ring has free slots.
-        const int lt = tid - 32;
+        // Threads 2 i and 2 i + 1 copy the two 8-channel halves of the same
+        // voxel's 16 channels, so that a warp reads whole 32-byte sectors and
+        // its 16-byte stores fall into different banks (a chunk plane is
+        // 720 words long); their voxels' offsets within a plane are fixed
+        // for a segment, a plane only moves the base.
+        const int lt = tid - 32, half = lt & 1;
+        const int na = max(0, min(Q.c8_hi, S.ca / 8) - Q.c8_lo) / 2, nb = c8p / 2 - na;   // 16-channel groups from a, b
+        const int ch_a = (Q.c8_lo + half) * 8, ch_b = (Q.c8_lo + 2 * na + half) * 8 - S.ca;
         uint32_t L = 0, slot = 0, ph = 0;             // plane, its ring slot and the slot's phase
         for (long long g = g_begin; g < g_end && !*fail;) {
             const WsSeg q = ws_segment(S, g, g_end, tiles_x, tiles_y);
             g += q.ze - q.zs;
+            long long oa[PS_LV], ob[PS_LV];
+            uint32_t in = 0;
+#pragma unroll
+            for (int j = 0; j < PS_LV; ++j) {
+                const int hv = (lt >> 1) + j * (WS_LOADERS / 2);
+                const int yy = q.y0 + hv / HALO_X - 1, xx = q.x0 + hv % HALO_X - 1;
+                const bool ok = (unsigned)yy < (unsigned)S.H && (unsigned)xx < (unsigned)S.W;
+                if (ok) in |= 1u << j;
+                oa[j] = ok ? ((long long)yy * S.W + xx) * S.ca + ch_a : 0;
+                ob[j] = ok && nb > 0 ? ((long long)(yy >> 1) * (S.W >> 1) + (xx >> 1)) * S.cb + ch_b : 0;
+            }
             for (int zz = q.zs - 1; zz <= q.ze && !*fail; ++zz, ++L, ring_next(slot, ph, R)) {
                 if (L >= R && !mbar_wait_or_fail(&empty[slot], ph ^ 1u, fail)) break;
-                const uint32_t base = sbase + slot * slot16 * 16;
-                for (int i = lt; i < c8p * RING_V; i += WS_LOADERS) {
-                    const int c8 = i / RING_V, hv = i - c8 * RING_V;
-                    const int yy = q.y0 + hv / HALO_X - 1, xx = q.x0 + hv % HALO_X - 1;
-                    const int ch = (Q.c8_lo + c8) * 8;
-                    uint32_t bytes = 0;
-                    const void* src = S.a;
-                    if ((unsigned)zz < (unsigned)S.D && (unsigned)yy < (unsigned)S.H && (unsigned)xx < (unsigned)S.W) {
-                        bytes = 16;
-                        if (ch < S.ca) {
-                            src = S.a + ((((size_t)q.n * S.D + zz) * S.H + yy) * S.W + xx) * S.ca + ch;
-                        } else {
-                            const size_t cv = (((size_t)q.n * (S.D >> 1) + (zz >> 1)) * (S.H >> 1) + (yy >> 1)) *
-                                                  (S.W >> 1) + (xx >> 1);
-                            src = S.b + cv * S.cb + (ch - S.ca);
-                        }
-                    }
-                    cp_async16_cg(base + (uint32_t)i * 16, src, bytes);
+                const uint32_t dst0 = sbase + (slot * slot16 + (uint32_t)(half * RING_V + (lt >> 1))) * 16;
+                const bool zin = (unsigned)zz < (unsigned)S.D;
+                const __nv_bfloat16* pa = S.a + (zin ? ((size_t)q.n * S.D + zz) * S.H * S.W * S.ca : 0);
+                const __nv_bfloat16* pb =
+                    nb > 0 ? S.b + (zin ? ((size_t)q.n * (S.D >> 1) + (zz >> 1)) * (S.H >> 1) * (S.W >> 1) * S.cb : 0)
+                           : nullptr;
+#pragma unroll
+                for (int j = 0; j < PS_LV; ++j) {
+                    if ((lt >> 1) + j * (WS_LOADERS / 2) >= RING_V) break;
+                    const uint32_t bytes = zin && ((in >> j) & 1u) ? 16u : 0u;
+                    uint32_t dst = dst0 + (uint32_t)(j * (WS_LOADERS / 2)) * 16;
+                    const __nv_bfloat16* src = pa + oa[j];
+                    for (int c = 0; c < na; ++c, dst += 2 * RING_V * 16) cp_async16_cg(dst, src + (bytes ? c * 16 : 0), bytes);
+                    src = pb + ob[j];
+                    for (int c = 0; c < nb; ++c, dst += 2 * RING_V * 16) cp_async16_cg(dst, src + (bytes ? c * 16 : 0), bytes);
                 }
                 cp_async_arrive_noinc(&full[slot]);
             }
@@ -1275,84 +1299,119 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
         if (L > 0) mbar_wait(&rfull[rs == 0 ? NQ - 1 : rs - 1], rs == 0 ? rph ^ 1u : rph);
     } else if (warp >= 4) {
         // ---- epilogue: output z = D_{z-1}[dz 0] + D_z[dz 1] + D_{z+1}[dz 2]; row m, lane quarter warp - 4 ----
+        // The voxel's other operands (mask, partial sum, head input) are read
+        // before the wait for the tensor core, the biases once per CTA; a
+        // region is handed back as soon as its values are in registers.
         const int qw = warp - 4, m = qw * 32 + lane;
         const uint32_t lq = (uint32_t)(qw * 32) << 16;
+        float bias[NO];
+#pragma unroll
+        for (int c = 0; c < NO; ++c) bias[c] = P.bias && !Q.part_out ? __ldg(P.bias + Q.co_lo + c) : 0.0f;
         // region and phase of plane z + 1, and the regions of planes z and z - 1
         uint32_t r1 = 0, ph1 = 0;
         ring_next(r1, ph1, NQ);
         ring_next(r1, ph1, NQ);                                // the first output reads planes 0, 1, 2
-        for (long long g = g_begin; g < g_end && !*fail;) {
+        bool ok = true;
+        for (long long g = g_begin; g < g_end && ok;) {
             const WsSeg q = ws_segment(S, g, g_end, tiles_x, tiles_y);
             g += q.ze - q.zs;
             const int y = q.y0 + (m >> 3), x = q.x0 + (m & 7);
             const bool in = y < S.H && x < S.W;
-            bool ok = true;
-            for (int z = q.zs; z < q.ze; ++z, ring_next(r1, ph1, NQ)) {
+            long long v = (((long long)q.n * S.D + q.zs) * S.H + y) * S.W + x;
+            for (int z = q.zs; z < q.ze; ++z, v += (long long)S.H * S.W, ring_next(r1, ph1, NQ)) {
                 const uint32_t r0i = r1 == 0 ? NQ - 1 : r1 - 1, rmi = r0i == 0 ? NQ - 1 : r0i - 1;
-                int w = 1;
-                if (lane == 0) w = mbar_wait_or_fail(&rfull[r1], ph1, fail) ? 1 : 0;
-                if (!__shfl_sync(0xffffffffu, w, 0)) {
-                    ok = false;
-                    break;
+                // the head: x + b, then + w_j a_j in channel order (the head kernel's FP32 sequence)
+                const bool head = NO == 16 && P.head && in;
+                float hsum = head ? P.head_x[v] + __ldg(P.head + 16) : 0.0f;
+                // output channels [c0, c0 + 8) of this launch go to out0 or out1 (split is a multiple of 8)
+                uint4 mk[NO / 8];
+                if (P.mask0 && in && !Q.part_out) {
+#pragma unroll
+                    for (int h = 0; h < NO / 8; ++h)
+                        if (Q.co_lo + 8 * h < P.split)
+                            mk[h] = __ldg(reinterpret_cast<const uint4*>(P.mask0 + (size_t)v * P.split + Q.co_lo + 8 * h));
                 }
+                float4 part[NO / 4];
+                if (Q.part_in && in) {
+#pragma unroll
+                    for (int h = 0; h < NO / 4; ++h)
+                        part[h] = __ldg(reinterpret_cast<const float4*>(Q.part_in + (size_t)v * NO) + h);
+                }
+                ok = warp_wait_or_fail(&rfull[r1], ph1, fail);
+                if (!ok) break;
                 tc_fence_after();
                 const uint32_t rm = tmem + rmi * RC + lq;
                 const uint32_t r0 = tmem + r0i * RC + NO + lq;
                 const uint32_t rp = tmem + r1 * RC + 2 * NO + lq;
-                const long long v = (((long long)q.n * S.D + z) * S.H + y) * S.W + x;
-                // the head: x + b, then + w_j a_j in channel order (the head kernel's FP32 sequence)
-                const bool head = NO == 16 && P.head && in;
-                float hsum = head ? P.head_x[v] + __ldg(P.head + 16) : 0.0f;
-                // the three regions' loads of 16 channels in flight together
 #pragma unroll
                 for (int c0 = 0; c0 < NO; c0 += 16) {
-                    uint32_t u[6][8];
-                    tmem_ld8_nw(rm + (uint32_t)c0, u[0]);
-                    tmem_ld8_nw(r0 + (uint32_t)c0, u[1]);
-                    tmem_ld8_nw(rp + (uint32_t)c0, u[2]);
-                    tmem_ld8_nw(rm + (uint32_t)c0 + 8, u[3]);
-                    tmem_ld8_nw(r0 + (uint32_t)c0 + 8, u[4]);
-                    tmem_ld8_nw(rp + (uint32_t)c0 + 8, u[5]);
+                    uint32_t um[16], u0[16], up[16];
+                    tmem_ld16_nw(rm + (uint32_t)c0, um);
+                    tmem_ld16_nw(r0 + (uint32_t)c0, u0);
+                    tmem_ld16_nw(rp + (uint32_t)c0, up);
                     tmem_wait_ld();
-                    if (!in) continue;
+                    // the uses below stay behind the wait
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int c = c0 + 8 * h;
-                        float f[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            f[j] = (__uint_as_float(u[3 * h][j]) + __uint_as_float(u[3 * h + 1][j])) +
-                                   __uint_as_float(u[3 * h + 2][j]);
-                        if (Q.part_in) {
-                            const float4* pi = reinterpret_cast<const float4*>(Q.part_in + (size_t)v * NO + c);
-                            const float4 u0 = __ldg(pi), u1 = __ldg(pi + 1);
-                            f[0] += u0.x, f[1] += u0.y, f[2] += u0.z, f[3] += u0.w;
-                            f[4] += u1.x, f[5] += u1.y, f[6] += u1.z, f[7] += u1.w;
-                        }
-                        if (Q.part_out) {
-                            float4* po = reinterpret_cast<float4*>(Q.part_out + (size_t)v * NO + c);
-                            po[0] = make_float4(f[0], f[1], f[2], f[3]);
-                            po[1] = make_float4(f[4], f[5], f[6], f[7]);
-                        } else {
-                            conv_store(P, v, Q.co_lo + c, Q.n_out, f);
-                            if (head) {
-#pragma unroll
-                                for (int j = 0; j < 8; ++j)
-                                    hsum = fmaf(__ldg(P.head + c + j), __bfloat162float(__float2bfloat16_rn(f[j])),
-                                                hsum);
+                    for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(um[j]), "+r"(u0[j]), "+r"(up[j]));
+                    if (c0 + 16 == NO) {                       // plane z - 1: last reader done
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) {
+                            mbar_arrive(&rfree[rmi]);
+                            if (z == q.ze - 1) {
+                                mbar_arrive(&rfree[r0i]);
+                                mbar_arrive(&rfree[r1]);
                             }
                         }
                     }
+                    if (in) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int c = c0 + 8 * h, co = Q.co_lo + c;
+                            float f[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                f[j] = (__uint_as_float(um[8 * h + j]) + __uint_as_float(u0[8 * h + j])) +
+                                       __uint_as_float(up[8 * h + j]);
+                            if (Q.part_in) {
+                                const float4 p0 = part[c / 4], p1 = part[c / 4 + 1];
+                                f[0] += p0.x, f[1] += p0.y, f[2] += p0.z, f[3] += p0.w;
+                                f[4] += p1.x, f[5] += p1.y, f[6] += p1.z, f[7] += p1.w;
+                            }
+                            if (Q.part_out) {
+                                float4* po = reinterpret_cast<float4*>(Q.part_out + (size_t)v * NO + c);
+                                po[0] = make_float4(f[0], f[1], f[2], f[3]);
+                                po[1] = make_float4(f[4], f[5], f[6], f[7]);
+                                continue;
+                            }
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                if (P.bias) f[j] += bias[c + j];
+                                if (P.relu) f[j] = fmaxf(f[j], 0.0f);
+                            }
+                            if (co < P.split) {
+                                if (P.mask0) {
+                                    float t[8];
+                                    unpack_bf16x8(mk[c / 8], t);
+#pragma unroll
+                                    for (int j = 0; j < 8; ++j) f[j] = t[j] > 0.0f ? f[j] : 0.0f;
+                                }
+                                if (P.out0) *reinterpret_cast<uint4*>(P.out0 + (size_t)v * P.split + co) = pack_bf16x8(f);
+                            } else {
+                                *reinterpret_cast<uint4*>(P.out1 + (size_t)v * (Q.n_out - P.split) + (co - P.split)) =
+                                    pack_bf16x8(f);
+                            }
+                            if (head) {
+#pragma unroll
+                                for (int j = 0; j < 8; ++j)
+                                    hsum = fmaf(__ldg(P.head + c + j), __bfloat162float(__float2bfloat16_rn(f[j])), hsum);
+                            }
+                        }
+                    }
+                    __syncwarp();                              // the next loads are warp-wide
                 }
                 if (head) P.head_out[v] = hsum;
-                tc_fence_before();
-                mbar_arrive(&rfree[rmi]);                               // plane z - 1: last reader done
-                if (z == q.ze - 1) {
-                    mbar_arrive(&rfree[r0i]);
-                    mbar_arrive(&rfree[r1]);
-                }
             }
-            if (!ok) break;
             // the next segment's first output reads its planes 0 .. 2: two planes on
             ring_next(r1, ph1, NQ);
             ring_next(r1, ph1, NQ);
