@@ -223,6 +223,19 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b
         ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
 
+// mma_bf16 with each descriptor as its low word (start address and leading
+// offset, the part that moves) and its high word (constant): 32-bit adds.
+__device__ __forceinline__ void mma_bf16_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                            uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %2};\n\t"
+        "mov.b64 db, {%3, %4};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc));
+}
+
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                      smem_u32(bar))
@@ -255,6 +268,24 @@ __device__ __forceinline__ void tmem_ld16_nw(uint32_t taddr, uint32_t r[16]) {
                  : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// N consecutive columns (8 or 16) without the wait
+template <int N>
+__device__ __forceinline__ void tmem_ld_nw(uint32_t taddr, uint32_t r[N]) {
+    if constexpr (N == 16) tmem_ld16_nw(taddr, r);
+    else tmem_ld8_nw(taddr, r);
+}
+
+// Two FP32 sums in one instruction, each rounded as a single add.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 a, b, c;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+        "add.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
 
 __device__ __forceinline__ uint4 pack_bf16x8(const float f[8]) {
     uint4 u;
@@ -1100,6 +1131,8 @@ __global__ void __launch_bounds__(THREADS, 4) conv_ws_kernel(const ConvP P, int 
 // a layer with more (64 output channels: two slices of 32).
 constexpr int PS_REGIONS_MAX = 8;
 constexpr int PS_GROUP_MAX = 3;
+constexpr int PS_THREADS = 384;             // warp 0 MMA, 1-3 loaders, 4-11 epilogue
+constexpr int PS_EPI_WARPS = 8;
 constexpr int PS_LV = (RING_V + WS_LOADERS / 2 - 1) / (WS_LOADERS / 2);     // halo voxels of a loader thread
 
 // tensor-memory columns of one region: 3 x cout
@@ -1132,8 +1165,22 @@ struct PsPass {
     float* part_out;           // FP32 sums [v][NO] out (no bias / ReLU / BF16), or null
 };
 
-template <int NO, int G>
-__global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, const PsPass Q, int ring) {
+// An epilogue warp is done with the region of plane z - 1 and, at a
+// segment's end, with those of planes z and z + 1.
+__device__ __forceinline__ void ps_release(uint64_t* rfree, int lane, uint32_t rm, uint32_t r0, uint32_t rp, bool last) {
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) {
+        mbar_arrive(&rfree[rm]);
+        if (last) {
+            mbar_arrive(&rfree[r0]);
+            mbar_arrive(&rfree[rp]);
+        }
+    }
+}
+
+template <int NO, int G, int C8P>
+__global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_ps_kernel(const ConvP P, const PsPass Q, int ring) {
     constexpr int NP = 3 * NO;                                // MMA N: the three dz weight planes
     constexpr uint32_t RC = ps_region_cols(NO);
     constexpr uint32_t NQ = (uint32_t)ps_regions(G), TCOLS = ps_tmem_cols(NO, G);
@@ -1144,7 +1191,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
     __shared__ int s_fail;
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const Src& S = P.src;
-    const int c8n = (S.ca + S.cb) / 8, c8p = Q.c8_hi - Q.c8_lo;
+    const int c8n = (S.ca + S.cb) / 8, c8p = C8P > 0 ? C8P : Q.c8_hi - Q.c8_lo;
     const int tiles_x = (S.W + 7) / 8, tiles_y = (S.H + 15) / 16;
     const long long total = (long long)S.B * tiles_y * tiles_x * S.D;
     const long long g_begin = total * blockIdx.x / gridDim.x, g_end = total * (blockIdx.x + 1) / gridDim.x;
@@ -1160,14 +1207,14 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
         }
         for (uint32_t r = 0; r < NQ; ++r) {
             mbar_init(&rfull[r], 1);
-            mbar_init(&rfree[r], 4);                // one arrival per epilogue warp
+            mbar_init(&rfree[r], PS_EPI_WARPS);
         }
         s_fail = 0;
         mbar_init_fence();
     }
     // weights: packed chunk (tap * c8n + c8, co_lo + co) -> (t9 * c8p + c8 - c8_lo, dz * NO + co)
     const uint32_t sbase = smem_u32(smem), swt = sbase + R * slot16 * 16;
-    for (int i = tid; i < 9 * c8p * NP; i += THREADS) {
+    for (int i = tid; i < 9 * c8p * NP; i += PS_THREADS) {
         const int r = i % NP, g = i / NP;
         const int t9 = g / c8p, c8 = Q.c8_lo + g % c8p, dz = r / NO, co = r % NO;
         const int src = ((dz * 9 + t9) * c8n + c8) * Q.n_out + Q.co_lo + co;
@@ -1194,38 +1241,44 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
         const int lt = tid - 32, half = lt & 1;
         const int na = max(0, min(Q.c8_hi, S.ca / 8) - Q.c8_lo) / 2, nb = c8p / 2 - na;   // 16-channel groups from a, b
         const int ch_a = (Q.c8_lo + half) * 8, ch_b = (Q.c8_lo + 2 * na + half) * 8 - S.ca;
+        const long long step_a = (long long)S.H * S.W * S.ca;                  // elements of a plane of a, of b
+        const long long step_b = (long long)(S.H >> 1) * (S.W >> 1) * S.cb;
         uint32_t L = 0, slot = 0, ph = 0;             // plane, its ring slot and the slot's phase
         for (long long g = g_begin; g < g_end && !*fail;) {
             const WsSeg q = ws_segment(S, g, g_end, tiles_x, tiles_y);
             g += q.ze - q.zs;
-            long long oa[PS_LV], ob[PS_LV];
-            uint32_t in = 0;
+            // this thread's voxels in plane zs - 1 (read only where they lie inside the volume)
+            const __nv_bfloat16 *pa[PS_LV], *pb[PS_LV];
+            uint32_t bytes[PS_LV];
 #pragma unroll
             for (int j = 0; j < PS_LV; ++j) {
                 const int hv = (lt >> 1) + j * (WS_LOADERS / 2);
                 const int yy = q.y0 + hv / HALO_X - 1, xx = q.x0 + hv % HALO_X - 1;
                 const bool ok = (unsigned)yy < (unsigned)S.H && (unsigned)xx < (unsigned)S.W;
-                if (ok) in |= 1u << j;
-                oa[j] = ok ? ((long long)yy * S.W + xx) * S.ca + ch_a : 0;
-                ob[j] = ok && nb > 0 ? ((long long)(yy >> 1) * (S.W >> 1) + (xx >> 1)) * S.cb + ch_b : 0;
+                bytes[j] = ok ? 16u : 0u;
+                pa[j] = S.a + ((long long)q.n * S.D + q.zs - 1) * step_a + (ok ? ((long long)yy * S.W + xx) * S.ca : 0) + ch_a;
+                pb[j] = nb > 0 ? S.b + ((long long)q.n * (S.D >> 1) + ((q.zs - 1) >> 1)) * step_b +
+                                     (ok ? ((long long)(yy >> 1) * (S.W >> 1) + (xx >> 1)) * S.cb : 0) + ch_b
+                               : nullptr;
             }
-            for (int zz = q.zs - 1; zz <= q.ze && !*fail; ++zz, ++L, ring_next(slot, ph, R)) {
+            for (int zz = q.zs - 1; zz <= q.ze; ++zz, ++L, ring_next(slot, ph, R)) {
                 if (L >= R && !mbar_wait_or_fail(&empty[slot], ph ^ 1u, fail)) break;
                 const uint32_t dst0 = sbase + (slot * slot16 + (uint32_t)(half * RING_V + (lt >> 1))) * 16;
                 const bool zin = (unsigned)zz < (unsigned)S.D;
-                const __nv_bfloat16* pa = S.a + (zin ? ((size_t)q.n * S.D + zz) * S.H * S.W * S.ca : 0);
-                const __nv_bfloat16* pb =
-                    nb > 0 ? S.b + (zin ? ((size_t)q.n * (S.D >> 1) + (zz >> 1)) * (S.H >> 1) * (S.W >> 1) * S.cb : 0)
-                           : nullptr;
 #pragma unroll
                 for (int j = 0; j < PS_LV; ++j) {
-                    if ((lt >> 1) + j * (WS_LOADERS / 2) >= RING_V) break;
-                    const uint32_t bytes = zin && ((in >> j) & 1u) ? 16u : 0u;
-                    uint32_t dst = dst0 + (uint32_t)(j * (WS_LOADERS / 2)) * 16;
-                    const __nv_bfloat16* src = pa + oa[j];
-                    for (int c = 0; c < na; ++c, dst += 2 * RING_V * 16) cp_async16_cg(dst, src + (bytes ? c * 16 : 0), bytes);
-                    src = pb + ob[j];
-                    for (int c = 0; c < nb; ++c, dst += 2 * RING_V * 16) cp_async16_cg(dst, src + (bytes ? c * 16 : 0), bytes);
+                    const uint32_t dst = dst0 + (uint32_t)(j * (WS_LOADERS / 2)) * 16, by = zin ? bytes[j] : 0u;
+                    const __nv_bfloat16 *sa = by ? pa[j] : S.a, *sb = by && nb > 0 ? pb[j] : S.a;
+                    if ((lt >> 1) + j * (WS_LOADERS / 2) < RING_V) {
+                        // a read of no bytes takes its address from the tensor's first channels
+#pragma unroll
+                        for (int c = 0; c < c8p / 2; ++c) {
+                            const __nv_bfloat16* src = c < na ? sa + (by ? c * 16 : 0) : sb + (by ? (c - na) * 16 : 0);
+                            cp_async16_cg(dst + (uint32_t)(c * 2 * RING_V * 16), src, by);
+                        }
+                    }
+                    pa[j] += step_a;
+                    if (nb > 0 && (zz & 1)) pb[j] += step_b;
                 }
                 cp_async_arrive_noinc(&full[slot]);
             }
@@ -1268,7 +1321,21 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
             if (!ok) break;
             fence_proxy_async();              // the loaders' copies, seen through the barrier, to the tensor core
             tc_fence_after();
-            if (elect_one()) {
+            if (G == 1 && C8P > 0) {
+                // every tap and channel group at a constant offset: no address arithmetic between the MMAs
+                if (elect_one()) {
+                    const uint32_t al = (uint32_t)a0 + so[0], bl = (uint32_t)b0;
+#pragma unroll
+                    for (int t9 = 0; t9 < 9; ++t9)
+#pragma unroll
+                        for (int j = 0; j < C8P / 2; ++j)
+                            mma_bf16_lo(d[0], al + (uint32_t)((t9 / 3) * HALO_X + t9 % 3 + 2 * j * RING_V),
+                                        (uint32_t)(a0 >> 32), bl + (uint32_t)((t9 * C8P + 2 * j) * NP),
+                                        (uint32_t)(b0 >> 32), IDESC, (t9 > 0 || j > 0) ? 1u : 0u);
+                    mma_commit(&rfull[rsk[0]]);
+                    mma_commit(&empty[fsk[0]]);
+                }
+            } else if (elect_one()) {
 #pragma unroll
                 for (int t9 = 0; t9 < 9; ++t9) {
                     const uint32_t ta = (uint32_t)((t9 / 3) * HALO_X + t9 % 3);
@@ -1302,11 +1369,22 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
         // The voxel's other operands (mask, partial sum, head input) are read
         // before the wait for the tensor core, the biases once per CTA; a
         // region is handed back as soon as its values are in registers.
-        const int qw = warp - 4, m = qw * 32 + lane;
+        // Eight warps, two per lane quarter: each takes half of the channels
+        // of every output plane, or, with the head (whose sum runs over all
+        // channels in order), all channels of every other plane.  Either way
+        // every warp waits for every plane and arrives once per region.
+        constexpr int CW = NO / 2;                             // channels per step
+        const int qw = warp & 3, grp = (warp - 4) >> 2, m = qw * 32 + lane;
         const uint32_t lq = (uint32_t)(qw * 32) << 16;
-        float bias[NO];
+        const bool heads = NO == 16 && P.head != nullptr;
+        float2 bias[CW / 2];
+        if (P.bias && !heads && !Q.part_out) {
 #pragma unroll
-        for (int c = 0; c < NO; ++c) bias[c] = P.bias && !Q.part_out ? __ldg(P.bias + Q.co_lo + c) : 0.0f;
+            for (int j = 0; j < CW / 2; ++j) {
+                const float* bp = P.bias + Q.co_lo + grp * CW + 2 * j;
+                bias[j] = make_float2(__ldg(bp), __ldg(bp + 1));
+            }
+        }
         // region and phase of plane z + 1, and the regions of planes z and z - 1
         uint32_t r1 = 0, ph1 = 0;
         ring_next(r1, ph1, NQ);
@@ -1317,99 +1395,103 @@ __global__ void __launch_bounds__(THREADS, 1) conv_ps_kernel(const ConvP P, cons
             g += q.ze - q.zs;
             const int y = q.y0 + (m >> 3), x = q.x0 + (m & 7);
             const bool in = y < S.H && x < S.W;
-            long long v = (((long long)q.n * S.D + q.zs) * S.H + y) * S.W + x;
-            for (int z = q.zs; z < q.ze; ++z, v += (long long)S.H * S.W, ring_next(r1, ph1, NQ)) {
+            uint32_t v = (uint32_t)((((long long)q.n * S.D + q.zs) * S.H + y) * S.W + x);
+            for (int z = q.zs; z < q.ze; ++z, v += (uint32_t)(S.H * S.W), ring_next(r1, ph1, NQ)) {
                 const uint32_t r0i = r1 == 0 ? NQ - 1 : r1 - 1, rmi = r0i == 0 ? NQ - 1 : r0i - 1;
+                const int c_lo = heads ? 0 : grp * CW;
+                const int c_hi = heads ? ((z & 1) == grp ? NO : 0) : c_lo + CW;
                 // the head: x + b, then + w_j a_j in channel order (the head kernel's FP32 sequence)
-                const bool head = NO == 16 && P.head && in;
+                const bool head = heads && in && c_hi > 0;
                 float hsum = head ? P.head_x[v] + __ldg(P.head + 16) : 0.0f;
-                // output channels [c0, c0 + 8) of this launch go to out0 or out1 (split is a multiple of 8)
-                uint4 mk[NO / 8];
-                if (P.mask0 && in && !Q.part_out) {
+                // output channels [c, c + 8) of this launch go to out0 or out1 (split is a multiple of 8)
+                uint4 mk[CW / 8];
+                if (P.mask0 && in && !Q.part_out && !heads) {
 #pragma unroll
-                    for (int h = 0; h < NO / 8; ++h)
-                        if (Q.co_lo + 8 * h < P.split)
-                            mk[h] = __ldg(reinterpret_cast<const uint4*>(P.mask0 + (size_t)v * P.split + Q.co_lo + 8 * h));
+                    for (int h = 0; h < CW / 8; ++h)
+                        if (Q.co_lo + c_lo + 8 * h < P.split)
+                            mk[h] = __ldg(reinterpret_cast<const uint4*>(P.mask0 + (size_t)v * P.split + Q.co_lo + c_lo + 8 * h));
                 }
-                float4 part[NO / 4];
+                float4 part[CW / 4];
                 if (Q.part_in && in) {
 #pragma unroll
-                    for (int h = 0; h < NO / 4; ++h)
-                        part[h] = __ldg(reinterpret_cast<const float4*>(Q.part_in + (size_t)v * NO) + h);
+                    for (int h = 0; h < CW / 4; ++h)
+                        part[h] = __ldg(reinterpret_cast<const float4*>(Q.part_in + (size_t)v * NO + c_lo) + h);
                 }
                 ok = warp_wait_or_fail(&rfull[r1], ph1, fail);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t rm = tmem + rmi * RC + lq;
-                const uint32_t r0 = tmem + r0i * RC + NO + lq;
-                const uint32_t rp = tmem + r1 * RC + 2 * NO + lq;
-#pragma unroll
-                for (int c0 = 0; c0 < NO; c0 += 16) {
-                    uint32_t um[16], u0[16], up[16];
-                    tmem_ld16_nw(rm + (uint32_t)c0, um);
-                    tmem_ld16_nw(r0 + (uint32_t)c0, u0);
-                    tmem_ld16_nw(rp + (uint32_t)c0, up);
+                for (int c0 = c_lo; c0 < c_hi; c0 += CW) {
+                    uint32_t um[CW], u0[CW], up[CW];
+                    tmem_ld_nw<CW>(tmem + rmi * RC + lq + (uint32_t)c0, um);
+                    tmem_ld_nw<CW>(tmem + r0i * RC + NO + lq + (uint32_t)c0, u0);
+                    tmem_ld_nw<CW>(tmem + r1 * RC + 2 * NO + lq + (uint32_t)c0, up);
                     tmem_wait_ld();
                     // the uses below stay behind the wait
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(um[j]), "+r"(u0[j]), "+r"(up[j]));
-                    if (c0 + 16 == NO) {                       // plane z - 1: last reader done
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) {
-                            mbar_arrive(&rfree[rmi]);
-                            if (z == q.ze - 1) {
-                                mbar_arrive(&rfree[r0i]);
-                                mbar_arrive(&rfree[r1]);
+                    for (int j = 0; j < CW; ++j) asm volatile("" : "+r"(um[j]), "+r"(u0[j]), "+r"(up[j]));
+                    if (c0 + CW == c_hi) ps_release(rfree, lane, rmi, r0i, r1, z == q.ze - 1);
+                    if (in) {
+                        float2 f[CW / 2];
+#pragma unroll
+                        for (int j = 0; j < CW / 2; ++j)
+                            f[j] = add2(add2(make_float2(__uint_as_float(um[2 * j]), __uint_as_float(um[2 * j + 1])),
+                                             make_float2(__uint_as_float(u0[2 * j]), __uint_as_float(u0[2 * j + 1]))),
+                                        make_float2(__uint_as_float(up[2 * j]), __uint_as_float(up[2 * j + 1])));
+                        if (Q.part_in) {
+#pragma unroll
+                            for (int j = 0; j < CW / 4; ++j) {
+                                f[2 * j] = add2(f[2 * j], make_float2(part[j].x, part[j].y));
+                                f[2 * j + 1] = add2(f[2 * j + 1], make_float2(part[j].z, part[j].w));
                             }
                         }
-                    }
-                    if (in) {
+                        if (Q.part_out) {
+                            float4* po = reinterpret_cast<float4*>(Q.part_out + (size_t)v * NO + c0);
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const int c = c0 + 8 * h, co = Q.co_lo + c;
-                            float f[8];
+                            for (int j = 0; j < CW / 4; ++j)
+                                po[j] = make_float4(f[2 * j].x, f[2 * j].y, f[2 * j + 1].x, f[2 * j + 1].y);
+                        } else {
+                            if (P.bias) {
 #pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                f[j] = (__uint_as_float(um[8 * h + j]) + __uint_as_float(u0[8 * h + j])) +
-                                       __uint_as_float(up[8 * h + j]);
-                            if (Q.part_in) {
-                                const float4 p0 = part[c / 4], p1 = part[c / 4 + 1];
-                                f[0] += p0.x, f[1] += p0.y, f[2] += p0.z, f[3] += p0.w;
-                                f[4] += p1.x, f[5] += p1.y, f[6] += p1.z, f[7] += p1.w;
-                            }
-                            if (Q.part_out) {
-                                float4* po = reinterpret_cast<float4*>(Q.part_out + (size_t)v * NO + c);
-                                po[0] = make_float4(f[0], f[1], f[2], f[3]);
-                                po[1] = make_float4(f[4], f[5], f[6], f[7]);
-                                continue;
-                            }
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                if (P.bias) f[j] += bias[c + j];
-                                if (P.relu) f[j] = fmaxf(f[j], 0.0f);
-                            }
-                            if (co < P.split) {
-                                if (P.mask0) {
-                                    float t[8];
-                                    unpack_bf16x8(mk[c / 8], t);
-#pragma unroll
-                                    for (int j = 0; j < 8; ++j) f[j] = t[j] > 0.0f ? f[j] : 0.0f;
+                                for (int j = 0; j < CW / 2; ++j) {
+                                    const float* bp = P.bias + c0 + 2 * j;
+                                    f[j] = add2(f[j], heads ? make_float2(__ldg(bp), __ldg(bp + 1)) : bias[j]);
                                 }
-                                if (P.out0) *reinterpret_cast<uint4*>(P.out0 + (size_t)v * P.split + co) = pack_bf16x8(f);
-                            } else {
-                                *reinterpret_cast<uint4*>(P.out1 + (size_t)v * (Q.n_out - P.split) + (co - P.split)) =
-                                    pack_bf16x8(f);
                             }
-                            if (head) {
 #pragma unroll
-                                for (int j = 0; j < 8; ++j)
-                                    hsum = fmaf(__ldg(P.head + c + j), __bfloat162float(__float2bfloat16_rn(f[j])), hsum);
+                            for (int h = 0; h < CW / 8; ++h) {
+                                const int co = Q.co_lo + c0 + 8 * h;
+                                float t[8];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) t[2 * j] = f[4 * h + j].x, t[2 * j + 1] = f[4 * h + j].y;
+                                if (P.relu) {
+#pragma unroll
+                                    for (int j = 0; j < 8; ++j) t[j] = fmaxf(t[j], 0.0f);
+                                }
+                                if (co < P.split) {
+                                    if (P.mask0) {
+                                        float k[8];
+                                        unpack_bf16x8(mk[h], k);
+#pragma unroll
+                                        for (int j = 0; j < 8; ++j) t[j] = k[j] > 0.0f ? t[j] : 0.0f;
+                                    }
+                                    if (P.out0)
+                                        *reinterpret_cast<uint4*>(P.out0 + (size_t)v * P.split + co) = pack_bf16x8(t);
+                                } else {
+                                    *reinterpret_cast<uint4*>(P.out1 + (size_t)v * (Q.n_out - P.split) + (co - P.split)) =
+                                        pack_bf16x8(t);
+                                }
+                                if (head) {
+#pragma unroll
+                                    for (int j = 0; j < 8; ++j)
+                                        hsum = fmaf(__ldg(P.head + c0 + 8 * h + j),
+                                                    __bfloat162float(__float2bfloat16_rn(t[j])), hsum);
+                                }
                             }
                         }
                     }
                     __syncwarp();                              // the next loads are warp-wide
                 }
+                if (c_hi == 0) ps_release(rfree, lane, rmi, r0i, r1, z == q.ze - 1);
                 if (head) P.head_out[v] = hsum;
             }
             // the next segment's first output reads its planes 0 .. 2: two planes on
@@ -2137,7 +2219,7 @@ bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 // the CTAs resident on one SM never ask for more than its 512 tensor-memory
 // columns together (an allocation beyond that would wait for another CTA).
 template <typename K>
-int tc_launch_smem(K kernel, size_t stages_bytes, uint32_t cols, size_t& smem) {
+int tc_launch_smem(K kernel, size_t stages_bytes, uint32_t cols, size_t& smem, int threads = THREADS) {
     smem = stages_bytes;
     const int max_ctas = (int)(512u / cols);
     int dev = 0;
@@ -2151,7 +2233,7 @@ int tc_launch_smem(K kernel, size_t stages_bytes, uint32_t cols, size_t& smem) {
     CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   (int)cudaSharedmemCarveoutMaxShared));
     int occ = 0;
-    CU_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, THREADS, smem));
+    CU_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem));
     if (occ * (int)cols > 512) return set_error(CCU_E_INVALID, "tensor-memory budget per SM exceeded");
     if (occ < 1) return set_error(CCU_E_INVALID, "kernel does not fit on an SM");
     return CCU_OK;
@@ -2208,20 +2290,20 @@ int ps_passes(int n_out, int cin) {
     return 0;
 }
 
-// Resident CTAs per SM of a kernel launched with THREADS threads and this
+// Resident CTAs per SM of a kernel launched with this many threads and
 // dynamic shared memory: shared memory (1 KB of it reserved per CTA), the
 // registers of its threads, the 512 tensor-memory columns and the 2048
 // threads of an SM.
 template <typename Kern>
-int resident_ctas(Kern kernel, size_t smem, uint32_t cols, int& resident) {
+int resident_ctas(Kern kernel, size_t smem, uint32_t cols, int& resident, int threads = THREADS) {
     int dev = 0, per_sm = 0;
     CU_CHECK(cudaGetDevice(&dev));
     CU_CHECK(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     cudaFuncAttributes fa;
     CU_CHECK(cudaFuncGetAttributes(&fa, kernel));
     const int regs = ((std::max(fa.numRegs, 1) + 7) / 8) * 8;      // allocated per thread in steps of 8
-    resident = std::max(1, std::min({(int)((size_t)per_sm / (smem + 1024)), 65536 / (regs * THREADS),
-                                     (int)(512u / cols), 2048 / THREADS}));
+    resident = std::max(1, std::min({(int)((size_t)per_sm / (smem + 1024)), 65536 / (regs * threads),
+                                     (int)(512u / cols), 2048 / threads}));
     return CCU_OK;
 }
 
@@ -2314,6 +2396,32 @@ int ps_workspace(size_t bytes, cudaStream_t st, float*& ws) {
     return rc;
 }
 
+// One launch: the pass's channel groups and output slice.
+template <int NO, int G, int C8P>
+int launch_conv_ps_pass(const ConvP& P, const PsPass& Q, long long planes, int sms, cudaStream_t st) {
+    const auto kernel = conv_ps_kernel<NO, G, C8P>;
+    const int c8p = Q.c8_hi - Q.c8_lo;
+    const uint32_t cols = ps_tmem_cols(NO, G);
+    // deepest ring (group + 1 .. WS_RING_MAX planes) that keeps the CTAs per SM the tensor memory allows
+    int ring = 0, best_res = 0, rc = CCU_OK;
+    size_t smem = 0;
+    for (int r = G + 1; r <= WS_RING_MAX && ps_smem_bytes(NO, c8p, r) <= 200 * 1024; ++r) {
+        int res = 1;
+        rc = resident_ctas(kernel, (size_t)ps_smem_bytes(NO, c8p, r) + 1024, cols, res, PS_THREADS);
+        if (rc != CCU_OK) return rc;
+        if (res >= best_res) best_res = res, ring = r;
+    }
+    if (ring == 0) return set_error(CCU_E_INVALID, "plane-stationary pass does not fit shared memory");
+    rc = tc_launch_smem(kernel, ps_smem_bytes(NO, c8p, ring), cols, smem, PS_THREADS);
+    if (rc != CCU_OK) return rc;
+    int resident = 1;
+    if ((rc = resident_ctas(kernel, smem, cols, resident, PS_THREADS)) != CCU_OK) return rc;
+    const long long grid = std::min<long long>(planes, (long long)sms * resident);
+    kernel<<<(unsigned)grid, PS_THREADS, smem, st>>>(P, Q, ring);
+    CU_CHECK(cudaGetLastError());
+    return CCU_OK;
+}
+
 template <int NO, int G>
 int launch_conv_ps_g(const ConvP& P, int n_out, int passes, cudaStream_t st) {
     const int c8n = (P.src.ca + P.src.cb) / 8;
@@ -2337,25 +2445,15 @@ int launch_conv_ps_g(const ConvP& P, int n_out, int passes, cudaStream_t st) {
         Q.c8_hi = std::min(c8n, lo + c8p_max);
         Q.part_in = k > 0 ? ws : nullptr;
         Q.part_out = Q.c8_hi < c8n ? ws : nullptr;
-        const int c8p = Q.c8_hi - Q.c8_lo;
-        const uint32_t cols = ps_tmem_cols(NO, G);
-        // deepest ring (group + 1 .. WS_RING_MAX planes) that keeps the CTAs per SM the tensor memory allows
-        int ring = 0, best_res = 0;
-        size_t smem = 0;
-        for (int r = G + 1; r <= WS_RING_MAX && ps_smem_bytes(NO, c8p, r) <= 200 * 1024; ++r) {
-            int res = 1;
-            const int rc = resident_ctas(conv_ps_kernel<NO, G>, (size_t)ps_smem_bytes(NO, c8p, r) + 1024, cols, res);
-            if (rc != CCU_OK) return rc;
-            if (res >= best_res) best_res = res, ring = r;
+        int rc = CCU_OK;
+        switch (G == 1 ? Q.c8_hi - Q.c8_lo : 0) {          // 16 to 64 input channels per pass: unrolled issue
+            case 2: rc = launch_conv_ps_pass<NO, G, G == 1 ? 2 : 0>(P, Q, planes, sms, st); break;
+            case 4: rc = launch_conv_ps_pass<NO, G, G == 1 ? 4 : 0>(P, Q, planes, sms, st); break;
+            case 6: rc = launch_conv_ps_pass<NO, G, G == 1 ? 6 : 0>(P, Q, planes, sms, st); break;
+            case 8: rc = launch_conv_ps_pass<NO, G, G == 1 ? 8 : 0>(P, Q, planes, sms, st); break;
+            default: rc = launch_conv_ps_pass<NO, G, 0>(P, Q, planes, sms, st); break;
         }
-        if (ring == 0) return set_error(CCU_E_INVALID, "plane-stationary pass does not fit shared memory");
-        int rc = tc_launch_smem(conv_ps_kernel<NO, G>, ps_smem_bytes(NO, c8p, ring), cols, smem);
         if (rc != CCU_OK) return rc;
-        int resident = 1;
-        if ((rc = resident_ctas(conv_ps_kernel<NO, G>, smem, cols, resident)) != CCU_OK) return rc;
-        const long long grid = std::min<long long>(planes, (long long)sms * resident);
-        conv_ps_kernel<NO, G><<<(unsigned)grid, THREADS, smem, st>>>(P, Q, ring);
-        CU_CHECK(cudaGetLastError());
     }
     return CCU_OK;
 }
