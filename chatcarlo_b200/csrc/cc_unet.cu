@@ -127,8 +127,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 
 // mbar_wait that also gives up once another thread of the CTA has set
 // *fail (its own wait ran out); sets *fail itself when its WAIT_NS run out.
-__device__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity, volatile int* fail) {
-    if (mbar_try_wait(bar, parity)) return true;
+// The polls stay a clock read apart: without it the waiting warps' polls
+// take the issue slots of the working ones.
+__device__ __noinline__ bool mbar_wait_or_fail_slow(uint64_t* bar, uint32_t parity, volatile int* fail) {
     const unsigned long long t0 = global_ns();
     while (true) {
         if (mbar_try_wait(bar, parity)) return true;
@@ -139,11 +140,15 @@ __device__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity, volatile int* 
         }
     }
 }
+__device__ __forceinline__ bool mbar_wait_or_fail(uint64_t* bar, uint32_t parity, volatile int* fail) {
+    return mbar_try_wait(bar, parity) || mbar_wait_or_fail_slow(bar, parity, fail);
+}
 
 // mbar_wait_or_fail by a whole converged warp: true where every lane saw
 // the phase complete, the same for all lanes.
 __device__ __forceinline__ bool warp_wait_or_fail(uint64_t* bar, uint32_t parity, volatile int* fail) {
-    return __all_sync(0xffffffffu, mbar_wait_or_fail(bar, parity, fail)) != 0;
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait_or_fail_slow(bar, parity, fail)) != 0;
 }
 
 // The mbarrier receives one arrival when all of this thread's earlier
@@ -1127,11 +1132,14 @@ __global__ void __launch_bounds__(THREADS, 4) conv_ws_kernel(const ConvP P, int 
 // weights do not fit shared memory run as several passes: every pass but
 // the last adds into an FP32 partial sum [v][NO] (part_out), the last adds
 // the partial (part_in) before bias, ReLU, mask and the BF16 store.
+// PLAIN: no mask, partial sums, head or second output (a forward layer in
+// one pass): the epilogue without their tests.
 // Output slices: a launch computes output channels [co_lo, co_lo + NO) of
 // a layer with more (64 output channels: two slices of 32).
 constexpr int PS_REGIONS_MAX = 8;
 constexpr int PS_GROUP_MAX = 3;
-constexpr int PS_THREADS = 384;             // warp 0 MMA, 1-3 loaders, 4-11 epilogue
+constexpr int PS_THREADS = 416;             // warps 0, 1 MMA, 2-4 loaders, 5-12 epilogue
+constexpr int PS_ISSUERS = 2, PS_EPI_WARP0 = PS_ISSUERS + WS_LOADERS / 32;
 constexpr int PS_EPI_WARPS = 8;
 constexpr int PS_LV = (RING_V + WS_LOADERS / 2 - 1) / (WS_LOADERS / 2);     // halo voxels of a loader thread
 
@@ -1179,7 +1187,7 @@ __device__ __forceinline__ void ps_release(uint64_t* rfree, int lane, uint32_t r
     }
 }
 
-template <int NO, int G, int C8P>
+template <int NO, int G, int C8P, bool PLAIN>
 __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_ps_kernel(const ConvP P, const PsPass Q, int ring) {
     constexpr int NP = 3 * NO;                                // MMA N: the three dz weight planes
     constexpr uint32_t RC = ps_region_cols(NO);
@@ -1228,7 +1236,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
-    if (warp >= 1 && warp <= 3) {
+    if (warp >= PS_ISSUERS && warp < PS_EPI_WARP0) {
         // ---- loaders: planes zs - 1 .. ze of each segment, channel groups of the pass ----
         // Each thread's copies of a plane arrive on the slot's "full" barrier
         // when they land, so the loaders never wait for their own copies:
@@ -1238,7 +1246,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         // its 16-byte stores fall into different banks (a chunk plane is
         // 720 words long); their voxels' offsets within a plane are fixed
         // for a segment, a plane only moves the base.
-        const int lt = tid - 32, half = lt & 1;
+        const int lt = tid - 32 * PS_ISSUERS, half = lt & 1;
         const int na = max(0, min(Q.c8_hi, S.ca / 8) - Q.c8_lo) / 2, nb = c8p / 2 - na;   // 16-channel groups from a, b
         const int ch_a = (Q.c8_lo + half) * 8, ch_b = (Q.c8_lo + 2 * na + half) * 8 - S.ca;
         const long long step_a = (long long)S.H * S.W * S.ca;                  // elements of a plane of a, of b
@@ -1284,9 +1292,13 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
             }
         }
         cp_async_wait<0>();
-    } else if (warp == 0) {
+    } else if (warp < (G == 1 ? PS_ISSUERS : 1)) {
         // ---- MMA issuer: per input plane one chain of 9 x c8p / 2 MMAs; the chains of a
-        // group of planes are issued tap by tap in turn ----
+        // group of planes are issued tap by tap in turn.  With G = 1 two warps
+        // take alternate planes: the tensor core's queue is short, so one
+        // warp's waits and commits between two planes would leave it idle
+        // where a CTA has the SM to itself ----
+        constexpr uint32_t STEP = G == 1 ? PS_ISSUERS : G;
         const uint64_t a0 = smem_desc(sbase, RING_V * 16, HALO_X * 16);
         const uint64_t b0 = smem_desc(swt, NP * 16, 128);
         constexpr uint32_t IDESC = idesc_bf16(TILE_M, NP, 0, 0);
@@ -1298,7 +1310,12 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         }
         // plane L's ring slot and region with their phases, advanced without divisions
         uint32_t L = 0, fs = 0, fph = 0, rs = 0, rph = 0;
+        uint32_t last_r = NQ, last_ph = 0;          // region and phase of the last plane issued
         bool ok = true;
+        for (; L < (uint32_t)warp; ++L) {
+            ring_next(fs, fph, R);
+            ring_next(rs, rph, NQ);
+        }
         while (L < n_planes && ok) {
             const uint32_t gn = min((uint32_t)G, n_planes - L);      // G but for the CTA's last group
             uint32_t d[G], so[G], fsk[G], rsk[G];
@@ -1356,15 +1373,26 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                     }
             }
             __syncwarp();
-            for (uint32_t k = 0; k < gn; ++k) {
+            last_r = rsk[0];
+            last_ph = rph;
+            if (G > 1) {                                   // the group's last plane
+#pragma unroll
+                for (int k = 1; k < G; ++k)
+                    if ((uint32_t)k < gn) {
+                        if (rsk[k] == 0) last_ph ^= 1u;
+                        last_r = rsk[k];
+                    }
+            }
+            L += STEP;
+#pragma unroll
+            for (uint32_t k = 0; k < STEP; ++k) {
                 ring_next(fs, fph, R);
                 ring_next(rs, rph, NQ);
             }
-            L += gn;
         }
-        // every issued MMA has finished before the tensor memory can be freed: plane L - 1's phase
-        if (L > 0) mbar_wait(&rfull[rs == 0 ? NQ - 1 : rs - 1], rs == 0 ? rph ^ 1u : rph);
-    } else if (warp >= 4) {
+        // every MMA that this warp issued has finished before the tensor memory can be freed
+        if (last_r < NQ) mbar_wait(&rfull[last_r], last_ph);
+    } else if (warp >= PS_EPI_WARP0) {
         // ---- epilogue: output z = D_{z-1}[dz 0] + D_z[dz 1] + D_{z+1}[dz 2]; row m, lane quarter warp - 4 ----
         // The voxel's other operands (mask, partial sum, head input) are read
         // before the wait for the tensor core, the biases once per CTA; a
@@ -1374,11 +1402,11 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         // channels in order), all channels of every other plane.  Either way
         // every warp waits for every plane and arrives once per region.
         constexpr int CW = NO / 2;                             // channels per step
-        const int qw = warp & 3, grp = (warp - 4) >> 2, m = qw * 32 + lane;
+        const int qw = warp & 3, grp = (warp - PS_EPI_WARP0) >> 2, m = qw * 32 + lane;
         const uint32_t lq = (uint32_t)(qw * 32) << 16;
-        const bool heads = NO == 16 && P.head != nullptr;
+        const bool heads = !PLAIN && NO == 16 && P.head != nullptr;
         float2 bias[CW / 2];
-        if (P.bias && !heads && !Q.part_out) {
+        if (P.bias && !heads && (PLAIN || !Q.part_out)) {
 #pragma unroll
             for (int j = 0; j < CW / 2; ++j) {
                 const float* bp = P.bias + Q.co_lo + grp * CW + 2 * j;
@@ -1396,6 +1424,10 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
             const int y = q.y0 + (m >> 3), x = q.x0 + (m & 7);
             const bool in = y < S.H && x < S.W;
             uint32_t v = (uint32_t)((((long long)q.n * S.D + q.zs) * S.H + y) * S.W + x);
+            // each plane's wait below covers every earlier plane of its own
+            // issuer; the segment's second plane is the other issuer's
+            ok = warp_wait_or_fail(&rfull[r1 == 0 ? NQ - 1 : r1 - 1], r1 == 0 ? ph1 ^ 1u : ph1, fail);
+            if (!ok) break;
             for (int z = q.zs; z < q.ze; ++z, v += (uint32_t)(S.H * S.W), ring_next(r1, ph1, NQ)) {
                 const uint32_t r0i = r1 == 0 ? NQ - 1 : r1 - 1, rmi = r0i == 0 ? NQ - 1 : r0i - 1;
                 const int c_lo = heads ? 0 : grp * CW;
@@ -1405,14 +1437,14 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                 float hsum = head ? P.head_x[v] + __ldg(P.head + 16) : 0.0f;
                 // output channels [c, c + 8) of this launch go to out0 or out1 (split is a multiple of 8)
                 uint4 mk[CW / 8];
-                if (P.mask0 && in && !Q.part_out && !heads) {
+                if (!PLAIN && P.mask0 && in && !Q.part_out && !heads) {
 #pragma unroll
                     for (int h = 0; h < CW / 8; ++h)
                         if (Q.co_lo + c_lo + 8 * h < P.split)
                             mk[h] = __ldg(reinterpret_cast<const uint4*>(P.mask0 + (size_t)v * P.split + Q.co_lo + c_lo + 8 * h));
                 }
                 float4 part[CW / 4];
-                if (Q.part_in && in) {
+                if (!PLAIN && Q.part_in && in) {
 #pragma unroll
                     for (int h = 0; h < CW / 4; ++h)
                         part[h] = __ldg(reinterpret_cast<const float4*>(Q.part_in + (size_t)v * NO + c_lo) + h);
@@ -1437,14 +1469,14 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                             f[j] = add2(add2(make_float2(__uint_as_float(um[2 * j]), __uint_as_float(um[2 * j + 1])),
                                              make_float2(__uint_as_float(u0[2 * j]), __uint_as_float(u0[2 * j + 1]))),
                                         make_float2(__uint_as_float(up[2 * j]), __uint_as_float(up[2 * j + 1])));
-                        if (Q.part_in) {
+                        if (!PLAIN && Q.part_in) {
 #pragma unroll
                             for (int j = 0; j < CW / 4; ++j) {
                                 f[2 * j] = add2(f[2 * j], make_float2(part[j].x, part[j].y));
                                 f[2 * j + 1] = add2(f[2 * j + 1], make_float2(part[j].z, part[j].w));
                             }
                         }
-                        if (Q.part_out) {
+                        if (!PLAIN && Q.part_out) {
                             float4* po = reinterpret_cast<float4*>(Q.part_out + (size_t)v * NO + c0);
 #pragma unroll
                             for (int j = 0; j < CW / 4; ++j)
@@ -1467,14 +1499,14 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
 #pragma unroll
                                     for (int j = 0; j < 8; ++j) t[j] = fmaxf(t[j], 0.0f);
                                 }
-                                if (co < P.split) {
-                                    if (P.mask0) {
+                                if (PLAIN || co < P.split) {
+                                    if (!PLAIN && P.mask0) {
                                         float k[8];
                                         unpack_bf16x8(mk[h], k);
 #pragma unroll
                                         for (int j = 0; j < 8; ++j) t[j] = k[j] > 0.0f ? t[j] : 0.0f;
                                     }
-                                    if (P.out0)
+                                    if (PLAIN || P.out0)
                                         *reinterpret_cast<uint4*>(P.out0 + (size_t)v * P.split + co) = pack_bf16x8(t);
                                 } else {
                                     *reinterpret_cast<uint4*>(P.out1 + (size_t)v * (Q.n_out - P.split) + (co - P.split)) =
@@ -2397,9 +2429,13 @@ int ps_workspace(size_t bytes, cudaStream_t st, float*& ws) {
 }
 
 // One launch: the pass's channel groups and output slice.
-template <int NO, int G, int C8P>
+template <int NO, int G, int C8P, bool PLAIN = false>
 int launch_conv_ps_pass(const ConvP& P, const PsPass& Q, long long planes, int sms, cudaStream_t st) {
-    const auto kernel = conv_ps_kernel<NO, G, C8P>;
+    if constexpr (G == 1 && C8P > 0 && !PLAIN) {
+        if (!P.mask0 && !P.head && !Q.part_in && !Q.part_out && P.out0 && Q.co_lo + NO <= P.split)
+            return launch_conv_ps_pass<NO, G, C8P, true>(P, Q, planes, sms, st);
+    }
+    const auto kernel = conv_ps_kernel<NO, G, C8P, PLAIN>;
     const int c8p = Q.c8_hi - Q.c8_lo;
     const uint32_t cols = ps_tmem_cols(NO, G);
     // deepest ring (group + 1 .. WS_RING_MAX planes) that keeps the CTAs per SM the tensor memory allows
