@@ -1166,6 +1166,37 @@ __device__ __forceinline__ void ring_next(uint32_t& i, uint32_t& phase, uint32_t
     }
 }
 
+// The (column, plane) segments of one CTA.  Whole columns first, one per CTA
+// and round, so that the CTAs walk down neighbouring columns together and
+// the halo that two of them read is still in L2; the columns left over
+// after the full rounds are cut into equal ranges of planes.
+struct PsWalk {
+    long long col, cols_full, g, g_end;      // next whole column; position and end in the left-over planes
+    int grid, tiles_x, tiles_y;
+
+    __device__ __forceinline__ PsWalk(const Src& S) {
+        tiles_x = (S.W + 7) / 8;
+        tiles_y = (S.H + 15) / 16;
+        grid = (int)gridDim.x;
+        const long long cols = (long long)S.B * tiles_y * tiles_x, left = cols % grid * S.D;
+        cols_full = cols - cols % grid;
+        col = blockIdx.x;
+        g = left * blockIdx.x / grid;
+        g_end = left * (blockIdx.x + 1) / grid;
+    }
+    __device__ __forceinline__ bool next(const Src& S, WsSeg& q) {
+        if (col < cols_full) {
+            q = ws_segment(S, col * S.D, (col + 1) * S.D, tiles_x, tiles_y);
+            col += grid;
+            return true;
+        }
+        if (g >= g_end) return false;
+        q = ws_segment(S, cols_full * S.D + g, cols_full * S.D + g_end, tiles_x, tiles_y);
+        g += q.ze - q.zs;
+        return true;
+    }
+};
+
 struct PsPass {
     int c8_lo, c8_hi;          // input channel groups of this pass
     int co_lo, n_out;          // output channels [co_lo, co_lo + NO) of the layer's n_out
@@ -1200,9 +1231,6 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const Src& S = P.src;
     const int c8n = (S.ca + S.cb) / 8, c8p = C8P > 0 ? C8P : Q.c8_hi - Q.c8_lo;
-    const int tiles_x = (S.W + 7) / 8, tiles_y = (S.H + 15) / 16;
-    const long long total = (long long)S.B * tiles_y * tiles_x * S.D;
-    const long long g_begin = total * blockIdx.x / gridDim.x, g_end = total * (blockIdx.x + 1) / gridDim.x;
     const uint32_t R = (uint32_t)ring;
     const uint32_t slot16 = (uint32_t)c8p * RING_V;           // one ring slot, 16-byte units
     volatile int* fail = &s_fail;
@@ -1252,9 +1280,8 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         const long long step_a = (long long)S.H * S.W * S.ca;                  // elements of a plane of a, of b
         const long long step_b = (long long)(S.H >> 1) * (S.W >> 1) * S.cb;
         uint32_t L = 0, slot = 0, ph = 0;             // plane, its ring slot and the slot's phase
-        for (long long g = g_begin; g < g_end && !*fail;) {
-            const WsSeg q = ws_segment(S, g, g_end, tiles_x, tiles_y);
-            g += q.ze - q.zs;
+        PsWalk walk(S);
+        for (WsSeg q; !*fail && walk.next(S, q);) {
             // this thread's voxels in plane zs - 1 (read only where they lie inside the volume)
             const __nv_bfloat16 *pa[PS_LV], *pb[PS_LV];
             uint32_t bytes[PS_LV];
@@ -1303,9 +1330,8 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         const uint64_t b0 = smem_desc(swt, NP * 16, 128);
         constexpr uint32_t IDESC = idesc_bf16(TILE_M, NP, 0, 0);
         uint32_t n_planes = 0;                       // planes of the CTA's sequence: each segment's zs - 1 .. ze
-        for (long long g = g_begin; g < g_end;) {
-            const WsSeg q = ws_segment(S, g, g_end, tiles_x, tiles_y);
-            g += q.ze - q.zs;
+        PsWalk walk(S);
+        for (WsSeg q; walk.next(S, q);) {
             n_planes += (uint32_t)(q.ze - q.zs) + 2;
         }
         // plane L's ring slot and region with their phases, advanced without divisions
@@ -1418,9 +1444,8 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         ring_next(r1, ph1, NQ);
         ring_next(r1, ph1, NQ);                                // the first output reads planes 0, 1, 2
         bool ok = true;
-        for (long long g = g_begin; g < g_end && ok;) {
-            const WsSeg q = ws_segment(S, g, g_end, tiles_x, tiles_y);
-            g += q.ze - q.zs;
+        PsWalk walk(S);
+        for (WsSeg q; ok && walk.next(S, q);) {
             const int y = q.y0 + (m >> 3), x = q.x0 + (m & 7);
             const bool in = y < S.H && x < S.W;
             uint32_t v = (uint32_t)((((long long)q.n * S.D + q.zs) * S.H + y) * S.W + x);
