@@ -213,6 +213,9 @@ __device__ __forceinline__ uint64_t smem_desc_sw(uint32_t addr, uint32_t lbo, ui
     return smem_desc(addr, lbo, sbo) | ((uint64_t)(layout & 7u) << 61);
 }
 
+// descriptor layout type of rows of `bytes` (32, 64 or 128)
+__host__ __device__ constexpr uint32_t swizzle_layout(int bytes) { return bytes == 32 ? 6u : (bytes == 64 ? 4u : 2u); }
+
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B,
 // A/B K-major (0) or MN-major (1), N >> 3, M >> 4.
 __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, int a_mn, int b_mn) {
@@ -1141,6 +1144,12 @@ constexpr int PS_GROUP_MAX = 3;
 constexpr int PS_THREADS = 416;             // warps 0, 1 MMA, 2-4 loaders, 5-12 epilogue
 constexpr int PS_ISSUERS = 2, PS_EPI_WARP0 = PS_ISSUERS + WS_LOADERS / 32;
 constexpr int PS_EPI_WARPS = 8;
+// A ring slot holds 16-channel groups of a halo plane, 180 voxel rows of 32
+// bytes under the 32-byte swizzle (16-byte half h of voxel v at half
+// h ^ ((v >> 2) & 1): the pattern repeats every 256 bytes, to which groups
+// are padded), the K-major layout of one K = 16 MMA step.
+constexpr int PS_ROWS_BYTES = RING_V * 32;
+constexpr int PS_GROUP_BYTES = (PS_ROWS_BYTES + 255) / 256 * 256;
 constexpr int PS_LV = (RING_V + WS_LOADERS / 2 - 1) / (WS_LOADERS / 2);     // halo voxels of a loader thread
 
 // tensor-memory columns of one region: 3 x cout
@@ -1155,7 +1164,7 @@ __host__ __device__ constexpr uint32_t ps_tmem_cols(int n, int g) {
 }
 __host__ __device__ constexpr uint32_t ps_weight_bytes(int n, int c8p) { return 9u * (uint32_t)c8p * 3u * n * 16u; }
 __host__ __device__ constexpr uint32_t ps_smem_bytes(int n, int c8p, int ring) {
-    return (uint32_t)ring * (uint32_t)c8p * RING_V * 16 + ps_weight_bytes(n, c8p);
+    return (uint32_t)ring * (uint32_t)(c8p / 2) * PS_GROUP_BYTES + ps_weight_bytes(n, c8p) + 256;   // 256: alignment
 }
 
 // next index of a ring of n entries, flipping the phase bit on wrap-around
@@ -1219,7 +1228,7 @@ __device__ __forceinline__ void ps_release(uint64_t* rfree, int lane, uint32_t r
 }
 
 template <int NO, int G, int C8P, bool PLAIN>
-__global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_ps_kernel(const ConvP P, const PsPass Q, int ring) {
+__global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_ps_kernel(const __grid_constant__ CUtensorMap amap, const ConvP P, const PsPass Q, int ring) {
     constexpr int NP = 3 * NO;                                // MMA N: the three dz weight planes
     constexpr uint32_t RC = ps_region_cols(NO);
     constexpr uint32_t NQ = (uint32_t)ps_regions(G), TCOLS = ps_tmem_cols(NO, G);
@@ -1232,13 +1241,16 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
     const Src& S = P.src;
     const int c8n = (S.ca + S.cb) / 8, c8p = C8P > 0 ? C8P : Q.c8_hi - Q.c8_lo;
     const uint32_t R = (uint32_t)ring;
-    const uint32_t slot16 = (uint32_t)c8p * RING_V;           // one ring slot, 16-byte units
+    constexpr uint32_t GROUP16 = PS_GROUP_BYTES / 16;         // one 16-channel group, 16-byte units
+    const uint32_t slot16 = (uint32_t)(c8p / 2) * GROUP16;    // one ring slot
+    // 16-channel groups of the pass from a (tile loads) and from b (gathered)
+    const int na = max(0, min(Q.c8_hi, S.ca / 8) - Q.c8_lo) / 2, nb = c8p / 2 - na;
     volatile int* fail = &s_fail;
 
     if (warp == 0) tmem_alloc(&s_tmem, TCOLS);
     if (tid == 0) {
         for (uint32_t r = 0; r < R; ++r) {
-            mbar_init(&full[r], WS_LOADERS);
+            mbar_init(&full[r], (na > 0 ? 1 : 0) + (nb > 0 ? WS_LOADERS : 0));
             mbar_init(&empty[r], 1);
         }
         for (uint32_t r = 0; r < NQ; ++r) {
@@ -1249,7 +1261,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         mbar_init_fence();
     }
     // weights: packed chunk (tap * c8n + c8, co_lo + co) -> (t9 * c8p + c8 - c8_lo, dz * NO + co)
-    const uint32_t sbase = smem_u32(smem), swt = sbase + R * slot16 * 16;
+    const uint32_t sbase = (smem_u32(smem) + 255u) & ~255u, swt = sbase + R * slot16 * 16;
     for (int i = tid; i < 9 * c8p * NP; i += PS_THREADS) {
         const int r = i % NP, g = i / NP;
         const int t9 = g / c8p, c8 = Q.c8_lo + g % c8p, dz = r / NO, co = r % NO;
@@ -1266,59 +1278,74 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
 
     if (warp >= PS_ISSUERS && warp < PS_EPI_WARP0) {
         // ---- loaders: planes zs - 1 .. ze of each segment, channel groups of the pass ----
-        // Each thread's copies of a plane arrive on the slot's "full" barrier
-        // when they land, so the loaders never wait for their own copies:
-        // as many planes are in flight as the ring has free slots.
-        // Threads 2 i and 2 i + 1 copy the two 8-channel halves of the same
-        // voxel's 16 channels, so that a warp reads whole 32-byte sectors and
-        // its 16-byte stores fall into different banks (a chunk plane is
-        // 720 words long); their voxels' offsets within a plane are fixed
-        // for a segment, a plane only moves the base.
+        // The groups of a are tile loads (box {16 channels, 10, 18, 1, 1};
+        // coordinates outside the volume read the padding's zeros), issued
+        // by one lane of the first loader warp and completing on the slot's
+        // "full" barrier: gathered by 16-byte cp.async copies, the same planes
+        // ran at 4.8 TB/s of L2 traffic, bound by the copies in flight.
+        // b, read nearest-upsampled, is gathered by all three warps: threads
+        // 2 i and 2 i + 1 copy the 16-byte halves of the same voxel's 16
+        // channels, so that a warp reads whole 32-byte sectors; each thread's
+        // copies arrive on the barrier when they land.  No loader waits for
+        // its own copies: as many planes are in flight as the ring has slots.
         const int lt = tid - 32 * PS_ISSUERS, half = lt & 1;
-        const int na = max(0, min(Q.c8_hi, S.ca / 8) - Q.c8_lo) / 2, nb = c8p / 2 - na;   // 16-channel groups from a, b
-        const int ch_a = (Q.c8_lo + half) * 8, ch_b = (Q.c8_lo + 2 * na + half) * 8 - S.ca;
-        const long long step_a = (long long)S.H * S.W * S.ca;                  // elements of a plane of a, of b
-        const long long step_b = (long long)(S.H >> 1) * (S.W >> 1) * S.cb;
+        const bool tiles = na > 0 && warp == PS_ISSUERS;
+        const int ch_b = (Q.c8_lo + 2 * na + half) * 8 - S.ca;
+        const long long step_b = (long long)(S.H >> 1) * (S.W >> 1) * S.cb;       // elements of a plane of b
         uint32_t L = 0, slot = 0, ph = 0;             // plane, its ring slot and the slot's phase
         PsWalk walk(S);
-        for (WsSeg q; !*fail && walk.next(S, q);) {
+        bool ok = tiles || nb > 0;
+        for (WsSeg q; ok && walk.next(S, q);) {
             // this thread's voxels in plane zs - 1 (read only where they lie inside the volume)
-            const __nv_bfloat16 *pa[PS_LV], *pb[PS_LV];
+            const __nv_bfloat16* pb[PS_LV];
             uint32_t bytes[PS_LV];
-#pragma unroll
-            for (int j = 0; j < PS_LV; ++j) {
-                const int hv = (lt >> 1) + j * (WS_LOADERS / 2);
-                const int yy = q.y0 + hv / HALO_X - 1, xx = q.x0 + hv % HALO_X - 1;
-                const bool ok = (unsigned)yy < (unsigned)S.H && (unsigned)xx < (unsigned)S.W;
-                bytes[j] = ok ? 16u : 0u;
-                pa[j] = S.a + ((long long)q.n * S.D + q.zs - 1) * step_a + (ok ? ((long long)yy * S.W + xx) * S.ca : 0) + ch_a;
-                pb[j] = nb > 0 ? S.b + ((long long)q.n * (S.D >> 1) + ((q.zs - 1) >> 1)) * step_b +
-                                     (ok ? ((long long)(yy >> 1) * (S.W >> 1) + (xx >> 1)) * S.cb : 0) + ch_b
-                               : nullptr;
-            }
-            for (int zz = q.zs - 1; zz <= q.ze; ++zz, ++L, ring_next(slot, ph, R)) {
-                if (L >= R && !mbar_wait_or_fail(&empty[slot], ph ^ 1u, fail)) break;
-                const uint32_t dst0 = sbase + (slot * slot16 + (uint32_t)(half * RING_V + (lt >> 1))) * 16;
-                const bool zin = (unsigned)zz < (unsigned)S.D;
+            if (nb > 0) {
 #pragma unroll
                 for (int j = 0; j < PS_LV; ++j) {
-                    const uint32_t dst = dst0 + (uint32_t)(j * (WS_LOADERS / 2)) * 16, by = zin ? bytes[j] : 0u;
-                    const __nv_bfloat16 *sa = by ? pa[j] : S.a, *sb = by && nb > 0 ? pb[j] : S.a;
-                    if ((lt >> 1) + j * (WS_LOADERS / 2) < RING_V) {
-                        // a read of no bytes takes its address from the tensor's first channels
-#pragma unroll
-                        for (int c = 0; c < c8p / 2; ++c) {
-                            const __nv_bfloat16* src = c < na ? sa + (by ? c * 16 : 0) : sb + (by ? (c - na) * 16 : 0);
-                            cp_async16_cg(dst + (uint32_t)(c * 2 * RING_V * 16), src, by);
-                        }
-                    }
-                    pa[j] += step_a;
-                    if (nb > 0 && (zz & 1)) pb[j] += step_b;
+                    const int hv = (lt >> 1) + j * (WS_LOADERS / 2);
+                    const int yy = q.y0 + hv / HALO_X - 1, xx = q.x0 + hv % HALO_X - 1;
+                    const bool in = (unsigned)yy < (unsigned)S.H && (unsigned)xx < (unsigned)S.W;
+                    bytes[j] = in ? 16u : 0u;
+                    pb[j] = S.b + ((long long)q.n * (S.D >> 1) + ((q.zs - 1) >> 1)) * step_b +
+                            (in ? ((long long)(yy >> 1) * (S.W >> 1) + (xx >> 1)) * S.cb : 0) + ch_b;
                 }
-                cp_async_arrive_noinc(&full[slot]);
+            }
+            for (int zz = q.zs - 1; zz <= q.ze; ++zz, ++L, ring_next(slot, ph, R)) {
+                if (L >= R) ok = warp_wait_or_fail(&empty[slot], ph ^ 1u, fail);
+                if (!ok) break;
+                const uint32_t dst0 = sbase + slot * slot16 * 16;
+                if (tiles) {
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&full[slot], (uint32_t)(na * PS_ROWS_BYTES));
+                        for (int c = 0; c < na; ++c)
+                            tma_load_5d(dst0 + (uint32_t)(c * PS_GROUP_BYTES), &amap, &full[slot], Q.c8_lo * 8 + 16 * c,
+                                        q.x0 - 1, q.y0 - 1, zz, q.n);
+                    }
+                    __syncwarp();
+                }
+                if (nb > 0) {
+                    const bool zin = (unsigned)zz < (unsigned)S.D;
+#pragma unroll
+                    for (int j = 0; j < PS_LV; ++j) {
+                        const int hv = (lt >> 1) + j * (WS_LOADERS / 2);
+                        const uint32_t by = zin ? bytes[j] : 0u;
+                        const uint32_t dst = dst0 + (uint32_t)(na * PS_GROUP_BYTES + hv * 32 + ((half ^ ((hv >> 2) & 1)) << 4));
+                        if (hv < RING_V) {
+                            const __nv_bfloat16* src = by ? pb[j] : S.b;      // a read of no bytes: any address of b
+#pragma unroll
+                            for (int c = 0; c < c8p / 2; ++c)
+                                if (c < nb) cp_async16_cg(dst + (uint32_t)(c * PS_GROUP_BYTES), src + (by ? c * 16 : 0), by);
+                        }
+                        if (zz & 1) pb[j] += step_b;
+                    }
+                    cp_async_arrive_noinc(&full[slot]);
+                }
             }
         }
         cp_async_wait<0>();
+        // after a failure, the tile loads still in flight land before the CTA ends
+        if (tiles && *fail)
+            for (uint32_t p = L > R ? L - R : 0; p < L; ++p) mbar_wait(&full[p % R], (p / R) & 1u);
     } else if (warp < (G == 1 ? PS_ISSUERS : 1)) {
         // ---- MMA issuer: per input plane one chain of 9 x c8p / 2 MMAs; the chains of a
         // group of planes are issued tap by tap in turn.  With G = 1 two warps
@@ -1326,7 +1353,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         // warp's waits and commits between two planes would leave it idle
         // where a CTA has the SM to itself ----
         constexpr uint32_t STEP = G == 1 ? PS_ISSUERS : G;
-        const uint64_t a0 = smem_desc(sbase, RING_V * 16, HALO_X * 16);
+        const uint64_t a0 = smem_desc_sw(sbase, 16, HALO_X * 32, swizzle_layout(32));   // 8 x-neighbours, then the next y row
         const uint64_t b0 = smem_desc(swt, NP * 16, 128);
         constexpr uint32_t IDESC = idesc_bf16(TILE_M, NP, 0, 0);
         uint32_t n_planes = 0;                       // planes of the CTA's sequence: each segment's zs - 1 .. ze
@@ -1372,7 +1399,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                     for (int t9 = 0; t9 < 9; ++t9)
 #pragma unroll
                         for (int j = 0; j < C8P / 2; ++j)
-                            mma_bf16_lo(d[0], al + (uint32_t)((t9 / 3) * HALO_X + t9 % 3 + 2 * j * RING_V),
+                            mma_bf16_lo(d[0], al + (uint32_t)(((t9 / 3) * HALO_X + t9 % 3) * 2 + j * (int)GROUP16),
                                         (uint32_t)(a0 >> 32), bl + (uint32_t)((t9 * C8P + 2 * j) * NP),
                                         (uint32_t)(b0 >> 32), IDESC, (t9 > 0 || j > 0) ? 1u : 0u);
                     mma_commit(&rfull[rsk[0]]);
@@ -1381,14 +1408,14 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
             } else if (elect_one()) {
 #pragma unroll
                 for (int t9 = 0; t9 < 9; ++t9) {
-                    const uint32_t ta = (uint32_t)((t9 / 3) * HALO_X + t9 % 3);
+                    const uint32_t ta = (uint32_t)((t9 / 3) * HALO_X + t9 % 3) * 2;
                     for (int j = 0; j < c8p / 2; ++j) {
                         const uint64_t bd = b0 + (uint32_t)((t9 * c8p + 2 * j) * NP);
                         const uint32_t acc = (t9 > 0 || j > 0) ? 1u : 0u;
 #pragma unroll
                         for (int k = 0; k < G; ++k)
                             if (G == 1 || (uint32_t)k < gn)
-                                mma_bf16(d[k], a0 + so[k] + ta + (uint32_t)(2 * j * RING_V), bd, IDESC, acc);
+                                mma_bf16(d[k], a0 + so[k] + ta + (uint32_t)j * GROUP16, bd, IDESC, acc);
                     }
                 }
 #pragma unroll
@@ -1748,8 +1775,6 @@ struct WgradT {
 };
 
 __host__ __device__ constexpr int wgrad_tma_stages(int n) { return n <= 16 ? 6 : (n <= 32 ? 5 : (n <= 64 ? 4 : 3)); }
-// descriptor layout type of rows of `bytes` (32, 64 or 128)
-__host__ __device__ constexpr uint32_t swizzle_layout(int bytes) { return bytes == 32 ? 6u : (bytes == 64 ? 4u : 2u); }
 
 template <int N>
 __global__ void __launch_bounds__(THREADS) wgrad_tma_kernel(const __grid_constant__ CUtensorMap xmap,
@@ -2453,12 +2478,53 @@ int ps_workspace(size_t bytes, cudaStream_t st, float*& ws) {
     return rc;
 }
 
+// cuTensorMapEncodeTiled from the driver (the runtime is linked statically,
+// the driver API is reached through its entry point).
+using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                       const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                       CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+TensorMapEncodeFn tensor_map_encoder() {
+    static std::once_flag once;
+    static TensorMapEncodeFn fn = nullptr;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
+                cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = (TensorMapEncodeFn)p;
+    });
+    return fn;
+}
+
+// 5D map of a [batch][d][h][w][c] BF16 tensor with boxes {bc, bx, by, 1, 1}
+// (bc = 16, 32 or 64 channels: rows of 32, 64 or 128 bytes, written with the
+// swizzle of that width); coordinates outside it read zeros.
+int volume_map(CUtensorMap* m, const void* base, int c, int batch, int d, int h, int w, int bc, int bx, int by) {
+    TensorMapEncodeFn enc = tensor_map_encoder();
+    if (!enc) return set_error(CCU_E_DEVICE, "cuTensorMapEncodeTiled is not available from the driver");
+    const cuuint64_t dims[5] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)d, (cuuint64_t)batch};
+    const cuuint64_t strides[4] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2,
+                                   (cuuint64_t)d * h * w * c * 2};
+    const cuuint32_t box[5] = {(cuuint32_t)bc, (cuuint32_t)bx, (cuuint32_t)by, 1u, 1u};
+    const cuuint32_t estride[5] = {1u, 1u, 1u, 1u, 1u};
+    const CUtensorMapSwizzle sw = bc == 16 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                           : (bc == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
+    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box,
+                           estride, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error(CCU_E_INVALID, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
+    return CCU_OK;
+}
+
 // One launch: the pass's channel groups and output slice.
 template <int NO, int G, int C8P, bool PLAIN = false>
-int launch_conv_ps_pass(const ConvP& P, const PsPass& Q, long long planes, int sms, cudaStream_t st) {
+int launch_conv_ps_pass(const CUtensorMap& amap, const ConvP& P, const PsPass& Q, long long planes, int sms,
+                        cudaStream_t st) {
     if constexpr (G == 1 && C8P > 0 && !PLAIN) {
         if (!P.mask0 && !P.head && !Q.part_in && !Q.part_out && P.out0 && Q.co_lo + NO <= P.split)
-            return launch_conv_ps_pass<NO, G, C8P, true>(P, Q, planes, sms, st);
+            return launch_conv_ps_pass<NO, G, C8P, true>(amap, P, Q, planes, sms, st);
     }
     const auto kernel = conv_ps_kernel<NO, G, C8P, PLAIN>;
     const int c8p = Q.c8_hi - Q.c8_lo;
@@ -2478,7 +2544,7 @@ int launch_conv_ps_pass(const ConvP& P, const PsPass& Q, long long planes, int s
     int resident = 1;
     if ((rc = resident_ctas(kernel, smem, cols, resident, PS_THREADS)) != CCU_OK) return rc;
     const long long grid = std::min<long long>(planes, (long long)sms * resident);
-    kernel<<<(unsigned)grid, PS_THREADS, smem, st>>>(P, Q, ring);
+    kernel<<<(unsigned)grid, PS_THREADS, smem, st>>>(amap, P, Q, ring);
     CU_CHECK(cudaGetLastError());
     return CCU_OK;
 }
@@ -2491,6 +2557,9 @@ int launch_conv_ps_g(const ConvP& P, int n_out, int passes, cudaStream_t st) {
     CU_CHECK(cudaGetDevice(&dev));
     CU_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const long long planes = (long long)P.src.B * ((P.src.H + 15) / 16) * ((P.src.W + 7) / 8) * P.src.D;
+    CUtensorMap amap;
+    const int map_rc = volume_map(&amap, P.src.a, P.src.ca, P.src.B, P.src.D, P.src.H, P.src.W, 16, HALO_X, HALO_Y);
+    if (map_rc != CCU_OK) return map_rc;
     float* ws = nullptr;
     if (passes > 1) {
         const int rc = ps_workspace((size_t)P.n_vox * NO * sizeof(float), st, ws);
@@ -2508,11 +2577,11 @@ int launch_conv_ps_g(const ConvP& P, int n_out, int passes, cudaStream_t st) {
         Q.part_out = Q.c8_hi < c8n ? ws : nullptr;
         int rc = CCU_OK;
         switch (G == 1 ? Q.c8_hi - Q.c8_lo : 0) {          // 16 to 64 input channels per pass: unrolled issue
-            case 2: rc = launch_conv_ps_pass<NO, G, G == 1 ? 2 : 0>(P, Q, planes, sms, st); break;
-            case 4: rc = launch_conv_ps_pass<NO, G, G == 1 ? 4 : 0>(P, Q, planes, sms, st); break;
-            case 6: rc = launch_conv_ps_pass<NO, G, G == 1 ? 6 : 0>(P, Q, planes, sms, st); break;
-            case 8: rc = launch_conv_ps_pass<NO, G, G == 1 ? 8 : 0>(P, Q, planes, sms, st); break;
-            default: rc = launch_conv_ps_pass<NO, G, 0>(P, Q, planes, sms, st); break;
+            case 2: rc = launch_conv_ps_pass<NO, G, G == 1 ? 2 : 0>(amap, P, Q, planes, sms, st); break;
+            case 4: rc = launch_conv_ps_pass<NO, G, G == 1 ? 4 : 0>(amap, P, Q, planes, sms, st); break;
+            case 6: rc = launch_conv_ps_pass<NO, G, G == 1 ? 6 : 0>(amap, P, Q, planes, sms, st); break;
+            case 8: rc = launch_conv_ps_pass<NO, G, G == 1 ? 8 : 0>(amap, P, Q, planes, sms, st); break;
+            default: rc = launch_conv_ps_pass<NO, G, 0>(amap, P, Q, planes, sms, st); break;
         }
         if (rc != CCU_OK) return rc;
     }
@@ -2551,46 +2620,6 @@ int launch_wgrad(const WgradP& P, int slices, int cin, cudaStream_t st) {
     dim3 grid((unsigned)((27 * cin + TILE_M - 1) / TILE_M), (unsigned)slices);
     wgrad_kernel<N><<<grid, THREADS, smem, st>>>(P);
     CU_CHECK(cudaGetLastError());
-    return CCU_OK;
-}
-
-// cuTensorMapEncodeTiled from the driver (the runtime is linked statically,
-// the driver API is reached through its entry point).
-using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                       const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                       CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-TensorMapEncodeFn tensor_map_encoder() {
-    static std::once_flag once;
-    static TensorMapEncodeFn fn = nullptr;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (TensorMapEncodeFn)p;
-    });
-    return fn;
-}
-
-// 5D map of a [batch][d][h][w][c] BF16 tensor with boxes {bc, bx, by, 1, 1}
-// (bc = 16, 32 or 64 channels: rows of 32, 64 or 128 bytes, written with the
-// swizzle of that width); coordinates outside it read zeros.
-int volume_map(CUtensorMap* m, const void* base, int c, int batch, int d, int h, int w, int bc, int bx, int by) {
-    TensorMapEncodeFn enc = tensor_map_encoder();
-    if (!enc) return set_error(CCU_E_DEVICE, "cuTensorMapEncodeTiled is not available from the driver");
-    const cuuint64_t dims[5] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)d, (cuuint64_t)batch};
-    const cuuint64_t strides[4] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2,
-                                   (cuuint64_t)d * h * w * c * 2};
-    const cuuint32_t box[5] = {(cuuint32_t)bc, (cuuint32_t)bx, (cuuint32_t)by, 1u, 1u};
-    const cuuint32_t estride[5] = {1u, 1u, 1u, 1u, 1u};
-    const CUtensorMapSwizzle sw = bc == 16 ? CU_TENSOR_MAP_SWIZZLE_32B
-                                           : (bc == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
-    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box,
-                           estride, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return set_error(CCU_E_INVALID, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
     return CCU_OK;
 }
 
