@@ -1741,66 +1741,76 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradP P) {
 }
 
 // ---------------------------------------------------------------------------
-// weight gradient from tensor-memory-accelerator tile loads
+// weight gradient from halo planes
 // ---------------------------------------------------------------------------
 
-// The GEMM of wgrad_kernel -- M = 128 (tap, ci) rows, N = output channels,
-// K = voxels -- for inputs that are not concatenated, with both operands
-// copied by the tensor memory accelerator instead of gathered by threads.
-// A K stage is a block of bx x by = 64 voxels at one z (bx a power of two
-// that divides W).  A box {c channels, bx, by, 1, 1} of the input, c =
-// min(cin, 64), at the stage's coordinates shifted by one tap holds the
-// A operand of c rows (tap, ci0 .. ci0 + c - 1) of the M tile: 64 voxel
-// rows of 2c bytes, written with the 32-, 64- or 128-byte swizzle that
-// matches its row length, which is the MN-major swizzled layout of the MMA
-// (the M tile's 128 / c boxes are its atom columns, 128 c bytes apart; K
-// groups of 8 rows are 16 c bytes apart).  The copy engine handles a box
-// row per cycle or so, so rows of whole voxels (32 bytes and more) move
-// more bytes per row than 16-byte channel groups would.  Coordinates
-// outside the volume read zeros, the convolution's zero padding.  The
-// output-gradient operand is the same kind of box of dz at the unshifted
-// coordinates (min(N, 64) channels), so K runs over the same voxels in the
-// same order in both.  Warp 0 issues the copies (lanes 0 .. 7: A boxes;
-// lanes 16, 17: dz boxes) once lane 0 has set the stage's expected bytes;
-// one thread of warp 1 issues the MMAs and commits the stage's "empty"
-// barrier; every warp then reads the accumulator and adds it into dw.
-struct WgradT {
-    float* dw;                   // [27][N][ld], accumulated at columns c_off .. c_off + cin - 1
-    int ld, c_off;               // columns of dw (all input channels of the layer), first column here
-    int cin, rows;               // input channels of this operand, 27 x cin
-    int a_ch;                    // channels of an A box: min(cin, 64)
-    int D, ny_blk, nx_blk;       // depth, y blocks (of by), x blocks (of bx)
-    int bx, by;                  // a stage's voxels along x and y (bx x by = KSTAGE)
-    long long stages;            // volumes x D x ny_blk x nx_blk
+// dW[dz, dy, dx][co][ci] = sum_v dz[v][co] X[v + (dz, dy, dx)][ci] as a GEMM
+// with K = voxels and both operands MN-major, for one group of CI input
+// channels and one of CO output channels (blockIdx.y).  A CTA walks down
+// 16 (y) x 8 (x) columns as the plane-stationary convolution does; per step
+// it loads one plane of the output gradient (128 rows of CO channels) and
+// one 18 x 10 halo plane of X (180 rows of CI channels), each voxel row
+// written with the swizzle of its length, and reads the halo plane under
+// shifted starts for all nine in-plane taps:
+//   M: four atoms of CI rows one voxel apart along x (dx = 0, 1, 2 and one
+//      unused, to fill M = 64 or 128), LBO = one voxel row;
+//   N: the gradient's planes z - 1, z, z + 1 (the taps dz = 2, 1, 0 of the X
+//      plane z), CO columns each, LBO = one ring slot;
+//   K: 16 voxels (two y rows of 8) per MMA, SBO = one y row of the operand;
+// and one accumulator of 3 CO columns per dy.  So an X plane crosses L2 once
+// per CTA instead of once per tap, which bounded the kernel that this
+// replaced (boxes of 64 voxels per tap: 223 us for 16 -> 16 channels on
+// 4 x 64^3), and per 128 voxels the tensor core runs 24 MMAs of M = 64, N = 48
+// (28 cycles each, bound by reading the operands from shared memory).
+// The gradient ring repeats its first two slots behind its last one, so that
+// the three planes of a window are one slot apart wherever it starts.
+// Warp 0 loads; warps 1 and 2 issue (dy = 0 and 1; dy = 2: separate
+// accumulators); every warp then adds the accumulators into dw.
+// Voxels outside the volume read zeros in both operands (an infinite X next
+// to a zero gradient row of the padding gives NaN, as it does next to a
+// zero inside the volume).
+struct WgradH {
+    Src vol;                     // sizes only
+    float* dw;                   // [27][cout][ld], accumulated at columns c_off ..
+    int ld, c_off, cout;
+    int ci_groups;               // blockIdx.y = co group * ci_groups + ci group
 };
 
-__host__ __device__ constexpr int wgrad_tma_stages(int n) { return n <= 16 ? 6 : (n <= 32 ? 5 : (n <= 64 ? 4 : 3)); }
+constexpr int WH_RING_MAX = 12;
+constexpr int WH_DY = 3;
+// bytes of a ring slot: X halo plane (padded to the swizzle pattern's 256 or
+// 512 bytes; the unused dx = 3 atom reads one row into the padding), gradient plane
+__host__ __device__ constexpr uint32_t wh_x_bytes(int ci) { return (uint32_t)(RING_V * ci * 2 + 511) / 512 * 512; }
+__host__ __device__ constexpr uint32_t wh_z_bytes(int co) { return (uint32_t)(TILE_M * co * 2); }
+__host__ __device__ constexpr uint32_t wh_smem_bytes(int ci, int co, int ring) {
+    return (uint32_t)ring * wh_x_bytes(ci) + (uint32_t)(ring + 2) * wh_z_bytes(co) + 1024;
+}
+__host__ __device__ constexpr uint32_t wh_tmem_cols(int co) { return co <= 16 ? 256u : 512u; }
 
-template <int N>
-__global__ void __launch_bounds__(THREADS) wgrad_tma_kernel(const __grid_constant__ CUtensorMap xmap,
-                                                            const __grid_constant__ CUtensorMap zmap,
-                                                            const WgradT P) {
-    constexpr int NS = wgrad_tma_stages(N);
-    constexpr int B_CH = N < 64 ? N : 64;                      // channels of a dz box
-    constexpr uint32_t A_BYTES = TILE_M * KSTAGE * 2, STAGE = wgrad_stage_bytes(N);
-    static_assert(STAGE % 1024 == 0, "stages keep the 1 KB alignment of the swizzle patterns");
+template <int CI, int CO>
+__global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_constant__ CUtensorMap xmap,
+                                                             const __grid_constant__ CUtensorMap zmap,
+                                                             const WgradH P, int ring) {
+    constexpr int M = 4 * CI, NP = 3 * CO;
+    constexpr uint32_t XB = wh_x_bytes(CI), ZB = wh_z_bytes(CO), AR = 2u * CI, BR = 2u * CO;
+    static_assert((M == 64 || M == 128) && WH_DY * NP <= 512, "four atoms of 16 or 32 rows");
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ uint64_t full[NS], empty[NS], done;
+    __shared__ uint64_t full[WH_RING_MAX], empty[WH_RING_MAX], done;
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
-    const int r0 = blockIdx.x * TILE_M;
-    const long long s_begin = P.stages * blockIdx.y / gridDim.y;
-    const int n_st = (int)(P.stages * (blockIdx.y + 1) / gridDim.y - s_begin);
+    const Src& S = P.vol;
+    const uint32_t R = (uint32_t)ring;
+    const int ci_lo = (int)(blockIdx.y % P.ci_groups) * CI, co_lo = (int)(blockIdx.y / P.ci_groups) * CO;
     volatile int* fail = &s_fail;
 
-    if (warp == 0) tmem_alloc(&s_tmem, tmem_cols(N));
+    if (warp == 0) tmem_alloc(&s_tmem, wh_tmem_cols(CO));
     if (tid == 0) {
-        for (int i = 0; i < NS; ++i) {
+        for (uint32_t i = 0; i < R; ++i) {
             mbar_init(&full[i], 1);
-            mbar_init(&empty[i], 1);
+            mbar_init(&empty[i], 2);                           // one commit per issuing warp
         }
-        mbar_init(&done, 1);
+        mbar_init(&done, 2);
         s_fail = 0;
         mbar_init_fence();
     }
@@ -1808,93 +1818,90 @@ __global__ void __launch_bounds__(THREADS) wgrad_tma_kernel(const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
-    const uint32_t sbase = (smem_u32(smem) + 1023u) & ~1023u;     // the launch adds 1 KB of slack
+    const uint32_t xbase = (smem_u32(smem) + 1023u) & ~1023u, zbase = xbase + R * XB;
 
+    PsWalk walk(S);
+    uint32_t L = 0, slot = 0, ph = 0;                          // step, its ring slot and the slot's phase
     if (warp == 0) {
-        // ---- copies: this lane's box, fixed for the CTA ----
-        int c0 = 0, ox = 0, oy = 0, oz = 0;
-        uint32_t dst = 0, box = 0;                                // box bytes, 0: no box
-        const CUtensorMap* map = &xmap;
-        if (lane < TILE_M / P.a_ch) {
-            const int r = r0 + lane * P.a_ch;
-            if (r < P.rows) {
-                const int tap = r / P.cin;
-                c0 = r - tap * P.cin;
-                oz = tap / 9 - 1;
-                oy = (tap / 3) % 3 - 1;
-                ox = tap % 3 - 1;
-                box = (uint32_t)(KSTAGE * 2 * P.a_ch);
-                dst = (uint32_t)lane * box;
+        // ---- loads: step i of a segment of X planes [zs, ze) brings the gradient's plane
+        // zs - 1 + i and, from i = 2 on, the X plane zs + i - 2 ----
+        bool ok = true;
+        for (WsSeg q; ok && walk.next(S, q);) {
+            for (int i = 0; i < q.ze - q.zs + 2; ++i, ++L, ring_next(slot, ph, R)) {
+                if (L >= R) ok = warp_wait_or_fail(&empty[slot], ph ^ 1u, fail);
+                if (!ok) break;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&full[slot], ZB * (slot < 2 ? 2u : 1u) + (i >= 2 ? RING_V * AR : 0u));
+                    tma_load_5d(zbase + slot * ZB, &zmap, &full[slot], co_lo, q.x0, q.y0, q.zs - 1 + i, q.n);
+                    if (slot < 2)
+                        tma_load_5d(zbase + (R + slot) * ZB, &zmap, &full[slot], co_lo, q.x0, q.y0, q.zs - 1 + i, q.n);
+                    if (i >= 2)
+                        tma_load_5d(xbase + slot * XB, &xmap, &full[slot], ci_lo, q.x0 - 1, q.y0 - 1, q.zs + i - 2, q.n);
+                }
+                __syncwarp();
             }
-        } else if (lane >= 16 && lane < 16 + N / B_CH) {
-            c0 = (lane - 16) * B_CH;
-            box = (uint32_t)(KSTAGE * 2 * B_CH);
-            dst = A_BYTES + (uint32_t)(lane - 16) * box;
-            map = &zmap;
-        }
-        const uint32_t bytes = __reduce_add_sync(0xffffffffu, box);
-        int issued = 0;
-        for (int s = 0; s < n_st; ++s) {
-            const int slot = s % NS;
-            int ok = 1;
-            // the slot's previous stage has been read by its MMAs
-            if (lane == 0 && s >= NS) ok = mbar_wait_or_fail(&empty[slot], (uint32_t)((s / NS) - 1) & 1u, fail);
-            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-            long long q = s_begin + s;
-            const int xb = (int)(q % P.nx_blk);
-            q /= P.nx_blk;
-            const int yb = (int)(q % P.ny_blk);
-            q /= P.ny_blk;
-            const int z = (int)(q % P.D), n = (int)(q / P.D);
-            if (lane == 0) mbar_arrive_expect_tx(&full[slot], bytes);
-            __syncwarp();
-            if (box)
-                tma_load_5d(sbase + (uint32_t)slot * STAGE + dst, map, &full[slot], c0, xb * P.bx + ox,
-                            yb * P.by + oy, z + oz, n);
-            issued = s + 1;
         }
         // after a failure, the copies still in flight land before the CTA ends
-        if (lane == 0 && *fail)
-            for (int s = max(0, issued - NS); s < issued; ++s) mbar_wait(&full[s % NS], (uint32_t)(s / NS) & 1u);
-    } else if (warp == 1) {
-        // ---- MMAs: four of K = 16 voxels per stage ----
-        constexpr uint32_t IDESC = idesc_bf16(TILE_M, N, 1, 1);
-        const uint32_t ar = 2u * (uint32_t)P.a_ch, al = swizzle_layout((int)ar);      // A row bytes, layout
-        constexpr uint32_t BR = 2u * B_CH, BL = swizzle_layout(2 * B_CH);
-        for (int s = 0; s < n_st; ++s) {
-            const int slot = s % NS;
-            if (!warp_wait_or_fail(&full[slot], (uint32_t)(s / NS) & 1u, fail)) break;
-            tc_fence_after();
-            const uint32_t a0 = sbase + (uint32_t)slot * STAGE, b0 = a0 + A_BYTES;
-            if (elect_one()) {
+        if (*fail)
+            for (uint32_t p = L > R ? L - R : 0; p < L; ++p) mbar_wait(&full[p % R], (p / R) & 1u);
+    } else if (warp <= 2) {
+        // ---- MMAs: from a segment's third step on, the window of gradient planes of steps i - 2 .. i ----
+        const uint64_t a0 = smem_desc_sw(xbase, AR, HALO_X * AR, swizzle_layout((int)AR));
+        const uint64_t b0 = smem_desc_sw(zbase, ZB, 8 * BR, swizzle_layout((int)BR));
+        constexpr uint32_t IDESC = idesc_bf16(M, NP, 1, 1);
+        const int dy0 = warp == 1 ? 0 : 2, dyn = warp == 1 ? 2 : 1;
+        uint32_t acc = 0;
+        uint32_t s1 = 0, s2 = 0;                               // slots of the steps before
+        bool ok = true;
+        for (WsSeg q; ok && walk.next(S, q);) {
+            for (int i = 0; i < q.ze - q.zs + 2; ++i, ++L, ring_next(slot, ph, R)) {
+                ok = warp_wait_or_fail(&full[slot], ph, fail);
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
+                    if (i >= 2) {
+                        const uint32_t al = (uint32_t)a0 + slot * (XB / 16) + (uint32_t)dy0 * (HALO_X * AR / 16);
+                        const uint32_t bl = (uint32_t)b0 + s2 * (ZB / 16);
 #pragma unroll
-                for (int k = 0; k < KSTAGE / 16; ++k)
-                    mma_bf16(tmem, smem_desc_sw(a0 + k * 16 * ar, KSTAGE * ar, 8 * ar, al),
-                             smem_desc_sw(b0 + k * 16 * BR, KSTAGE * BR, 8 * BR, BL), IDESC,
-                             (s > 0 || k > 0) ? 1u : 0u);
-                mma_commit(&empty[slot]);
+                        for (int k = 0; k < TILE_M / 16; ++k)
+#pragma unroll
+                            for (int y = 0; y < 2; ++y)
+                                if (y < dyn)
+                                    mma_bf16_lo(tmem + (uint32_t)((dy0 + y) * NP),
+                                                al + (uint32_t)((2 * k + y) * (int)(HALO_X * AR / 16)),
+                                                (uint32_t)(a0 >> 32), bl + (uint32_t)(k * (int)BR), (uint32_t)(b0 >> 32),
+                                                IDESC, k > 0 ? 1u : acc);
+                    }
+                    if (L >= 2) mma_commit(&empty[s2]);
+                }
+                __syncwarp();
+                if (i >= 2) acc = 1;
+                s2 = s1;
+                s1 = slot;
             }
-            __syncwarp();
         }
-        if (elect_one()) mma_commit(&done);          // arrives once every MMA issued above has finished
+        if (elect_one()) mma_commit(&done);                    // arrives once every MMA issued above has finished
         __syncwarp();
     }
-    // ---- epilogue: the accumulator into dw ----
-    if (lane == 0) mbar_wait_or_fail(&done, 0u, fail);
+    // ---- epilogue: the accumulators into dw; lane quarter q holds dx = q ----
+    mbar_wait_or_fail(&done, 0u, fail);
     __syncthreads();
     tc_fence_after();
-    const bool good = !*fail && n_st > 0;
-    if (good) {
-        const int q = warp & 3, half = warp >> 2;
-        const int rr = r0 + q * 32 + lane;
-        const int tp = rr / P.cin, cc = rr - tp * P.cin;
-        for (int c0 = half * 8; c0 < N; c0 += 16) {
-            float f[8];
-            tmem_ld8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, f);
-            if (rr < P.rows) {
+    PsWalk any(S);
+    WsSeg first;
+    if (!*fail && any.next(S, first)) {
+        const int dx = warp & 3, half = warp >> 2;
+        if (dx < 3) {
+            for (int g = half; g < WH_DY * NP / 8; g += 2) {
+                const int col = 8 * g, dy = col / NP, z = 2 - (col / CO) % 3, co = co_lo + col % CO;
+                float f[8];
+                tmem_ld8(tmem + ((uint32_t)(dx * 32) << 16) + (uint32_t)col, f);
+                if (lane < CI) {
+                    float* d = P.dw + ((size_t)((z * 3 + dy) * 3 + dx) * P.cout + co) * P.ld + P.c_off + ci_lo + lane;
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    atomicAdd(P.dw + ((size_t)tp * N + c0 + j) * P.ld + P.c_off + cc, f[j]);
+                    for (int j = 0; j < 8; ++j) atomicAdd(d + (size_t)j * P.ld, f[j]);
+                }
+                __syncwarp();
             }
         }
     } else if (*fail && tid == 0) {
@@ -1902,7 +1909,7 @@ __global__ void __launch_bounds__(THREADS) wgrad_tma_kernel(const __grid_constan
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, tmem_cols(N));
+    if (warp == 0) tmem_dealloc(tmem, wh_tmem_cols(CO));
 }
 
 // Nearest 2x upsampling, channels-last: out[n][z][y][x] = b[n][z/2][y/2][x/2]
@@ -2623,41 +2630,45 @@ int launch_wgrad(const WgradP& P, int slices, int cin, cudaStream_t st) {
     return CCU_OK;
 }
 
-template <int N>
-int launch_wgrad_tma(const void* a, int ca, int batch, int d, int h, int w, const void* dz, float* dw, int ld,
-                     int c_off, int slices, cudaStream_t st) {
-    int bx = KSTAGE;
-    while (w % bx) bx >>= 1;                        // >= 8: checked by the caller
-    const int by = KSTAGE / bx;
-    const int a_ch = std::min(ca, 64);             // ca: 16, 32 or a multiple of 64, checked by the caller
+// dW of one input operand x (channels c_off .. c_off + cx - 1 of the layer's ld).
+template <int CI, int CO>
+int launch_wgrad_halo(const void* x, int cx, int batch, int d, int h, int w, const void* dz, int cout, float* dw, int ld,
+                      int c_off, int slices, cudaStream_t st) {
     CUtensorMap xmap, zmap;
-    int rc = volume_map(&xmap, a, ca, batch, d, h, w, a_ch, bx, by);
-    if (rc == CCU_OK) rc = volume_map(&zmap, dz, N, batch, d, h, w, std::min(N, 64), bx, by);
+    int rc = volume_map(&xmap, x, cx, batch, d, h, w, CI, HALO_X, HALO_Y);
+    if (rc == CCU_OK) rc = volume_map(&zmap, dz, cout, batch, d, h, w, CO, 8, 16);
     if (rc != CCU_OK) return rc;
-    WgradT P;
+    int dev = 0, sms = 0;
+    CU_CHECK(cudaGetDevice(&dev));
+    CU_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const auto kernel = wgrad_halo_kernel<CI, CO>;
+    const uint32_t cols = wh_tmem_cols(CO);
+    // deepest ring (a window of three planes and one in flight at least) that keeps
+    // the CTAs per SM the tensor memory allows
+    int ring = 0, best = 0;
+    for (int r = 4; r <= WH_RING_MAX && wh_smem_bytes(CI, CO, r) <= 200 * 1024; ++r) {
+        int res = 1;
+        if ((rc = resident_ctas(kernel, wh_smem_bytes(CI, CO, r) + 1024, cols, res)) != CCU_OK) return rc;
+        if (res >= best) best = res, ring = r;
+    }
+    size_t smem = 0;
+    if ((rc = tc_launch_smem(kernel, wh_smem_bytes(CI, CO, ring), cols, smem)) != CCU_OK) return rc;
+    int resident = 1;
+    if ((rc = resident_ctas(kernel, smem, cols, resident)) != CCU_OK) return rc;
+    WgradH P;
+    P.vol = Src{nullptr, nullptr, 0, 0, batch, d, h, w};
     P.dw = dw;
     P.ld = ld;
     P.c_off = c_off;
-    P.cin = ca;
-    P.rows = 27 * ca;
-    P.a_ch = a_ch;
-    P.D = d;
-    P.bx = bx;
-    P.by = by;
-    P.nx_blk = w / bx;
-    P.ny_blk = (h + by - 1) / by;
-    P.stages = (long long)batch * d * P.ny_blk * P.nx_blk;
-    size_t smem = 0;
-    rc = tc_launch_smem(wgrad_tma_kernel<N>, (size_t)wgrad_tma_stages(N) * wgrad_stage_bytes(N) + 1024, tmem_cols(N),
-                        smem);
-    if (rc != CCU_OK) return rc;
-    // at least four CTAs per SM over the M tiles when the stages allow it
-    // (the deep levels have few voxels), else the caller's split
-    const int mtiles = (P.rows + TILE_M - 1) / TILE_M;
-    const long long want = std::max<long long>(slices, (4LL * sm_count() + mtiles - 1) / mtiles);
-    const long long splits = std::max(1LL, std::min<long long>(want, P.stages));
-    dim3 grid((unsigned)mtiles, (unsigned)splits);
-    wgrad_tma_kernel<N><<<grid, THREADS, smem, st>>>(xmap, zmap, P);
+    P.cout = cout;
+    P.ci_groups = cx / CI;
+    // plane ranges per channel-group pair: at least the caller's split (the
+    // voxels of one FP32 accumulator), in whole waves of the resident CTAs
+    const long long planes = (long long)batch * ((h + 15) / 16) * ((w + 7) / 8) * d;
+    const long long jobs = (long long)P.ci_groups * (cout / CO), room = (long long)sms * resident;
+    const long long waves = (std::max<long long>(slices, 1) * jobs + room - 1) / room;
+    const long long splits = std::max(1LL, std::min(planes, std::max(1LL, waves * room / jobs)));
+    kernel<<<dim3((unsigned)splits, (unsigned)jobs), THREADS, smem, st>>>(xmap, zmap, P, ring);
     CU_CHECK(cudaGetLastError());
     return CCU_OK;
 }
@@ -2786,21 +2797,21 @@ int ccu_conv3d_wgrad(const void* a, int ca, const void* b, int cb, int batch, in
     if (rc != CCU_OK) return rc;
     if (!dz || !dw || !aligned16(dz) || slices <= 0) return set_error(CCU_E_INVALID, "bad gradient arguments");
     cudaStream_t st = (cudaStream_t)stream;
+    if (cout != 16 && cout != 32 && cout != 64 && cout != 128)
+        return set_error(CCU_E_INVALID, "output channels must be one of 16, 32, 64, 128");
+    // a concatenated layer reads its upsampled part from a copy in a
+    // per-device buffer: only for the shapes documented to use that buffer
     auto box_channels = [](int c) { return c == 16 || c == 32 || c % 64 == 0; };
-    if (g_wgrad_path == 0 && w % 8 == 0 && box_channels(ca) && (cb == 0 || box_channels(cb))) {
-        if (cout != 16 && cout != 32 && cout != 64 && cout != 128)
-            return set_error(CCU_E_INVALID, "output channels must be one of 16, 32, 64, 128");
+    if (g_wgrad_path == 0 && (cb == 0 || (w % 8 == 0 && box_channels(ca) && box_channels(cb)))) {
         auto run = [&](const void* x, int cx, int c_off) {
-            switch (cout) {
-                case 16: return launch_wgrad_tma<16>(x, cx, batch, d, h, w, dz, dw, ca + cb, c_off, slices, st);
-                case 32: return launch_wgrad_tma<32>(x, cx, batch, d, h, w, dz, dw, ca + cb, c_off, slices, st);
-                case 64: return launch_wgrad_tma<64>(x, cx, batch, d, h, w, dz, dw, ca + cb, c_off, slices, st);
-                default: return launch_wgrad_tma<128>(x, cx, batch, d, h, w, dz, dw, ca + cb, c_off, slices, st);
-            }
+            if (cx % 32 == 0)
+                return cout == 16 ? launch_wgrad_halo<32, 16>(x, cx, batch, d, h, w, dz, cout, dw, ca + cb, c_off, slices, st)
+                                  : launch_wgrad_halo<32, 32>(x, cx, batch, d, h, w, dz, cout, dw, ca + cb, c_off, slices, st);
+            return cout == 16 ? launch_wgrad_halo<16, 16>(x, cx, batch, d, h, w, dz, cout, dw, ca + cb, c_off, slices, st)
+                              : launch_wgrad_halo<16, 32>(x, cx, batch, d, h, w, dz, cout, dw, ca + cb, c_off, slices, st);
         };
         if (cb == 0) return run(a, ca, 0);
-        // a concatenated layer: the skip part from a, the upsampled part
-        // from its full-resolution copy in a per-device buffer
+        // the skip part from a, the upsampled part from its full-resolution copy
         void* up = nullptr;
         const long long n_vox = (long long)batch * d * h * w;
         rc = grow_buffer(g_up_ws, (size_t)n_vox * cb * 2, st, up);
