@@ -1137,13 +1137,14 @@ __global__ void __launch_bounds__(THREADS, 4) conv_ws_kernel(const ConvP P, int 
 // the partial (part_in) before bias, ReLU, mask and the BF16 store.
 // PLAIN: no mask, partial sums, head or second output (a forward layer in
 // one pass): the epilogue without their tests.
-// Output slices: a launch computes output channels [co_lo, co_lo + NO) of
-// a layer with more (64 output channels: two slices of 32).
+// Output slices: CTA row blockIdx.y computes output channels [co_lo, co_lo +
+// NO), co_lo = the launch's first + blockIdx.y NO, of a layer with more.
 constexpr int PS_REGIONS_MAX = 8;
 constexpr int PS_GROUP_MAX = 3;
 constexpr int PS_THREADS = 416;             // warps 0, 1 MMA, 2-4 loaders, 5-12 epilogue
 constexpr int PS_ISSUERS = 2, PS_EPI_WARP0 = PS_ISSUERS + WS_LOADERS / 32;
 constexpr int PS_EPI_WARPS = 8;
+constexpr uint32_t PS_SMEM_MAX = 220 * 1024;
 // A ring slot holds 16-channel groups of a halo plane, 180 voxel rows of 32
 // bytes under the 32-byte swizzle (16-byte half h of voxel v at half
 // h ^ ((v >> 2) & 1): the pattern repeats every 256 bytes, to which groups
@@ -1208,9 +1209,9 @@ struct PsWalk {
 
 struct PsPass {
     int c8_lo, c8_hi;          // input channel groups of this pass
-    int co_lo, n_out;          // output channels [co_lo, co_lo + NO) of the layer's n_out
-    const float* part_in;      // FP32 partial sums [v][NO] to add, or null
-    float* part_out;           // FP32 sums [v][NO] out (no bias / ReLU / BF16), or null
+    int co_lo, n_out;          // first output channel of the launch's slices, the layer's output channels
+    const float* part_in;      // FP32 partial sums [slice][v][NO] to add, or null
+    float* part_out;           // FP32 sums [slice][v][NO] out (no bias / ReLU / BF16), or null
 };
 
 // An epilogue warp is done with the region of plane z - 1 and, at a
@@ -1246,6 +1247,10 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
     // 16-channel groups of the pass from a (tile loads) and from b (gathered)
     const int na = max(0, min(Q.c8_hi, S.ca / 8) - Q.c8_lo) / 2, nb = c8p / 2 - na;
     volatile int* fail = &s_fail;
+    // this CTA's output slice and its partial sums
+    const int co_lo = Q.co_lo + (int)blockIdx.y * NO;
+    const float* part_in = Q.part_in ? Q.part_in + (size_t)blockIdx.y * P.n_vox * NO : nullptr;
+    float* part_out = Q.part_out ? Q.part_out + (size_t)blockIdx.y * P.n_vox * NO : nullptr;
 
     if (warp == 0) tmem_alloc(&s_tmem, TCOLS);
     if (tid == 0) {
@@ -1265,7 +1270,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
     for (int i = tid; i < 9 * c8p * NP; i += PS_THREADS) {
         const int r = i % NP, g = i / NP;
         const int t9 = g / c8p, c8 = Q.c8_lo + g % c8p, dz = r / NO, co = r % NO;
-        const int src = ((dz * 9 + t9) * c8n + c8) * Q.n_out + Q.co_lo + co;
+        const int src = ((dz * 9 + t9) * c8n + c8) * Q.n_out + co_lo + co;
         cp_async16(swt + (uint32_t)i * 16, P.w + (size_t)src * 8, 16u);
     }
     cp_async_commit();
@@ -1459,10 +1464,10 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         const uint32_t lq = (uint32_t)(qw * 32) << 16;
         const bool heads = !PLAIN && NO == 16 && P.head != nullptr;
         float2 bias[CW / 2];
-        if (P.bias && !heads && (PLAIN || !Q.part_out)) {
+        if (P.bias && !heads && (PLAIN || !part_out)) {
 #pragma unroll
             for (int j = 0; j < CW / 2; ++j) {
-                const float* bp = P.bias + Q.co_lo + grp * CW + 2 * j;
+                const float* bp = P.bias + co_lo + grp * CW + 2 * j;
                 bias[j] = make_float2(__ldg(bp), __ldg(bp + 1));
             }
         }
@@ -1489,17 +1494,17 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                 float hsum = head ? P.head_x[v] + __ldg(P.head + 16) : 0.0f;
                 // output channels [c, c + 8) of this launch go to out0 or out1 (split is a multiple of 8)
                 uint4 mk[CW / 8];
-                if (!PLAIN && P.mask0 && in && !Q.part_out && !heads) {
+                if (!PLAIN && P.mask0 && in && !part_out && !heads) {
 #pragma unroll
                     for (int h = 0; h < CW / 8; ++h)
-                        if (Q.co_lo + c_lo + 8 * h < P.split)
-                            mk[h] = __ldg(reinterpret_cast<const uint4*>(P.mask0 + (size_t)v * P.split + Q.co_lo + c_lo + 8 * h));
+                        if (co_lo + c_lo + 8 * h < P.split)
+                            mk[h] = __ldg(reinterpret_cast<const uint4*>(P.mask0 + (size_t)v * P.split + co_lo + c_lo + 8 * h));
                 }
                 float4 part[CW / 4];
-                if (!PLAIN && Q.part_in && in) {
+                if (!PLAIN && part_in && in) {
 #pragma unroll
                     for (int h = 0; h < CW / 4; ++h)
-                        part[h] = __ldg(reinterpret_cast<const float4*>(Q.part_in + (size_t)v * NO + c_lo) + h);
+                        part[h] = __ldg(reinterpret_cast<const float4*>(part_in + (size_t)v * NO + c_lo) + h);
                 }
                 ok = warp_wait_or_fail(&rfull[r1], ph1, fail);
                 if (!ok) break;
@@ -1521,15 +1526,15 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                             f[j] = add2(add2(make_float2(__uint_as_float(um[2 * j]), __uint_as_float(um[2 * j + 1])),
                                              make_float2(__uint_as_float(u0[2 * j]), __uint_as_float(u0[2 * j + 1]))),
                                         make_float2(__uint_as_float(up[2 * j]), __uint_as_float(up[2 * j + 1])));
-                        if (!PLAIN && Q.part_in) {
+                        if (!PLAIN && part_in) {
 #pragma unroll
                             for (int j = 0; j < CW / 4; ++j) {
                                 f[2 * j] = add2(f[2 * j], make_float2(part[j].x, part[j].y));
                                 f[2 * j + 1] = add2(f[2 * j + 1], make_float2(part[j].z, part[j].w));
                             }
                         }
-                        if (!PLAIN && Q.part_out) {
-                            float4* po = reinterpret_cast<float4*>(Q.part_out + (size_t)v * NO + c0);
+                        if (!PLAIN && part_out) {
+                            float4* po = reinterpret_cast<float4*>(part_out + (size_t)v * NO + c0);
 #pragma unroll
                             for (int j = 0; j < CW / 4; ++j)
                                 po[j] = make_float4(f[2 * j].x, f[2 * j].y, f[2 * j + 1].x, f[2 * j + 1].y);
@@ -1543,7 +1548,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                             }
 #pragma unroll
                             for (int h = 0; h < CW / 8; ++h) {
-                                const int co = Q.co_lo + c0 + 8 * h;
+                                const int co = co_lo + c0 + 8 * h;
                                 float t[8];
 #pragma unroll
                                 for (int j = 0; j < 4; ++j) t[2 * j] = f[4 * h + j].x, t[2 * j + 1] = f[4 * h + j].y;
@@ -2317,7 +2322,7 @@ int tc_launch_smem(K kernel, size_t stages_bytes, uint32_t cols, size_t& smem, i
     CU_CHECK(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     const size_t floor_smem = (size_t)per_sm / (size_t)(max_ctas + 1) + 1024;
     if (smem < floor_smem) smem = floor_smem;
-    if (smem > 200 * 1024) return set_error(CCU_E_INVALID, "stages too large for shared memory");
+    if (smem > PS_SMEM_MAX) return set_error(CCU_E_INVALID, "stages too large for shared memory");
     CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   (int)cudaSharedmemCarveoutMaxShared));
@@ -2358,25 +2363,38 @@ bool stream_applies(const ConvP& P, int n_out) {
            stream_smem_bytes(n_out, cin) <= 200 * 1024;
 }
 
-// Channel passes of the plane-stationary kernel for cin input channels: the
-// fewest passes of equal 16-channel-aligned groups whose weights and a
-// ring of 3 planes fit 200 KB of shared memory (0: does not apply).
-// Output slices of the plane-stationary kernel: one of 16 or 32 channels,
-// two of 32 for 64 (0: does not apply).
-int ps_slice(int n_out) {
-    if (g_conv_path != 0) return 0;
-    return n_out == 16 ? 16 : (n_out == 32 || n_out == 64) ? 32 : 0;
-}
+// How the plane-stationary kernel runs a layer of n_out output and cin input
+// channels (no = 0: it does not apply): slices of no = 32 or 16 output
+// channels (one CTA row each, and a last slice of 16 where 32 does not
+// divide n_out), and the fewest passes of equal 16-channel-aligned groups of
+// input channels whose weights and a ring of 3 planes fit 200 KB of shared
+// memory.  Passes exchange partial sums through a per-device workspace, so
+// layers beyond 16, 32 and 64 output channels are only taken in one pass:
+// with slices of 16 where the weights of 32 do not fit (128 input channels:
+// 108 KB and two ring slots; 8 x 8^3 volumes 128 -> 128 in 14 us against 67 us
+// in the gathering kernel, whose 32 CTAs each step through 54 stages).
+struct PsPlan {
+    int no = 0, passes = 0;
+};
 
-int ps_passes(int n_out, int cin) {
-    const int no = ps_slice(n_out);
-    if (!no || cin % 16) return 0;
+PsPlan ps_plan(int n_out, int cin) {
+    PsPlan p;
+    if (g_conv_path != 0 || cin % 16) return p;
     const int c16 = cin / 16;
-    for (int passes = 1; passes <= c16; ++passes) {
-        const int c8p = 2 * ((c16 + passes - 1) / passes);
-        if (ps_smem_bytes(no, c8p, 3) <= 200 * 1024) return passes;
+    const bool split = n_out == 16 || n_out == 32 || n_out == 64;
+    const int no = n_out == 16 ? 16 : 32;
+    if (split || n_out == 48 || n_out == 96 || n_out == 128 || n_out == 192) {
+        for (int passes = 1; passes <= (split ? c16 : 1); ++passes) {
+            const int c8p = 2 * ((c16 + passes - 1) / passes);
+            if (ps_smem_bytes(no, c8p, 3) <= 200 * 1024) {
+                p.no = no;
+                p.passes = passes;
+                return p;
+            }
+        }
+        if (!split && ps_smem_bytes(16, 2 * c16, 2) <= PS_SMEM_MAX) p.no = 16, p.passes = 1;
     }
-    return 0;
+    return p;
 }
 
 // Resident CTAs per SM of a kernel launched with this many threads and
@@ -2525,13 +2543,13 @@ int volume_map(CUtensorMap* m, const void* base, int c, int batch, int d, int h,
     return CCU_OK;
 }
 
-// One launch: the pass's channel groups and output slice.
+// One launch: the pass's channel groups and `slices` output slices.
 template <int NO, int G, int C8P, bool PLAIN = false>
-int launch_conv_ps_pass(const CUtensorMap& amap, const ConvP& P, const PsPass& Q, long long planes, int sms,
+int launch_conv_ps_pass(const CUtensorMap& amap, const ConvP& P, const PsPass& Q, int slices, long long planes, int sms,
                         cudaStream_t st) {
     if constexpr (G == 1 && C8P > 0 && !PLAIN) {
-        if (!P.mask0 && !P.head && !Q.part_in && !Q.part_out && P.out0 && Q.co_lo + NO <= P.split)
-            return launch_conv_ps_pass<NO, G, C8P, true>(amap, P, Q, planes, sms, st);
+        if (!P.mask0 && !P.head && !Q.part_in && !Q.part_out && P.out0 && Q.co_lo + slices * NO <= P.split)
+            return launch_conv_ps_pass<NO, G, C8P, true>(amap, P, Q, slices, planes, sms, st);
     }
     const auto kernel = conv_ps_kernel<NO, G, C8P, PLAIN>;
     const int c8p = Q.c8_hi - Q.c8_lo;
@@ -2539,7 +2557,7 @@ int launch_conv_ps_pass(const CUtensorMap& amap, const ConvP& P, const PsPass& Q
     // deepest ring (group + 1 .. WS_RING_MAX planes) that keeps the CTAs per SM the tensor memory allows
     int ring = 0, best_res = 0, rc = CCU_OK;
     size_t smem = 0;
-    for (int r = G + 1; r <= WS_RING_MAX && ps_smem_bytes(NO, c8p, r) <= 200 * 1024; ++r) {
+    for (int r = G + 1; r <= WS_RING_MAX && ps_smem_bytes(NO, c8p, r) <= PS_SMEM_MAX; ++r) {
         int res = 1;
         rc = resident_ctas(kernel, (size_t)ps_smem_bytes(NO, c8p, r) + 1024, cols, res, PS_THREADS);
         if (rc != CCU_OK) return rc;
@@ -2550,30 +2568,27 @@ int launch_conv_ps_pass(const CUtensorMap& amap, const ConvP& P, const PsPass& Q
     if (rc != CCU_OK) return rc;
     int resident = 1;
     if ((rc = resident_ctas(kernel, smem, cols, resident, PS_THREADS)) != CCU_OK) return rc;
-    const long long grid = std::min<long long>(planes, (long long)sms * resident);
-    kernel<<<(unsigned)grid, PS_THREADS, smem, st>>>(amap, P, Q, ring);
+    const long long grid = std::min<long long>(planes, std::max(1, sms * resident / slices));
+    kernel<<<dim3((unsigned)grid, (unsigned)slices), PS_THREADS, smem, st>>>(amap, P, Q, ring);
     CU_CHECK(cudaGetLastError());
     return CCU_OK;
 }
 
+// Output channels [co_lo, co_lo + slices NO) of the layer, in channel passes.
 template <int NO, int G>
-int launch_conv_ps_g(const ConvP& P, int n_out, int passes, cudaStream_t st) {
+int launch_conv_ps_g(const CUtensorMap& amap, const ConvP& P, int n_out, int co_lo, int slices, int passes,
+                     cudaStream_t st) {
     const int c8n = (P.src.ca + P.src.cb) / 8;
     const int c8p_max = 2 * ((c8n / 2 + passes - 1) / passes);
     int dev = 0, sms = 0;
     CU_CHECK(cudaGetDevice(&dev));
     CU_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const long long planes = (long long)P.src.B * ((P.src.H + 15) / 16) * ((P.src.W + 7) / 8) * P.src.D;
-    CUtensorMap amap;
-    const int map_rc = volume_map(&amap, P.src.a, P.src.ca, P.src.B, P.src.D, P.src.H, P.src.W, 16, HALO_X, HALO_Y);
-    if (map_rc != CCU_OK) return map_rc;
     float* ws = nullptr;
     if (passes > 1) {
-        const int rc = ps_workspace((size_t)P.n_vox * NO * sizeof(float), st, ws);
+        const int rc = ps_workspace((size_t)P.n_vox * NO * slices * sizeof(float), st, ws);
         if (rc != CCU_OK) return rc;
     }
-    // output slices one after the other (they share the partial-sum workspace), channel passes within each
-    for (int co_lo = 0; co_lo < n_out; co_lo += NO)
     for (int k = 0, lo = 0; lo < c8n; ++k, lo += c8p_max) {
         PsPass Q;
         Q.co_lo = co_lo;
@@ -2583,28 +2598,38 @@ int launch_conv_ps_g(const ConvP& P, int n_out, int passes, cudaStream_t st) {
         Q.part_in = k > 0 ? ws : nullptr;
         Q.part_out = Q.c8_hi < c8n ? ws : nullptr;
         int rc = CCU_OK;
-        switch (G == 1 ? Q.c8_hi - Q.c8_lo : 0) {          // 16 to 64 input channels per pass: unrolled issue
-            case 2: rc = launch_conv_ps_pass<NO, G, G == 1 ? 2 : 0>(amap, P, Q, planes, sms, st); break;
-            case 4: rc = launch_conv_ps_pass<NO, G, G == 1 ? 4 : 0>(amap, P, Q, planes, sms, st); break;
-            case 6: rc = launch_conv_ps_pass<NO, G, G == 1 ? 6 : 0>(amap, P, Q, planes, sms, st); break;
-            case 8: rc = launch_conv_ps_pass<NO, G, G == 1 ? 8 : 0>(amap, P, Q, planes, sms, st); break;
-            default: rc = launch_conv_ps_pass<NO, G, 0>(amap, P, Q, planes, sms, st); break;
+        switch (G == 1 ? Q.c8_hi - Q.c8_lo : 0) {          // 16 to 64, or 128, input channels per pass: unrolled issue
+            case 2: rc = launch_conv_ps_pass<NO, G, G == 1 ? 2 : 0>(amap, P, Q, slices, planes, sms, st); break;
+            case 4: rc = launch_conv_ps_pass<NO, G, G == 1 ? 4 : 0>(amap, P, Q, slices, planes, sms, st); break;
+            case 6: rc = launch_conv_ps_pass<NO, G, G == 1 ? 6 : 0>(amap, P, Q, slices, planes, sms, st); break;
+            case 8: rc = launch_conv_ps_pass<NO, G, G == 1 ? 8 : 0>(amap, P, Q, slices, planes, sms, st); break;
+            case 16:
+                rc = launch_conv_ps_pass<NO, G, G == 1 && NO == 16 ? 16 : 0>(amap, P, Q, slices, planes, sms, st);
+                break;
+            default: rc = launch_conv_ps_pass<NO, G, 0>(amap, P, Q, slices, planes, sms, st); break;
         }
         if (rc != CCU_OK) return rc;
     }
     return CCU_OK;
 }
 
-// The requested issue group (by default 1: for 16 output channels one chain
-// on each of two CTAs per SM measured 1.4x faster than three interleaved
-// chains on one CTA), down to the largest whose regions fit 512
-// tensor-memory columns (1 for 32 output channels).
-template <int NO>
-int launch_conv_ps(const ConvP& P, int n_out, int passes, cudaStream_t st) {
-    const int group = g_conv_group > 0 ? g_conv_group : 1;
-    if (NO == 16 && group == 3) return launch_conv_ps_g<16, 3>(P, n_out, passes, st);
-    if (NO == 16 && group == 2) return launch_conv_ps_g<16, 2>(P, n_out, passes, st);
-    return launch_conv_ps_g<NO, 1>(P, n_out, passes, st);
+// The layer's slices.  A 16-channel layer takes the requested issue group
+// (by default 1: one chain on each of two CTAs per SM measured 1.4x faster
+// than three interleaved chains on one CTA), whose regions must fit 512
+// tensor-memory columns; the others take 1.
+int launch_conv_ps(const ConvP& P, int n_out, const PsPlan& plan, cudaStream_t st) {
+    CUtensorMap amap;
+    int rc = volume_map(&amap, P.src.a, P.src.ca, P.src.B, P.src.D, P.src.H, P.src.W, 16, HALO_X, HALO_Y);
+    if (rc != CCU_OK) return rc;
+    if (plan.no == 16) {
+        if (n_out == 16 && g_conv_group == 3) return launch_conv_ps_g<16, 3>(amap, P, n_out, 0, 1, plan.passes, st);
+        if (n_out == 16 && g_conv_group == 2) return launch_conv_ps_g<16, 2>(amap, P, n_out, 0, 1, plan.passes, st);
+        return launch_conv_ps_g<16, 1>(amap, P, n_out, 0, n_out / 16, plan.passes, st);
+    }
+    rc = launch_conv_ps_g<32, 1>(amap, P, n_out, 0, n_out / 32, plan.passes, st);
+    if (rc == CCU_OK && n_out % 32)
+        rc = launch_conv_ps_g<16, 1>(amap, P, n_out, n_out / 32 * 32, 1, plan.passes, st);
+    return rc;
 }
 
 template <int N>
@@ -2727,10 +2752,7 @@ int ccu_conv3d(const void* a, int ca, const void* b, int cb, int batch, int d, i
     P.head_x = nullptr;
     P.head_out = nullptr;
     cudaStream_t st = (cudaStream_t)stream;
-    if (const int passes = ps_passes(cout, ca + cb)) {
-        if (ps_slice(cout) == 16) return launch_conv_ps<16>(P, cout, passes, st);
-        return launch_conv_ps<32>(P, cout, passes, st);
-    }
+    if (const PsPlan plan = ps_plan(cout, ca + cb); plan.no) return launch_conv_ps(P, cout, plan, st);
     if (stream_applies(P, cout)) {
         switch (cout) {
             case 16: return launch_conv_stream<16>(P, st);
@@ -2768,7 +2790,7 @@ int ccu_conv3d_head(const void* a, int ca, int batch, int d, int h, int w, const
     if (!aligned16(weight) || (act && !aligned16(act))) return set_error(CCU_E_INVALID, "tensors must be 16-byte aligned");
     const long long n_vox = (long long)batch * d * h * w;
     cudaStream_t st = (cudaStream_t)stream;
-    if (ps_passes(16, ca) == 1) {
+    if (const PsPlan plan = ps_plan(16, ca); plan.passes == 1) {
         ConvP P;
         P.src = Src{(const __nv_bfloat16*)a, nullptr, ca, 0, batch, d, h, w};
         P.w = (const __nv_bfloat16*)weight;
@@ -2782,7 +2804,7 @@ int ccu_conv3d_head(const void* a, int ca, int batch, int d, int h, int w, const
         P.head = head;
         P.head_x = xlog;
         P.head_out = out;
-        return launch_conv_ps<16>(P, 16, 1, st);
+        return launch_conv_ps(P, 16, plan, st);
     }
     // not fusable (another convolution path): the convolution into act, then the head kernel
     if (!act) return set_error(CCU_E_INVALID, "the activation buffer is needed when the head is not fused");

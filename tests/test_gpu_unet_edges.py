@@ -51,3 +51,44 @@ def test_weight_gradient_halo_planes(U, ca, cout, dims, slices):
         v = v.reshape(n, ca)
         bound = (n + 1) * 2.0 ** -23 * (z.abs().T @ v.abs())
         assert bool(((dw[t].double() - z.T @ v).abs() <= bound).all()), t
+
+
+@pytest.mark.parametrize("cin,cout,split,dims", [
+    (16, 48, 16, (1, 3, 17, 9)),            # slices of 32 and 16, the output split inside the first
+    (32, 96, 32, (2, 2, 16, 8)),            # three slices of 32
+    (64, 192, 64, (1, 5, 7, 11)),           # six slices of 32
+    (64, 128, 128, (1, 1, 1, 1)),           # four slices, one voxel
+    (128, 128, 128, (2, 4, 9, 17)),         # eight slices of 16, a ring of two planes
+    (128, 96, 40, (1, 3, 16, 16)),          # six slices of 16, split inside a slice
+])
+@pytest.mark.parametrize("masked", [False, True])
+def test_convolution_output_slices(U, cin, cout, split, dims, masked):
+    """Sums of 27 cin products, exact in FP32, err by at most 2^-23 of the sum
+    of their magnitudes per addition; the BF16 store rounds once (2^-8)."""
+    g = torch.Generator(device="cuda").manual_seed(cin + cout + dims[2])
+    n = dims[0] * dims[1] * dims[2] * dims[3]
+    x = torch.randn(*dims, cin, generator=g, device="cuda").to(torch.bfloat16)
+    w32 = torch.randn(27, cout, cin, generator=g, device="cuda") * 0.05
+    w = torch.empty(U.lib().ccu_packed_weight_elems(cout, cin), dtype=torch.bfloat16, device="cuda")
+    bias = torch.randn(cout, generator=g, device="cuda")
+    mask = torch.randn(n, split, generator=g, device="cuda").to(torch.bfloat16)
+    out0 = torch.empty(n, split, dtype=torch.bfloat16, device="cuda")
+    out1 = torch.empty(n, max(cout - split, 8), dtype=torch.bfloat16, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    U.check(U.lib().ccu_pack_weights(w32.data_ptr(), cout, cin, w.data_ptr(), None, st))
+    U.check(U.lib().ccu_conv3d(x.data_ptr(), cin, None, 0, *dims, w.data_ptr(), bias.data_ptr(), cout, 0,
+                               out0.data_ptr(), split, mask.data_ptr() if masked else None,
+                               out1.data_ptr() if split < cout else None, st))
+    torch.cuda.synchronize()
+    assert U.status() == 0
+    wd = w32.to(torch.bfloat16).double()
+    ref = bias.double().expand(n, cout).clone()
+    mag = ref.abs()
+    for t, v in _taps(x.double()):
+        v = v.reshape(n, cin)
+        ref += v @ wd[t].T
+        mag += v.abs() @ wd[t].abs().T
+    if masked:
+        ref[:, :split] *= mask > 0
+    got = torch.cat([out0, out1], 1)[:, :cout].double() if split < cout else out0.double()
+    assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + (27 * cin + 4) * 2.0 ** -23 * mag).all())
