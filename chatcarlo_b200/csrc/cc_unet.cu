@@ -1207,6 +1207,11 @@ struct PsWalk {
     }
 };
 
+template <int N>
+struct PsInt {
+    static constexpr int value = N;
+};
+
 struct PsPass {
     int c8_lo, c8_hi;          // input channel groups of this pass
     int co_lo, n_out;          // first output channel of the launch's slices, the layer's output channels
@@ -1215,17 +1220,20 @@ struct PsPass {
 };
 
 // An epilogue warp is done with the region of plane z - 1 and, at a
-// segment's end, with those of planes z and z + 1.
-__device__ __forceinline__ void ps_release(uint64_t* rfree, int lane, uint32_t rm, uint32_t r0, uint32_t rp, bool last) {
+// segment's end, with those of planes z and z + 1.  One elected lane arrives,
+// predicated rather than branched to: the warp's tensor-memory reads are
+// complete for all its lanes behind tcgen05.wait.
+__device__ __forceinline__ void ps_release(uint64_t* rfree, uint32_t rm, uint32_t r0, uint32_t rp, bool last) {
     tc_fence_before();
-    __syncwarp();
-    if (lane == 0) {
-        mbar_arrive(&rfree[rm]);
-        if (last) {
-            mbar_arrive(&rfree[r0]);
-            mbar_arrive(&rfree[rp]);
-        }
-    }
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 st;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "@p mbarrier.arrive.shared::cta.b64 st, [%0];\n\t"
+        "setp.ne.and.b32 q, %3, 0, p;\n\t"
+        "@q mbarrier.arrive.shared::cta.b64 st, [%1];\n\t"
+        "@q mbarrier.arrive.shared::cta.b64 st, [%2];\n\t}" ::"r"(smem_u32(rfree + rm)),
+        "r"(smem_u32(rfree + r0)), "r"(smem_u32(rfree + rp)), "r"((int)last)
+        : "memory");
 }
 
 template <int NO, int G, int C8P, bool PLAIN>
@@ -1452,140 +1460,158 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         if (last_r < NQ) mbar_wait(&rfull[last_r], last_ph);
     } else if (warp >= PS_EPI_WARP0) {
         // ---- epilogue: output z = D_{z-1}[dz 0] + D_z[dz 1] + D_{z+1}[dz 2]; row m, lane quarter warp - 4 ----
-        // The voxel's other operands (mask, partial sum, head input) are read
-        // before the wait for the tensor core, the biases once per CTA; a
-        // region is handed back as soon as its values are in registers.
         // Eight warps, two per lane quarter: each takes half of the channels
         // of every output plane, or, with the head (whose sum runs over all
         // channels in order), all channels of every other plane.  Either way
-        // every warp waits for every plane and arrives once per region.
-        constexpr int CW = NO / 2;                             // channels per step
+        // it waits for every plane and arrives once per region, as soon as
+        // the values are in registers.  An output costs a warp some 600 cycles
+        // of latency however few channels it has; what it reads beside the
+        // sums (mask, partial sum) is therefore read a plane ahead: read in
+        // the same plane it cost another 400.
+        constexpr int CW = NO / 2;                             // channels per warp
         const int qw = warp & 3, grp = (warp - PS_EPI_WARP0) >> 2, m = qw * 32 + lane;
         const uint32_t lq = (uint32_t)(qw * 32) << 16;
         const bool heads = !PLAIN && NO == 16 && P.head != nullptr;
+        const bool masked = !PLAIN && P.mask0 && !part_out && !heads;
+        const int c0 = grp * CW, co0 = co_lo + c0;
+        const uint32_t plane = (uint32_t)(S.H * S.W);
         float2 bias[CW / 2];
-        if (P.bias && !heads && (PLAIN || !part_out)) {
+        if (P.bias && (PLAIN || !part_out)) {
 #pragma unroll
-            for (int j = 0; j < CW / 2; ++j) {
-                const float* bp = P.bias + co_lo + grp * CW + 2 * j;
-                bias[j] = make_float2(__ldg(bp), __ldg(bp + 1));
-            }
+            for (int j = 0; j < CW / 2; ++j)
+                bias[j] = make_float2(__ldg(P.bias + co0 + 2 * j), __ldg(P.bias + co0 + 2 * j + 1));
         }
-        // region and phase of plane z + 1, and the regions of planes z and z - 1
-        uint32_t r1 = 0, ph1 = 0;
-        ring_next(r1, ph1, NQ);
-        ring_next(r1, ph1, NQ);                                // the first output reads planes 0, 1, 2
+        // regions of planes z - 1, z and z + 1 and the phase of the last
+        uint32_t rm = 0, r0 = 1, r1 = 2, ph1 = 0;
         bool ok = true;
         PsWalk walk(S);
         for (WsSeg q; ok && walk.next(S, q);) {
             const int y = q.y0 + (m >> 3), x = q.x0 + (m & 7);
             const bool in = y < S.H && x < S.W;
             uint32_t v = (uint32_t)((((long long)q.n * S.D + q.zs) * S.H + y) * S.W + x);
-            // each plane's wait below covers every earlier plane of its own
-            // issuer; the segment's second plane is the other issuer's
-            ok = warp_wait_or_fail(&rfull[r1 == 0 ? NQ - 1 : r1 - 1], r1 == 0 ? ph1 ^ 1u : ph1, fail);
-            if (!ok) break;
-            for (int z = q.zs; z < q.ze; ++z, v += (uint32_t)(S.H * S.W), ring_next(r1, ph1, NQ)) {
-                const uint32_t r0i = r1 == 0 ? NQ - 1 : r1 - 1, rmi = r0i == 0 ? NQ - 1 : r0i - 1;
-                const int c_lo = heads ? 0 : grp * CW;
-                const int c_hi = heads ? ((z & 1) == grp ? NO : 0) : c_lo + CW;
-                // the head: x + b, then + w_j a_j in channel order (the head kernel's FP32 sequence)
-                const bool head = heads && in && c_hi > 0;
-                float hsum = head ? P.head_x[v] + __ldg(P.head + 16) : 0.0f;
-                // output channels [c, c + 8) of this launch go to out0 or out1 (split is a multiple of 8)
-                uint4 mk[CW / 8];
-                if (!PLAIN && P.mask0 && in && !part_out && !heads) {
+            uint4 mk[CW / 8];
+            float4 part[CW / 4];
+            auto read_ahead = [&](uint32_t u) {
+                if (masked) {
 #pragma unroll
                     for (int h = 0; h < CW / 8; ++h)
-                        if (co_lo + c_lo + 8 * h < P.split)
-                            mk[h] = __ldg(reinterpret_cast<const uint4*>(P.mask0 + (size_t)v * P.split + co_lo + c_lo + 8 * h));
+                        if (co0 + 8 * h < P.split)
+                            mk[h] = __ldg(reinterpret_cast<const uint4*>(P.mask0 + (size_t)u * P.split + co0 + 8 * h));
                 }
-                float4 part[CW / 4];
-                if (!PLAIN && part_in && in) {
+                if (part_in) {
 #pragma unroll
                     for (int h = 0; h < CW / 4; ++h)
-                        part[h] = __ldg(reinterpret_cast<const float4*>(part_in + (size_t)v * NO + c_lo) + h);
+                        part[h] = __ldg(reinterpret_cast<const float4*>(part_in + (size_t)u * NO + c0) + h);
                 }
+            };
+            if (!PLAIN && in) read_ahead(v);
+            // each plane's wait below covers every earlier plane of its own
+            // issuer; the segment's second plane is the other issuer's
+            ok = warp_wait_or_fail(&rfull[r0], r1 == 0 ? ph1 ^ 1u : ph1, fail);
+            for (int z = q.zs; ok && z < q.ze; ++z, v += plane) {
                 ok = warp_wait_or_fail(&rfull[r1], ph1, fail);
                 if (!ok) break;
                 tc_fence_after();
-                for (int c0 = c_lo; c0 < c_hi; c0 += CW) {
-                    uint32_t um[CW], u0[CW], up[CW];
-                    tmem_ld_nw<CW>(tmem + rmi * RC + lq + (uint32_t)c0, um);
-                    tmem_ld_nw<CW>(tmem + r0i * RC + NO + lq + (uint32_t)c0, u0);
-                    tmem_ld_nw<CW>(tmem + r1 * RC + 2 * NO + lq + (uint32_t)c0, up);
+                // the sums of CN channels from c on
+                auto sums = [&](auto cn, int c, bool release, float2* f) {
+                    constexpr int CN = decltype(cn)::value;
+                    uint32_t um[CN], u0[CN], up[CN];
+                    tmem_ld_nw<CN>(tmem + rm * RC + lq + (uint32_t)c, um);
+                    tmem_ld_nw<CN>(tmem + r0 * RC + NO + lq + (uint32_t)c, u0);
+                    tmem_ld_nw<CN>(tmem + r1 * RC + 2 * NO + lq + (uint32_t)c, up);
                     tmem_wait_ld();
                     // the uses below stay behind the wait
 #pragma unroll
-                    for (int j = 0; j < CW; ++j) asm volatile("" : "+r"(um[j]), "+r"(u0[j]), "+r"(up[j]));
-                    if (c0 + CW == c_hi) ps_release(rfree, lane, rmi, r0i, r1, z == q.ze - 1);
-                    if (in) {
-                        float2 f[CW / 2];
+                    for (int j = 0; j < CN; ++j) asm volatile("" : "+r"(um[j]), "+r"(u0[j]), "+r"(up[j]));
+                    if (release) ps_release(rfree, rm, r0, r1, z == q.ze - 1);
 #pragma unroll
-                        for (int j = 0; j < CW / 2; ++j)
-                            f[j] = add2(add2(make_float2(__uint_as_float(um[2 * j]), __uint_as_float(um[2 * j + 1])),
-                                             make_float2(__uint_as_float(u0[2 * j]), __uint_as_float(u0[2 * j + 1]))),
-                                        make_float2(__uint_as_float(up[2 * j]), __uint_as_float(up[2 * j + 1])));
-                        if (!PLAIN && part_in) {
+                    for (int j = 0; j < CN / 2; ++j)
+                        f[j] = add2(add2(make_float2(__uint_as_float(um[2 * j]), __uint_as_float(um[2 * j + 1])),
+                                         make_float2(__uint_as_float(u0[2 * j]), __uint_as_float(u0[2 * j + 1]))),
+                                    make_float2(__uint_as_float(up[2 * j]), __uint_as_float(up[2 * j + 1])));
+                };
+                if (heads) {
+                    if ((z & 1) != grp) {
+                        ps_release(rfree, rm, r0, r1, z == q.ze - 1);
+                    } else {
+                        // x + b, then + w_j a_j in channel order (the head kernel's FP32 sequence)
+                        float hsum = in ? P.head_x[v] + __ldg(P.head + 16) : 0.0f;
 #pragma unroll
-                            for (int j = 0; j < CW / 4; ++j) {
-                                f[2 * j] = add2(f[2 * j], make_float2(part[j].x, part[j].y));
-                                f[2 * j + 1] = add2(f[2 * j + 1], make_float2(part[j].z, part[j].w));
+                        for (int c = 0; c < NO; c += 8) {
+                            float2 f[4];
+                            float t[8];
+                            sums(PsInt<8>{}, c, c + 8 == NO, f);
+                            if (in) {
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) t[2 * j] = f[j].x, t[2 * j + 1] = f[j].y;
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) {
+                                    if (P.bias) t[j] += __ldg(P.bias + c + j);
+                                    if (P.relu) t[j] = fmaxf(t[j], 0.0f);
+                                    hsum = fmaf(__ldg(P.head + c + j), __bfloat162float(__float2bfloat16_rn(t[j])), hsum);
+                                }
+                                if (P.out0) *reinterpret_cast<uint4*>(P.out0 + (size_t)v * P.split + c) = pack_bf16x8(t);
                             }
+                            __syncwarp();                      // the next loads are warp-wide
                         }
-                        if (!PLAIN && part_out) {
+                        if (in) P.head_out[v] = hsum;
+                    }
+                } else {
+                    float2 f[CW / 2];
+                    sums(PsInt<CW>{}, c0, true, f);
+                    if (!PLAIN && part_in) {
+#pragma unroll
+                        for (int j = 0; j < CW / 4; ++j) {
+                            f[2 * j] = add2(f[2 * j], make_float2(part[j].x, part[j].y));
+                            f[2 * j + 1] = add2(f[2 * j + 1], make_float2(part[j].z, part[j].w));
+                        }
+                    }
+                    if (!PLAIN && part_out) {
+                        if (in) {
                             float4* po = reinterpret_cast<float4*>(part_out + (size_t)v * NO + c0);
 #pragma unroll
                             for (int j = 0; j < CW / 4; ++j)
                                 po[j] = make_float4(f[2 * j].x, f[2 * j].y, f[2 * j + 1].x, f[2 * j + 1].y);
-                        } else {
-                            if (P.bias) {
+                        }
+                    } else {
+                        if (P.bias) {
 #pragma unroll
-                                for (int j = 0; j < CW / 2; ++j) {
-                                    const float* bp = P.bias + c0 + 2 * j;
-                                    f[j] = add2(f[j], heads ? make_float2(__ldg(bp), __ldg(bp + 1)) : bias[j]);
-                                }
+                            for (int j = 0; j < CW / 2; ++j) f[j] = add2(f[j], bias[j]);
+                        }
+#pragma unroll
+                        for (int h = 0; h < CW / 8; ++h) {
+                            // output channels [co, co + 8) go to out0 or out1 (split is a multiple of 8)
+                            const int co = co0 + 8 * h;
+                            const bool first = PLAIN || co < P.split;
+                            float t[8];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) t[2 * j] = f[4 * h + j].x, t[2 * j + 1] = f[4 * h + j].y;
+                            if (P.relu) {
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) t[j] = fmaxf(t[j], 0.0f);
                             }
+                            if (masked && first) {
+                                float k[8];
+                                unpack_bf16x8(mk[h], k);
 #pragma unroll
-                            for (int h = 0; h < CW / 8; ++h) {
-                                const int co = co_lo + c0 + 8 * h;
-                                float t[8];
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) t[2 * j] = f[4 * h + j].x, t[2 * j + 1] = f[4 * h + j].y;
-                                if (P.relu) {
-#pragma unroll
-                                    for (int j = 0; j < 8; ++j) t[j] = fmaxf(t[j], 0.0f);
-                                }
-                                if (PLAIN || co < P.split) {
-                                    if (!PLAIN && P.mask0) {
-                                        float k[8];
-                                        unpack_bf16x8(mk[h], k);
-#pragma unroll
-                                        for (int j = 0; j < 8; ++j) t[j] = k[j] > 0.0f ? t[j] : 0.0f;
-                                    }
-                                    if (PLAIN || P.out0)
-                                        *reinterpret_cast<uint4*>(P.out0 + (size_t)v * P.split + co) = pack_bf16x8(t);
-                                } else {
-                                    *reinterpret_cast<uint4*>(P.out1 + (size_t)v * (Q.n_out - P.split) + (co - P.split)) =
-                                        pack_bf16x8(t);
-                                }
-                                if (head) {
-#pragma unroll
-                                    for (int j = 0; j < 8; ++j)
-                                        hsum = fmaf(__ldg(P.head + c0 + 8 * h + j),
-                                                    __bfloat162float(__float2bfloat16_rn(t[j])), hsum);
-                                }
+                                for (int j = 0; j < 8; ++j) t[j] = k[j] > 0.0f ? t[j] : 0.0f;
                             }
+                            __nv_bfloat16* o = first ? P.out0 + ((size_t)v * P.split + co)
+                                                     : P.out1 + ((size_t)v * (Q.n_out - P.split) + (co - P.split));
+                            if (in) *reinterpret_cast<uint4*>(o) = pack_bf16x8(t);
                         }
                     }
-                    __syncwarp();                              // the next loads are warp-wide
+                    if (!PLAIN && in && z + 1 < q.ze) read_ahead(v + plane);
                 }
-                if (c_hi == 0) ps_release(rfree, lane, rmi, r0i, r1, z == q.ze - 1);
-                if (head) P.head_out[v] = hsum;
+                rm = r0, r0 = r1;
+                ring_next(r1, ph1, NQ);
             }
             // the next segment's first output reads its planes 0 .. 2: two planes on
-            ring_next(r1, ph1, NQ);
-            ring_next(r1, ph1, NQ);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                rm = r0, r0 = r1;
+                ring_next(r1, ph1, NQ);
+            }
         }
     }
     __syncthreads();
