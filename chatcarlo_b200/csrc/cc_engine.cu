@@ -183,7 +183,8 @@ struct KRun {
     long long first;          // global index of the first history
     long long batch_size;     // histories per scratch buffer
     int n_scratch;
-    int chunk;                // histories a warp takes from the global counter at once
+    int group;                // batches whose units alternate (see HIST_UNIT)
+    int copy_shift;           // log2 of the scratch copies of a batch's slot
     int fluorescence;
     unsigned long long seed;
     long long max_steps;
@@ -198,7 +199,7 @@ struct KRun {
     double* edep;             // [n_scratch][n_mat]
     unsigned long long* counters;   // absorbed, escaped, scatter_sum, n_fluor, steps, voxel visits,
                                     // [6] history counter, [7] segments offered to the queue
-    unsigned long long* work;       // global history counter
+    unsigned long long* work;       // global unit counter
     unsigned* status;
     struct SegRec* seg;             // track-segment queue of the deferred tally
     long long seg_cap;              // its capacity (records)
@@ -732,7 +733,7 @@ struct SegRec {
     real p[3], d[3];
     real t0, t1;
     phys wk, wh;
-    int batch, m;           // scratch slot; pieces of at most TALLY_PIECE visits
+    int slot, m;            // scratch slot; pieces of at most TALLY_PIECE visits
 };
 
 // ---------------------------------------------------------------------------
@@ -855,17 +856,25 @@ __device__ __forceinline__ void sample_source(const KSource& S, HistoryRng& rng,
 // the transport kernel
 // ---------------------------------------------------------------------------
 
-// Histories a warp takes from the global counter at once.  The histories in
-// flight span warps x chunk indices, i.e. several batches, and every batch
-// scores into its own scratch slot.  A small grid (a slot of a few MB) wants
-// that spread: the hot voxels then have several copies in L2 and their
-// atomics contend less.  A grid whose slot is near the L2 size wants the
-// opposite, fewer slots in flight, or its atomics miss in L2.  Measured on
-// the room workload (6 MB slots) 32 histories per chunk were 1.9x slower than
-// 256, on the CT workload (246 MB slots) 9 % faster.
-constexpr int HIST_CHUNK_SPREAD = 256;
-constexpr int HIST_CHUNK_COMPACT = 32;
-constexpr size_t SLOT_BYTES_COMPACT = (size_t)32 << 20;     // slots above this use the compact chunk
+// A warp takes HIST_UNIT consecutive histories of one batch at a time from the
+// launch's counter, so that no warp is left with a long chunk while the others
+// have run dry.  Every batch scores into its own scratch slot, and the order
+// of the units decides how many slots are scored at once.  A small grid (a
+// slot of a few MB) wants several: all histories cross the few voxels next to
+// the source, and reductions on one address follow one another (one slot at a
+// time ran the room workload at 2.8e8 histories/s), so the units go
+// round-robin over groups of SPREAD_SLOTS batches, and a launch of fewer
+// batches scores each into copies of its slot that the fold adds up.  Room
+// workload, transport kernel, 1e5 / 1e6 / 4e6 histories: 0.88 / 4.0 / 14.3 ms
+// with 1 slot at a time, 0.51 / 2.56 / 7.2 with 4, 0.45 / 1.98 / 6.5 with 8,
+// 0.39 / 1.87 / 6.4 with 16, 0.39 / 1.78 / 6.4 with 32 (whose copies cost the
+// fold of small runs more); chunks of 256 consecutive histories per warp, the
+// order before, 1.26 / 2.26 / 6.8, with most warps idle in small runs.
+// A grid whose slot is near the L2 size wants the opposite, one batch after
+// the other, or its reductions miss in L2.
+constexpr int HIST_UNIT = 32;
+constexpr int SPREAD_SLOTS = 16;
+constexpr size_t SLOT_BYTES_COMPACT = (size_t)32 << 20;     // slots above this are scored one after the other
 // Voxel visits per piece when a warp splits its track segments.  The split
 // of a segment depends on that segment alone, never on the warp's other
 // lanes, so every piece -- and every length it scores -- is the same
@@ -920,7 +929,7 @@ __device__ __forceinline__ void score_warp_segments(const KGrid& G, const SegRec
         const int k = u - pre[lo];
         real ta, tz;
         piece_range(q.t0, q.t1, q.m, k, ta, tz);
-        int nv = walk_range<CELL>(G, G.tally + (size_t)q.batch * 2 * G.nvox, q.p, q.d, ta, tz, q.wk, q.wh);
+        int nv = walk_range<CELL>(G, G.tally + (size_t)q.slot * 2 * G.nvox, q.p, q.d, ta, tz, q.wk, q.wh);
         c_vox += max(nv - (k > 0 ? 1 : 0), 0);   // a cut voxel is one visit
     }
     __syncwarp();
@@ -954,6 +963,24 @@ __device__ __forceinline__ void score_warp_segments(const KGrid& G, const SegRec
 // voxel walk, which keeps the loop's code small.
 constexpr int TV_DEFER = 3;
 
+// The next unit of the launch's counter: histories [first, end) of one batch
+// (empty beyond a short last batch) and their scratch slot; first < 0: none left.
+__device__ __forceinline__ void take_unit(const KRun& R, long long& first, long long& end, int& slot) {
+    const long long per = (R.batch_size + HIST_UNIT - 1) / HIST_UNIT;
+    const long long k = (long long)atomicAdd(R.work, 1ull);
+    first = end = -1;
+    if (k >= per * R.n_scratch) return;
+    const long long in_group = per * R.group;
+    const int g = (int)(k / in_group) * R.group;                       // the group's first batch
+    const long long r = k % in_group;
+    const int members = min(R.group, R.n_scratch - g);
+    const long long unit = r / members;
+    const int batch = g + (int)(r - unit * members);
+    first = (long long)batch * R.batch_size + unit * HIST_UNIT;
+    end = max(first, min(first + HIST_UNIT, min((long long)(batch + 1) * R.batch_size, R.n)));
+    slot = (batch << R.copy_shift) | ((int)unit & ((1 << R.copy_shift) - 1));
+}
+
 template <bool FROM_SOURCE, bool TALLY, bool HEEL = false, int TV = CELL_FP64>
 __global__ void __launch_bounds__(BLOCK, CC_MIN_BLOCKS)
 transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource SRC, const KRun R) {
@@ -972,16 +999,14 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
     // thread hands them to the block's 64-bit counters before they near 2^31
     unsigned c_abs = 0, c_esc = 0, c_sc = 0, c_fl = 0, c_steps = 0, c_vox = 0;
 
-    // a launch that leaves the chunk unset takes the spread default (a zero
-    // chunk would never advance the counter)
-    const int chunk = R.chunk > 0 ? R.chunk : HIST_CHUNK_SPREAD;
-    // warp-local pool [pool_next, pool_end)
+    // warp-local pool [pool_next, pool_end), histories of one unit, and its scratch slot
     long long pool_next = 0, pool_end = 0;
+    int pool_slot = 0;
     bool live = false;
     long long h = 0;
     real p[3], d[3];
     phys E = P(0.), tau = P(0.);
-    int nsc = 0, mat = -1, batch = 0;
+    int nsc = 0, mat = -1, slot = 0;
     int steps = 0;
     HistoryRng rng;
 
@@ -990,12 +1015,11 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
         unsigned need = __ballot_sync(FULL, !live);
         while (need) {
             if (pool_next >= pool_end) {
-                long long base = 0;
-                if (lane == 0) base = (long long)atomicAdd(R.work, (unsigned long long)chunk);
-                base = __shfl_sync(FULL, base, 0);
-                if (base >= R.n) break;
-                pool_next = base;
-                pool_end = min(base + chunk, R.n);
+                if (lane == 0) take_unit(R, pool_next, pool_end, pool_slot);
+                pool_next = __shfl_sync(FULL, pool_next, 0);
+                pool_end = __shfl_sync(FULL, pool_end, 0);
+                pool_slot = __shfl_sync(FULL, pool_slot, 0);
+                if (pool_next < 0) break;
             }
             int rank = __popc(need & ((1u << lane) - 1u));
             long long avail = pool_end - pool_next;
@@ -1005,8 +1029,7 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
                 live = true;
                 long long gh = R.first + h;
                 rng.init(R.seed, (unsigned long long)gh, 0u);
-                batch = (int)(h / R.batch_size);
-                if (batch >= R.n_scratch) batch = R.n_scratch - 1;
+                slot = pool_slot;
                 if (FROM_SOURCE) {
                     sample_source<HEEL>(SRC, rng, p, d, E);
                 } else {
@@ -1081,13 +1104,13 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
                         SegRec& r = R.seg[idx];
                         r.p[0] = p[0]; r.p[1] = p[1]; r.p[2] = p[2];
                         r.d[0] = d[0]; r.d[1] = d[1]; r.d[2] = d[2];
-                        r.t0 = t0; r.t1 = t1; r.wk = wk; r.wh = wh; r.batch = batch; r.m = m;
+                        r.t0 = t0; r.t1 = t1; r.wk = wk; r.wh = wh; r.slot = slot; r.m = m;
                     } else {
                         // queue full: this lane walks the same pieces itself
                         for (int k = 0; k < m; ++k) {
                             real ta, tz;
                             piece_range(t0, t1, m, k, ta, tz);
-                            int nv = walk_range(G, G.tally + (size_t)batch * 2 * G.nvox, p, d, ta, tz, wk, wh);
+                            int nv = walk_range(G, G.tally + (size_t)slot * 2 * G.nvox, p, d, ta, tz, wk, wh);
                             c_vox += max(nv - (k > 0 ? 1 : 0), 0);
                         }
                     }
@@ -1100,7 +1123,7 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
                     SegRec& r = s_seg[warp][lane];
                     r.p[0] = p[0]; r.p[1] = p[1]; r.p[2] = p[2];
                     r.d[0] = d[0]; r.d[1] = d[1]; r.d[2] = d[2];
-                    r.t0 = t0; r.t1 = t1; r.wk = wk; r.wh = wh; r.batch = batch; r.m = m;
+                    r.t0 = t0; r.t1 = t1; r.wk = wk; r.wh = wh; r.slot = slot; r.m = m;
                 }
                 score_warp_segments<TV == TV_DEFER ? CELL_RUNTIME : TV>(G, s_seg[warp], s_pre[warp], lane, m, c_vox);
             }
@@ -1130,11 +1153,11 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
             // The element draw, the new direction and the new free path are
             // common to the three interactions; they run outside the branches
             // so that every interacting lane of the warp executes them together.
-            const int slot = pick_element(T, M, L, kind, uni(rng));
+            const int el = pick_element(T, M, L, kind, uni(rng));
             phys cost = P(1.0), e_new = E, dep = P(0.0);
             if (kind == 0) {
                 // photoelectric, K fluorescence (physics.py:155-212, transport.py:174-198)
-                const phys e_line = sample_k_line(T.elems[slot], E, R.fluorescence, rng);
+                const phys e_line = sample_k_line(T.elems[el], E, R.fluorescence, rng);
                 const bool emit = e_line > P(0.0);
                 dep = emit ? E - e_line : E;
                 if (emit) {
@@ -1146,17 +1169,17 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
                 }
             } else if (kind == 1) {
                 phys eps;
-                sample_compton(T.sq + (size_t)slot * TABLE_N, E, rng, eps, cost);
+                sample_compton(T.sq + (size_t)el * TABLE_N, E, rng, eps, cost);
                 e_new = E * eps;
                 dep = E - e_new;
-            } else if (!sample_rayleigh(T.rx + (size_t)slot * TABLE_N, T.ra + (size_t)slot * TABLE_N,
-                                        T.ray_bucket + (size_t)slot * (RAY_BUCKETS + 1), T.elems[slot].ray_scale,
+            } else if (!sample_rayleigh(T.rx + (size_t)el * TABLE_N, T.ra + (size_t)el * TABLE_N,
+                                        T.ray_bucket + (size_t)el * (RAY_BUCKETS + 1), T.elems[el].ray_scale,
                                         E, rng, cost)) {
                 atomicOr(R.status, ST_RAYLEIGH_Q);
                 live = false;
                 continue;
             }
-            if (kind < 2) atomicAdd(&s_edep[batch * T.n_mat + mat], (double)dep);
+            if (kind < 2) atomicAdd(&s_edep[(slot >> R.copy_shift) * T.n_mat + mat], (double)dep);
             if (!done) {
                 if (kind == 0) isotropic(d, rng);                     // the fluorescence photon
                 else scatter_direction(d, cost, TWO_PI * uni(rng));
@@ -1555,9 +1578,25 @@ __global__ void fold_kernel(double2* __restrict__ total, double2* __restrict__ q
 // read and written once per launch instead of once per batch.  The
 // additions per voxel happen in the same order as slot-by-slot folds.
 struct FoldSlots {
-    double inv_nb[MAX_SCRATCH];     // 1 / histories of each batch; 0 skips the slot
-    int n;
+    double inv_nb[MAX_SCRATCH];     // 1 / histories of each batch; 0 skips the batch
+    int n, copies;                  // batches, scratch copies of each (added before the batch is squared)
 };
+
+// A batch's cell: the sum of its copies, which are cleared.
+__device__ __forceinline__ double2 take_cells(double2* __restrict__ scratch, long long nvox, long long i, int copies,
+                                              int cell32) {
+    double2 v = make_double2(0.0, 0.0);
+    for (int c = 0; c < copies; ++c) {
+        double2* sc = scratch + (size_t)c * nvox;
+        const double2 u = cell_read(sc, i, cell32);
+        if (u.x != 0.0 || u.y != 0.0) {
+            v.x += u.x;
+            v.y += u.y;
+            sc[i] = make_double2(0.0, 0.0);
+        }
+    }
+    return v;
+}
 
 __global__ void fold_slots_kernel(double2* __restrict__ total, double2* __restrict__ q, int* __restrict__ nhit,
                                   double2* __restrict__ scratch, long long nvox, const FoldSlots F, int cell32) {
@@ -1569,15 +1608,13 @@ __global__ void fold_slots_kernel(double2* __restrict__ total, double2* __restri
         bool loaded = false;
         for (int s = 0; s < F.n; ++s) {
             if (F.inv_nb[s] == 0.0) continue;
-            double2* sc = scratch + (size_t)s * nvox;
-            const double2 v = cell_read(sc, i, cell32);
+            const double2 v = take_cells(scratch + (size_t)s * F.copies * nvox, nvox, i, F.copies, cell32);
             if (v.x != 0.0 || v.y != 0.0) {
                 if (!loaded) { t = total[i]; qq = q[i]; h = nhit[i]; loaded = true; }
                 t.x += v.x; t.y += v.y;
                 qq.x += v.x * v.x * F.inv_nb[s];
                 qq.y += v.y * v.y * F.inv_nb[s];
                 h += 1;
-                sc[i] = make_double2(0.0, 0.0);
             }
         }
         if (loaded) { total[i] = t; q[i] = qq; nhit[i] = h; }
@@ -2503,14 +2540,16 @@ static int fold_plain(cc_grid* g, int n_slots, int cell32) {
     return CC_OK;
 }
 
-static int fold_batches(cc_grid* g, int n_slots, const long long* counts, int cell32) {
+// `copies` scratch cells per batch and voxel, added before the batch is squared.
+static int fold_batches(cc_grid* g, int n_slots, const long long* counts, int cell32, int copies = 1) {
     cc_ctx* c = g->ctx;
     int threads = 256;
     int blocks = std::max(1, std::min((int)((g->k.nvox + threads - 1) / threads), c->sm_count * 8));
-    if (n_slots > 1 && n_slots <= MAX_SCRATCH) {
+    if ((n_slots > 1 || copies > 1) && n_slots <= MAX_SCRATCH) {
         FoldSlots F;
         memset(&F, 0, sizeof(F));
         F.n = n_slots;
+        F.copies = copies;
         for (int s = 0; s < n_slots; ++s) {
             if (counts[s] <= 0) continue;
             F.inv_nb[s] = 1.0 / (double)counts[s];
@@ -2744,12 +2783,13 @@ static int ensure_ring(cc_ctx* c) {
 // a ring record, queued on the context's stream without waiting.
 static int enqueue_launch(cc_ctx* c, const cc_scene* scene, const cc_tables* tables, const KSource* src,
                           cc_grid* grid, double* tally_base, int n_slots, long long batch_size, KRun R,
-                          int cell32, cc_ctx::LaunchRec& rec) {
+                          int cell32, cc_ctx::LaunchRec& rec, int copy_shift = 0) {
     const KTables& T = tables->k;
     R.n_scratch = n_slots;
     R.batch_size = batch_size;
     const bool big_grid = grid && (size_t)grid->k.nvox * 16 > SLOT_BYTES_COMPACT;
-    R.chunk = big_grid ? HIST_CHUNK_COMPACT : HIST_CHUNK_SPREAD;
+    R.group = big_grid ? 1 : SPREAD_SLOTS;
+    R.copy_shift = copy_shift;
     R.max_steps = c->max_steps;
     R.status = c->d_status;
     R.counters = c->d_counters;
@@ -3082,7 +3122,9 @@ int cc_run(cc_ctx* c, const cc_scene* scene, const cc_tables* tables, const cc_s
         size_t per = (size_t)grid->k.nvox * 2 * sizeof(double);
         size_t budget = (size_t)8 << 30;
         slots = (int)std::max<size_t>(1, std::min<size_t>(slots, budget / per));
-        int rc = grid_alloc_scratch(grid, slots);
+        // slots of all batches of a launch, and of the copies of a launch of few
+        const bool spread = per <= SLOT_BYTES_COMPACT;
+        int rc = grid_alloc_scratch(grid, spread ? std::max(slots, (int)std::min<size_t>(SPREAD_SLOTS, budget / per)) : slots);
         if (rc != CC_OK) return rc;
     }
     long long done = 0;
@@ -3130,6 +3172,9 @@ int cc_run(cc_ctx* c, const cc_scene* scene, const cc_tables* tables, const cc_s
         int ns = slots;
         long long n_launch = std::min<long long>(n_hist - done, (long long)ns * batch_size);
         ns = (int)((n_launch + batch_size - 1) / batch_size);
+        int copy_shift = 0;
+        if (grid && (size_t)grid->k.nvox * 16 <= SLOT_BYTES_COMPACT)
+            while ((ns << (copy_shift + 1)) <= std::min(+SPREAD_SLOTS, grid->n_scratch)) ++copy_shift;
         KRun R;
         memset(&R, 0, sizeof(R));
         R.n = n_launch;
@@ -3144,7 +3189,7 @@ int cc_run(cc_ctx* c, const cc_scene* scene, const cc_tables* tables, const cc_s
             if (rc != CC_OK) { drain(ri + 1); return rc; }
         }
         rc = enqueue_launch(c, scene, tables, &src->k, grid, tally, slotted ? ns : 1,
-                            slotted ? batch_size : std::max<long long>(n_launch, 1), R, cell32, rec);
+                            slotted ? batch_size : std::max<long long>(n_launch, 1), R, cell32, rec, copy_shift);
         if (rc != CC_OK) { drain(ri + 1); cudaStreamSynchronize(c->stream); return rc; }
         rec.n = n_launch;     // rec.ns: its batches (one slot for all histories without a grid)
         ++li;
@@ -3153,11 +3198,11 @@ int cc_run(cc_ctx* c, const cc_scene* scene, const cc_tables* tables, const cc_s
         if (stats) {
             std::vector<long long> counts(ns);
             for (int b = 0; b < ns; ++b) counts[b] = std::min<long long>(batch_size, n_launch - (long long)b * batch_size);
-            rc = fold_batches(grid, ns, counts.data(), cell32);
+            rc = fold_batches(grid, ns, counts.data(), cell32, 1 << copy_shift);
             if (rc != CC_OK) { drain(ri + 1); return rc; }
             launches += ns > 1 ? 1 : ns;
         } else if (grid) {
-            rc = fold_plain(grid, ns, cell32);
+            rc = fold_plain(grid, ns << copy_shift, cell32);
             if (rc != CC_OK) { drain(ri + 1); return rc; }
             launches += ns > 1 ? 1 : ns;
         }
@@ -3336,6 +3381,7 @@ int cc_transport_photons_device_noalloc(const cc_scene* scene, const cc_tables* 
     R.pos = d_pos; R.dir = d_dir; R.energy = d_en;
     R.n_scatter = d_nsc; R.absorbed = d_abs; R.escaped = d_esc;
     R.n_scratch = 1;
+    R.group = 1;
     R.batch_size = n;
     R.max_steps = tables->ctx->max_steps;
     R.counters = scratch;
@@ -3535,6 +3581,7 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
                 FoldSlots F;
                 memset(&F, 0, sizeof(F));
                 F.n = slots;
+                F.copies = 1;
                 for (int sl = 0; sl < slots; ++sl)
                     if (b->slot_counts[i][sl] > 0) F.inv_nb[sl] = 1.0 / (double)b->slot_counts[i][sl];
                 fold_slots_kernel<<<nb, threads, 0, st>>>((double2*)g->d_total, (double2*)g->d_q, g->d_nhit,
