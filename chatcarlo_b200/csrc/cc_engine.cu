@@ -1934,6 +1934,11 @@ struct cc_grid {
     int* d_nhit = nullptr;
     double* d_scratch = nullptr;    // [n_scratch][nvox] double2; slot 0 is the pending batch
     int n_scratch = 0;
+    // whether a scratch cell may hold a score: set before a launch that scores,
+    // cleared once the folds of all its slots (which zero them) are queued, so
+    // that cc_grid_reset clears the slots (33 of 246 MB on the CT grid, 1.25 ms)
+    // only where something is left in them
+    bool scratch_dirty = false;
     char* d_out = nullptr;          // download staging: kerma, h10, kerma_sum2, h10_sum2 (f64), n_hit (i32)
     double* d_maps = nullptr;       // cc_grid_maps staging: 4 maps (f64), allocated on first use
     double origin64[3] = {0, 0, 0}; // the caller's FP64 origin and voxel edge (the kernels track in FP32)
@@ -2473,8 +2478,9 @@ int cc_grid_reset(cc_grid* g) {
     CC_CUDA(cudaMemsetAsync(g->d_total, 0, b2, st));
     if (g->d_q) CC_CUDA(cudaMemsetAsync(g->d_q, 0, b2, st));
     if (g->d_nhit) CC_CUDA(cudaMemsetAsync(g->d_nhit, 0, (size_t)g->k.nvox * sizeof(int), st));
-    if (g->d_scratch) CC_CUDA(cudaMemsetAsync(g->d_scratch, 0, (size_t)g->n_scratch * b2, st));
+    if (g->d_scratch && g->scratch_dirty) CC_CUDA(cudaMemsetAsync(g->d_scratch, 0, (size_t)g->n_scratch * b2, st));
     CC_CUDA(cudaStreamSynchronize(st));
+    g->scratch_dirty = false;
     g->n_batches = 0;
     g->n_histories = 0;
     return CC_OK;
@@ -2521,7 +2527,8 @@ static int cell32_for(const cc_ctx* c, long long histories_per_slot) {
 #endif
 }
 
-// Scratch slots [0, n_slots) into the totals without batch statistics.
+// Scratch slots [0, n_slots), all that the grid's launches since the last
+// fold scored, into the totals without batch statistics.
 static int fold_plain(cc_grid* g, int n_slots, int cell32) {
     cc_ctx* c = g->ctx;
     int threads = 256;
@@ -2530,6 +2537,7 @@ static int fold_plain(cc_grid* g, int n_slots, int cell32) {
         fold_plain_slots_kernel<<<blocks, threads, 0, c->stream>>>((double2*)g->d_total, (double2*)g->d_scratch,
                                                                    g->k.nvox, n_slots, cell32);
         CC_CUDA(cudaGetLastError());
+        g->scratch_dirty = false;
         return CC_OK;
     }
     for (int s = 0; s < n_slots; ++s) {
@@ -2537,6 +2545,7 @@ static int fold_plain(cc_grid* g, int n_slots, int cell32) {
             (double2*)g->d_total, (double2*)(g->d_scratch + (size_t)s * 2 * g->k.nvox), g->k.nvox, cell32);
         CC_CUDA(cudaGetLastError());
     }
+    g->scratch_dirty = false;
     return CC_OK;
 }
 
@@ -2559,6 +2568,7 @@ static int fold_batches(cc_grid* g, int n_slots, const long long* counts, int ce
         fold_slots_kernel<<<blocks, threads, 0, c->stream>>>((double2*)g->d_total, (double2*)g->d_q, g->d_nhit,
                                                              (double2*)g->d_scratch, g->k.nvox, F, cell32);
         CC_CUDA(cudaGetLastError());
+        g->scratch_dirty = false;
         return CC_OK;
     }
     for (int s = 0; s < n_slots; ++s) {
@@ -2570,6 +2580,7 @@ static int fold_batches(cc_grid* g, int n_slots, const long long* counts, int ce
         g->n_batches += 1;
         g->n_histories += counts[s];
     }
+    g->scratch_dirty = false;
     return CC_OK;
 }
 
@@ -2591,6 +2602,7 @@ int cc_grid_upload(cc_grid* g, const double* kerma, const double* h10, const dou
         CC_CUDA(cudaMemcpy(g->d_nhit, nhit, (size_t)nv * sizeof(int), cudaMemcpyHostToDevice));
     }
     if (g->d_scratch) CC_CUDA(cudaMemset(g->d_scratch, 0, (size_t)g->n_scratch * nv * 2 * sizeof(double)));
+    g->scratch_dirty = false;
     g->n_batches = n_batches;
     g->n_histories = n_histories;
     return CC_OK;
@@ -2831,6 +2843,7 @@ static int enqueue_launch(cc_ctx* c, const cc_scene* scene, const cc_tables* tab
         R.seg_cap = c->seg_alloc;
     }
     CC_CUDA(cudaEventRecord(rec.k0, st));
+    if (grid) grid->scratch_dirty = true;
     cudaError_t e;
     const bool heel = fs && S.heel_n > 0;
     if (fs && tl && heel) e = launch_transport<true, true, true>(c, T, scene->k, G, S, R, smem, blocks);
