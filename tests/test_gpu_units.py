@@ -34,3 +34,35 @@ def test_totals_do_not_depend_on_the_batches(n, batches):
         assert g.n_batches_hit.max() <= nb and np.array_equal(g.n_batches_hit > 0, g.kerma_keV > 0)
         if nb == 1:
             np.testing.assert_allclose(g.kerma_sum2, g.kerma_keV ** 2 / n, rtol=1e-14, atol=0)
+
+
+def test_reset_clears_what_the_last_run_left():
+    """Runs on one engine grid: batches folded away leave nothing to clear, a
+    pending batch (photons scored without a fold) is cleared by the reset."""
+    from chatcarlo_b200 import _native as N
+    from chatcarlo_b200 import workloads as W
+    from chatcarlo_b200.geometry import Geometry
+    from chatcarlo_b200.transport import DeviceGrid, default_engine, run_transport
+    eng = default_engine()
+    raw, spec = W.plain_mc(), W.PLAIN_MC_GRID
+    ref = run_transport(raw, n_histories=5_000, seed=3, dose_grid=True, grid=W.make_grid(spec)).grid
+    host = W.make_grid(spec)
+    geo = Geometry(raw["geometry"])
+    ts, th = eng.tables(geo.materials(), need_muen=True)
+    sh = eng.scene(geo, ts)
+    dg = DeviceGrid(eng, host, stats=True)
+    try:
+        pos, d, e = W.pencil_beam_arrays(1_000, [0.0, 0.0, -20.0], [0.0, 0.0, 1.0], 60.0)
+        edep = np.zeros(len(ts.names))
+        N.check(eng.lib.cc_transport_photons(eng.ctx, sh, th, dg.handle, 1_000, N.dptr(pos), N.dptr(d), N.dptr(e), 1, 0,
+                                             1, None, None, None, N.dptr(edep), None))
+        dg.download(host)
+        assert host.kerma_keV.sum() > 0                # pending
+        dg.reset()
+        dg.download(host)
+        assert host.kerma_keV.max() == 0.0
+    finally:
+        dg.close()
+        eng.lib.cc_scene_destroy(sh)
+    again = run_transport(raw, n_histories=5_000, seed=3, dose_grid=True, grid=W.make_grid(spec)).grid
+    np.testing.assert_allclose(again.kerma_keV, ref.kerma_keV, rtol=2.0 ** -36, atol=0)
