@@ -935,6 +935,63 @@ __device__ __forceinline__ void score_warp_segments(const KGrid& G, const SegRec
     __syncwarp();
 }
 
+// The inline tally's segments of one warp: a ring of records, each with the
+// number of the warp's first piece of it.  Pieces are walked 32 at a time, one
+// per lane, in the order of their numbers; fewer than 32 wait for the next
+// step's, so that every round but the last of the launch has a piece for
+// every lane (a room step has about 40: scored step by step, its second round
+// had 8).  At most 31 pieces wait, of at most 31 segments and the one whose
+// last piece was just walked, so SEG_RING holds a step's 32 beside them.
+constexpr int SEG_RING = 64;
+
+template <typename REC>
+struct SegQueue {
+    REC* seg;                       // [SEG_RING]
+    unsigned* start;                // [SEG_RING] piece number of a record's first piece
+    unsigned head = 0, tail = 0;    // next piece to walk, pieces so far
+    unsigned s_head = 0, s_tail = 0;     // oldest record in use, records so far
+
+    // The record for this lane's segment of m pieces; called by all lanes
+    // (m = 0: none).
+    __device__ __forceinline__ REC* push(int lane, int m) {
+        const unsigned have = __ballot_sync(FULL, m > 0);
+        const int incl = warp_inclusive_scan(m, lane);
+        REC* r = nullptr;
+        if (m > 0) {
+            const unsigned i = (s_tail + __popc(have & ((1u << lane) - 1u))) % SEG_RING;
+            start[i] = tail + (unsigned)(incl - m);
+            r = seg + i;
+        }
+        s_tail += __popc(have);
+        tail += (unsigned)__shfl_sync(FULL, incl, 31);
+        return r;
+    }
+
+    // walk(record, k): piece k of a record; every full round, and with
+    // `flush` the rest.
+    template <typename WALK>
+    __device__ __forceinline__ void rounds(int lane, bool flush, WALK walk) {
+        __syncwarp();
+        while (tail - head >= 32u || (flush && tail != head)) {
+            const unsigned n = min(32u, tail - head);
+            unsigned i = 0;
+            if ((unsigned)lane < n) {
+                const unsigned u = head + (unsigned)lane;
+                unsigned hi = s_tail - s_head;       // start[s_head + i] <= u < start[s_head + hi]
+                while (hi - i > 1) {
+                    const unsigned mid = (i + hi) >> 1;
+                    if ((int)(u - start[(s_head + mid) % SEG_RING]) >= 0) i = mid; else hi = mid;
+                }
+                i += s_head;
+                walk(seg[i % SEG_RING], (int)(u - start[i % SEG_RING]));
+            }
+            head += n;
+            s_head = __shfl_sync(FULL, i, (int)n - 1);
+        }
+        __syncwarp();
+    }
+};
+
 // Deferred tally (a context option, off by default): the transport kernel
 // appends its in-grid segments to a queue in HBM, and tally_kernel scores
 // them with full warps at its own occupancy.  Scores are the same pieces as
@@ -986,8 +1043,9 @@ __global__ void __launch_bounds__(BLOCK, CC_MIN_BLOCKS)
 transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource SRC, const KRun R) {
     extern __shared__ double s_edep[];             // [n_scratch][n_mat]
     __shared__ unsigned long long s_cnt[6];
-    __shared__ SegRec s_seg[TALLY ? WARPS_PER_BLOCK : 1][32];
-    __shared__ int s_pre[TALLY ? WARPS_PER_BLOCK : 1][33];
+    constexpr bool INLINE = TALLY && TV != TV_DEFER;
+    __shared__ SegRec s_seg[INLINE ? WARPS_PER_BLOCK : 1][INLINE ? SEG_RING : 1];
+    __shared__ unsigned s_start[INLINE ? WARPS_PER_BLOCK : 1][INLINE ? SEG_RING : 1];
     const int n_acc = R.n_scratch * T.n_mat;
     for (int i = threadIdx.x; i < n_acc; i += blockDim.x) s_edep[i] = 0.0;
     if (threadIdx.x < 6) s_cnt[threadIdx.x] = 0ull;
@@ -1002,6 +1060,14 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
     // warp-local pool [pool_next, pool_end), histories of one unit, and its scratch slot
     long long pool_next = 0, pool_end = 0;
     int pool_slot = 0;
+    SegQueue<SegRec> Q{s_seg[INLINE ? warp : 0], s_start[INLINE ? warp : 0]};
+    auto score_piece = [&](const SegRec& q, int k) {
+        real ta, tz;
+        piece_range(q.t0, q.t1, q.m, k, ta, tz);
+        const int nv = walk_range<TV == TV_DEFER ? CELL_RUNTIME : TV>(G, G.tally + (size_t)q.slot * 2 * G.nvox, q.p, q.d, ta,
+                                                                      tz, q.wk, q.wh);
+        c_vox += max(nv - (k > 0 ? 1 : 0), 0);   // a cut voxel is one visit
+    };
     bool live = false;
     long long h = 0;
     real p[3], d[3];
@@ -1117,16 +1183,13 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
                 }
             }
         } else if (TALLY) {
-            if (__any_sync(FULL, tal_n > 0)) {
-                int m = (tal_n + TALLY_PIECE - 1) / TALLY_PIECE;
-                if (m > 0) {
-                    SegRec& r = s_seg[warp][lane];
-                    r.p[0] = p[0]; r.p[1] = p[1]; r.p[2] = p[2];
-                    r.d[0] = d[0]; r.d[1] = d[1]; r.d[2] = d[2];
-                    r.t0 = t0; r.t1 = t1; r.wk = wk; r.wh = wh; r.slot = slot; r.m = m;
-                }
-                score_warp_segments<TV == TV_DEFER ? CELL_RUNTIME : TV>(G, s_seg[warp], s_pre[warp], lane, m, c_vox);
+            const int m = (tal_n + TALLY_PIECE - 1) / TALLY_PIECE;
+            if (SegRec* r = Q.push(lane, m)) {
+                r->p[0] = p[0]; r->p[1] = p[1]; r->p[2] = p[2];
+                r->d[0] = d[0]; r->d[1] = d[1]; r->d[2] = d[2];
+                r->t0 = t0; r->t1 = t1; r->wk = wk; r->wh = wh; r->slot = slot; r->m = m;
             }
+            Q.rounds(lane, false, score_piece);
         }
         if (TALLY && c_vox >= COUNTER_FLUSH) {
             atomicAdd(&s_cnt[5], (unsigned long long)c_vox);
@@ -1219,6 +1282,7 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
             live = false;
         }
     }
+    if (INLINE) Q.rounds(lane, true, score_piece);
     // ---- reductions ----
     atomicAdd(&s_cnt[0], (unsigned long long)c_abs);
     atomicAdd(&s_cnt[1], (unsigned long long)c_esc);
