@@ -185,6 +185,7 @@ struct KRun {
     int n_scratch;
     int group;                // batches whose units alternate (see HIST_UNIT)
     int copy_shift;           // log2 of the scratch copies of a batch's slot
+    int lockstep;             // the block's warps step together (LOCKSTEP_PER_LANE)
     int fluorescence;
     unsigned long long seed;
     long long max_steps;
@@ -951,6 +952,16 @@ struct SegQueue {
     unsigned head = 0, tail = 0;    // next piece to walk, pieces so far
     unsigned s_head = 0, s_tail = 0;     // oldest record in use, records so far
 
+    // shared memory of a block of this many threads, and warp w's ring in it
+    static __host__ __device__ size_t bytes(int threads) {
+        return (size_t)(threads / 32) * SEG_RING * (sizeof(REC) + sizeof(unsigned));
+    }
+    __device__ __forceinline__ SegQueue(void* mem, int w) {
+        char* m = static_cast<char*>(mem) + (size_t)w * SEG_RING * (sizeof(REC) + sizeof(unsigned));
+        seg = reinterpret_cast<REC*>(m);
+        start = reinterpret_cast<unsigned*>(m + SEG_RING * sizeof(REC));
+    }
+
     // The record for this lane's segment of m pieces; called by all lanes
     // (m = 0: none).
     __device__ __forceinline__ REC* push(int lane, int m) {
@@ -1008,6 +1019,15 @@ struct SegQueue {
 //      lanes walk the pieces round-robin, so every lane walks about the same
 //      number of voxels;
 //   3. lanes move their photon and sample the interaction, if any.
+// Instruction fetch is the kernel's top stall (4.8 of 15.5 cycles per issue):
+// its loop is far larger than the innermost instruction cache, and 32 warps
+// roam it at will.  With R.lockstep the eight warps of a block meet before
+// phases 1b and 3, so that they fetch the same code (room workload, 4e6
+// histories: 5.83 -> 5.42 ms; blocks of 512: 5.65).  A launch with few
+// histories per lane loses more waiting than it gains (1e5: 0.39 -> 0.43), as
+// do launches without a tally (shorter code; 1e6 photons 0.93 -> 1.04) and
+// with one block per SM (CT 5.83 -> 5.97); they run free.
+constexpr int LOCKSTEP_PER_LANE = 4;
 // Four 256-thread blocks per SM: the register budget (<= 64) that this asks
 // for costs no spills and hides more latency than two or three blocks.
 #ifndef CC_MIN_BLOCKS
@@ -1041,11 +1061,9 @@ __device__ __forceinline__ void take_unit(const KRun& R, long long& first, long 
 template <bool FROM_SOURCE, bool TALLY, bool HEEL = false, int TV = CELL_FP64>
 __global__ void __launch_bounds__(BLOCK, CC_MIN_BLOCKS)
 transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource SRC, const KRun R) {
-    extern __shared__ double s_edep[];             // [n_scratch][n_mat]
+    extern __shared__ double s_edep[];             // [n_scratch][n_mat], then the warps' segment rings
     __shared__ unsigned long long s_cnt[6];
     constexpr bool INLINE = TALLY && TV != TV_DEFER;
-    __shared__ SegRec s_seg[INLINE ? WARPS_PER_BLOCK : 1][INLINE ? SEG_RING : 1];
-    __shared__ unsigned s_start[INLINE ? WARPS_PER_BLOCK : 1][INLINE ? SEG_RING : 1];
     const int n_acc = R.n_scratch * T.n_mat;
     for (int i = threadIdx.x; i < n_acc; i += blockDim.x) s_edep[i] = 0.0;
     if (threadIdx.x < 6) s_cnt[threadIdx.x] = 0ull;
@@ -1060,7 +1078,7 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
     // warp-local pool [pool_next, pool_end), histories of one unit, and its scratch slot
     long long pool_next = 0, pool_end = 0;
     int pool_slot = 0;
-    SegQueue<SegRec> Q{s_seg[INLINE ? warp : 0], s_start[INLINE ? warp : 0]};
+    SegQueue<SegRec> Q(s_edep + n_acc, warp);
     auto score_piece = [&](const SegRec& q, int k) {
         real ta, tz;
         piece_range(q.t0, q.t1, q.m, k, ta, tz);
@@ -1113,7 +1131,11 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
             pool_next += take;
             need = __ballot_sync(FULL, !live);
         }
-        if (__all_sync(FULL, !live)) break;
+        if (INLINE && R.lockstep) {
+            if (!__syncthreads_or(live)) break;
+        } else if (__all_sync(FULL, !live)) {
+            break;
+        }
 
         // ---- phase 1b: material, mu, next boundary ----
         bool go = live;
@@ -1195,6 +1217,7 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
             atomicAdd(&s_cnt[5], (unsigned long long)c_vox);
             c_vox = 0;
         }
+        if (INLINE && R.lockstep) __syncthreads();
         if (!go) continue;
 
         // ---- phase 3: move, cross or interact ----
@@ -1394,11 +1417,15 @@ __device__ __forceinline__ void add_scene_counts(const KBatch& B, bool ended, in
     }
 }
 
+// Three blocks per SM: with 64 registers (four blocks) this kernel, which also
+// reads its scene through pointers, spills 164 bytes; 24 scenes of 3.2e6
+// histories: 5.14 ms with four, 4.96 with three.
+constexpr int BATCH_MIN_BLOCKS = CC_MIN_BLOCKS < 3 ? CC_MIN_BLOCKS : 3;
+
 template <bool TALLY, bool HEEL = false>
-__global__ void __launch_bounds__(BLOCK, CC_MIN_BLOCKS)
+__global__ void __launch_bounds__(BLOCK, BATCH_MIN_BLOCKS)
 batch_kernel(const KTables T, const KBatch B, const KRun R) {
-    __shared__ SegRecB s_seg[TALLY ? WARPS_PER_BLOCK : 1][32];
-    __shared__ int s_pre[TALLY ? WARPS_PER_BLOCK : 1][33];
+    extern __shared__ double s_rings[];            // the warps' segment rings
     __shared__ unsigned long long s_cnt[2];
     if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
     __syncthreads();
@@ -1407,6 +1434,14 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
     const unsigned long long seed = __ldg(B.run);
     const int fluorescence = (int)__ldg(B.run + 1);
     unsigned c_steps = 0, c_vox = 0;            // 32-bit, handed on before they near 2^31
+    SegQueue<SegRecB> Q(s_rings, warp);
+    auto score_piece = [&](const SegRecB& q, int k) {
+        real ta, tz;
+        piece_range(q.t0, q.t1, q.m, k, ta, tz);
+        const KGrid& G = B.grids[q.scene];
+        const int nv = walk_range(G, G.tally + (size_t)q.slot * 2 * G.nvox, q.p, q.d, ta, tz, q.wk, q.wh);
+        c_vox += max(nv - (k > 0 ? 1 : 0), 0);   // a cut voxel is one visit
+    };
 
     long long pool_next = 0, pool_end = 0;
     int pool_scene = 0;
@@ -1452,7 +1487,11 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
             pool_next += take;
             need = __ballot_sync(FULL, !live);
         }
-        if (__all_sync(FULL, !live)) break;
+        if (TALLY && R.lockstep) {
+            if (!__syncthreads_or(live)) break;
+        } else if (__all_sync(FULL, !live)) {
+            break;
+        }
 
         // ---- phase 1 ----
         const KScene& S = B.scenes[sc];
@@ -1498,41 +1537,20 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
 
         // ---- phase 2: the warp scores its segments together ----
         if (TALLY) {
-            if (__any_sync(FULL, tal_n > 0)) {
-                int m = (tal_n + TALLY_PIECE - 1) / TALLY_PIECE;
-                if (m > 0) {
-                    SegRecB& r = s_seg[warp][lane];
-                    r.p[0] = p[0]; r.p[1] = p[1]; r.p[2] = p[2];
-                    r.d[0] = d[0]; r.d[1] = d[1]; r.d[2] = d[2];
-                    r.t0 = t0; r.t1 = t1; r.wk = wk; r.wh = wh; r.scene = sc; r.slot = slot; r.m = m;
-                }
-                int incl = warp_inclusive_scan(m, lane);
-                s_pre[warp][lane] = incl - m;
-                if (lane == 31) s_pre[warp][32] = incl;
-                __syncwarp();
-                const int U = s_pre[warp][32];
-                for (int u = lane; u < U; u += 32) {
-                    int lo = 0, hi = 32;
-                    while (hi - lo > 1) {
-                        int mid = (lo + hi) >> 1;
-                        if (s_pre[warp][mid] <= u) lo = mid; else hi = mid;
-                    }
-                    const SegRecB& q = s_seg[warp][lo];
-                    int k = u - s_pre[warp][lo];
-                    real dt = (q.t1 - q.t0) / (real)q.m;
-                    real ta = q.t0 + dt * (real)k;
-                    real tz = (k == q.m - 1) ? q.t1 : ta + dt;
-                    const KGrid& G = B.grids[q.scene];
-                    int nv = walk_range(G, G.tally + (size_t)q.slot * 2 * G.nvox, q.p, q.d, ta, tz, q.wk, q.wh);
-                    c_vox += max(nv - (k > 0 ? 1 : 0), 0);   // a cut voxel is one visit
-                }
-                __syncwarp();
-                if (c_vox >= COUNTER_FLUSH) {
-                    atomicAdd(&s_cnt[1], (unsigned long long)c_vox);
-                    c_vox = 0;
-                }
+            const int m = (tal_n + TALLY_PIECE - 1) / TALLY_PIECE;
+            if (SegRecB* r = Q.push(lane, m)) {
+                r->p[0] = p[0]; r->p[1] = p[1]; r->p[2] = p[2];
+                r->d[0] = d[0]; r->d[1] = d[1]; r->d[2] = d[2];
+                r->t0 = t0; r->t1 = t1; r->wk = wk; r->wh = wh; r->scene = sc; r->slot = slot; r->m = m;
+            }
+            Q.rounds(lane, false, score_piece);
+            if (c_vox >= COUNTER_FLUSH) {
+                atomicAdd(&s_cnt[1], (unsigned long long)c_vox);
+                c_vox = 0;
             }
         }
+
+        if (TALLY && R.lockstep) __syncthreads();
 
         // ---- phase 3 ----
         bool ended = false, esc = false, absd = false;
@@ -1598,6 +1616,7 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
             }
         }
     }
+    if (TALLY) Q.rounds(lane, true, score_piece);
     atomicAdd(&s_cnt[0], (unsigned long long)c_steps);
     atomicAdd(&s_cnt[1], (unsigned long long)c_vox);
     __syncthreads();
@@ -2023,20 +2042,31 @@ static int dev_upload(std::vector<void*>& allocs, const std::vector<T>& v, const
     return CC_OK;
 }
 
+// Shared memory beyond 48 KB has to be asked for (the FP64 build's records).
+template <typename K>
+static cudaError_t allow_smem(K kernel, size_t smem) {
+    if (smem <= (size_t)48 << 10) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
+template <bool FS, bool TL, bool HEEL, int TV>
+static cudaError_t launch_variant(cc_ctx* c, const KTables& T, const KScene& S, const KGrid& G, const KSource& SRC,
+                                  const KRun& R, size_t smem, int grid_blocks) {
+    const auto kernel = transport_kernel<FS, TL, HEEL, TV>;
+    const cudaError_t e = allow_smem(kernel, smem);
+    if (e != cudaSuccess) return e;
+    kernel<<<grid_blocks, c->block, smem, c->stream>>>(T, S, G, SRC, R);
+    return cudaGetLastError();
+}
+
 template <bool FS, bool TL, bool HEEL = false>
 static cudaError_t launch_transport(cc_ctx* c, const KTables& T, const KScene& S, const KGrid& G,
                                     const KSource& SRC, const KRun& R, size_t smem, int grid_blocks) {
     if constexpr (TL) {
-        if (R.defer)
-            transport_kernel<FS, TL, HEEL, TV_DEFER><<<grid_blocks, c->block, smem, c->stream>>>(T, S, G, SRC, R);
-        else if (G.tally32)
-            transport_kernel<FS, TL, HEEL, CELL_FP32><<<grid_blocks, c->block, smem, c->stream>>>(T, S, G, SRC, R);
-        else
-            transport_kernel<FS, TL, HEEL, CELL_FP64><<<grid_blocks, c->block, smem, c->stream>>>(T, S, G, SRC, R);
-    } else {
-        transport_kernel<FS, TL, HEEL><<<grid_blocks, c->block, smem, c->stream>>>(T, S, G, SRC, R);
+        if (R.defer) return launch_variant<FS, TL, HEEL, TV_DEFER>(c, T, S, G, SRC, R, smem, grid_blocks);
+        if (G.tally32) return launch_variant<FS, TL, HEEL, CELL_FP32>(c, T, S, G, SRC, R, smem, grid_blocks);
     }
-    return cudaGetLastError();
+    return launch_variant<FS, TL, HEEL, CELL_FP64>(c, T, S, G, SRC, R, smem, grid_blocks);
 }
 
 extern "C" {
@@ -2823,7 +2853,11 @@ static int grid_blocks_for(cc_ctx* c, size_t smem, bool fs, bool tl, bool big_gr
     if (per_sm == 0) {
         int occ = 0;
         cudaError_t e;
-        if (fs && tl) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<true, true>, c->block, smem);
+        // (beyond 48 KB the occupancy of a kernel that has not asked for it is an error)
+        e = fs ? (tl ? allow_smem(transport_kernel<true, true>, smem) : cudaSuccess)
+               : (tl ? allow_smem(transport_kernel<false, true>, smem) : cudaSuccess);
+        if (e != cudaSuccess) occ = 0;
+        else if (fs && tl) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<true, true>, c->block, smem);
         else if (fs) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<true, false>, c->block, smem);
         else if (tl) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<false, true>, c->block, smem);
         else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<false, false>, c->block, smem);
@@ -2885,8 +2919,9 @@ static int enqueue_launch(cc_ctx* c, const cc_scene* scene, const cc_tables* tab
     memset(&S, 0, sizeof(S));
     bool fs = src != nullptr;
     if (fs) S = *src;
-    size_t smem = n_acc * sizeof(double);
+    size_t smem = n_acc * sizeof(double) + (tl && !c->tally_queue ? SegQueue<SegRec>::bytes(c->block) : 0);
     int blocks = grid_blocks_for(c, smem, fs, tl, big_grid);
+    R.lockstep = tl && !big_grid && R.n >= (long long)LOCKSTEP_PER_LANE * blocks * c->block ? 1 : 0;
     const bool defer = tl && c->tally_queue;
     R.defer = defer ? 1 : 0;
     if (defer) {
@@ -3625,23 +3660,33 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
     R.status = b->d_status;
     R.counters = b->d_counters;
     R.work = b->d_counters + 6;
+    const size_t smem = b->tally ? SegQueue<SegRecB>::bytes(c->block) : 0;
+    if (b->tally) {
+        e = heel ? allow_smem(batch_kernel<true, true>, smem) : allow_smem(batch_kernel<true>, smem);
+        if (e != cudaSuccess) { batch_free(b); return set_error(CC_E_DEVICE, std::string("batch launch: ") + cudaGetErrorString(e)); }
+    }
     // launch shape: the context's block size and blocks per SM (the autotuner sets them)
     int per_sm = c->blocks_per_sm;
     if (per_sm == 0) {
         int occ = 0;
-        cudaError_t oe = b->tally ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<true>, c->block, 0)
+        cudaError_t oe = b->tally ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<true>, c->block, smem)
                                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<false>, c->block, 0);
         per_sm = (oe == cudaSuccess && occ > 0) ? occ : 1;
     }
     b->blocks = c->sm_count * per_sm;
+    {
+        long long all = 0;
+        for (long long n : b->nhist) all += n;
+        R.lockstep = b->tally && all >= (long long)LOCKSTEP_PER_LANE * b->blocks * c->block ? 1 : 0;
+    }
     // capture: clear the counters, take the seed, transport, fold the batches
     e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->d_mem + o_cnt, 0, sizeof(unsigned long long) * 4 * n_scenes, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->d_mem + o_c8, 0, total - o_c8, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_mem + o_run, b->h_run, 2 * sizeof(unsigned long long), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
-        if (b->tally && heel) batch_kernel<true, true><<<b->blocks, c->block, 0, st>>>(tables->k, k, R);
-        else if (b->tally) batch_kernel<true><<<b->blocks, c->block, 0, st>>>(tables->k, k, R);
+        if (b->tally && heel) batch_kernel<true, true><<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
+        else if (b->tally) batch_kernel<true><<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
         else if (heel) batch_kernel<false, true><<<b->blocks, c->block, 0, st>>>(tables->k, k, R);
         else batch_kernel<false><<<b->blocks, c->block, 0, st>>>(tables->k, k, R);
         e = cudaGetLastError();
