@@ -697,12 +697,14 @@ __device__ __forceinline__ int walk_range(const KGrid& G, double* tally, const r
     walk_axis(G.o[1], G.h, G.inv_h, G.ny, p[1], d[1], t0, iy, sy, my, dy);
     walk_axis(G.o[2], G.h, G.inv_h, G.nz, p[2], d[2], t0, iz, sz, mz, dz);
     real t = t0;
-    int guard = G.nx + G.ny + G.nz + 4;
     int visits = 0;
+    // face crossings left before the ray leaves the grid along each axis
+    int rx = sx > 0 ? G.nx - 1 - ix : ix, ry = sy > 0 ? G.ny - 1 - iy : iy, rz = sz > 0 ? G.nz - 1 - iz : iz;
     // flat index (C order, tally.py:292) updated incrementally; grids are < 2^31 voxels
     const int vx = sx * G.ny * G.nz, vy = sy * G.nz, vz = sz;
     int v = (ix * G.ny + iy) * G.nz + iz;
-    while (t < t1 && guard-- > 0) {
+    while (t < t1) {                 // every turn but the last uses up a crossing
+
         // the axis whose face comes first; ties go to the later axis, except
         // that x beats z only when strictly first
         const bool ax0 = (mx < my) && (mx < mz);
@@ -716,10 +718,10 @@ __device__ __forceinline__ int walk_range(const KGrid& G, double* tally, const r
         }
         t = tn;
         if (t >= t1) break;
-        ix += ax0 ? sx : 0;
-        iy += ax1 ? sy : 0;
-        iz += ax2 ? sz : 0;
-        if ((unsigned)ix >= (unsigned)G.nx || (unsigned)iy >= (unsigned)G.ny || (unsigned)iz >= (unsigned)G.nz) break;
+        rx -= ax0;
+        ry -= ax1;
+        rz -= ax2;
+        if ((ax0 ? rx : (ax1 ? ry : rz)) < 0) break;
         v += ax0 ? vx : (ax1 ? vy : vz);
         if (ax0) mx += dx;
         if (ax1) my += dy;
