@@ -92,3 +92,17 @@ def test_convolution_output_slices(U, cin, cout, split, dims, masked):
         ref[:, :split] *= mask > 0
     got = torch.cat([out0, out1], 1)[:, :cout].double() if split < cout else out0.double()
     assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + (27 * cin + 4) * 2.0 ** -23 * mag).all())
+
+
+@pytest.mark.parametrize("c,n,offset", [(1, 1000, 0), (4, 77, 0), (8, 1, 0), (16, 4097, 0), (64, 333, 0), (256, 50, 0),
+                                        (16, 4097, 1)])           # offset 1: dz is not 16-byte aligned
+def test_bias_gradient_widths(U, c, n, offset):
+    """Every one of at most n additions errs by at most 2^-24 of the running sum of magnitudes."""
+    g = torch.Generator(device="cuda").manual_seed(c + n)
+    buf = torch.randn(n * c + offset, generator=g, device="cuda").to(torch.bfloat16)
+    dz = buf[offset:].view(n, c)
+    db = torch.ones(c, device="cuda")
+    U.check(U.lib().ccu_bias_grad(dz.data_ptr(), n, c, db.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    ref, mag = 1.0 + dz.double().sum(0), 1.0 + dz.double().abs().sum(0)
+    assert bool(((db.double() - ref).abs() <= (n + 1) * 2.0 ** -24 * mag).all())
