@@ -177,6 +177,25 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
+// Programmatic dependent launch: a kernel launched by launch_dependent may
+// start once the blocks of the kernel before it on the stream have ended,
+// before that kernel's writes are visible and its completion is known.  It must
+// call this before it touches global memory: the wait returns when they are.
+// Its launch, barriers and tensor-memory allocation overlap the end of the
+// kernel before (gradient of a 4 x 64^3 minibatch, some 110 kernels: 1.29 ->
+// 1.13 ms).  No kernel lets the next one start earlier (launch_dependents): the
+// waiting blocks took the places of the last ones' neighbours, and 16 -> 16
+// channels on 320x320x152 went from 280 to 320 us.
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A pointer whose loads the compiler cannot move above the wait (reads of
+// constant data, __ldg or const __restrict__, are otherwise free to).
+template <typename T>
+__device__ __forceinline__ T* behind_wait(T* p) {
+    asm volatile("" : "+l"(p));
+    return p;
+}
+
 __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
@@ -1273,7 +1292,10 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         s_fail = 0;
         mbar_init_fence();
     }
+    wait_for_previous_kernel();
     // weights: packed chunk (tap * c8n + c8, co_lo + co) -> (t9 * c8p + c8 - c8_lo, dz * NO + co)
+    // (all threads: as 16-byte copies; 256- and 512-byte bulk copies, issued one by one, took 8 us longer
+    // for 128 input channels)
     const uint32_t sbase = (smem_u32(smem) + 255u) & ~255u, swt = sbase + R * slot16 * 16;
     for (int i = tid; i < 9 * c8p * NP; i += PS_THREADS) {
         const int r = i % NP, g = i / NP;
@@ -1468,18 +1490,21 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         // of latency however few channels it has; what it reads beside the
         // sums (mask, partial sum) is therefore read a plane ahead: read in
         // the same plane it cost another 400.
+        const float *bias_p = behind_wait(P.bias), *head_p = behind_wait(P.head), *head_x = behind_wait(P.head_x);
+        const __nv_bfloat16* mask0 = behind_wait(P.mask0);
+        const float* part_rd = behind_wait(part_in);
         constexpr int CW = NO / 2;                             // channels per warp
         const int qw = warp & 3, grp = (warp - PS_EPI_WARP0) >> 2, m = qw * 32 + lane;
         const uint32_t lq = (uint32_t)(qw * 32) << 16;
-        const bool heads = !PLAIN && NO == 16 && P.head != nullptr;
-        const bool masked = !PLAIN && P.mask0 && !part_out && !heads;
+        const bool heads = !PLAIN && NO == 16 && head_p != nullptr;
+        const bool masked = !PLAIN && mask0 && !part_out && !heads;
         const int c0 = grp * CW, co0 = co_lo + c0;
         const uint32_t plane = (uint32_t)(S.H * S.W);
         float2 bias[CW / 2];
-        if (P.bias && (PLAIN || !part_out)) {
+        if (bias_p && (PLAIN || !part_out)) {
 #pragma unroll
             for (int j = 0; j < CW / 2; ++j)
-                bias[j] = make_float2(__ldg(P.bias + co0 + 2 * j), __ldg(P.bias + co0 + 2 * j + 1));
+                bias[j] = make_float2(__ldg(bias_p + co0 + 2 * j), __ldg(bias_p + co0 + 2 * j + 1));
         }
         // regions of planes z - 1, z and z + 1 and the phase of the last
         uint32_t rm = 0, r0 = 1, r1 = 2, ph1 = 0;
@@ -1496,12 +1521,12 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
 #pragma unroll
                     for (int h = 0; h < CW / 8; ++h)
                         if (co0 + 8 * h < P.split)
-                            mk[h] = __ldg(reinterpret_cast<const uint4*>(P.mask0 + (size_t)u * P.split + co0 + 8 * h));
+                            mk[h] = __ldg(reinterpret_cast<const uint4*>(mask0 + (size_t)u * P.split + co0 + 8 * h));
                 }
-                if (part_in) {
+                if (part_rd) {
 #pragma unroll
                     for (int h = 0; h < CW / 4; ++h)
-                        part[h] = __ldg(reinterpret_cast<const float4*>(part_in + (size_t)u * NO + c0) + h);
+                        part[h] = __ldg(reinterpret_cast<const float4*>(part_rd + (size_t)u * NO + c0) + h);
                 }
             };
             if (!PLAIN && in) read_ahead(v);
@@ -1535,7 +1560,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                         ps_release(rfree, rm, r0, r1, z == q.ze - 1);
                     } else {
                         // x + b, then + w_j a_j in channel order (the head kernel's FP32 sequence)
-                        float hsum = in ? P.head_x[v] + __ldg(P.head + 16) : 0.0f;
+                        float hsum = in ? head_x[v] + __ldg(head_p + 16) : 0.0f;
 #pragma unroll
                         for (int c = 0; c < NO; c += 8) {
                             float2 f[4];
@@ -1546,9 +1571,9 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                                 for (int j = 0; j < 4; ++j) t[2 * j] = f[j].x, t[2 * j + 1] = f[j].y;
 #pragma unroll
                                 for (int j = 0; j < 8; ++j) {
-                                    if (P.bias) t[j] += __ldg(P.bias + c + j);
+                                    if (bias_p) t[j] += __ldg(bias_p + c + j);
                                     if (P.relu) t[j] = fmaxf(t[j], 0.0f);
-                                    hsum = fmaf(__ldg(P.head + c + j), __bfloat162float(__float2bfloat16_rn(t[j])), hsum);
+                                    hsum = fmaf(__ldg(head_p + c + j), __bfloat162float(__float2bfloat16_rn(t[j])), hsum);
                                 }
                                 if (P.out0) *reinterpret_cast<uint4*>(P.out0 + (size_t)v * P.split + c) = pack_bf16x8(t);
                             }
@@ -1559,7 +1584,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                 } else {
                     float2 f[CW / 2];
                     sums(PsInt<CW>{}, c0, true, f);
-                    if (!PLAIN && part_in) {
+                    if (!PLAIN && part_rd) {
 #pragma unroll
                         for (int j = 0; j < CW / 4; ++j) {
                             f[2 * j] = add2(f[2 * j], make_float2(part[j].x, part[j].y));
@@ -1574,7 +1599,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                                 po[j] = make_float4(f[2 * j].x, f[2 * j].y, f[2 * j + 1].x, f[2 * j + 1].y);
                         }
                     } else {
-                        if (P.bias) {
+                        if (bias_p) {
 #pragma unroll
                             for (int j = 0; j < CW / 2; ++j) f[j] = add2(f[j], bias[j]);
                         }
@@ -1845,6 +1870,7 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
         s_fail = 0;
         mbar_init_fence();
     }
+    wait_for_previous_kernel();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1947,6 +1973,8 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
 // (the second input of a concatenated layer, spelled out for the tile loads).
 __global__ void upsample_kernel(const uint4* __restrict__ b, uint4* __restrict__ out, int batch, int d, int h,
                                 int w, int c8) {
+    wait_for_previous_kernel();
+    b = behind_wait(b);
     const long long total = (long long)batch * d * h * w * c8;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
@@ -1996,6 +2024,8 @@ __global__ void bias_grad_narrow_kernel(const __nv_bfloat16* __restrict__ dz, lo
 // channels of 4 x 16^3: 13.4 and 5.4 us.
 __global__ void __launch_bounds__(256) bias_grad_kernel(const uint4* __restrict__ dz, long long n_chunks, int c8,
                                                         float* __restrict__ db) {
+    wait_for_previous_kernel();
+    dz = behind_wait(dz);
     __shared__ float s_acc[256];
     s_acc[threadIdx.x] = 0.0f;
     __syncthreads();
@@ -2027,6 +2057,8 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const uint4* __restrict_
 // y[n, z, y, x, c] = mean of the 2x2x2 children (D, H, W of x even)
 __global__ void avgpool_kernel(const __nv_bfloat16* __restrict__ x, int B, int D, int H, int W, int c,
                                __nv_bfloat16* __restrict__ y) {
+    wait_for_previous_kernel();
+    x = behind_wait(x);
     const int D2 = D >> 1, H2 = H >> 1, W2 = W >> 1;
     const long long total = (long long)B * D2 * H2 * W2 * (c >> 3);
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -2057,6 +2089,10 @@ __global__ void avgpool_kernel(const __nv_bfloat16* __restrict__ x, int B, int D
 // dz_x[v][c] += (x_act[v][c] > 0) * gy[parent(v)][c] / 8   (x at full resolution)
 __global__ void pool_backward_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* __restrict__ x_act,
                                      int B, int D, int H, int W, int c, __nv_bfloat16* __restrict__ dz_x) {
+    wait_for_previous_kernel();
+    gy = behind_wait(gy);
+    x_act = behind_wait(x_act);
+    dz_x = behind_wait(dz_x);
     const long long total = (long long)B * D * H * W * (c >> 3);
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
@@ -2084,6 +2120,9 @@ __global__ void pool_backward_kernel(const __nv_bfloat16* __restrict__ gy, const
 // (g_full at full resolution D, H, W)
 __global__ void up_reduce_kernel(const __nv_bfloat16* __restrict__ g_full, const __nv_bfloat16* __restrict__ coarse,
                                  int B, int D, int H, int W, int c, __nv_bfloat16* __restrict__ dz_c) {
+    wait_for_previous_kernel();
+    g_full = behind_wait(g_full);
+    coarse = behind_wait(coarse);
     const int D2 = D >> 1, H2 = H >> 1, W2 = W >> 1;
     const long long total = (long long)B * D2 * H2 * W2 * (c >> 3);
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -2124,6 +2163,12 @@ __global__ void head_kernel(const __nv_bfloat16* __restrict__ d0, const float* _
                             const float* __restrict__ tgt, const float* __restrict__ wgt,
                             const float* __restrict__ head, float inv_wsum, long long n_vox, float* __restrict__ out,
                             __nv_bfloat16* __restrict__ dz, float* __restrict__ dhead, float* __restrict__ loss) {
+    wait_for_previous_kernel();
+    d0 = behind_wait(d0);
+    xlog = behind_wait(xlog);
+    tgt = behind_wait(tgt);
+    wgt = behind_wait(wgt);
+    head = behind_wait(head);
     __shared__ float s_acc[18];
     if (threadIdx.x < 18) s_acc[threadIdx.x] = 0.0f;
     __syncthreads();
@@ -2370,6 +2415,50 @@ int grid_for(long long work, int threads) {
     return (int)(b < 1 ? 1 : b);
 }
 
+// Launch of a kernel that starts with wait_for_previous_kernel().
+template <typename... A, typename... B>
+int launch_dependent(void (*kernel)(A...), dim3 grid, int threads, size_t smem, cudaStream_t st, B&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CU_CHECK(cudaLaunchKernelEx(&cfg, kernel, std::forward<B>(args)...));
+    return CCU_OK;
+}
+
+// How a kernel is launched on a device, worked out on its first launch
+// there: the shared-memory attributes it needs are then set, and the
+// occupancy queries (a dozen per launch, 6 us) are not repeated.
+struct LaunchPlan {
+    int ring = 0, resident = 1, sms = 0;
+    size_t smem = 0;
+};
+struct PlanCache {
+    std::mutex mu;
+    bool have[64] = {};
+    LaunchPlan plan[64];
+};
+template <typename Make>
+int device_plan(PlanCache* cache, LaunchPlan& out, Make make) {
+    int dev = 0;
+    CU_CHECK(cudaGetDevice(&dev));
+    if (!cache || dev < 0 || dev >= 64) return make(dev, out);
+    std::lock_guard<std::mutex> lk(cache->mu);
+    if (!cache->have[dev]) {
+        const int rc = make(dev, cache->plan[dev]);
+        if (rc != CCU_OK) return rc;
+        cache->have[dev] = true;
+    }
+    out = cache->plan[dev];
+    return CCU_OK;
+}
+
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 // Shared memory per CTA: the pipeline stages, raised where needed so that
@@ -2608,33 +2697,34 @@ int volume_map(CUtensorMap* m, const void* base, int c, int batch, int d, int h,
 
 // One launch: the pass's channel groups and `slices` output slices.
 template <int NO, int G, int C8P, bool PLAIN = false>
-int launch_conv_ps_pass(const CUtensorMap& amap, const ConvP& P, const PsPass& Q, int slices, long long planes, int sms,
+int launch_conv_ps_pass(const CUtensorMap& amap, const ConvP& P, const PsPass& Q, int slices, long long planes,
                         cudaStream_t st) {
     if constexpr (G == 1 && C8P > 0 && !PLAIN) {
         if (!P.mask0 && !P.head && !Q.part_in && !Q.part_out && P.out0 && Q.co_lo + slices * NO <= P.split)
-            return launch_conv_ps_pass<NO, G, C8P, true>(amap, P, Q, slices, planes, sms, st);
+            return launch_conv_ps_pass<NO, G, C8P, true>(amap, P, Q, slices, planes, st);
     }
     const auto kernel = conv_ps_kernel<NO, G, C8P, PLAIN>;
     const int c8p = Q.c8_hi - Q.c8_lo;
-    const uint32_t cols = ps_tmem_cols(NO, G);
-    // deepest ring (group + 1 .. WS_RING_MAX planes) that keeps the CTAs per SM the tensor memory allows
-    int ring = 0, best_res = 0, rc = CCU_OK;
-    size_t smem = 0;
-    for (int r = G + 1; r <= WS_RING_MAX && ps_smem_bytes(NO, c8p, r) <= PS_SMEM_MAX; ++r) {
-        int res = 1;
-        rc = resident_ctas(kernel, (size_t)ps_smem_bytes(NO, c8p, r) + 1024, cols, res, PS_THREADS);
-        if (rc != CCU_OK) return rc;
-        if (res >= best_res) best_res = res, ring = r;
-    }
-    if (ring == 0) return set_error(CCU_E_INVALID, "plane-stationary pass does not fit shared memory");
-    rc = tc_launch_smem(kernel, ps_smem_bytes(NO, c8p, ring), cols, smem, PS_THREADS);
+    static PlanCache cache;                     // one ring depth per kernel where the channel groups are fixed
+    LaunchPlan plan;
+    int rc = device_plan(C8P > 0 ? &cache : nullptr, plan, [&](int dev, LaunchPlan& p) {
+        const uint32_t cols = ps_tmem_cols(NO, G);
+        CU_CHECK(cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev));
+        // deepest ring (group + 1 .. WS_RING_MAX planes) that keeps the CTAs per SM the tensor memory allows
+        int best = 0, r_c = CCU_OK;
+        for (int r = G + 1; r <= WS_RING_MAX && ps_smem_bytes(NO, c8p, r) <= PS_SMEM_MAX; ++r) {
+            int res = 1;
+            r_c = resident_ctas(kernel, (size_t)ps_smem_bytes(NO, c8p, r) + 1024, cols, res, PS_THREADS);
+            if (r_c != CCU_OK) return r_c;
+            if (res >= best) best = res, p.ring = r;
+        }
+        if (p.ring == 0) return set_error(CCU_E_INVALID, "plane-stationary pass does not fit shared memory");
+        r_c = tc_launch_smem(kernel, ps_smem_bytes(NO, c8p, p.ring), cols, p.smem, PS_THREADS);
+        return r_c == CCU_OK ? resident_ctas(kernel, p.smem, cols, p.resident, PS_THREADS) : r_c;
+    });
     if (rc != CCU_OK) return rc;
-    int resident = 1;
-    if ((rc = resident_ctas(kernel, smem, cols, resident, PS_THREADS)) != CCU_OK) return rc;
-    const long long grid = std::min<long long>(planes, std::max(1, sms * resident / slices));
-    kernel<<<dim3((unsigned)grid, (unsigned)slices), PS_THREADS, smem, st>>>(amap, P, Q, ring);
-    CU_CHECK(cudaGetLastError());
-    return CCU_OK;
+    const long long grid = std::min<long long>(planes, std::max(1, plan.sms * plan.resident / slices));
+    return launch_dependent(kernel, dim3((unsigned)grid, (unsigned)slices), PS_THREADS, plan.smem, st, amap, P, Q, plan.ring);
 }
 
 // Output channels [co_lo, co_lo + slices NO) of the layer, in channel passes.
@@ -2643,9 +2733,6 @@ int launch_conv_ps_g(const CUtensorMap& amap, const ConvP& P, int n_out, int co_
                      cudaStream_t st) {
     const int c8n = (P.src.ca + P.src.cb) / 8;
     const int c8p_max = 2 * ((c8n / 2 + passes - 1) / passes);
-    int dev = 0, sms = 0;
-    CU_CHECK(cudaGetDevice(&dev));
-    CU_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const long long planes = (long long)P.src.B * ((P.src.H + 15) / 16) * ((P.src.W + 7) / 8) * P.src.D;
     float* ws = nullptr;
     if (passes > 1) {
@@ -2662,14 +2749,14 @@ int launch_conv_ps_g(const CUtensorMap& amap, const ConvP& P, int n_out, int co_
         Q.part_out = Q.c8_hi < c8n ? ws : nullptr;
         int rc = CCU_OK;
         switch (G == 1 ? Q.c8_hi - Q.c8_lo : 0) {          // 16 to 64, or 128, input channels per pass: unrolled issue
-            case 2: rc = launch_conv_ps_pass<NO, G, G == 1 ? 2 : 0>(amap, P, Q, slices, planes, sms, st); break;
-            case 4: rc = launch_conv_ps_pass<NO, G, G == 1 ? 4 : 0>(amap, P, Q, slices, planes, sms, st); break;
-            case 6: rc = launch_conv_ps_pass<NO, G, G == 1 ? 6 : 0>(amap, P, Q, slices, planes, sms, st); break;
-            case 8: rc = launch_conv_ps_pass<NO, G, G == 1 ? 8 : 0>(amap, P, Q, slices, planes, sms, st); break;
+            case 2: rc = launch_conv_ps_pass<NO, G, G == 1 ? 2 : 0>(amap, P, Q, slices, planes, st); break;
+            case 4: rc = launch_conv_ps_pass<NO, G, G == 1 ? 4 : 0>(amap, P, Q, slices, planes, st); break;
+            case 6: rc = launch_conv_ps_pass<NO, G, G == 1 ? 6 : 0>(amap, P, Q, slices, planes, st); break;
+            case 8: rc = launch_conv_ps_pass<NO, G, G == 1 ? 8 : 0>(amap, P, Q, slices, planes, st); break;
             case 16:
-                rc = launch_conv_ps_pass<NO, G, G == 1 && NO == 16 ? 16 : 0>(amap, P, Q, slices, planes, sms, st);
+                rc = launch_conv_ps_pass<NO, G, G == 1 && NO == 16 ? 16 : 0>(amap, P, Q, slices, planes, st);
                 break;
-            default: rc = launch_conv_ps_pass<NO, G, 0>(amap, P, Q, slices, planes, sms, st); break;
+            default: rc = launch_conv_ps_pass<NO, G, 0>(amap, P, Q, slices, planes, st); break;
         }
         if (rc != CCU_OK) return rc;
     }
@@ -2726,23 +2813,24 @@ int launch_wgrad_halo(const void* x, int cx, int batch, int d, int h, int w, con
     int rc = volume_map(&xmap, x, cx, batch, d, h, w, CI, HALO_X, HALO_Y);
     if (rc == CCU_OK) rc = volume_map(&zmap, dz, cout, batch, d, h, w, CO, 8, 16);
     if (rc != CCU_OK) return rc;
-    int dev = 0, sms = 0;
-    CU_CHECK(cudaGetDevice(&dev));
-    CU_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const auto kernel = wgrad_halo_kernel<CI, CO>;
-    const uint32_t cols = wh_tmem_cols(CO);
-    // deepest ring (a window of three planes and one in flight at least) that keeps
-    // the CTAs per SM the tensor memory allows
-    int ring = 0, best = 0;
-    for (int r = 4; r <= WH_RING_MAX && wh_smem_bytes(CI, CO, r) <= 200 * 1024; ++r) {
-        int res = 1;
-        if ((rc = resident_ctas(kernel, wh_smem_bytes(CI, CO, r) + 1024, cols, res)) != CCU_OK) return rc;
-        if (res >= best) best = res, ring = r;
-    }
-    size_t smem = 0;
-    if ((rc = tc_launch_smem(kernel, wh_smem_bytes(CI, CO, ring), cols, smem)) != CCU_OK) return rc;
-    int resident = 1;
-    if ((rc = resident_ctas(kernel, smem, cols, resident)) != CCU_OK) return rc;
+    static PlanCache cache;
+    LaunchPlan plan;
+    rc = device_plan(&cache, plan, [&](int dev, LaunchPlan& p) {
+        const uint32_t cols = wh_tmem_cols(CO);
+        CU_CHECK(cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev));
+        // deepest ring (a window of three planes and one in flight at least) that keeps
+        // the CTAs per SM the tensor memory allows
+        int best = 0, r_c = CCU_OK;
+        for (int r = 4; r <= WH_RING_MAX && wh_smem_bytes(CI, CO, r) <= 200 * 1024; ++r) {
+            int res = 1;
+            if ((r_c = resident_ctas(kernel, wh_smem_bytes(CI, CO, r) + 1024, cols, res)) != CCU_OK) return r_c;
+            if (res >= best) best = res, p.ring = r;
+        }
+        r_c = tc_launch_smem(kernel, wh_smem_bytes(CI, CO, p.ring), cols, p.smem);
+        return r_c == CCU_OK ? resident_ctas(kernel, p.smem, cols, p.resident) : r_c;
+    });
+    if (rc != CCU_OK) return rc;
     WgradH P;
     P.vol = Src{nullptr, nullptr, 0, 0, batch, d, h, w};
     P.dw = dw;
@@ -2753,12 +2841,10 @@ int launch_wgrad_halo(const void* x, int cx, int batch, int d, int h, int w, con
     // plane ranges per channel-group pair: at least the caller's split (the
     // voxels of one FP32 accumulator), in whole waves of the resident CTAs
     const long long planes = (long long)batch * ((h + 15) / 16) * ((w + 7) / 8) * d;
-    const long long jobs = (long long)P.ci_groups * (cout / CO), room = (long long)sms * resident;
+    const long long jobs = (long long)P.ci_groups * (cout / CO), room = (long long)plan.sms * plan.resident;
     const long long waves = (std::max<long long>(slices, 1) * jobs + room - 1) / room;
     const long long splits = std::max(1LL, std::min(planes, std::max(1LL, waves * room / jobs)));
-    kernel<<<dim3((unsigned)splits, (unsigned)jobs), THREADS, smem, st>>>(xmap, zmap, P, ring);
-    CU_CHECK(cudaGetLastError());
-    return CCU_OK;
+    return launch_dependent(kernel, dim3((unsigned)splits, (unsigned)jobs), THREADS, plan.smem, st, xmap, zmap, P, plan.ring);
 }
 
 int g_wgrad_path = 0;       // 0: tile loads where they apply, 1: the gathering kernel
@@ -2901,9 +2987,9 @@ int ccu_conv3d_wgrad(const void* a, int ca, const void* b, int cb, int batch, in
         const long long n_vox = (long long)batch * d * h * w;
         rc = grow_buffer(g_up_ws, (size_t)n_vox * cb * 2, st, up);
         if (rc != CCU_OK) return rc;
-        upsample_kernel<<<grid_for(n_vox * (cb / 8), 256), 256, 0, st>>>((const uint4*)b, (uint4*)up, batch, d, h, w,
-                                                                        cb / 8);
-        CU_CHECK(cudaGetLastError());
+        rc = launch_dependent(upsample_kernel, dim3((unsigned)grid_for(n_vox * (cb / 8), 256)), 256, 0, st, (const uint4*)b,
+                              (uint4*)up, batch, d, h, w, cb / 8);
+        if (rc != CCU_OK) return rc;
         rc = run(a, ca, 0);
         if (rc != CCU_OK) return rc;
         return run(up, cb, ca);
@@ -2932,7 +3018,8 @@ int ccu_bias_grad(const void* dz, long long n_vox, int c, float* db, void* strea
     if (c % 8 == 0 && aligned16(dz)) {
         const long long chunks = n_vox * (c / 8);
         const int blocks = (int)std::max(1LL, std::min((chunks + 1023) / 1024, 4LL * sm_count()));
-        bias_grad_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const uint4*)dz, chunks, c / 8, db);
+        return launch_dependent(bias_grad_kernel, dim3((unsigned)blocks), 256, 0, (cudaStream_t)stream, (const uint4*)dz, chunks,
+                                c / 8, db);
     } else {
         bias_grad_narrow_kernel<<<grid_for(n_vox * c, 256), 256, c * sizeof(float), (cudaStream_t)stream>>>(
             (const __nv_bfloat16*)dz, n_vox, c, db);
@@ -2944,10 +3031,8 @@ int ccu_bias_grad(const void* dz, long long n_vox, int c, float* db, void* strea
 int ccu_avgpool(const void* x, int batch, int d, int h, int w, int c, void* y, void* stream) {
     if (!x || !y || c % 8 || d % 2 || h % 2 || w % 2) return set_error(CCU_E_INVALID, "bad pooling arguments");
     long long work = (long long)batch * (d / 2) * (h / 2) * (w / 2) * (c / 8);
-    avgpool_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, batch, d, h, w, c,
-                                                                          (__nv_bfloat16*)y);
-    CU_CHECK(cudaGetLastError());
-    return CCU_OK;
+    return launch_dependent(avgpool_kernel, dim3((unsigned)grid_for(work, 256)), 256, 0, (cudaStream_t)stream,
+                            (const __nv_bfloat16*)x, batch, d, h, w, c, (__nv_bfloat16*)y);
 }
 
 int ccu_pool_backward(const void* gy, const void* x_act, int batch, int d, int h, int w, int c, void* dz_x,
@@ -2955,10 +3040,8 @@ int ccu_pool_backward(const void* gy, const void* x_act, int batch, int d, int h
     if (!gy || !x_act || !dz_x || c % 8 || d % 2 || h % 2 || w % 2)
         return set_error(CCU_E_INVALID, "bad pooling arguments");
     long long work = (long long)batch * d * h * w * (c / 8);
-    pool_backward_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)gy, (const __nv_bfloat16*)x_act, batch, d, h, w, c, (__nv_bfloat16*)dz_x);
-    CU_CHECK(cudaGetLastError());
-    return CCU_OK;
+    return launch_dependent(pool_backward_kernel, dim3((unsigned)grid_for(work, 256)), 256, 0, (cudaStream_t)stream,
+                            (const __nv_bfloat16*)gy, (const __nv_bfloat16*)x_act, batch, d, h, w, c, (__nv_bfloat16*)dz_x);
 }
 
 int ccu_up_reduce(const void* g_full, const void* coarse_act, int batch, int d, int h, int w, int c, void* dz_coarse,
@@ -2966,10 +3049,9 @@ int ccu_up_reduce(const void* g_full, const void* coarse_act, int batch, int d, 
     if (!g_full || !coarse_act || !dz_coarse || c % 8 || d % 2 || h % 2 || w % 2)
         return set_error(CCU_E_INVALID, "bad upsampling arguments");
     long long work = (long long)batch * (d / 2) * (h / 2) * (w / 2) * (c / 8);
-    up_reduce_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)g_full, (const __nv_bfloat16*)coarse_act, batch, d, h, w, c, (__nv_bfloat16*)dz_coarse);
-    CU_CHECK(cudaGetLastError());
-    return CCU_OK;
+    return launch_dependent(up_reduce_kernel, dim3((unsigned)grid_for(work, 256)), 256, 0, (cudaStream_t)stream,
+                            (const __nv_bfloat16*)g_full, (const __nv_bfloat16*)coarse_act, batch, d, h, w, c,
+                            (__nv_bfloat16*)dz_coarse);
 }
 
 int ccu_head(const void* d0, const float* xlog, const float* target, const float* weight, const float* head,
@@ -2978,10 +3060,8 @@ int ccu_head(const void* d0, const float* xlog, const float* target, const float
     // with the loss, every block ends in 18 reductions: no more blocks than four
     // per SM (16 per SM: 37 us on 4 x 64^3 voxels, 4: 25 us)
     const int blocks = target ? std::min(grid_for(n_vox, 256), 4 * sm_count()) : grid_for(n_vox, 256);
-    head_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)d0, xlog, target, weight, head, inv_wsum, n_vox, out, (__nv_bfloat16*)dz, dhead, loss);
-    CU_CHECK(cudaGetLastError());
-    return CCU_OK;
+    return launch_dependent(head_kernel, dim3((unsigned)blocks), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)d0, xlog,
+                            target, weight, head, inv_wsum, n_vox, out, (__nv_bfloat16*)dz, dhead, loss);
 }
 
 int ccu_input(const float* xlog, const float* density, const uint8_t* mat, int n_mat, const float* unc,
