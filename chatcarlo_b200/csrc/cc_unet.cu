@@ -1160,9 +1160,11 @@ __global__ void __launch_bounds__(THREADS, 4) conv_ws_kernel(const ConvP P, int 
 // NO), co_lo = the launch's first + blockIdx.y NO, of a layer with more.
 constexpr int PS_REGIONS_MAX = 8;
 constexpr int PS_GROUP_MAX = 3;
-constexpr int PS_THREADS = 416;             // warps 0, 1 MMA, 2-4 loaders, 5-12 epilogue
+// Warps 0 and 1 issue MMAs, 2 to 4 load, the others are the epilogue: eight
+// for slices of 16 output channels (two CTAs share an SM), sixteen for 32.
+__host__ __device__ constexpr int ps_epi_warps(int n) { return n == 16 ? 8 : 16; }
 constexpr int PS_ISSUERS = 2, PS_EPI_WARP0 = PS_ISSUERS + WS_LOADERS / 32;
-constexpr int PS_EPI_WARPS = 8;
+__host__ __device__ constexpr int ps_threads(int n) { return 32 * (PS_EPI_WARP0 + ps_epi_warps(n)); }
 constexpr uint32_t PS_SMEM_MAX = 220 * 1024;
 // A ring slot holds 16-channel groups of a halo plane, 180 voxel rows of 32
 // bytes under the 32-byte swizzle (16-byte half h of voxel v at half
@@ -1226,6 +1228,20 @@ struct PsWalk {
     }
 };
 
+// Region and phase of a plane of the CTA's sequence.
+struct PsRegion {
+    uint32_t r = 0, ph = 0;
+    __device__ __forceinline__ PsRegion ahead(uint32_t k, uint32_t n) const {      // k <= n planes on
+        PsRegion o{r + k, ph};
+        if (o.r >= n) o.r -= n, o.ph ^= 1u;
+        return o;
+    }
+    __device__ __forceinline__ PsRegion ahead_any(uint32_t k, uint32_t n) const {
+        const uint32_t t = r + k;
+        return PsRegion{t % n, ph ^ ((t / n) & 1u)};
+    }
+};
+
 template <int N>
 struct PsInt {
     static constexpr int value = N;
@@ -1238,11 +1254,11 @@ struct PsPass {
     float* part_out;           // FP32 sums [slice][v][NO] out (no bias / ReLU / BF16), or null
 };
 
-// An epilogue warp is done with the region of plane z - 1 and, at a
-// segment's end, with those of planes z and z + 1.  One elected lane arrives,
-// predicated rather than branched to: the warp's tensor-memory reads are
-// complete for all its lanes behind tcgen05.wait.
-__device__ __forceinline__ void ps_release(uint64_t* rfree, uint32_t rm, uint32_t r0, uint32_t rp, bool last) {
+// One arrival of an epilogue warp on the "free" barriers of regions ra, and
+// where b and c ask for it rb and rc.  One elected lane arrives, predicated
+// rather than branched to: the warp's tensor-memory reads are complete for all
+// its lanes behind tcgen05.wait.
+__device__ __forceinline__ void ps_release(uint64_t* rfree, uint32_t ra, uint32_t rb, bool b, uint32_t rc, bool c) {
     tc_fence_before();
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t.reg .b64 st;\n\t"
@@ -1250,13 +1266,14 @@ __device__ __forceinline__ void ps_release(uint64_t* rfree, uint32_t rm, uint32_
         "@p mbarrier.arrive.shared::cta.b64 st, [%0];\n\t"
         "setp.ne.and.b32 q, %3, 0, p;\n\t"
         "@q mbarrier.arrive.shared::cta.b64 st, [%1];\n\t"
-        "@q mbarrier.arrive.shared::cta.b64 st, [%2];\n\t}" ::"r"(smem_u32(rfree + rm)),
-        "r"(smem_u32(rfree + r0)), "r"(smem_u32(rfree + rp)), "r"((int)last)
+        "setp.ne.and.b32 q, %4, 0, p;\n\t"
+        "@q mbarrier.arrive.shared::cta.b64 st, [%2];\n\t}" ::"r"(smem_u32(rfree + ra)),
+        "r"(smem_u32(rfree + rb)), "r"(smem_u32(rfree + rc)), "r"((int)b), "r"((int)c)
         : "memory");
 }
 
 template <int NO, int G, int C8P, bool PLAIN>
-__global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_ps_kernel(const __grid_constant__ CUtensorMap amap, const ConvP P, const PsPass Q, int ring) {
+__global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8 ? 2 : 1) conv_ps_kernel(const __grid_constant__ CUtensorMap amap, const ConvP P, const PsPass Q, int ring) {
     constexpr int NP = 3 * NO;                                // MMA N: the three dz weight planes
     constexpr uint32_t RC = ps_region_cols(NO);
     constexpr uint32_t NQ = (uint32_t)ps_regions(G), TCOLS = ps_tmem_cols(NO, G);
@@ -1287,7 +1304,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         }
         for (uint32_t r = 0; r < NQ; ++r) {
             mbar_init(&rfull[r], 1);
-            mbar_init(&rfree[r], PS_EPI_WARPS);
+            mbar_init(&rfree[r], ps_epi_warps(NO));
         }
         s_fail = 0;
         mbar_init_fence();
@@ -1297,7 +1314,7 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
     // (all threads: as 16-byte copies; 256- and 512-byte bulk copies, issued one by one, took 8 us longer
     // for 128 input channels)
     const uint32_t sbase = (smem_u32(smem) + 255u) & ~255u, swt = sbase + R * slot16 * 16;
-    for (int i = tid; i < 9 * c8p * NP; i += PS_THREADS) {
+    for (int i = tid; i < 9 * c8p * NP; i += ps_threads(NO)) {
         const int r = i % NP, g = i / NP;
         const int t9 = g / c8p, c8 = Q.c8_lo + g % c8p, dz = r / NO, co = r % NO;
         const int src = ((dz * 9 + t9) * c8n + c8) * Q.n_out + co_lo + co;
@@ -1431,12 +1448,16 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                 if (elect_one()) {
                     const uint32_t al = (uint32_t)a0 + so[0], bl = (uint32_t)b0;
 #pragma unroll
-                    for (int t9 = 0; t9 < 9; ++t9)
+                    for (int t9 = 0; t9 < 9; ++t9) {
+                        uint32_t bt = bl + (uint32_t)(t9 * C8P * NP);
+                        // many groups: the constants of all MMAs kept across planes would spill
+                        if (C8P >= 6) asm volatile("" : "+r"(bt));
 #pragma unroll
                         for (int j = 0; j < C8P / 2; ++j)
                             mma_bf16_lo(d[0], al + (uint32_t)(((t9 / 3) * HALO_X + t9 % 3) * 2 + j * (int)GROUP16),
-                                        (uint32_t)(a0 >> 32), bl + (uint32_t)((t9 * C8P + 2 * j) * NP),
-                                        (uint32_t)(b0 >> 32), IDESC, (t9 > 0 || j > 0) ? 1u : 0u);
+                                        (uint32_t)(a0 >> 32), bt + (uint32_t)(2 * j * NP), (uint32_t)(b0 >> 32), IDESC,
+                                        (t9 > 0 || j > 0) ? 1u : 0u);
+                    }
                     mma_commit(&rfull[rsk[0]]);
                     mma_commit(&empty[fsk[0]]);
                 }
@@ -1482,23 +1503,32 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
         if (last_r < NQ) mbar_wait(&rfull[last_r], last_ph);
     } else if (warp >= PS_EPI_WARP0) {
         // ---- epilogue: output z = D_{z-1}[dz 0] + D_z[dz 1] + D_{z+1}[dz 2]; row m, lane quarter warp - 4 ----
-        // Eight warps, two per lane quarter: each takes half of the channels
-        // of every output plane, or, with the head (whose sum runs over all
-        // channels in order), all channels of every other plane.  Either way
-        // it waits for every plane and arrives once per region, as soon as
-        // the values are in registers.  An output costs a warp some 600 cycles
-        // of latency however few channels it has; what it reads beside the
-        // sums (mask, partial sum) is therefore read a plane ahead: read in
-        // the same plane it cost another 400.
+        // A warp takes CW channels of its lane quarter.  Slices of 16: two
+        // groups of four warps, each half of the channels of every plane (or,
+        // with the head, whose sum runs over all channels in order, all
+        // channels of every other plane).  Slices of 32, with the SM to
+        // themselves: four groups, half of the channels of every other plane
+        // each; an output costs a warp some 700 cycles of latency (1,000 with a
+        // mask) however few channels it has, against 500 to 1,000 of MMAs.
+        // Either way every warp arrives exactly once on a plane's "free"
+        // barrier, after it has seen that plane's MMAs complete and read what
+        // it reads of it: a group that takes every output arrives for plane
+        // z - 1 after output z, one that takes every other for z - 1 and z
+        // (it reads z + 1 again for z + 2), and at a segment's ends for the
+        // planes without a reader of its own.
+        // What an output reads beside the sums (mask, partial sum) is read
+        // an output ahead: read with it, its latency was added to the output's.
+        constexpr int CW = NO / 2, GROUPS = ps_epi_warps(NO) / 4;
+        constexpr bool EVERY_OTHER = GROUPS == 4;
         const float *bias_p = behind_wait(P.bias), *head_p = behind_wait(P.head), *head_x = behind_wait(P.head_x);
         const __nv_bfloat16* mask0 = behind_wait(P.mask0);
         const float* part_rd = behind_wait(part_in);
-        constexpr int CW = NO / 2;                             // channels per warp
         const int qw = warp & 3, grp = (warp - PS_EPI_WARP0) >> 2, m = qw * 32 + lane;
+        const int half = grp & 1, own = EVERY_OTHER ? grp >> 1 : 0, step = EVERY_OTHER ? 2 : 1;
         const uint32_t lq = (uint32_t)(qw * 32) << 16;
         const bool heads = !PLAIN && NO == 16 && head_p != nullptr;
         const bool masked = !PLAIN && mask0 && !part_out && !heads;
-        const int c0 = grp * CW, co0 = co_lo + c0;
+        const int c0 = half * CW, co0 = co_lo + c0;
         const uint32_t plane = (uint32_t)(S.H * S.W);
         float2 bias[CW / 2];
         if (bias_p && (PLAIN || !part_out)) {
@@ -1506,14 +1536,14 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
             for (int j = 0; j < CW / 2; ++j)
                 bias[j] = make_float2(__ldg(bias_p + co0 + 2 * j), __ldg(bias_p + co0 + 2 * j + 1));
         }
-        // regions of planes z - 1, z and z + 1 and the phase of the last
-        uint32_t rm = 0, r0 = 1, r1 = 2, ph1 = 0;
+        PsRegion base;                                         // the segment's first plane, zs - 1
         bool ok = true;
+        auto wait_plane = [&](PsRegion a) { return warp_wait_or_fail(&rfull[a.r], a.ph, fail); };
         PsWalk walk(S);
         for (WsSeg q; ok && walk.next(S, q);) {
-            const int y = q.y0 + (m >> 3), x = q.x0 + (m & 7);
+            const int y = q.y0 + (m >> 3), x = q.x0 + (m & 7), n = q.ze - q.zs;
             const bool in = y < S.H && x < S.W;
-            uint32_t v = (uint32_t)((((long long)q.n * S.D + q.zs) * S.H + y) * S.W + x);
+            uint32_t v = (uint32_t)((((long long)q.n * S.D + q.zs + own) * S.H + y) * S.W + x);
             uint4 mk[CW / 8];
             float4 part[CW / 4];
             auto read_ahead = [&](uint32_t u) {
@@ -1529,26 +1559,30 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                         part[h] = __ldg(reinterpret_cast<const float4*>(part_rd + (size_t)u * NO + c0) + h);
                 }
             };
-            if (!PLAIN && in) read_ahead(v);
-            // each plane's wait below covers every earlier plane of its own
-            // issuer; the segment's second plane is the other issuer's
-            ok = warp_wait_or_fail(&rfull[r0], r1 == 0 ? ph1 ^ 1u : ph1, fail);
-            for (int z = q.zs; ok && z < q.ze; ++z, v += plane) {
-                ok = warp_wait_or_fail(&rfull[r1], ph1, fail);
+            if (!PLAIN && in && own < n) read_ahead(v);
+            PsRegion rm = base.ahead((uint32_t)own, NQ);       // planes z - 1, z and z + 1 of the next output
+            // a wait for a plane covers every earlier plane of its own issuer;
+            // the two issuers take alternate planes
+            ok = wait_plane(base) && wait_plane(base.ahead(1, NQ));
+            if (ok && own == 1) ps_release(rfree, base.r, 0, false, 0, false);       // the first plane: not read
+            for (int i = own; ok && i < n; i += step, v += step * plane, rm = rm.ahead((uint32_t)step, NQ)) {
+                const PsRegion r0 = rm.ahead(1, NQ), rp = rm.ahead(2, NQ);
+                ok = (!EVERY_OTHER || wait_plane(r0)) && wait_plane(rp);
                 if (!ok) break;
                 tc_fence_after();
+                const bool last = i == n - 1;
                 // the sums of CN channels from c on
                 auto sums = [&](auto cn, int c, bool release, float2* f) {
                     constexpr int CN = decltype(cn)::value;
                     uint32_t um[CN], u0[CN], up[CN];
-                    tmem_ld_nw<CN>(tmem + rm * RC + lq + (uint32_t)c, um);
-                    tmem_ld_nw<CN>(tmem + r0 * RC + NO + lq + (uint32_t)c, u0);
-                    tmem_ld_nw<CN>(tmem + r1 * RC + 2 * NO + lq + (uint32_t)c, up);
+                    tmem_ld_nw<CN>(tmem + rm.r * RC + lq + (uint32_t)c, um);
+                    tmem_ld_nw<CN>(tmem + r0.r * RC + NO + lq + (uint32_t)c, u0);
+                    tmem_ld_nw<CN>(tmem + rp.r * RC + 2 * NO + lq + (uint32_t)c, up);
                     tmem_wait_ld();
                     // the uses below stay behind the wait
 #pragma unroll
                     for (int j = 0; j < CN; ++j) asm volatile("" : "+r"(um[j]), "+r"(u0[j]), "+r"(up[j]));
-                    if (release) ps_release(rfree, rm, r0, r1, z == q.ze - 1);
+                    if (release) ps_release(rfree, rm.r, r0.r, EVERY_OTHER || last, rp.r, last);
 #pragma unroll
                     for (int j = 0; j < CN / 2; ++j)
                         f[j] = add2(add2(make_float2(__uint_as_float(um[2 * j]), __uint_as_float(um[2 * j + 1])),
@@ -1556,8 +1590,8 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                                     make_float2(__uint_as_float(up[2 * j]), __uint_as_float(up[2 * j + 1])));
                 };
                 if (heads) {
-                    if ((z & 1) != grp) {
-                        ps_release(rfree, rm, r0, r1, z == q.ze - 1);
+                    if ((i & 1) != half) {
+                        ps_release(rfree, rm.r, r0.r, last, rp.r, last);
                     } else {
                         // x + b, then + w_j a_j in channel order (the head kernel's FP32 sequence)
                         float hsum = in ? head_x[v] + __ldg(head_p + 16) : 0.0f;
@@ -1581,62 +1615,62 @@ __global__ void __launch_bounds__(PS_THREADS, NO == 16 && G == 1 ? 2 : 1) conv_p
                         }
                         if (in) P.head_out[v] = hsum;
                     }
-                } else {
-                    float2 f[CW / 2];
-                    sums(PsInt<CW>{}, c0, true, f);
-                    if (!PLAIN && part_rd) {
-#pragma unroll
-                        for (int j = 0; j < CW / 4; ++j) {
-                            f[2 * j] = add2(f[2 * j], make_float2(part[j].x, part[j].y));
-                            f[2 * j + 1] = add2(f[2 * j + 1], make_float2(part[j].z, part[j].w));
-                        }
-                    }
-                    if (!PLAIN && part_out) {
-                        if (in) {
-                            float4* po = reinterpret_cast<float4*>(part_out + (size_t)v * NO + c0);
-#pragma unroll
-                            for (int j = 0; j < CW / 4; ++j)
-                                po[j] = make_float4(f[2 * j].x, f[2 * j].y, f[2 * j + 1].x, f[2 * j + 1].y);
-                        }
-                    } else {
-                        if (bias_p) {
-#pragma unroll
-                            for (int j = 0; j < CW / 2; ++j) f[j] = add2(f[j], bias[j]);
-                        }
-#pragma unroll
-                        for (int h = 0; h < CW / 8; ++h) {
-                            // output channels [co, co + 8) go to out0 or out1 (split is a multiple of 8)
-                            const int co = co0 + 8 * h;
-                            const bool first = PLAIN || co < P.split;
-                            float t[8];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) t[2 * j] = f[4 * h + j].x, t[2 * j + 1] = f[4 * h + j].y;
-                            if (P.relu) {
-#pragma unroll
-                                for (int j = 0; j < 8; ++j) t[j] = fmaxf(t[j], 0.0f);
-                            }
-                            if (masked && first) {
-                                float k[8];
-                                unpack_bf16x8(mk[h], k);
-#pragma unroll
-                                for (int j = 0; j < 8; ++j) t[j] = k[j] > 0.0f ? t[j] : 0.0f;
-                            }
-                            __nv_bfloat16* o = first ? P.out0 + ((size_t)v * P.split + co)
-                                                     : P.out1 + ((size_t)v * (Q.n_out - P.split) + (co - P.split));
-                            if (in) *reinterpret_cast<uint4*>(o) = pack_bf16x8(t);
-                        }
-                    }
-                    if (!PLAIN && in && z + 1 < q.ze) read_ahead(v + plane);
+                    continue;
                 }
-                rm = r0, r0 = r1;
-                ring_next(r1, ph1, NQ);
-            }
-            // the next segment's first output reads its planes 0 .. 2: two planes on
+                float2 f[CW / 2];
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                rm = r0, r0 = r1;
-                ring_next(r1, ph1, NQ);
+                for (int c = 0; c < CW; c += 8) sums(PsInt<8>{}, c0 + c, c + 8 == CW, f + c / 2);
+                if (!PLAIN && part_rd) {
+#pragma unroll
+                    for (int j = 0; j < CW / 4; ++j) {
+                        f[2 * j] = add2(f[2 * j], make_float2(part[j].x, part[j].y));
+                        f[2 * j + 1] = add2(f[2 * j + 1], make_float2(part[j].z, part[j].w));
+                    }
+                }
+                if (!PLAIN && part_out) {
+                    if (in) {
+                        float4* po = reinterpret_cast<float4*>(part_out + (size_t)v * NO + c0);
+#pragma unroll
+                        for (int j = 0; j < CW / 4; ++j)
+                            po[j] = make_float4(f[2 * j].x, f[2 * j].y, f[2 * j + 1].x, f[2 * j + 1].y);
+                    }
+                } else {
+                    if (bias_p) {
+#pragma unroll
+                        for (int j = 0; j < CW / 2; ++j) f[j] = add2(f[j], bias[j]);
+                    }
+#pragma unroll
+                    for (int h = 0; h < CW / 8; ++h) {
+                        // output channels [co, co + 8) go to out0 or out1 (split is a multiple of 8)
+                        const int co = co0 + 8 * h;
+                        const bool first = PLAIN || co < P.split;
+                        float t[8];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) t[2 * j] = f[4 * h + j].x, t[2 * j + 1] = f[4 * h + j].y;
+                        if (P.relu) {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) t[j] = fmaxf(t[j], 0.0f);
+                        }
+                        if (masked && first) {
+                            float k[8];
+                            unpack_bf16x8(mk[h], k);
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) t[j] = k[j] > 0.0f ? t[j] : 0.0f;
+                        }
+                        __nv_bfloat16* o = first ? P.out0 + ((size_t)v * P.split + co)
+                                                 : P.out1 + ((size_t)v * (Q.n_out - P.split) + (co - P.split));
+                        if (in) *reinterpret_cast<uint4*>(o) = pack_bf16x8(t);
+                    }
+                }
+                if (!PLAIN && in && i + step < n) read_ahead(v + step * plane);
             }
+            // the group without the last output: the last two planes
+            if (EVERY_OTHER && ok && ((n - 1) & 1) != own) {
+                const PsRegion before = base.ahead_any((uint32_t)n, NQ), end = base.ahead_any((uint32_t)n + 1, NQ);
+                ok = wait_plane(before) && wait_plane(end);
+                if (ok) ps_release(rfree, before.r, end.r, true, 0, false);
+            }
+            base = base.ahead_any((uint32_t)n + 2, NQ);
         }
     }
     __syncthreads();
@@ -2714,17 +2748,17 @@ int launch_conv_ps_pass(const CUtensorMap& amap, const ConvP& P, const PsPass& Q
         int best = 0, r_c = CCU_OK;
         for (int r = G + 1; r <= WS_RING_MAX && ps_smem_bytes(NO, c8p, r) <= PS_SMEM_MAX; ++r) {
             int res = 1;
-            r_c = resident_ctas(kernel, (size_t)ps_smem_bytes(NO, c8p, r) + 1024, cols, res, PS_THREADS);
+            r_c = resident_ctas(kernel, (size_t)ps_smem_bytes(NO, c8p, r) + 1024, cols, res, ps_threads(NO));
             if (r_c != CCU_OK) return r_c;
             if (res >= best) best = res, p.ring = r;
         }
         if (p.ring == 0) return set_error(CCU_E_INVALID, "plane-stationary pass does not fit shared memory");
-        r_c = tc_launch_smem(kernel, ps_smem_bytes(NO, c8p, p.ring), cols, p.smem, PS_THREADS);
-        return r_c == CCU_OK ? resident_ctas(kernel, p.smem, cols, p.resident, PS_THREADS) : r_c;
+        r_c = tc_launch_smem(kernel, ps_smem_bytes(NO, c8p, p.ring), cols, p.smem, ps_threads(NO));
+        return r_c == CCU_OK ? resident_ctas(kernel, p.smem, cols, p.resident, ps_threads(NO)) : r_c;
     });
     if (rc != CCU_OK) return rc;
     const long long grid = std::min<long long>(planes, std::max(1, plan.sms * plan.resident / slices));
-    return launch_dependent(kernel, dim3((unsigned)grid, (unsigned)slices), PS_THREADS, plan.smem, st, amap, P, Q, plan.ring);
+    return launch_dependent(kernel, dim3((unsigned)grid, (unsigned)slices), ps_threads(NO), plan.smem, st, amap, P, Q, plan.ring);
 }
 
 // Output channels [co_lo, co_lo + slices NO) of the layer, in channel passes.
