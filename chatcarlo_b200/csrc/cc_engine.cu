@@ -85,7 +85,8 @@ __device__ __forceinline__ PNode ldg_node(const PNode* p) {
 #endif
 }
 // a uniform draw in (0, 1] of the build's precision from the next 32 bits
-__device__ __forceinline__ phys uni(HistoryRng& r) {
+template <typename RNG>
+__device__ __forceinline__ phys uni(RNG& r) {
 #ifdef CC_TRACK_FP64
     return r.uniform_d();
 #else
@@ -481,7 +482,8 @@ __device__ __forceinline__ phys s_over_z(const phys* s, phys q) {
 }
 
 // Bound Compton: Kahn-type KN proposal with S(Z,q)/Z rejection (physics.py:41-56, 95-135).
-__device__ __forceinline__ void sample_compton(const phys* sz, phys E, HistoryRng& rng, phys& eps_out, phys& cos_out) {
+template <typename RNG>
+__device__ __forceinline__ void sample_compton(const phys* sz, phys E, RNG& rng, phys& eps_out, phys& cos_out) {
     phys alpha = E / MEC2;
     phys emin = P(1.0) / (P(1.0) + P(2.0) * alpha);
     phys env = P(1.0) / emin + emin;
@@ -502,8 +504,9 @@ __device__ __forceinline__ void sample_compton(const phys* sz, phys E, HistoryRn
 // Rayleigh: inverse of A(x) then (1+cos^2)/2 rejection (physics.py:281-351).
 // The row of a target A comes from a uniform-in-A bucket index, then a
 // short binary search inside the bucket.
+template <typename RNG>
 __device__ __forceinline__ bool sample_rayleigh(const phys* rx, const phys* ra, const int* bucket, phys scale,
-                                             phys E, HistoryRng& rng, phys& cos_out) {
+                                             phys E, RNG& rng, phys& cos_out) {
     phys xmax = (E / HC) * (E / HC);
     if (xmax > __ldg(rx + TABLE_N - 1)) return false;
     // A(x_max): x grid is q^2 with q uniform on [0, 20]
@@ -539,7 +542,8 @@ __device__ __forceinline__ bool sample_rayleigh(const phys* rx, const phys* ra, 
 // relaxes radiatively with probability omega_K and emits one of the K lines
 // (cumulative line probabilities), which leaves only when at or above the
 // 5 keV cut-off.  Returns the emitted line's energy, 0 when none.
-__device__ __forceinline__ phys sample_k_line(const DevElement& el, phys E, int fluorescence, HistoryRng& rng) {
+template <typename RNG>
+__device__ __forceinline__ phys sample_k_line(const DevElement& el, phys E, int fluorescence, RNG& rng) {
     if (!(fluorescence && el.emits && E > el.k_edge)) return P(0.0);
     const bool is_k = uni(rng) < el.k_prob;
     const bool is_rad = uni(rng) < el.omega;
@@ -577,7 +581,8 @@ __device__ __forceinline__ void scatter_direction(real d[3], phys cost, phys phi
     d[0] = r.x; d[1] = r.y; d[2] = r.z;
 }
 
-__device__ __forceinline__ void isotropic(real d[3], HistoryRng& rng) {
+template <typename RNG>
+__device__ __forceinline__ void isotropic(real d[3], RNG& rng) {
     phys c = P(2.0) * uni(rng) - P(1.0);
     phys s = sqrt(fmax(P(0.0), P(1.0) - c * c));
     phys sp, cp;
@@ -768,7 +773,8 @@ __device__ __forceinline__ phys heel_fluence(const KSource& S, phys s) {
 
 // Energy of a photon at heel coordinate s: the alias table of its bin,
 // clamped to the bins that have fluence (source.py:195-207).
-__device__ __forceinline__ phys heel_energy(const KSource& S, phys s, HistoryRng& rng) {
+template <typename RNG>
+__device__ __forceinline__ phys heel_energy(const KSource& S, phys s, RNG& rng) {
     int b = (int)((s + S.span) / S.bin_w);
     b = min(max(b, 0), S.heel_n - 1);
     b = min(max(b, S.heel_lo), S.heel_hi);
@@ -783,8 +789,8 @@ constexpr int HEEL_MAX_TRIALS = 100000;
 
 // HEEL: the source may carry the heel effect (a separate instantiation, so
 // that the kernels of sources without it keep their registers).
-template <bool HEEL>
-__device__ __forceinline__ void sample_source(const KSource& S, HistoryRng& rng, real p[3], real d[3], phys& E) {
+template <bool HEEL, typename RNG>
+__device__ __forceinline__ void sample_source(const KSource& S, RNG& rng, real p[3], real d[3], phys& E) {
     phys pos[3] = {S.pos[0], S.pos[1], S.pos[2]};
     phys dir[3] = {S.dir[0], S.dir[1], S.dir[2]};
     phys u[3] = {S.u[0], S.u[1], S.u[2]};
@@ -886,7 +892,7 @@ constexpr size_t SLOT_BYTES_COMPACT = (size_t)32 << 20;     // slots above this 
 #ifndef TALLY_PIECE
 #define TALLY_PIECE 16
 #endif
-constexpr int BLOCK = 256;
+constexpr int BLOCK = RNG_THREADS;
 constexpr int WARPS_PER_BLOCK = BLOCK / 32;
 // A thread's 32-bit counters go to the block's 64-bit ones once any reaches
 // 2^30: one history adds far less than the remaining 2^31 (its steps are
@@ -1063,7 +1069,7 @@ __device__ __forceinline__ void take_unit(const KRun& R, long long& first, long 
 template <bool FROM_SOURCE, bool TALLY, bool HEEL = false, int TV = CELL_FP64>
 __global__ void __launch_bounds__(BLOCK, CC_MIN_BLOCKS)
 transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource SRC, const KRun R) {
-    extern __shared__ double s_edep[];             // [n_scratch][n_mat], then the warps' segment rings
+    extern __shared__ double s_edep[];             // [n_scratch][n_mat], the random words, the warps' segment rings
     __shared__ unsigned long long s_cnt[6];
     constexpr bool INLINE = TALLY && TV != TV_DEFER;
     const int n_acc = R.n_scratch * T.n_mat;
@@ -1080,7 +1086,8 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
     // warp-local pool [pool_next, pool_end), histories of one unit, and its scratch slot
     long long pool_next = 0, pool_end = 0;
     int pool_slot = 0;
-    SegQueue<SegRec> Q(s_edep + n_acc, warp);
+    uint32_t* const s_words = reinterpret_cast<uint32_t*>(s_edep + n_acc);
+    SegQueue<SegRec> Q(s_words + RNG_BYTES / sizeof(uint32_t), warp);
     auto score_piece = [&](const SegRec& q, int k) {
         real ta, tz;
         piece_range(q.t0, q.t1, q.m, k, ta, tz);
@@ -1094,7 +1101,8 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
     phys E = P(0.), tau = P(0.);
     int nsc = 0, mat = -1, slot = 0;
     int steps = 0;
-    HistoryRng rng;
+    RingRng rng;
+    rng.ring = s_words + threadIdx.x;
 
     while (true) {
         // ---- phase 1a: regeneration ----
@@ -1114,7 +1122,7 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
                 h = pool_next + rank;
                 live = true;
                 long long gh = R.first + h;
-                rng.init(R.seed, (unsigned long long)gh, 0u);
+                rng.init(R.seed, (unsigned long long)gh);
                 slot = pool_slot;
                 if (FROM_SOURCE) {
                     sample_source<HEEL>(SRC, rng, p, d, E);
@@ -1235,6 +1243,7 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
             phys ph, co, ra;
             parts(T, M, L, ph, co, ra);
             phys tot = ph + co + ra;
+            rng.top_up(5);                     // kind, element and a first Compton trial
             phys r = uni(rng) * tot;
             ++nsc;
             const int kind = r < ph ? 0 : (r < ph + co ? 1 : 2);
@@ -1269,6 +1278,7 @@ transport_kernel(const KTables T, const KScene S, const KGrid G, const KSource S
             }
             if (kind < 2) atomicAdd(&s_edep[(slot >> R.copy_shift) * T.n_mat + mat], (double)dep);
             if (!done) {
+                rng.top_up(3);
                 if (kind == 0) isotropic(d, rng);                     // the fluorescence photon
                 else scatter_direction(d, cost, TWO_PI * uni(rng));
                 E = e_new;
@@ -1427,7 +1437,7 @@ constexpr int BATCH_MIN_BLOCKS = CC_MIN_BLOCKS < 3 ? CC_MIN_BLOCKS : 3;
 template <bool TALLY, bool HEEL = false>
 __global__ void __launch_bounds__(BLOCK, BATCH_MIN_BLOCKS)
 batch_kernel(const KTables T, const KBatch B, const KRun R) {
-    extern __shared__ double s_rings[];            // the warps' segment rings
+    extern __shared__ double s_rings[];            // the random words, the warps' segment rings
     __shared__ unsigned long long s_cnt[2];
     if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
     __syncthreads();
@@ -1436,7 +1446,8 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
     const unsigned long long seed = __ldg(B.run);
     const int fluorescence = (int)__ldg(B.run + 1);
     unsigned c_steps = 0, c_vox = 0;            // 32-bit, handed on before they near 2^31
-    SegQueue<SegRecB> Q(s_rings, warp);
+    uint32_t* const s_words = reinterpret_cast<uint32_t*>(s_rings);
+    SegQueue<SegRecB> Q(s_words + RNG_BYTES / sizeof(uint32_t), warp);
     auto score_piece = [&](const SegRecB& q, int k) {
         real ta, tz;
         piece_range(q.t0, q.t1, q.m, k, ta, tz);
@@ -1454,7 +1465,8 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
     phys E = P(0.), tau = P(0.);
     int nsc = 0, mat = -1;
     int steps = 0;
-    HistoryRng rng;
+    RingRng rng;
+    rng.ring = s_words + threadIdx.x;
 
     while (true) {
         // ---- regeneration ----
@@ -1477,7 +1489,7 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
                 li = pool_next + rank;
                 sc = pool_scene;
                 live = true;
-                rng.init(seed, ((unsigned long long)sc << 40) + (unsigned long long)li, 0u);
+                rng.init(seed, ((unsigned long long)sc << 40) + (unsigned long long)li);
                 long long nh = __ldg(B.n_hist + sc);
                 slot = (int)((li * B.slots) / nh);
                 sample_source<HEEL>(B.sources[sc], rng, p, d, E);
@@ -1566,6 +1578,7 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
             } else {
                 phys ph, co, ra;
                 parts(T, M, L, ph, co, ra);
+                rng.top_up(5);                 // kind, element and a first Compton trial
                 phys r = uni(rng) * (ph + co + ra);
                 ++nsc;
                 const int kind = r < ph ? 0 : (r < ph + co ? 1 : 2);
@@ -1595,6 +1608,7 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
                     ok = false;
                 }
                 if (ok && !ended) {
+                    rng.top_up(3);
                     if (kind == 0) isotropic(d, rng);                   // the fluorescence photon
                     else scatter_direction(d, cost, TWO_PI * uni(rng));
                     E = e_new;
@@ -2921,7 +2935,7 @@ static int enqueue_launch(cc_ctx* c, const cc_scene* scene, const cc_tables* tab
     memset(&S, 0, sizeof(S));
     bool fs = src != nullptr;
     if (fs) S = *src;
-    size_t smem = n_acc * sizeof(double) + (tl && !c->tally_queue ? SegQueue<SegRec>::bytes(c->block) : 0);
+    size_t smem = n_acc * sizeof(double) + RNG_BYTES + (tl && !c->tally_queue ? SegQueue<SegRec>::bytes(c->block) : 0);
     int blocks = grid_blocks_for(c, smem, fs, tl, big_grid);
     R.lockstep = tl && !big_grid && R.n >= (long long)LOCKSTEP_PER_LANE * blocks * c->block ? 1 : 0;
     const bool defer = tl && c->tally_queue;
@@ -3506,7 +3520,7 @@ int cc_transport_photons_device_noalloc(const cc_scene* scene, const cc_tables* 
     memset(&G, 0, sizeof(G));
     KSource S;
     memset(&S, 0, sizeof(S));
-    const size_t smem = (size_t)tables->n_mat * sizeof(double);
+    const size_t smem = (size_t)tables->n_mat * sizeof(double) + RNG_BYTES;
     int sms = 0, occ = 0;
     CC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<false, false>, BLOCK, smem) != cudaSuccess ||
@@ -3662,7 +3676,7 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
     R.status = b->d_status;
     R.counters = b->d_counters;
     R.work = b->d_counters + 6;
-    const size_t smem = b->tally ? SegQueue<SegRecB>::bytes(c->block) : 0;
+    const size_t smem = RNG_BYTES + (b->tally ? SegQueue<SegRecB>::bytes(c->block) : 0);
     if (b->tally) {
         e = heel ? allow_smem(batch_kernel<true, true>, smem) : allow_smem(batch_kernel<true>, smem);
         if (e != cudaSuccess) { batch_free(b); return set_error(CC_E_DEVICE, std::string("batch launch: ") + cudaGetErrorString(e)); }
@@ -3672,7 +3686,7 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
     if (per_sm == 0) {
         int occ = 0;
         cudaError_t oe = b->tally ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<true>, c->block, smem)
-                                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<false>, c->block, 0);
+                                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<false>, c->block, smem);
         per_sm = (oe == cudaSuccess && occ > 0) ? occ : 1;
     }
     b->blocks = c->sm_count * per_sm;
@@ -3689,8 +3703,8 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
     if (e == cudaSuccess) {
         if (b->tally && heel) batch_kernel<true, true><<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
         else if (b->tally) batch_kernel<true><<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
-        else if (heel) batch_kernel<false, true><<<b->blocks, c->block, 0, st>>>(tables->k, k, R);
-        else batch_kernel<false><<<b->blocks, c->block, 0, st>>>(tables->k, k, R);
+        else if (heel) batch_kernel<false, true><<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
+        else batch_kernel<false><<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
         e = cudaGetLastError();
         b->launches = 1;
     }

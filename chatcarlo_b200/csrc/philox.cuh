@@ -104,4 +104,63 @@ struct HistoryRng {
     CC_HD double uniform_d() { return ((double)next_u32() + 1.0) * 2.3283064365386963e-10; }
 };
 
+#ifdef __CUDACC__
+// The same stream with its next words in shared memory: two blocks per thread
+// (word w of thread t at ring[w * RNG_THREADS + t]).  A thread of the transport
+// kernels that runs out of words in the middle of a rejection loop makes its
+// warp compute a block for it alone, and a history takes seven of them; with
+// two blocks held, the warp's threads top up together where they are converged
+// (before an interaction, before the new flight), and the four words and their
+// count no longer take registers.
+constexpr int RNG_THREADS = 256;                 // threads of a block at most
+constexpr int RNG_WORDS = 8;
+constexpr size_t RNG_BYTES = (size_t)RNG_WORDS * RNG_THREADS * sizeof(uint32_t);
+
+__device__ __noinline__ void philox_to_ring(uint32_t* ring, uint32_t block, uint32_t h0, uint32_t h1, uint32_t k0,
+                                            uint32_t k1) {
+    const u32x4 b = philox4x32_10(u32x4{block, 0u, h0, h1}, k0, k1);
+    uint32_t* w = ring + (block & 1u) * 4u * RNG_THREADS;
+    w[0] = b.x;
+    w[RNG_THREADS] = b.y;
+    w[2 * RNG_THREADS] = b.z;
+    w[3 * RNG_THREADS] = b.w;
+}
+
+struct RingRng {
+    uint32_t* ring;        // this thread's column
+    uint32_t k0, k1;       // seed
+    uint32_t h0, h1;       // history index
+    uint32_t block;        // next counter block
+    uint32_t pos;          // draws taken; 4 block - pos words are left
+
+    __device__ __forceinline__ void init(uint64_t seed, uint64_t history) {
+        k0 = (uint32_t)seed;
+        k1 = (uint32_t)(seed >> 32);
+        h0 = (uint32_t)history;
+        h1 = (uint32_t)(history >> 32);
+        block = pos = 0;
+        refill();
+        refill();
+    }
+    // Only with at most four words left: the block it replaces is used up.
+    __device__ __forceinline__ void refill() {
+        philox_to_ring(ring, block, h0, h1, k0, k1);
+        ++block;
+    }
+    // A refill now, with the warp's other threads, where fewer than `words`
+    // (1 .. 5) draws are left.
+    __device__ __forceinline__ void top_up(uint32_t words) {
+        if (4u * block - pos < words) refill();
+    }
+    __device__ __forceinline__ uint32_t next_u32() {
+        if (pos == 4u * block) refill();
+        const uint32_t r = ring[(pos % RNG_WORDS) * RNG_THREADS];
+        ++pos;
+        return r;
+    }
+    __device__ __forceinline__ float uniform() { return u01_oc(next_u32()); }
+    __device__ __forceinline__ double uniform_d() { return ((double)next_u32() + 1.0) * 2.3283064365386963e-10; }
+};
+#endif
+
 }  // namespace cc
