@@ -76,8 +76,8 @@ class BatchedRun:
             N.check(self.eng.lib.cc_ctx_set_launch(self.eng.ctx, 256, 0))
 
     def reset(self):
-        for d in self.dgrids:
-            d.reset()
+        if self.tally:
+            N.check(self.eng.lib.cc_batch_reset(self.plan))
 
     def run(self, seed: int, fluorescence: bool = True):
         counts = np.zeros((self.n, 4), dtype=np.int64)

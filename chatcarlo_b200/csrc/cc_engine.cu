@@ -1759,6 +1759,34 @@ __global__ void fold_plain_kernel(double2* __restrict__ total, double2* __restri
     }
 }
 
+// fold_plain_kernel on every scene of a batch (blockIdx.y): 24 launches of 3 us
+// each in the graph of a 24-scene batch otherwise.
+__global__ void fold_plain_scenes_kernel(const KGrid* __restrict__ grids, double2* const* __restrict__ totals) {
+    const KGrid& G = grids[blockIdx.y];
+    double2* const total = totals[blockIdx.y];
+    double2* const scratch = reinterpret_cast<double2*>(G.tally);
+    const long long nvox = G.nvox;
+    const int cell32 = G.tally32;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvox; i += (long long)gridDim.x * blockDim.x) {
+        const double2 s = cell_read(scratch, i, cell32);
+        if (s.x != 0.0 || s.y != 0.0) {
+            double2 t = total[i];
+            t.x += s.x;
+            t.y += s.y;
+            total[i] = t;
+            scratch[i] = make_double2(0.0, 0.0);
+        }
+    }
+}
+
+// The totals of every scene of a batch to zero (blockIdx.y).
+__global__ void zero_scenes_kernel(const KGrid* __restrict__ grids, double2* const* __restrict__ totals) {
+    double2* const total = totals[blockIdx.y];
+    const long long nvox = grids[blockIdx.y].nvox;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvox; i += (long long)gridDim.x * blockDim.x)
+        total[i] = make_double2(0.0, 0.0);
+}
+
 // Split the interleaved device grids into the caller's separate arrays
 // (totals include a pending, not yet folded batch, as VoxelGrid.kerma_keV does).
 __global__ void unpack_kernel(const double2* __restrict__ total, const double2* __restrict__ pending,
@@ -3564,6 +3592,8 @@ struct cc_batch {
     unsigned long long* h_run = nullptr;      // pinned: seed, fluorescence
     unsigned long long* d_counters = nullptr; // [8]: 4 steps, 5 voxel visits, 6 work
     unsigned* d_status = nullptr;
+    double2** d_totals = nullptr;             // [n_scenes] totals of the scenes' grids
+    long long max_vox = 0;                    // largest grid
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int blocks = 0;
@@ -3580,6 +3610,37 @@ static void batch_free(cc_batch* b) {
 }
 
 extern "C" {
+
+constexpr int SCENE_ROWS = 32768;             // scenes of one launch over all scenes (grid rows)
+
+// Blocks per scene of such a launch.
+static int scene_blocks(const cc_batch* b) {
+    const long long per_scene = std::max(1, b->ctx->sm_count * 8 / std::max(1, b->n_scenes));
+    return (int)std::max(1LL, std::min((b->max_vox + 255) / 256, std::max(per_scene, 8LL)));
+}
+
+int cc_batch_reset(cc_batch* b) {
+    if (!b) return set_error(CC_E_INVALID, "batch is NULL");
+    cc_ctx* c = b->ctx;
+    CC_CUDA(cudaSetDevice(c->device));
+    bool one = b->tally;
+    for (const cc_grid* g : b->grids) one = one && !g->d_q && !g->scratch_dirty;
+    if (!one) {                                // batch statistics or scores left over: grid by grid
+        for (cc_grid* g : b->grids) {
+            const int rc = cc_grid_reset(g);
+            if (rc != CC_OK) return rc;
+        }
+        return CC_OK;
+    }
+    for (int i0 = 0; i0 < b->n_scenes; i0 += SCENE_ROWS) {
+        const dim3 grid((unsigned)scene_blocks(b), (unsigned)std::min(SCENE_ROWS, b->n_scenes - i0));
+        zero_scenes_kernel<<<grid, 256, 0, c->stream>>>(b->kb.grids + i0, b->d_totals + i0);
+        CC_CUDA(cudaGetLastError());
+    }
+    CC_CUDA(cudaStreamSynchronize(c->stream));
+    for (cc_grid* g : b->grids) g->n_batches = g->n_histories = 0;
+    return CC_OK;
+}
 
 int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const cc_scene* const* scenes,
                     const cc_source* const* sources, cc_grid* const* grids, const int64_t* n_histories,
@@ -3598,6 +3659,7 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
     b->chunk = chunk;
     b->tally = grids != nullptr;
     bool heel = false;               // some source carries the heel effect
+    const size_t smem = RNG_BYTES + (b->tally ? SegQueue<SegRecB>::bytes(c->block) : 0);
     std::vector<KScene> hs(n_scenes);
     std::vector<KSource> hsrc(n_scenes);
     std::vector<KGrid> hg(n_scenes);
@@ -3621,7 +3683,6 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
             b->grids.push_back(g);
         }
         b->nhist[i] = n_histories[i];
-        cf[i + 1] = cf[i] + (n_histories[i] + chunk - 1) / chunk;
         std::vector<long long>& sc = b->slot_counts[i];
         sc.assign(slots, 0);
         // histories li with floor(li * slots / n) == k
@@ -3630,6 +3691,27 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
             sc[k] = hi - lo;
         }
     }
+    if (b->tally) {
+        const cudaError_t e = heel ? allow_smem(batch_kernel<true, true>, smem) : allow_smem(batch_kernel<true>, smem);
+        if (e != cudaSuccess) { batch_free(b); return set_error(CC_E_DEVICE, std::string("batch launch: ") + cudaGetErrorString(e)); }
+    }
+    // launch shape: the context's block size and blocks per SM (the autotuner sets them)
+    int per_sm = c->blocks_per_sm;
+    if (per_sm == 0) {
+        int occ = 0;
+        cudaError_t oe = b->tally ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<true>, c->block, smem)
+                                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<false>, c->block, smem);
+        per_sm = (oe == cudaSuccess && occ > 0) ? occ : 1;
+    }
+    b->blocks = c->sm_count * per_sm;
+    // a warp's chunk: what the caller asks for, less where a warp would get fewer
+    // than eight of them (24 scenes of 3.2e6 histories: 4.27 ms with chunks of
+    // 256, 4.02 with 96; 64 scenes of 2.5e7: 31.1 with 256, 31.5 with 64)
+    long long all = 0;
+    for (long long n : b->nhist) all += n;
+    const long long share = all / (8LL * b->blocks * (c->block / 32)) / 32 * 32;
+    chunk = (int)std::min<long long>(chunk, std::max(64LL, share));
+    for (int i = 0; i < n_scenes; ++i) cf[i + 1] = cf[i] + (n_histories[i] + chunk - 1) / chunk;
     // one device block for every table of the batch
     // every sub-array starts on a 256-byte boundary (KScene is 4-byte aligned,
     // KSource and KGrid hold 8-byte pointers)
@@ -3640,7 +3722,8 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
     size_t o_cf = al(o_g + sizeof(KGrid) * n_scenes);
     size_t o_nh = al(o_cf + sizeof(long long) * (n_scenes + 1));
     size_t o_cnt = al(o_nh + sizeof(long long) * n_scenes);
-    size_t o_run = al(o_cnt + sizeof(unsigned long long) * 4 * n_scenes);
+    size_t o_tot = al(o_cnt + sizeof(unsigned long long) * 4 * n_scenes);
+    size_t o_run = al(o_tot + sizeof(double2*) * n_scenes);
     size_t o_c8 = al(o_run + 2 * sizeof(unsigned long long));
     size_t o_st = o_c8 + 8 * sizeof(unsigned long long);
     size_t total = al(o_st + 16);
@@ -3653,6 +3736,13 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
     cudaError_t e = cudaMemcpy(b->d_mem + o_sc, hs.data(), sizeof(KScene) * n_scenes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_mem + o_src, hsrc.data(), sizeof(KSource) * n_scenes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && b->tally) e = cudaMemcpy(b->d_mem + o_g, hg.data(), sizeof(KGrid) * n_scenes, cudaMemcpyHostToDevice);
+    b->d_totals = (double2**)(b->d_mem + o_tot);
+    std::vector<double2*> totals(n_scenes, nullptr);
+    for (size_t i = 0; i < b->grids.size(); ++i) {
+        totals[i] = (double2*)b->grids[i]->d_total;
+        b->max_vox = std::max(b->max_vox, b->grids[i]->k.nvox);
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(b->d_totals, totals.data(), sizeof(double2*) * n_scenes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_mem + o_cf, cf.data(), sizeof(long long) * (n_scenes + 1), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_mem + o_nh, b->nhist.data(), sizeof(long long) * n_scenes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { batch_free(b); return set_error(CC_E_DEVICE, std::string("batch upload: ") + cudaGetErrorString(e)); }
@@ -3676,25 +3766,7 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
     R.status = b->d_status;
     R.counters = b->d_counters;
     R.work = b->d_counters + 6;
-    const size_t smem = RNG_BYTES + (b->tally ? SegQueue<SegRecB>::bytes(c->block) : 0);
-    if (b->tally) {
-        e = heel ? allow_smem(batch_kernel<true, true>, smem) : allow_smem(batch_kernel<true>, smem);
-        if (e != cudaSuccess) { batch_free(b); return set_error(CC_E_DEVICE, std::string("batch launch: ") + cudaGetErrorString(e)); }
-    }
-    // launch shape: the context's block size and blocks per SM (the autotuner sets them)
-    int per_sm = c->blocks_per_sm;
-    if (per_sm == 0) {
-        int occ = 0;
-        cudaError_t oe = b->tally ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<true>, c->block, smem)
-                                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<false>, c->block, smem);
-        per_sm = (oe == cudaSuccess && occ > 0) ? occ : 1;
-    }
-    b->blocks = c->sm_count * per_sm;
-    {
-        long long all = 0;
-        for (long long n : b->nhist) all += n;
-        R.lockstep = b->tally && all >= (long long)LOCKSTEP_PER_LANE * b->blocks * c->block ? 1 : 0;
-    }
+    R.lockstep = b->tally && all >= (long long)LOCKSTEP_PER_LANE * b->blocks * c->block ? 1 : 0;
     // capture: clear the counters, take the seed, transport, fold the batches
     e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->d_mem + o_cnt, 0, sizeof(unsigned long long) * 4 * n_scenes, st);
@@ -3708,37 +3780,28 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
         e = cudaGetLastError();
         b->launches = 1;
     }
-    if (e == cudaSuccess && b->tally) {
+    if (e == cudaSuccess && b->tally && slots == 1) {
+        for (int i0 = 0; i0 < n_scenes && e == cudaSuccess; i0 += SCENE_ROWS) {
+            const dim3 grid((unsigned)scene_blocks(b), (unsigned)std::min(SCENE_ROWS, n_scenes - i0));
+            fold_plain_scenes_kernel<<<grid, 256, 0, st>>>(k.grids + i0, b->d_totals + i0);
+            ++b->launches;
+            e = cudaGetLastError();
+        }
+    } else if (e == cudaSuccess && b->tally) {
         int threads = 256;
         for (int i = 0; i < n_scenes && e == cudaSuccess; ++i) {
             cc_grid* g = grids[i];
-            const int cell32 = hg[i].tally32;
             int nb = std::max(1, std::min((int)((g->k.nvox + threads - 1) / threads), c->sm_count * 8));
-            if (slots > 1) {
-                // all batch slots of the scene in one fold
-                FoldSlots F;
-                memset(&F, 0, sizeof(F));
-                F.n = slots;
-                F.copies = 1;
-                for (int sl = 0; sl < slots; ++sl)
-                    if (b->slot_counts[i][sl] > 0) F.inv_nb[sl] = 1.0 / (double)b->slot_counts[i][sl];
-                fold_slots_kernel<<<nb, threads, 0, st>>>((double2*)g->d_total, (double2*)g->d_q, g->d_nhit,
-                                                          (double2*)g->d_scratch, g->k.nvox, F, cell32);
-                ++b->launches;
-                e = cudaGetLastError();
-                continue;
-            }
-            for (int sl = 0; sl < slots; ++sl) {
-                long long cnt = b->slot_counts[i][sl];
-                if (cnt <= 0) continue;
-                double2* scr = (double2*)(g->d_scratch + (size_t)sl * 2 * g->k.nvox);
-                if (slots > 1)
-                    fold_kernel<<<nb, threads, 0, st>>>((double2*)g->d_total, (double2*)g->d_q, g->d_nhit, scr,
-                                                         g->k.nvox, 1.0 / (double)cnt, cell32);
-                else
-                    fold_plain_kernel<<<nb, threads, 0, st>>>((double2*)g->d_total, scr, g->k.nvox, cell32);
-                ++b->launches;
-            }
+            // all batch slots of the scene in one fold
+            FoldSlots F;
+            memset(&F, 0, sizeof(F));
+            F.n = slots;
+            F.copies = 1;
+            for (int sl = 0; sl < slots; ++sl)
+                if (b->slot_counts[i][sl] > 0) F.inv_nb[sl] = 1.0 / (double)b->slot_counts[i][sl];
+            fold_slots_kernel<<<nb, threads, 0, st>>>((double2*)g->d_total, (double2*)g->d_q, g->d_nhit,
+                                                      (double2*)g->d_scratch, g->k.nvox, F, hg[i].tally32);
+            ++b->launches;
             e = cudaGetLastError();
         }
     }

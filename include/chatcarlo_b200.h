@@ -331,7 +331,7 @@ int cc_transport_photons_device_noalloc(const cc_scene* scene, const cc_tables* 
 /* Batched multi-scene runs (no counterpart in the reference, which runs one
  * scene per run_transport call).  n_scenes scenes, each with its own source,
  * grid (grids may be NULL: no tallies) and history count, share one table
- * set and run in one persistent launch: warps take chunks of `chunk`
+ * set and run in one persistent launch: warps take chunks of up to `chunk`
  * histories that never span two scenes; history i of scene s draws the
  * Philox stream of history (s << 40) + i.  With slots > 1 (grids created
  * with CC_GRID_STATS) each scene's histories form `slots` batches for the
@@ -344,6 +344,8 @@ int cc_batch_create(cc_ctx* ctx, const cc_tables* tables, int32_t n_scenes, cons
                     int32_t slots, int32_t chunk, cc_batch** out);
 int cc_batch_run(cc_batch* batch, uint64_t seed, int32_t fluorescence, int64_t* scene_counts,
                  cc_run_out* out);
+/* cc_grid_reset of every grid of the batch, in one launch. */
+int cc_batch_reset(cc_batch* batch);
 int cc_batch_destroy(cc_batch* batch);
 
 /* Sample source photons only (tests of source.py parity). */
