@@ -1280,6 +1280,7 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
     static_assert(NQ <= PS_REGIONS_MAX && NQ * RC <= 512, "issue group too large for the tensor memory");
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t full[WS_RING_MAX], empty[WS_RING_MAX], rfull[PS_REGIONS_MAX], rfree[PS_REGIONS_MAX];
+    __shared__ uint64_t wfull;
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
@@ -1306,28 +1307,30 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
             mbar_init(&rfull[r], 1);
             mbar_init(&rfree[r], ps_epi_warps(NO));
         }
+        mbar_init(&wfull, ps_threads(NO) - WS_LOADERS);
         s_fail = 0;
         mbar_init_fence();
     }
     wait_for_previous_kernel();
-    // weights: packed chunk (tap * c8n + c8, co_lo + co) -> (t9 * c8p + c8 - c8_lo, dz * NO + co)
-    // (all threads: as 16-byte copies; 256- and 512-byte bulk copies, issued one by one, took 8 us longer
-    // for 128 input channels)
     const uint32_t sbase = (smem_u32(smem) + 255u) & ~255u, swt = sbase + R * slot16 * 16;
-    for (int i = tid; i < 9 * c8p * NP; i += ps_threads(NO)) {
-        const int r = i % NP, g = i / NP;
-        const int t9 = g / c8p, c8 = Q.c8_lo + g % c8p, dz = r / NO, co = r % NO;
-        const int src = ((dz * 9 + t9) * c8n + c8) * Q.n_out + co_lo + co;
-        cp_async16(swt + (uint32_t)i * 16, P.w + (size_t)src * 8, 16u);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-    fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
+    if (warp < PS_ISSUERS || warp >= PS_EPI_WARP0) {
+        // weights: packed chunk (tap * c8n + c8, co_lo + co) -> (t9 * c8p + c8 - c8_lo, dz * NO + co), by all
+        // threads but the loaders, which start on the planes at once (16-byte copies: 256- and 512-byte bulk
+        // copies, issued one by one, took 8 us longer for 128 input channels)
+        const int wt = warp < PS_ISSUERS ? tid : tid - WS_LOADERS;
+        for (int i = wt; i < 9 * c8p * NP; i += ps_threads(NO) - WS_LOADERS) {
+            const int r = i % NP, g = i / NP;
+            const int t9 = g / c8p, c8 = Q.c8_lo + g % c8p, dz = r / NO, co = r % NO;
+            const int src = ((dz * 9 + t9) * c8n + c8) * Q.n_out + co_lo + co;
+            cp_async16(swt + (uint32_t)i * 16, P.w + (size_t)src * 8, 16u);
+        }
+        cp_async_arrive_noinc(&wfull);
+    }
     if (warp >= PS_ISSUERS && warp < PS_EPI_WARP0) {
         // ---- loaders: planes zs - 1 .. ze of each segment, channel groups of the pass ----
         // The groups of a are tile loads (box {16 channels, 10, 18, 1, 1};
@@ -1416,7 +1419,7 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
         // plane L's ring slot and region with their phases, advanced without divisions
         uint32_t L = 0, fs = 0, fph = 0, rs = 0, rph = 0;
         uint32_t last_r = NQ, last_ph = 0;          // region and phase of the last plane issued
-        bool ok = true;
+        bool ok = warp_wait_or_fail(&wfull, 0u, fail);       // the proxy fence before the first MMA covers it too
         for (; L < (uint32_t)warp; ++L) {
             ring_next(fs, fph, R);
             ring_next(rs, rph, NQ);
@@ -1673,6 +1676,7 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
             base = base.ahead_any((uint32_t)n + 2, NQ);
         }
     }
+    cp_async_wait<0>();
     __syncthreads();
     if (tid == 0 && s_fail) atomicOr(&g_status, 1u);
     tc_fence_after();
