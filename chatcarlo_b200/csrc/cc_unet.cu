@@ -1154,6 +1154,21 @@ __global__ void __launch_bounds__(THREADS, 4) conv_ws_kernel(const ConvP P, int 
 // weights do not fit shared memory run as several passes: every pass but
 // the last adds into an FP32 partial sum [v][NO] (part_out), the last adds
 // the partial (part_in) before bias, ReLU, mask and the BF16 store.
+// PAIR (slices of 16 output channels, even width): the row of a tile is a pair
+// of x-neighbours instead of a voxel, so the halo planes are read for 256
+// voxels by MMAs of the same M, and bound by reading the halo rows (A) from
+// shared memory, the N = 48 MMAs of 16 channels gain most from that.  Seen as
+// pairs, the volume has W / 2 columns of twice the channels, [even voxel's |
+// odd voxel's]; an output plane's region holds [parity][dz][16 channels], and
+// per dy the taps of both parities are four steps over all input channels:
+//   pair x - 1, odd  -> even outputs (dx -1)               N = 48
+//   pair x, even     -> even (dx 0) and odd outputs (-1)   N = 96
+//   pair x, odd      -> even (dx +1) and odd outputs (0)   N = 96
+//   pair x + 1, even -> odd outputs (dx +1)                N = 48
+// so each output meets its taps and channels in the order of the kernel
+// without pairs (the sums are the same), at 13 MMAs (656 cycles) per 256
+// voxels and 16 input channels instead of 18 (842).  The upsampled input is the
+// same for both voxels of a pair and is held once.
 // PLAIN: no mask, partial sums, head or second output (a forward layer in
 // one pass): the epilogue without their tests.
 // Output slices: CTA row blockIdx.y computes output channels [co_lo, co_lo +
@@ -1187,6 +1202,12 @@ __host__ __device__ constexpr uint32_t ps_tmem_cols(int n, int g) {
 __host__ __device__ constexpr uint32_t ps_weight_bytes(int n, int c8p) { return 9u * (uint32_t)c8p * 3u * n * 16u; }
 __host__ __device__ constexpr uint32_t ps_smem_bytes(int n, int c8p, int ring) {
     return (uint32_t)ring * (uint32_t)(c8p / 2) * PS_GROUP_BYTES + ps_weight_bytes(n, c8p) + 256;   // 256: alignment
+}
+// PAIR: rows of the weight blocks of one dy and 16 input channels, in step order
+constexpr int PAIR_ROWS = 48 + 96 + 96 + 48;
+// a and b in groups of 16 channels; a's are held for both voxels of a pair
+__host__ __device__ constexpr uint32_t pair_smem_bytes(int a16, int b16, int ring) {
+    return (uint32_t)ring * (uint32_t)(2 * a16 + b16) * PS_GROUP_BYTES + 3u * (uint32_t)(a16 + b16) * PAIR_ROWS * 32u + 256;
 }
 
 // next index of a ring of n entries, flipping the phase bit on wrap-around
@@ -1272,11 +1293,12 @@ __device__ __forceinline__ void ps_release(uint64_t* rfree, uint32_t ra, uint32_
         : "memory");
 }
 
-template <int NO, int G, int C8P, bool PLAIN>
+template <int NO, int G, int C8P, bool PLAIN, bool PAIR = false>
 __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8 ? 2 : 1) conv_ps_kernel(const __grid_constant__ CUtensorMap amap, const ConvP P, const PsPass Q, int ring) {
     constexpr int NP = 3 * NO;                                // MMA N: the three dz weight planes
     constexpr uint32_t RC = ps_region_cols(NO);
     constexpr uint32_t NQ = (uint32_t)ps_regions(G), TCOLS = ps_tmem_cols(NO, G);
+    static_assert(!PAIR || (NO == 32 && G == 1 && C8P > 0), "pairs of 16 output channels each");
     static_assert(NQ <= PS_REGIONS_MAX && NQ * RC <= 512, "issue group too large for the tensor memory");
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t full[WS_RING_MAX], empty[WS_RING_MAX], rfull[PS_REGIONS_MAX], rfree[PS_REGIONS_MAX];
@@ -1288,12 +1310,12 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
     const int c8n = (S.ca + S.cb) / 8, c8p = C8P > 0 ? C8P : Q.c8_hi - Q.c8_lo;
     const uint32_t R = (uint32_t)ring;
     constexpr uint32_t GROUP16 = PS_GROUP_BYTES / 16;         // one 16-channel group, 16-byte units
-    const uint32_t slot16 = (uint32_t)(c8p / 2) * GROUP16;    // one ring slot
-    // 16-channel groups of the pass from a (tile loads) and from b (gathered)
-    const int na = max(0, min(Q.c8_hi, S.ca / 8) - Q.c8_lo) / 2, nb = c8p / 2 - na;
+    // 16-channel groups of the pass from a (tile loads; of both voxels of a pair) and from b (gathered)
+    const int na = PAIR ? S.ca / 8 : max(0, min(Q.c8_hi, S.ca / 8) - Q.c8_lo) / 2, nb = PAIR ? S.cb / 16 : c8p / 2 - na;
+    const uint32_t slot16 = (uint32_t)(na + nb) * GROUP16;    // one ring slot
     volatile int* fail = &s_fail;
     // this CTA's output slice and its partial sums
-    const int co_lo = Q.co_lo + (int)blockIdx.y * NO;
+    const int co_lo = Q.co_lo + (PAIR ? 0 : (int)blockIdx.y * NO);
     const float* part_in = Q.part_in ? Q.part_in + (size_t)blockIdx.y * P.n_vox * NO : nullptr;
     float* part_out = Q.part_out ? Q.part_out + (size_t)blockIdx.y * P.n_vox * NO : nullptr;
 
@@ -1323,6 +1345,22 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
         // threads but the loaders, which start on the planes at once (16-byte copies: 256- and 512-byte bulk
         // copies, issued one by one, took 8 us longer for 128 input channels)
         const int wt = warp < PS_ISSUERS ? tid : tid - WS_LOADERS;
+        if (PAIR) {
+            // block (dy, step, 16-channel group): [K half][row], rows (parity, dz, co) as described above
+            for (int i = wt; i < 3 * (C8P / 2) * PAIR_ROWS * 2; i += ps_threads(NO) - WS_LOADERS) {
+                const int dy = i / (C8P * PAIR_ROWS);
+                int r = i - dy * (C8P * PAIR_ROWS);
+                const int st = r < C8P * 48 ? 0 : (r < C8P * 144 ? 1 : (r < C8P * 240 ? 2 : 3));
+                r -= C8P * (st == 0 ? 0 : (st == 1 ? 48 : (st == 2 ? 144 : 240)));
+                const int rows = st == 0 || st == 3 ? 48 : 96, g = r / (2 * rows);
+                r -= g * 2 * rows;
+                const int kh = r / rows, row = r - kh * rows;
+                const int odd = st == 0 ? 0 : (st == 3 ? 1 : (row >= 48)), dz = row % 48 / 16, co = row % 16;
+                const int dx = st - odd;                       // step st is tap dx = st of even outputs, st - 1 of odd ones
+                const int src = ((dz * 9 + dy * 3 + dx) * c8n + 2 * g + kh) * Q.n_out + co_lo + co;
+                cp_async16(swt + (uint32_t)i * 16, P.w + (size_t)src * 8, 16u);
+            }
+        } else
         for (int i = wt; i < 9 * c8p * NP; i += ps_threads(NO) - WS_LOADERS) {
             const int r = i % NP, g = i / NP;
             const int t9 = g / c8p, c8 = Q.c8_lo + g % c8p, dz = r / NO, co = r % NO;
@@ -1345,8 +1383,9 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
         // its own copies: as many planes are in flight as the ring has slots.
         const int lt = tid - 32 * PS_ISSUERS, half = lt & 1;
         const bool tiles = na > 0 && warp == PS_ISSUERS;
-        const int ch_b = (Q.c8_lo + 2 * na + half) * 8 - S.ca;
-        const long long step_b = (long long)(S.H >> 1) * (S.W >> 1) * S.cb;       // elements of a plane of b
+        const int ch_b = PAIR ? half * 8 : (Q.c8_lo + 2 * na + half) * 8 - S.ca;
+        const int wb = PAIR ? S.W : S.W >> 1;                                    // a pair is one voxel of b
+        const long long step_b = (long long)(S.H >> 1) * wb * S.cb;             // elements of a plane of b
         uint32_t L = 0, slot = 0, ph = 0;             // plane, its ring slot and the slot's phase
         PsWalk walk(S);
         bool ok = tiles || nb > 0;
@@ -1362,7 +1401,7 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
                     const bool in = (unsigned)yy < (unsigned)S.H && (unsigned)xx < (unsigned)S.W;
                     bytes[j] = in ? 16u : 0u;
                     pb[j] = S.b + ((long long)q.n * (S.D >> 1) + ((q.zs - 1) >> 1)) * step_b +
-                            (in ? ((long long)(yy >> 1) * (S.W >> 1) + (xx >> 1)) * S.cb : 0) + ch_b;
+                            (in ? ((long long)(yy >> 1) * wb + (PAIR ? xx : xx >> 1)) * S.cb : 0) + ch_b;
                 }
             }
             for (int zz = q.zs - 1; zz <= q.ze; ++zz, ++L, ring_next(slot, ph, R)) {
@@ -1373,8 +1412,9 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
                     if (elect_one()) {
                         mbar_arrive_expect_tx(&full[slot], (uint32_t)(na * PS_ROWS_BYTES));
                         for (int c = 0; c < na; ++c)
-                            tma_load_5d(dst0 + (uint32_t)(c * PS_GROUP_BYTES), &amap, &full[slot], Q.c8_lo * 8 + 16 * c,
-                                        q.x0 - 1, q.y0 - 1, zz, q.n);
+                            tma_load_5d(dst0 + (uint32_t)(c * PS_GROUP_BYTES), &amap, &full[slot],
+                                        PAIR ? (c & 1) * S.ca + (c >> 1) * 16 : Q.c8_lo * 8 + 16 * c, q.x0 - 1, q.y0 - 1, zz,
+                                        q.n);
                     }
                     __syncwarp();
                 }
@@ -1446,7 +1486,45 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
             if (!ok) break;
             fence_proxy_async();              // the loaders' copies, seen through the barrier, to the tensor core
             tc_fence_after();
-            if (G == 1 && C8P > 0) {
+            if constexpr (PAIR) {
+                if (elect_one()) {
+                    constexpr uint32_t ID48 = idesc_bf16(TILE_M, 48, 0, 0), ID96 = idesc_bf16(TILE_M, 96, 0, 0);
+                    const uint32_t ah = (uint32_t)(a0 >> 32), al0 = (uint32_t)a0 + so[0];
+                    const uint32_t b48h = (uint32_t)(smem_desc(0, 48 * 16, 128) >> 32);
+                    const uint32_t b48 = (uint32_t)smem_desc(swt, 48 * 16, 128), b96 = (uint32_t)smem_desc(swt, 96 * 16, 128);
+                    const uint32_t even = d[0], odd = d[0] + 48;
+#pragma unroll
+                    for (int dy = 0; dy < 3; ++dy) {
+                        // the block of a step's first group, 16-byte units
+                        uint32_t wo = (uint32_t)(dy * C8P * PAIR_ROWS);
+                        asm volatile("" : "+r"(wo));           // constants of all MMAs kept across planes would spill
+#pragma unroll
+                        for (int st = 0; st < 4; ++st) {
+                            const int rows = st == 0 || st == 3 ? 48 : 96, first = st == 0 ? 0 : (st == 1 ? 48 : (st == 2 ? 144 : 240));
+                            const int ox = st == 0 ? 0 : (st == 3 ? 2 : 1), par = st == 0 || st == 2;   // pair offset + 1, voxel of the pair
+#pragma unroll
+                            for (int g = 0; g < C8P / 2; ++g) {
+                                const uint32_t grp = 2 * g < na ? (uint32_t)(2 * g + par) : (uint32_t)(na + g) - (uint32_t)(na / 2);
+                                const uint32_t aw = al0 + grp * GROUP16 + (uint32_t)((dy * HALO_X + ox) * 2);
+                                const uint32_t w0 = wo + (uint32_t)(C8P * first + g * 2 * rows);
+                                if (st == 0) {
+                                    mma_bf16_lo(even, aw, ah, b48 + w0, b48h, ID48, dy > 0 || g > 0 ? 1u : 0u);
+                                } else if (st == 3) {
+                                    mma_bf16_lo(odd, aw, ah, b48 + w0, b48h, ID48, 1u);
+                                } else if (dy == 0 && st == 1 && g == 0) {
+                                    // the odd outputs' first step
+                                    mma_bf16_lo(even, aw, ah, b96 + w0, b48h, ID48, 1u);
+                                    mma_bf16_lo(odd, aw, ah, b96 + w0 + 48, b48h, ID48, 0u);
+                                } else {
+                                    mma_bf16_lo(even, aw, ah, b96 + w0, b48h, ID96, 1u);
+                                }
+                            }
+                        }
+                    }
+                    mma_commit(&rfull[rsk[0]]);
+                    mma_commit(&empty[fsk[0]]);
+                }
+            } else if (G == 1 && C8P > 0) {
                 // every tap and channel group at a constant offset: no address arithmetic between the MMAs
                 if (elect_one()) {
                     const uint32_t al = (uint32_t)a0 + so[0], bl = (uint32_t)b0;
@@ -1531,8 +1609,10 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
         const uint32_t lq = (uint32_t)(qw * 32) << 16;
         const bool heads = !PLAIN && NO == 16 && head_p != nullptr;
         const bool masked = !PLAIN && mask0 && !part_out && !heads;
-        const int c0 = half * CW, co0 = co_lo + c0;
-        const uint32_t plane = (uint32_t)(S.H * S.W);
+        const int c0 = PAIR ? 0 : half * CW, co0 = co_lo + c0;        // PAIR: half is the voxel of the pair
+        // the warp's first column of a region's three dz parts
+        const uint32_t col_m = lq + (uint32_t)(PAIR ? 48 * half : c0), col_0 = col_m + (PAIR ? 16 : NO), col_p = col_0 + (PAIR ? 16 : NO);
+        const uint32_t plane = (uint32_t)(S.H * S.W) * (PAIR ? 2u : 1u);
         float2 bias[CW / 2];
         if (bias_p && (PLAIN || !part_out)) {
 #pragma unroll
@@ -1547,6 +1627,7 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
             const int y = q.y0 + (m >> 3), x = q.x0 + (m & 7), n = q.ze - q.zs;
             const bool in = y < S.H && x < S.W;
             uint32_t v = (uint32_t)((((long long)q.n * S.D + q.zs + own) * S.H + y) * S.W + x);
+            if (PAIR) v = 2 * v + (uint32_t)half;
             uint4 mk[CW / 8];
             float4 part[CW / 4];
             auto read_ahead = [&](uint32_t u) {
@@ -1578,9 +1659,9 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
                 auto sums = [&](auto cn, int c, bool release, float2* f) {
                     constexpr int CN = decltype(cn)::value;
                     uint32_t um[CN], u0[CN], up[CN];
-                    tmem_ld_nw<CN>(tmem + rm.r * RC + lq + (uint32_t)c, um);
-                    tmem_ld_nw<CN>(tmem + r0.r * RC + NO + lq + (uint32_t)c, u0);
-                    tmem_ld_nw<CN>(tmem + rp.r * RC + 2 * NO + lq + (uint32_t)c, up);
+                    tmem_ld_nw<CN>(tmem + rm.r * RC + col_m + (uint32_t)c, um);
+                    tmem_ld_nw<CN>(tmem + r0.r * RC + col_0 + (uint32_t)c, u0);
+                    tmem_ld_nw<CN>(tmem + rp.r * RC + col_p + (uint32_t)c, up);
                     tmem_wait_ld();
                     // the uses below stay behind the wait
 #pragma unroll
@@ -1602,7 +1683,7 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
                         for (int c = 0; c < NO; c += 8) {
                             float2 f[4];
                             float t[8];
-                            sums(PsInt<8>{}, c, c + 8 == NO, f);
+                            sums(PsInt<8>{}, c - c0, c + 8 == NO, f);
                             if (in) {
 #pragma unroll
                                 for (int j = 0; j < 4; ++j) t[2 * j] = f[j].x, t[2 * j + 1] = f[j].y;
@@ -1622,7 +1703,7 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
                 }
                 float2 f[CW / 2];
 #pragma unroll
-                for (int c = 0; c < CW; c += 8) sums(PsInt<8>{}, c0 + c, c + 8 == CW, f + c / 2);
+                for (int c = 0; c < CW; c += 8) sums(PsInt<8>{}, c, c + 8 == CW, f + c / 2);
                 if (!PLAIN && part_rd) {
 #pragma unroll
                     for (int j = 0; j < CW / 4; ++j) {
@@ -1642,6 +1723,9 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
 #pragma unroll
                         for (int j = 0; j < CW / 2; ++j) f[j] = add2(f[j], bias[j]);
                     }
+                    // PAIR with the head: all 16 channels of the voxel are here
+                    const bool pair_head = PAIR && !PLAIN && head_p != nullptr;
+                    float hsum = pair_head && in ? head_x[v] + __ldg(head_p + 16) : 0.0f;
 #pragma unroll
                     for (int h = 0; h < CW / 8; ++h) {
                         // output channels [co, co + 8) go to out0 or out1 (split is a multiple of 8)
@@ -1662,8 +1746,14 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
                         }
                         __nv_bfloat16* o = first ? P.out0 + ((size_t)v * P.split + co)
                                                  : P.out1 + ((size_t)v * (Q.n_out - P.split) + (co - P.split));
-                        if (in) *reinterpret_cast<uint4*>(o) = pack_bf16x8(t);
+                        if (in && !(pair_head && !P.out0)) *reinterpret_cast<uint4*>(o) = pack_bf16x8(t);
+                        if (pair_head) {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                hsum = fmaf(__ldg(head_p + 8 * h + j), __bfloat162float(__float2bfloat16_rn(t[j])), hsum);
+                        }
                     }
+                    if (pair_head && in) P.head_out[v] = hsum;
                 }
                 if (!PLAIN && in && i + step < n) read_ahead(v + step * plane);
             }
@@ -2733,6 +2823,70 @@ int volume_map(CUtensorMap* m, const void* base, int c, int batch, int d, int h,
     return CCU_OK;
 }
 
+// Whether a slice of 16 output channels runs on pairs of voxels: an even width;
+// 32 or 48 input channels (16 -> 16 on 320x320x152 took 228 us without pairs and
+// 261 with, its MMAs too few to cover a plane's handovers with one CTA per SM;
+// beyond 48 weights and ring do not fit); tiles of 16 voxels along x that waste
+// less than pairs gain (W = 24 would pad to 32); and planes enough per SM that
+// the gain passes the larger weights' load (us without pairs and with:
+//   48 channels: 8 x 32^3, 7 planes per SM, 20.4, 20.9; 4 x 48^3, 12 planes, 27.3,
+//     26.2; 4 x 64^3, 28 planes, 50.8, 44.0; 320x320x152 706, 550
+//   32 channels: 2 x 64^3, 14 planes, 21.9, 22.7; 3 x 64^3, 21 planes, 28.5, 28.9
+//     and with a mask 33.9, 30.3; 4 x 64^3 35.2, 34.3 and 41.3, 36.1).
+bool pair_applies(const ConvP& P, int sms) {
+    const int c16 = (P.src.ca + P.src.cb) / 16, w = P.src.W;
+    const long long planes = (long long)P.src.B * P.src.D * ((P.src.H + 15) / 16) * ((w + 15) / 16);
+    return g_conv_group == 0 && w % 2 == 0 && (c16 == 2 || c16 == 3) && (w + 15) / 16 * 16 * 5 <= (w + 7) / 8 * 8 * 6 &&
+           planes >= (long long)sms * (c16 == 3 ? 10 : 20);
+}
+
+template <int C8P, bool PLAIN>
+int launch_conv_pair_g(const ConvP& P, int n_out, int co_lo, cudaStream_t st) {
+    const int a16 = P.src.ca / 16, b16 = P.src.cb / 16;
+    ConvP V = P;
+    V.src.W = P.src.W / 2;
+    CUtensorMap amap;                            // the volume in pairs: twice the channels, half the width
+    int rc = volume_map(&amap, P.src.a, 2 * P.src.ca, P.src.B, P.src.D, P.src.H, V.src.W, 16, HALO_X, HALO_Y);
+    if (rc != CCU_OK) return rc;
+    const auto kernel = conv_ps_kernel<32, 1, C8P, PLAIN, true>;
+    static PlanCache caches[C8P / 2];            // by the groups of b
+    LaunchPlan plan;
+    rc = device_plan(&caches[b16], plan, [&](int dev, LaunchPlan& p) {
+        CU_CHECK(cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev));
+        p.ring = 2;
+        while (p.ring < WS_RING_MAX && pair_smem_bytes(a16, b16, p.ring + 1) <= PS_SMEM_MAX) ++p.ring;
+        const int r_c = tc_launch_smem(kernel, pair_smem_bytes(a16, b16, p.ring), ps_tmem_cols(32, 1), p.smem, ps_threads(32));
+        // one kernel serves several splits into a and b, each with its own ring: allow it the largest
+        CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS_SMEM_MAX));
+        return r_c == CCU_OK ? resident_ctas(kernel, p.smem, ps_tmem_cols(32, 1), p.resident, ps_threads(32)) : r_c;
+    });
+    if (rc != CCU_OK) return rc;
+    PsPass Q;
+    Q.co_lo = co_lo;
+    Q.n_out = n_out;
+    Q.c8_lo = 0;
+    Q.c8_hi = C8P;
+    Q.part_in = nullptr;
+    Q.part_out = nullptr;
+    const long long planes = (long long)V.src.B * ((V.src.H + 15) / 16) * ((V.src.W + 7) / 8) * V.src.D;
+    const long long grid = std::min<long long>(planes, (long long)plan.sms * plan.resident);
+    return launch_dependent(kernel, dim3((unsigned)grid), ps_threads(32), plan.smem, st, amap, V, Q, plan.ring);
+}
+
+template <int C8P>
+int launch_conv_pair_c(const ConvP& P, int n_out, int co_lo, cudaStream_t st) {
+    if (!P.mask0 && !P.head && P.out0 && co_lo + 16 <= P.split) return launch_conv_pair_g<C8P, true>(P, n_out, co_lo, st);
+    return launch_conv_pair_g<C8P, false>(P, n_out, co_lo, st);
+}
+
+// Output channels [co_lo, co_lo + 16) on pairs of voxels.
+int launch_conv_pair(const ConvP& P, int n_out, int co_lo, cudaStream_t st) {
+    switch ((P.src.ca + P.src.cb) / 16) {
+        case 2: return launch_conv_pair_c<4>(P, n_out, co_lo, st);
+        default: return launch_conv_pair_c<6>(P, n_out, co_lo, st);
+    }
+}
+
 // One launch: the pass's channel groups and `slices` output slices.
 template <int NO, int G, int C8P, bool PLAIN = false>
 int launch_conv_ps_pass(const CUtensorMap& amap, const ConvP& P, const PsPass& Q, int slices, long long planes,
@@ -2806,8 +2960,17 @@ int launch_conv_ps_g(const CUtensorMap& amap, const ConvP& P, int n_out, int co_
 // than three interleaved chains on one CTA), whose regions must fit 512
 // tensor-memory columns; the others take 1.
 int launch_conv_ps(const ConvP& P, int n_out, const PsPlan& plan, cudaStream_t st) {
+    static PlanCache cache;
+    LaunchPlan device;
+    int rc = device_plan(&cache, device, [](int dev, LaunchPlan& p) {
+        CU_CHECK(cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev));
+        return CCU_OK;
+    });
+    if (rc != CCU_OK) return rc;
+    const bool pairs = n_out % 32 == 16 && pair_applies(P, device.sms);
+    if (n_out == 16 && pairs) return launch_conv_pair(P, n_out, 0, st);
     CUtensorMap amap;
-    int rc = volume_map(&amap, P.src.a, P.src.ca, P.src.B, P.src.D, P.src.H, P.src.W, 16, HALO_X, HALO_Y);
+    rc = volume_map(&amap, P.src.a, P.src.ca, P.src.B, P.src.D, P.src.H, P.src.W, 16, HALO_X, HALO_Y);
     if (rc != CCU_OK) return rc;
     if (plan.no == 16) {
         if (n_out == 16 && g_conv_group == 3) return launch_conv_ps_g<16, 3>(amap, P, n_out, 0, 1, plan.passes, st);
@@ -2815,6 +2978,7 @@ int launch_conv_ps(const ConvP& P, int n_out, const PsPlan& plan, cudaStream_t s
         return launch_conv_ps_g<16, 1>(amap, P, n_out, 0, n_out / 16, plan.passes, st);
     }
     rc = launch_conv_ps_g<32, 1>(amap, P, n_out, 0, n_out / 32, plan.passes, st);
+    if (rc == CCU_OK && pairs) return launch_conv_pair(P, n_out, n_out / 32 * 32, st);
     if (rc == CCU_OK && n_out % 32)
         rc = launch_conv_ps_g<16, 1>(amap, P, n_out, n_out / 32 * 32, 1, plan.passes, st);
     return rc;

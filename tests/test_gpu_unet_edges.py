@@ -106,3 +106,45 @@ def test_bias_gradient_widths(U, c, n, offset):
     torch.cuda.synchronize()
     ref, mag = 1.0 + dz.double().sum(0), 1.0 + dz.double().abs().sum(0)
     assert bool(((db.double() - ref).abs() <= (n + 1) * 2.0 ** -24 * mag).all())
+
+
+@pytest.mark.parametrize("ca,cb,dims", [
+    (32, 0, (1, 1, 1, 16)), (32, 0, (2, 90, 37, 94)), (32, 0, (1, 3000, 1, 16)), (48, 0, (2, 62, 37, 94)),
+    (48, 0, (1, 380, 33, 30)), (16, 32, (2, 62, 38, 94)), (32, 16, (1, 380, 34, 32)), (48, 0, (1, 600, 33, 24)),
+])
+def test_sixteen_channels_on_pairs_of_voxels(U, ca, cb, dims):
+    """The kernel on pairs sums the same products in the same order as the one
+    without (an issue group set by hand keeps it off), so the values are equal."""
+    g = torch.Generator(device="cuda").manual_seed(ca + cb + dims[3])
+    n = dims[0] * dims[1] * dims[2] * dims[3]
+    a = torch.randn(n, ca, generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(n // 8, cb, generator=g, device="cuda").to(torch.bfloat16) if cb else None
+    w32 = torch.randn(27, 16, ca + cb, generator=g, device="cuda") * 0.1
+    w = torch.empty(U.lib().ccu_packed_weight_elems(16, ca + cb), dtype=torch.bfloat16, device="cuda")
+    bias = torch.randn(16, generator=g, device="cuda")
+    mask = torch.randn(n, 16, generator=g, device="cuda").to(torch.bfloat16)
+    head, x = torch.randn(17, generator=g, device="cuda"), torch.randn(n, generator=g, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    U.check(U.lib().ccu_pack_weights(w32.data_ptr(), 16, ca + cb, w.data_ptr(), None, st))
+    got = []
+    try:
+        for group in (0, 1):
+            U.check(U.lib().ccu_set_conv_group(group))
+            outs = []
+            for m, relu in ((None, 1), (mask.data_ptr(), 0)):
+                o = torch.empty(n, 16, dtype=torch.bfloat16, device="cuda")
+                U.check(U.lib().ccu_conv3d(a.data_ptr(), ca, b.data_ptr() if cb else None, cb, *dims, w.data_ptr(),
+                                           bias.data_ptr(), 16, relu, o.data_ptr(), 16, m, None, st))
+                outs.append(o)
+            if cb == 0:
+                h = torch.empty(n, device="cuda")
+                U.check(U.lib().ccu_conv3d_head(a.data_ptr(), ca, *dims, w.data_ptr(), bias.data_ptr(), head.data_ptr(),
+                                                x.data_ptr(), h.data_ptr(), None, 0, st))
+                outs.append(h)
+            got.append(outs)
+    finally:
+        U.check(U.lib().ccu_set_conv_group(0))
+    torch.cuda.synchronize()
+    assert U.status() == 0
+    for p, q in zip(*got):
+        assert torch.equal(p, q)
