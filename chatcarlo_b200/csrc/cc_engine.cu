@@ -879,11 +879,10 @@ __device__ __forceinline__ void sample_source(const KSource& S, RNG& rng, real p
 // 0.39 / 1.87 / 6.4 with 16, 0.39 / 1.78 / 6.4 with 32 (whose copies cost the
 // fold of small runs more); chunks of 256 consecutive histories per warp, the
 // order before, 1.26 / 2.26 / 6.8, with most warps idle in small runs.
-// A grid whose slot is near the L2 size wants the opposite, one batch after
-// the other, or its reductions miss in L2.
+// Where the beam is wide and the slots are large, fewer at once (SlotOrder).
 constexpr int HIST_UNIT = 32;
 constexpr int SPREAD_SLOTS = 16;
-constexpr size_t SLOT_BYTES_COMPACT = (size_t)32 << 20;     // slots above this are scored one after the other
+constexpr size_t SLOT_BYTES_COMPACT = (size_t)32 << 20;     // slots above this are large (SlotOrder)
 // Voxel visits per piece when a warp splits its track segments.  The split
 // of a segment depends on that segment alone, never on the warp's other
 // lanes, so every piece -- and every length it scores -- is the same
@@ -2884,15 +2883,87 @@ static int status_to_error(unsigned st) {
     return CC_OK;
 }
 
-// Blocks per SM of a launch whose grid's scratch slot exceeds
-// SLOT_BYTES_COMPACT, unless the context sets its own: fewer histories in
-// flight span fewer batch slots, whose scattered reductions then hit L2
-// more often.  Measured on the CT workload (246 MB slots, batches of
-// 200,000 histories): 2.89e8 histories/s with 1 block of 256 per SM, 2.68e8
-// with 2, 2.52e8 with 3, 2.46e8 with 4.
-constexpr int BIG_GRID_BLOCKS_PER_SM = 1;
+// How a launch's histories meet the scratch slots of its batches (see
+// HIST_UNIT).  Reductions on one address follow one another (4 ns each), so
+// histories that all cross the same few voxels want several slots at a time;
+// a beam that is spread over many voxels wants the slots in use to stay in L2.
+struct SlotOrder {
+    int group = SPREAD_SLOTS;     // batches scored at a time
+    bool copies = false;          // a launch of fewer scores copies of their slots
+    bool one_block = false;       // one block per SM: fewer histories, and so slots, in flight
+    bool lockstep = false;
+};
 
-static int grid_blocks_for(cc_ctx* c, size_t smem, bool fs, bool tl, bool big_grid) {
+// Voxel faces across the beam where it may first meet the grid: those of its
+// field at the least distance between the source (at any angle) and the grid.
+static double beam_faces(const KSource& S, const cc_grid* g) {
+    const double h = 1.0 / (double)g->k.inv_h;
+    const int n[3] = {g->k.nx, g->k.ny, g->k.nz};
+    if (S.field == CC_FIELD_PARALLEL) return (double)S.su * (double)S.sv / (h * h);
+    double near2 = 0, far2 = 0, r2 = 0;
+    for (int k = 0; k < 3; ++k) {
+        const double lo = g->origin64[k], hi = lo + n[k] * h, x = (double)S.pos[k], c = (double)S.iso[k];
+        const double out = std::max(0.0, std::max(lo - x, x - hi)), corner = std::max(std::abs(lo - c), std::abs(hi - c));
+        near2 += out * out;
+        far2 += corner * corner;
+        r2 += (x - c) * (x - c);
+    }
+    // a rotating source stays on a ring about the isocentre, moved along its axis by half the scan at most
+    const double dist = S.rotation ? std::max(0.0, std::sqrt(r2) - std::sqrt(far2) - 0.5 * (double)S.scan) : std::sqrt(near2);
+    if (S.field == CC_FIELD_CONE) {
+        const double c = (double)S.cos_half, t2 = c > 0.0 ? (1.0 - c * c) / (c * c) : 1.0;
+        return 3.14159265358979 * t2 * dist * dist / (h * h);
+    }
+    const double m = dist / std::max((double)S.sid, 1e-6);
+    return (double)S.su * m * (double)S.sv * m / (h * h);
+}
+
+// Beams of fewer voxel faces than NARROW_FACES score SPREAD_SLOTS slots at a
+// time whatever their size, the others as many as GROUP_BYTES hold, and with
+// slots above SLOT_BYTES_COMPACT one block per SM once those that the
+// histories of four (FULL_HISTORIES) reach exceed LIVE_BYTES.  Device time of
+// 1.4e6 histories in batches of 200,000 (ms; 1, 2, 4, 8 slots at a time with
+// four blocks per SM, and 1 slot with one block):
+//   room, source in the grid, slot  47 MB  9.4  7.8  6.4  5.5 | 10.0
+//                                  218 MB 33.2 26.8 19.2 13.6 | 33.3
+//   pencil beam, slot               34 MB  9.4  7.2  5.5  5.0 | 10.4
+//   CT fan, slot                    15 MB  1.15      1.18 1.20 | 2.03
+//                                   24 MB  1.27 1.30 1.42 2.05 | 2.16
+//                                   40 MB  1.73 1.92 2.30 2.90 | 2.30
+//                                   70 MB  2.81 3.03           | 2.54
+//                                  246 MB  5.90 6.07           | 5.05
+//   cone on a phantom, slot         19 MB  1.56 1.57 1.64 2.05 | 2.28 (2 slots)
+//                                   37 MB  2.12 2.37 3.06 4.53 | 2.51
+//                                   87 MB  4.84 5.56 6.80 7.97 | 3.39
+// Square parallel beams of 0.8 and 1.6 cm on a grid of 0.2 cm (16 and 64 faces):
+// 3.9 and 3.8 ms as narrow ones, 4.5 and 3.0 as wide ones.  Copies are worth
+// their fold up to some 16 KB per history (room, slots of 47 MB, 1, 2, 4, 8, 16
+// copies: 5000 histories 0.27 0.28 0.31 0.36 0.45 ms, 200,000 1.68 1.29 1.09
+// 1.04 1.10).  Photons of the caller have one slot; their beam is not known.
+constexpr double NARROW_FACES = 32;
+constexpr size_t GROUP_BYTES = (size_t)64 << 20, LIVE_BYTES = (size_t)96 << 20;
+constexpr double COPY_BYTES_PER_HISTORY = 16384;
+constexpr double FULL_HISTORIES = 4 * 148 * BLOCK;
+
+static SlotOrder slot_order(const KSource* src, const cc_grid* grid, long long batch_size) {
+    SlotOrder O;
+    if (!grid) return O;
+    const size_t per = (size_t)grid->k.nvox * 16;
+    const bool large = per > SLOT_BYTES_COMPACT;
+    if (!src) {
+        O.one_block = large;
+        O.lockstep = !large;
+    } else if (beam_faces(*src, grid) < NARROW_FACES) {
+        O.copies = O.lockstep = true;
+    } else {
+        O.group = (int)std::max<size_t>(1, std::min<size_t>(SPREAD_SLOTS, GROUP_BYTES / per));
+        O.one_block = large && (double)per * (1.0 + FULL_HISTORIES / (double)batch_size) > (double)LIVE_BYTES;
+        O.lockstep = !large;
+    }
+    return O;
+}
+
+static int grid_blocks_for(cc_ctx* c, size_t smem, bool fs, bool tl, bool one_block) {
     int per_sm = c->blocks_per_sm;
     if (per_sm == 0) {
         int occ = 0;
@@ -2906,7 +2977,7 @@ static int grid_blocks_for(cc_ctx* c, size_t smem, bool fs, bool tl, bool big_gr
         else if (tl) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<false, true>, c->block, smem);
         else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<false, false>, c->block, smem);
         if (e != cudaSuccess || occ < 1) occ = 1;
-        per_sm = big_grid ? std::min(occ, BIG_GRID_BLOCKS_PER_SM) : occ;
+        per_sm = one_block ? 1 : occ;
     }
     return c->sm_count * per_sm;
 }
@@ -2941,8 +3012,8 @@ static int enqueue_launch(cc_ctx* c, const cc_scene* scene, const cc_tables* tab
     const KTables& T = tables->k;
     R.n_scratch = n_slots;
     R.batch_size = batch_size;
-    const bool big_grid = grid && (size_t)grid->k.nvox * 16 > SLOT_BYTES_COMPACT;
-    R.group = big_grid ? 1 : SPREAD_SLOTS;
+    const SlotOrder order = slot_order(src, grid, batch_size);
+    R.group = order.group;
     R.copy_shift = copy_shift;
     R.max_steps = c->max_steps;
     R.status = c->d_status;
@@ -2964,8 +3035,8 @@ static int enqueue_launch(cc_ctx* c, const cc_scene* scene, const cc_tables* tab
     bool fs = src != nullptr;
     if (fs) S = *src;
     size_t smem = n_acc * sizeof(double) + RNG_BYTES + (tl && !c->tally_queue ? SegQueue<SegRec>::bytes(c->block) : 0);
-    int blocks = grid_blocks_for(c, smem, fs, tl, big_grid);
-    R.lockstep = tl && !big_grid && R.n >= (long long)LOCKSTEP_PER_LANE * blocks * c->block ? 1 : 0;
+    int blocks = grid_blocks_for(c, smem, fs, tl, order.one_block);
+    R.lockstep = tl && order.lockstep && R.n >= (long long)LOCKSTEP_PER_LANE * blocks * c->block ? 1 : 0;
     const bool defer = tl && c->tally_queue;
     R.defer = defer ? 1 : 0;
     if (defer) {
@@ -3274,13 +3345,18 @@ int cc_run(cc_ctx* c, const cc_scene* scene, const cc_tables* tables, const cc_s
     // statistics need that, and FP32 cells must not sum more than a batch)
     const bool slotted = grid != nullptr;
     const int cell32 = slotted ? cell32_for(c, batch_size) : 0;
+    const SlotOrder order = slot_order(&src->k, grid, batch_size);
     if (grid) {
         size_t per = (size_t)grid->k.nvox * 2 * sizeof(double);
         size_t budget = (size_t)8 << 30;
         slots = (int)std::max<size_t>(1, std::min<size_t>(slots, budget / per));
         // slots of all batches of a launch, and of the copies of a launch of few
-        const bool spread = per <= SLOT_BYTES_COMPACT;
-        int rc = grid_alloc_scratch(grid, spread ? std::max(slots, (int)std::min<size_t>(SPREAD_SLOTS, budget / per)) : slots);
+        const int spread = order.copies && per <= SLOT_BYTES_COMPACT ? std::max(slots, (int)std::min<size_t>(SPREAD_SLOTS, budget / per)) : slots;
+        int rc = grid_alloc_scratch(grid, spread);
+        if (rc == CC_E_DEVICE && spread > slots) {      // no room for the copies
+            cudaGetLastError();
+            rc = grid_alloc_scratch(grid, slots);
+        }
         if (rc != CC_OK) return rc;
     }
     long long done = 0;
@@ -3329,8 +3405,10 @@ int cc_run(cc_ctx* c, const cc_scene* scene, const cc_tables* tables, const cc_s
         long long n_launch = std::min<long long>(n_hist - done, (long long)ns * batch_size);
         ns = (int)((n_launch + batch_size - 1) / batch_size);
         int copy_shift = 0;
-        if (grid && (size_t)grid->k.nvox * 16 <= SLOT_BYTES_COMPACT)
-            while ((ns << (copy_shift + 1)) <= std::min(+SPREAD_SLOTS, grid->n_scratch)) ++copy_shift;
+        if (order.copies)
+            while ((ns << (copy_shift + 1)) <= std::min(+SPREAD_SLOTS, grid->n_scratch) &&
+                   (double)grid->k.nvox * 16 * (ns << (copy_shift + 1)) <= (double)n_launch * COPY_BYTES_PER_HISTORY)
+                ++copy_shift;
         KRun R;
         memset(&R, 0, sizeof(R));
         R.n = n_launch;

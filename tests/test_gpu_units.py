@@ -36,6 +36,37 @@ def test_totals_do_not_depend_on_the_batches(n, batches):
             np.testing.assert_allclose(g.kerma_sum2, g.kerma_keV ** 2 / n, rtol=1e-14, atol=0)
 
 
+@pytest.mark.parametrize("scene,voxel", [
+    ("plain_mc", 0.19),      # pencil beam, slots above 32 MB: copies of them
+    ("ct", 0.21),            # rotating fan: groups of 2 slots of 25 MB
+    ("ct", 0.18),            # 40 MB: four blocks per SM with one batch, one with many small ones
+    ("phantom", 0.29),       # cone: groups of 3 slots of 21 MB
+])
+def test_totals_do_not_depend_on_the_slots_in_use(scene, voxel):
+    from chatcarlo_b200 import phantoms as PH
+    from chatcarlo_b200 import workloads as W
+    from chatcarlo_b200.tally import VoxelGrid
+    from chatcarlo_b200.transport import run_transport
+    if scene == "phantom":
+        raw, spec = PH.phantom(np.random.default_rng(1))
+    else:
+        raw, spec = {"ct": W.ct, "plain_mc": W.plain_mc}[scene](), {"ct": W.CT_GRID, "plain_mc": W.PLAIN_MC_GRID}[scene]
+    shape = tuple(int(np.ceil(k * spec["voxel_cm"] / voxel)) for k in spec["shape"])
+    res = []
+    for b in (20_000, 2_900):
+        g = VoxelGrid(origin_cm=np.asarray(spec["origin"], dtype=float), shape=shape, voxel_size_cm=voxel,
+                      track_uncertainty=True)
+        r = run_transport(raw, n_histories=20_000, seed=5, batch_size=b, dose_grid=True, grid_resolution_cm=voxel, grid=g)
+        assert (g.n_batches, g.n_histories) == (-(-20_000 // b), 20_000)
+        res.append((r, g))
+    (r0, g0), (r1, g1) = res
+    assert r0.fraction_absorbed == r1.fraction_absorbed and r0.n_voxel_visits == r1.n_voxel_visits
+    for a, a0 in ((g1.kerma_keV, g0.kerma_keV), (g1.h10_track_pSv_cm3, g0.h10_track_pSv_cm3)):
+        # additions of positive FP64 numbers, as above
+        np.testing.assert_allclose(a, a0, rtol=2.0 ** -36, atol=0)
+    np.testing.assert_allclose(g0.kerma_sum2, g0.kerma_keV ** 2 / 20_000, rtol=1e-14, atol=0)
+
+
 def test_reset_clears_what_the_last_run_left():
     """Runs on one engine grid: batches folded away leave nothing to clear, a
     pending batch (photons scored without a fold) is cleared by the reset."""
