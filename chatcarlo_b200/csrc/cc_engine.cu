@@ -1035,8 +1035,9 @@ struct SegQueue {
 // do launches without a tally (shorter code; 1e6 photons 0.93 -> 1.04) and
 // with one block per SM (CT 5.83 -> 5.97); they run free.
 constexpr int LOCKSTEP_PER_LANE = 4;
-// Four 256-thread blocks per SM: the register budget (<= 64) that this asks
-// for costs no spills and hides more latency than two or three blocks.
+// Four 256-thread blocks per SM: the register budget (<= 64) that this asks for
+// costs no spills, and five (51 registers) are slower: room workload, 4e6
+// histories 4.95 ms with four, 5.5 with five.
 #ifndef CC_MIN_BLOCKS
 #define CC_MIN_BLOCKS 4
 #endif
@@ -1429,9 +1430,35 @@ __device__ __forceinline__ void add_scene_counts(const KBatch& B, bool ended, in
 }
 
 // Three blocks per SM: with 64 registers (four blocks) this kernel, which also
-// reads its scene through pointers, spills 164 bytes; 24 scenes of 3.2e6
-// histories: 5.14 ms with four, 4.96 with three.
+// reads its scene through pointers, spills 84 bytes; 24 scenes of 3.2e6
+// histories 4.06 ms with three, 4.10 with four, 8 scenes of 200,000 on 128^3
+// voxels 3.15 and 3.51.
 constexpr int BATCH_MIN_BLOCKS = CC_MIN_BLOCKS < 3 ? CC_MIN_BLOCKS : 3;
+// Its warps step together in groups of four, whose scenes differ less than a
+// block's (24 scenes of 3.2e6 histories: 4.06 ms in groups of eight warps, 3.93
+// in fours, 3.95 in twos; one scene in the transport kernel, room workload,
+// 4e6 histories: 4.99, 5.14, 5.37 ms).
+constexpr int BATCH_LOCKSTEP = 128;
+static_assert(BLOCK <= 2 * BATCH_LOCKSTEP, "two groups, barriers 1 and 2");
+// (barrier numbers known at compile time: with one in a register a block
+// reserves all 16, and six blocks of 128 threads no longer fit an SM)
+template <int ID>
+__device__ __forceinline__ bool group_any(bool v, int n) {
+    int any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, %2, %3, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+        : "=r"(any) : "r"((int)v), "n"(ID), "r"(n) : "memory");
+    return any != 0;
+}
+__device__ __forceinline__ bool group_any(bool v) {
+    if (threadIdx.x < BATCH_LOCKSTEP) return group_any<1>(v, min(BATCH_LOCKSTEP, (int)blockDim.x));
+    return group_any<2>(v, (int)blockDim.x - BATCH_LOCKSTEP);
+}
+__device__ __forceinline__ void group_sync() {
+    if (threadIdx.x < BATCH_LOCKSTEP) asm volatile("barrier.cta.sync 1, %0;" ::"r"(min(BATCH_LOCKSTEP, (int)blockDim.x)) : "memory");
+    else asm volatile("barrier.cta.sync 2, %0;" ::"r"((int)blockDim.x - BATCH_LOCKSTEP) : "memory");
+}
 
 template <bool TALLY, bool HEEL = false>
 __global__ void __launch_bounds__(BLOCK, BATCH_MIN_BLOCKS)
@@ -1501,7 +1528,7 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
             need = __ballot_sync(FULL, !live);
         }
         if (TALLY && R.lockstep) {
-            if (!__syncthreads_or(live)) break;
+            if (!group_any(live)) break;
         } else if (__all_sync(FULL, !live)) {
             break;
         }
@@ -1563,7 +1590,7 @@ batch_kernel(const KTables T, const KBatch B, const KRun R) {
             }
         }
 
-        if (TALLY && R.lockstep) __syncthreads();
+        if (TALLY && R.lockstep) group_sync();
 
         // ---- phase 3 ----
         bool ended = false, esc = false, absd = false;

@@ -97,3 +97,21 @@ def test_reset_clears_what_the_last_run_left():
         eng.lib.cc_scene_destroy(sh)
     again = run_transport(raw, n_histories=5_000, seed=3, dose_grid=True, grid=W.make_grid(spec)).grid
     np.testing.assert_allclose(again.kerma_keV, ref.kerma_keV, rtol=2.0 ** -36, atol=0)
+
+
+@pytest.mark.parametrize("block", [32, 128, 160, 256])
+def test_batch_groups_of_warps(block):
+    """Blocks of one, four, five and eight warps, stepped in groups of four
+    (enough histories per lane that they are): the same histories and scores."""
+    from chatcarlo_b200 import phantoms as PH
+    from chatcarlo_b200.batched import BatchedRun
+    scenes, specs = PH.phantoms(3, 4, side=16, voxel_cm=2.0)
+    got = []
+    for shape in ({"block": 256, "blocks_per_sm": 3, "chunk": 256}, {"block": block, "blocks_per_sm": 1, "chunk": 64}):
+        br = BatchedRun(scenes, specs, [70_000, 1, 120_001], shape=shape)
+        counts, _ = br.run(seed=9)
+        got.append((np.array(counts), [g.kerma_keV.copy() for g in br.download()]))
+    assert np.array_equal(got[0][0], got[1][0])
+    for a, b in zip(got[0][1], got[1][1]):
+        # additions of positive FP64 numbers, fewer than 2^20 per voxel
+        np.testing.assert_allclose(b, a, rtol=2.0 ** -33, atol=0)
