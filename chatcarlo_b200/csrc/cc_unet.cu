@@ -6,23 +6,21 @@
 //
 //   D[v, co] = sum_{tap, ci} X[v + off(tap), ci] * W[tap, co, ci]
 //
-// M = 128 output voxels per CTA, N = output channels, K = 27 taps x input
-// channels.  All 256 threads of the CTA gather the A tile (neighbour voxel
-// rows, zero outside the volume) and the B tile (weights of one tap) into
-// shared memory in the K-major, no-swizzle canonical layout; one thread
-// issues tcgen05.mma (kind::f16, BF16 inputs, FP32 accumulator in tensor
-// memory) and commits to an mbarrier, so the gather of the next stage runs
-// while the tensor core works on the current one (two stages).  The
-// epilogue reads the accumulator back with tcgen05.ld and applies bias and
-// ReLU (forward) or the ReLU mask of the layer below (backward data).
+// in tcgen05.mma instructions (kind::f16, BF16 inputs, FP32 accumulators in
+// tensor memory) of M = 128 output voxels.  The default kernel
+// (conv_ps_kernel) streams halo planes that the tensor memory accelerator
+// writes and reads a tap as a shifted start in them; the gathering kernel
+// (conv_kernel) copies neighbour voxel rows for every tap and takes any shape.
+// The epilogue reads the accumulators back with tcgen05.ld and applies bias
+// and ReLU (forward) or the ReLU mask of the layer below (backward data).
 //
 // A convolution input may be the channel concatenation of a full-resolution
 // tensor a and a half-resolution tensor b read nearest-upsampled (the U-Net
-// decoder's skip + upsampled path), fused into the gather.
+// decoder's skip + upsampled path), fused into the copies.
 //
-// The weight gradient is a second GEMM with M = 27 x C_in rows (tap, ci),
-// N = C_out and K = voxels, its operands MN-major in shared memory, split
-// over voxel ranges and reduced with FP32 atomics.
+// The weight gradient is a second GEMM with taps and input channels in M,
+// taps and output channels in N and K = voxels, its operands MN-major in
+// shared memory, split over voxel ranges and reduced with FP32 atomics.
 //
 // Every mbarrier wait is bounded by the global timer; a wait that runs out
 // sets a status bit that the host reads, and the CTA still frees its tensor
@@ -1126,14 +1124,14 @@ __global__ void __launch_bounds__(THREADS, 4) conv_ws_kernel(const ConvP P, int 
 }
 
 // ---------------------------------------------------------------------------
-// plane-stationary streaming convolution (16 or 32 output channels)
+// plane-stationary streaming convolution (slices of 16 or 32 output channels)
 // ---------------------------------------------------------------------------
 
-// A tcgen05.mma that accumulates into the accumulator of the previous one
-// waits for it: a chain of MMAs on one accumulator runs at one MMA per
-// ~125 cycles (A in shared memory) whatever N is, so 16 or 32 output
-// channels per MMA leave the tensor core mostly idle.  Here each input
-// plane p is read by ONE chain of 9 x cin/16 MMAs (the in-plane taps dy,
+// A tcgen05.mma of M = 128, K = 16 is bound by reading its operands from
+// shared memory, 128 bytes a cycle: 46.8 cycles at N = 48 (A 4 KB, B 1.5 KB),
+// 56.3 at N = 96, 96 at N = 192, where the arithmetic takes 24, 48 and 96.  An
+// output-stationary kernel reads A once per tap for N = 16 or 32 columns.
+// Here each input plane p is read by 9 x cin/16 MMAs (the in-plane taps dy,
 // dx) against the three weight planes dz stacked along N (N = 3 x cout):
 //     D_p[m][dz * cout + co] = sum_{dy, dx, ci} W[dz, dy, dx][co][ci] x_p(m + (dy, dx))[ci]
 // and output plane z is D_{z-1}[.., 0 | ..] + D_z[.., 1 | ..] + D_{z+1}[.., 2 | ..],
@@ -1141,10 +1139,19 @@ __global__ void __launch_bounds__(THREADS, 4) conv_ws_kernel(const ConvP P, int 
 // read a third as often as by the output-stationary kernels, and N is
 // three times wider.  Q = 5 regions of 3 x cout columns: the MMAs of
 // plane p + 1 and p + 2 overlap the epilogue of output p - 1.
-// Work split, ring of halo planes, warp roles and loader as conv_ws_kernel;
-// the barriers are: full / empty per ring slot (one MMA group reads each
-// plane), rfull per region (the plane's MMAs are done) and rfree per region
-// (the last output that reads the region, z + 1 for D_z, is stored).
+// Work split: PsWalk.  Roles: three loader warps (a's halo planes by tile
+// loads, one elected lane; b's voxels by 16-byte copies), two issuing warps and
+// eight or sixteen epilogue warps.  What bounds it (16 -> 16 channels on
+// 320x320x152): its MMAs' operand reads, 185 us; 197 without copies, 228 with
+// the inputs in turn from DRAM (708 -> 278 with L2 flushed, against gathered
+// halos, a divergent issue loop and four epilogue warps).  What gave it: issue
+// by a lane elected in a converged warp, its operands in uniform registers
+// (behind a divergent branch 2500 cycles per plane instead of 500), unrolled
+// taps, tile loads (369 -> 276), regions released before the stores, and masks
+// and partial sums read one output ahead.
+// Barriers: full / empty per ring slot (one MMA group reads each plane), rfull
+// per region (the plane's MMAs are done) and rfree per region (the last output
+// that reads the region, z + 1 for D_z, is read).
 // Issue groups: the MMA thread takes G consecutive planes at once and
 // interleaves their chains tap by tap, so that G independent accumulator
 // chains are in flight per CTA (one per plane); the CTA then holds
@@ -1953,9 +1960,14 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradP P) {
 // Voxels outside the volume read zeros in both operands (an infinite X next
 // to a zero gradient row of the padding gives NaN, as it does next to a
 // zero inside the volume).
+// Warps 4 to 7 add the gradient planes up for the bias gradient meanwhile (in
+// the CTAs of the first input channel group): a launch of its own per layer
+// took 60 of the 1085 us of a gradient of 4 x 64^3 voxels, this nothing that
+// shows (16 -> 16 channels 36.9 us either way).
 struct WgradH {
     Src vol;                     // sizes only
     float* dw;                   // [27][cout][ld], accumulated at columns c_off ..
+    float* db;                   // [cout], accumulated, or null
     int ld, c_off, cout;
     int ci_groups;               // blockIdx.y = co group * ci_groups + ci group
 };
@@ -1982,9 +1994,11 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
     __shared__ uint64_t full[WH_RING_MAX], empty[WH_RING_MAX], done;
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
+    __shared__ float s_db[CO];
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const Src& S = P.vol;
     const uint32_t R = (uint32_t)ring;
+    const bool sums = P.db != nullptr && blockIdx.y % P.ci_groups == 0;
     const int ci_lo = (int)(blockIdx.y % P.ci_groups) * CI, co_lo = (int)(blockIdx.y / P.ci_groups) * CO;
     volatile int* fail = &s_fail;
 
@@ -1992,12 +2006,13 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
     if (tid == 0) {
         for (uint32_t i = 0; i < R; ++i) {
             mbar_init(&full[i], 1);
-            mbar_init(&empty[i], 2);                           // one commit per issuing warp
+            mbar_init(&empty[i], sums ? 2 + 4 : 2);            // one commit per issuing warp, one arrival per summing warp
         }
         mbar_init(&done, 2);
         s_fail = 0;
         mbar_init_fence();
     }
+    if (tid < CO) s_db[tid] = 0.0f;
     wait_for_previous_kernel();
     tc_fence_before();
     __syncthreads();
@@ -2067,6 +2082,42 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
         }
         if (elect_one()) mma_commit(&done);                    // arrives once every MMA issued above has finished
         __syncwarp();
+    } else if (sums && warp >= 4) {
+        // ---- bias gradient: each plane [zs, ze) of the gradient once, 8 channels of every (128 / CH)-th row per thread ----
+        constexpr int CH = CO / 8;
+        const int chunk = lane % CH, row0 = (tid - 128) / CH;
+        float f[8] = {};
+        bool ok = true;
+        for (WsSeg q; ok && walk.next(S, q);) {
+            for (int i = 0; i < q.ze - q.zs + 2; ++i, ++L, ring_next(slot, ph, R)) {
+                ok = warp_wait_or_fail(&full[slot], ph, fail);
+                if (!ok) break;
+                if (i >= 1 && i <= q.ze - q.zs) {
+                    const uint8_t* plane = smem + (zbase - smem_u32(smem)) + slot * ZB;
+#pragma unroll
+                    for (int k = 0; k < CH; ++k) {
+                        const int row = row0 + k * (TILE_M / CH);
+                        const int at = chunk ^ (CO == 16 ? (row >> 2) & 1 : (row >> 1) & 3);       // the row's swizzle
+                        const uint4 v = *reinterpret_cast<const uint4*>(plane + row * (int)BR + at * 16);
+                        const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const float2 t = __bfloat1622float2(e[c]);
+                            f[2 * c] += t.x;
+                            f[2 * c + 1] += t.y;
+                        }
+                    }
+                }
+                __syncwarp();
+                if (elect_one()) mbar_arrive(&empty[slot]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+#pragma unroll
+            for (int m = CH; m < 32; m <<= 1) f[c] += __shfl_xor_sync(0xffffffffu, f[c], m);
+            if (lane < CH) atomicAdd(&s_db[8 * lane + c], f[c]);
+        }
     }
     // ---- epilogue: the accumulators into dw; lane quarter q holds dx = q ----
     mbar_wait_or_fail(&done, 0u, fail);
@@ -2075,6 +2126,7 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
     PsWalk any(S);
     WsSeg first;
     if (!*fail && any.next(S, first)) {
+        if (sums && tid < CO) atomicAdd(P.db + co_lo + tid, s_db[tid]);
         const int dx = warp & 3, half = warp >> 2;
         if (dx < 3) {
             for (int g = half; g < WH_DY * NP / 8; g += 2) {
@@ -2955,9 +3007,9 @@ int launch_conv_ps_g(const CUtensorMap& amap, const ConvP& P, int n_out, int co_
     return CCU_OK;
 }
 
-// The layer's slices.  A 16-channel layer takes the requested issue group
-// (by default 1: one chain on each of two CTAs per SM measured 1.4x faster
-// than three interleaved chains on one CTA), whose regions must fit 512
+// The layer's slices.  A 16-channel layer takes the requested issue group (by
+// default 1: two CTAs per SM; three interleaved chains on one CTA are 2.4x
+// slower, 32 -> 16 on 4 x 64^3 83 us against 35), whose regions must fit 512
 // tensor-memory columns; the others take 1.
 int launch_conv_ps(const ConvP& P, int n_out, const PsPlan& plan, cudaStream_t st) {
     static PlanCache cache;
@@ -3009,8 +3061,8 @@ int launch_wgrad(const WgradP& P, int slices, int cin, cudaStream_t st) {
 
 // dW of one input operand x (channels c_off .. c_off + cx - 1 of the layer's ld).
 template <int CI, int CO>
-int launch_wgrad_halo(const void* x, int cx, int batch, int d, int h, int w, const void* dz, int cout, float* dw, int ld,
-                      int c_off, int slices, cudaStream_t st) {
+int launch_wgrad_halo(const void* x, int cx, int batch, int d, int h, int w, const void* dz, int cout, float* dw,
+                      float* db, int ld, int c_off, int slices, cudaStream_t st) {
     CUtensorMap xmap, zmap;
     int rc = volume_map(&xmap, x, cx, batch, d, h, w, CI, HALO_X, HALO_Y);
     if (rc == CCU_OK) rc = volume_map(&zmap, dz, cout, batch, d, h, w, CO, 8, 16);
@@ -3036,6 +3088,7 @@ int launch_wgrad_halo(const void* x, int cx, int batch, int d, int h, int w, con
     WgradH P;
     P.vol = Src{nullptr, nullptr, 0, 0, batch, d, h, w};
     P.dw = dw;
+    P.db = db;
     P.ld = ld;
     P.c_off = c_off;
     P.cout = cout;
@@ -3166,6 +3219,11 @@ int ccu_conv3d_head(const void* a, int ca, int batch, int d, int h, int w, const
 
 int ccu_conv3d_wgrad(const void* a, int ca, const void* b, int cb, int batch, int d, int h, int w, const void* dz,
                      int cout, float* dw, int slices, void* stream) {
+    return ccu_conv3d_wgrad_bias(a, ca, b, cb, batch, d, h, w, dz, cout, dw, nullptr, slices, stream);
+}
+
+int ccu_conv3d_wgrad_bias(const void* a, int ca, const void* b, int cb, int batch, int d, int h, int w, const void* dz,
+                          int cout, float* dw, float* db, int slices, void* stream) {
     int rc = check_src(a, ca, b, cb, batch, d, h, w);
     if (rc != CCU_OK) return rc;
     if (!dz || !dw || !aligned16(dz) || slices <= 0) return set_error(CCU_E_INVALID, "bad gradient arguments");
@@ -3176,14 +3234,14 @@ int ccu_conv3d_wgrad(const void* a, int ca, const void* b, int cb, int batch, in
     // per-device buffer: only for the shapes documented to use that buffer
     auto box_channels = [](int c) { return c == 16 || c == 32 || c % 64 == 0; };
     if (g_wgrad_path == 0 && (cb == 0 || (w % 8 == 0 && box_channels(ca) && box_channels(cb)))) {
-        auto run = [&](const void* x, int cx, int c_off) {
+        auto run = [&](const void* x, int cx, int c_off, float* sums) {
             if (cx % 32 == 0)
-                return cout == 16 ? launch_wgrad_halo<32, 16>(x, cx, batch, d, h, w, dz, cout, dw, ca + cb, c_off, slices, st)
-                                  : launch_wgrad_halo<32, 32>(x, cx, batch, d, h, w, dz, cout, dw, ca + cb, c_off, slices, st);
-            return cout == 16 ? launch_wgrad_halo<16, 16>(x, cx, batch, d, h, w, dz, cout, dw, ca + cb, c_off, slices, st)
-                              : launch_wgrad_halo<16, 32>(x, cx, batch, d, h, w, dz, cout, dw, ca + cb, c_off, slices, st);
+                return cout == 16 ? launch_wgrad_halo<32, 16>(x, cx, batch, d, h, w, dz, cout, dw, sums, ca + cb, c_off, slices, st)
+                                  : launch_wgrad_halo<32, 32>(x, cx, batch, d, h, w, dz, cout, dw, sums, ca + cb, c_off, slices, st);
+            return cout == 16 ? launch_wgrad_halo<16, 16>(x, cx, batch, d, h, w, dz, cout, dw, sums, ca + cb, c_off, slices, st)
+                              : launch_wgrad_halo<16, 32>(x, cx, batch, d, h, w, dz, cout, dw, sums, ca + cb, c_off, slices, st);
         };
-        if (cb == 0) return run(a, ca, 0);
+        if (cb == 0) return run(a, ca, 0, db);
         // the skip part from a, the upsampled part from its full-resolution copy
         void* up = nullptr;
         const long long n_vox = (long long)batch * d * h * w;
@@ -3192,10 +3250,11 @@ int ccu_conv3d_wgrad(const void* a, int ca, const void* b, int cb, int batch, in
         rc = launch_dependent(upsample_kernel, dim3((unsigned)grid_for(n_vox * (cb / 8), 256)), 256, 0, st, (const uint4*)b,
                               (uint4*)up, batch, d, h, w, cb / 8);
         if (rc != CCU_OK) return rc;
-        rc = run(a, ca, 0);
+        rc = run(a, ca, 0, db);
         if (rc != CCU_OK) return rc;
-        return run(up, cb, ca);
+        return run(up, cb, ca, nullptr);
     }
+    if (db && (rc = ccu_bias_grad(dz, (long long)batch * d * h * w, cout, db, stream)) != CCU_OK) return rc;
     WgradP P;
     P.src = Src{(const __nv_bfloat16*)a, (const __nv_bfloat16*)b, ca, cb, batch, d, h, w};
     P.dz = (const __nv_bfloat16*)dz;

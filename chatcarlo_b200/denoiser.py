@@ -283,9 +283,8 @@ class UNet3D:
         n = B * d * h * w
         if slices is None:
             slices = max(1, min(256, n // 2048))
-        self._call(lib.ccu_conv3d_wgrad, self._ptr(a), L.ca, self._ptr(b) if b is not None else None, L.cb, B, d, h, w,
-                   self._ptr(dz), L.cout, self._ptr(self.g, o), slices, st)
-        self._call(lib.ccu_bias_grad, self._ptr(dz), n, L.cout, self._ptr(self.g, bo), st)
+        self._call(lib.ccu_conv3d_wgrad_bias, self._ptr(a), L.ca, self._ptr(b) if b is not None else None, L.cb,
+                   B, d, h, w, self._ptr(dz), L.cout, self._ptr(self.g, o), self._ptr(self.g, bo), slices, st)
         if out0 is not None:
             self._call(lib.ccu_conv3d, self._ptr(dz), L.cout, None, 0, B, d, h, w, self._ptr(self.wt[L.name]), None,
                        L.cin, 0, self._ptr(out0), L.ca, self._ptr(mask0) if mask0 is not None else None,

@@ -65,6 +65,12 @@ int ccu_conv3d_head(const void* a, int ca, int batch, int d, int h, int w, const
 int ccu_conv3d_wgrad(const void* a, int ca, const void* b, int cb, int batch, int d, int h, int w, const void* dz,
                      int cout, float* dw, int slices, void* stream);
 
+/* ccu_conv3d_wgrad and, when db is not NULL, db[cout] (FP32) += sum over
+ * voxels of dz[v][co] in the same pass over dz (by ccu_bias_grad where the
+ * gathering kernel runs). */
+int ccu_conv3d_wgrad_bias(const void* a, int ca, const void* b, int cb, int batch, int d, int h, int w,
+                          const void* dz, int cout, float* dw, float* db, int slices, void* stream);
+
 /* db[c] += sum over voxels of dz[v][c]; c divides 256. */
 int ccu_bias_grad(const void* dz, long long n_vox, int c, float* db, void* stream);
 
@@ -123,10 +129,11 @@ long long ccu_packed_weight_elems(int n, int c);
 int ccu_pack_weights(const float* w32, int cout, int cin, void* w, void* wt, void* stream);
 
 /* Which convolution kernel ccu_conv3d uses: 0 (default) the
- * plane-stationary kernel for 16 or 32 output channels (in channel passes
- * with an FP32 partial sum when the weights do not fit shared memory at
- * once; the partial lives in a per-device workspace of n_vox x cout x 4
- * bytes that the first such call allocates and the process keeps), else the
+ * plane-stationary kernel for 16, 32 or 64 output channels (in channel
+ * passes with an FP32 partial sum when the weights do not fit shared memory
+ * at once; the partial lives in a per-device workspace of n_vox x cout x 4
+ * bytes that the first such call allocates and the process keeps) and for
+ * 48, 96, 128 or 192 where one pass holds the weights, else the
  * persistent halo kernel that streams z-planes through a shared-memory ring
  * where it applies (input and output channels <= 48), else the gathering
  * kernel; 1 always the gathering kernel; 2 the one-tile halo kernel where
@@ -146,12 +153,12 @@ int ccu_set_wgrad_path(int path);
  * with CCU_E_INVALID).  Process-wide. */
 int ccu_set_conv_ring(int ring);
 
-/* Issue group of the plane-stationary kernel (path 0, 16 or 32 output
- * channels): 0 (default) chosen per layer, else 1 .. 3 input planes whose
- * MMA chains one thread interleaves (more independent accumulators in
- * flight, fewer CTAs per SM), reduced per layer to the largest group whose
- * tensor-memory regions fit 512 columns (3 for 16 output channels, 1 for
- * 32).  Process-wide. */
+/* Issue group of the plane-stationary kernel (path 0): 0 (default) chosen
+ * per layer (one plane; slices of 16 output channels of large volumes on
+ * pairs of voxels, with the same sums), else 1 .. 3 input planes whose MMA
+ * chains are interleaved (more independent accumulators in flight, fewer
+ * CTAs per SM) by a layer of 16 output channels; others take one, without
+ * pairs.  Process-wide. */
 int ccu_set_conv_group(int group);
 
 /* cudaMemsetAsync(p, 0, bytes) on the stream (gradient buffers). */

@@ -148,3 +148,34 @@ def test_sixteen_channels_on_pairs_of_voxels(U, ca, cb, dims):
     assert U.status() == 0
     for p, q in zip(*got):
         assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("ca,cb,cout,dims,slices,path", [
+    (16, 0, 16, (1, 1, 1, 1), 1, 0),            # one voxel
+    (16, 0, 16, (2, 3, 17, 9), 1, 0),           # one row and one column beyond a tile
+    (32, 0, 128, (1, 5, 16, 8), 64, 0),         # four output groups, more splits than planes
+    (64, 0, 32, (3, 19, 33, 7), 2, 0),          # two input groups: the first alone sums; the ring wraps
+    (32, 64, 16, (1, 4, 18, 16), 3, 0),         # concatenated: the first part's launch alone sums
+    (16, 32, 64, (1, 2, 6, 10), 2, 0),          # concatenated, gathering kernel
+    (16, 0, 32, (2, 4, 9, 11), 4, 1),           # gathering kernel by choice
+])
+def test_bias_gradient_beside_the_weight_gradient(U, ca, cb, cout, dims, slices, path):
+    """At most n additions of exactly converted values in FP32, each erring by
+    at most 2^-24 of the sum of the magnitudes."""
+    g = torch.Generator(device="cuda").manual_seed(ca + cout + dims[2])
+    n = dims[0] * dims[1] * dims[2] * dims[3]
+    a = torch.randn(n, ca, generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(max(1, n // 8), max(1, cb), generator=g, device="cuda").to(torch.bfloat16)
+    dz = torch.randn(n, cout, generator=g, device="cuda").to(torch.bfloat16)
+    dw, db = torch.zeros(27, cout, ca + cb, device="cuda"), torch.ones(cout, device="cuda")
+    try:
+        U.check(U.lib().ccu_set_wgrad_path(path))
+        U.check(U.lib().ccu_conv3d_wgrad_bias(a.data_ptr(), ca, b.data_ptr() if cb else None, cb, *dims, dz.data_ptr(), cout,
+                                              dw.data_ptr(), db.data_ptr(), slices, torch.cuda.current_stream().cuda_stream))
+    finally:
+        U.check(U.lib().ccu_set_wgrad_path(0))
+    torch.cuda.synchronize()
+    assert U.status() == 0
+    ref, mag = 1.0 + dz.double().sum(0), 1.0 + dz.double().abs().sum(0)
+    assert bool(((db.double() - ref).abs() <= (n + 1) * 2.0 ** -24 * mag).all())
+    assert bool((dw.abs().sum((0, 2)) > 0).all())
