@@ -21,11 +21,12 @@ LIB_DIR = PKG / "lib"
 LIB_PATH = LIB_DIR / "libccb200.so"
 HEADER = PKG.parent / "include" / "chatcarlo_b200.h"
 SOURCES = [CSRC / "cc_engine.cu", CSRC / "cc_atomics.cu"]
-DEPS = SOURCES + [CSRC / "philox.cuh", HEADER]
+RULES = CSRC / "launch_rules.h"
+DEPS = SOURCES + [CSRC / "philox.cuh", RULES, HEADER]
 FP64_LIB_PATH = LIB_DIR / "libccb200_fp64.so"
 UNET_LIB_PATH = LIB_DIR / "libccunet.so"
 UNET_SOURCES = [CSRC / "cc_unet.cu"]
-UNET_DEPS = UNET_SOURCES + [PKG.parent / "include" / "chatcarlo_b200_unet.h"]
+UNET_DEPS = UNET_SOURCES + [RULES, PKG.parent / "include" / "chatcarlo_b200_unet.h"]
 
 # --use_fast_math: FP32 tracking tolerates approximate division, square root and
 # transcendentals (the surface band is 8 ulps of the world extent); tallies are

@@ -37,6 +37,7 @@
 #include <string>
 
 #include "../../include/chatcarlo_b200_unet.h"
+#include "launch_rules.h"
 
 namespace {
 
@@ -1188,6 +1189,8 @@ __host__ __device__ constexpr int ps_epi_warps(int n) { return n == 16 ? 8 : 16;
 constexpr int PS_ISSUERS = 2, PS_EPI_WARP0 = PS_ISSUERS + WS_LOADERS / 32;
 __host__ __device__ constexpr int ps_threads(int n) { return 32 * (PS_EPI_WARP0 + ps_epi_warps(n)); }
 constexpr uint32_t PS_SMEM_MAX = 220 * 1024;
+// (one warp issues groups of planes, two take single planes in turn)
+__host__ __device__ constexpr int ps_issuers(int g) { return g == 1 ? PS_ISSUERS : 1; }
 // A ring slot holds 16-channel groups of a halo plane, 180 voxel rows of 32
 // bytes under the 32-byte swizzle (16-byte half h of voxel v at half
 // h ^ ((v >> 2) & 1): the pattern repeats every 256 bytes, to which groups
@@ -1206,6 +1209,7 @@ __host__ __device__ constexpr int ps_regions(int g) { return g <= 1 ? 5 : 2 * g 
 __host__ __device__ constexpr uint32_t ps_tmem_cols(int n, int g) {
     return (uint32_t)ps_regions(g) * ps_region_cols(n) <= 256u ? 256u : 512u;
 }
+constexpr bool ps_ring_allowed(int ring, int g) { return cc::issue_ring_allowed(ring, ps_issuers(g), ps_regions(g)); }
 __host__ __device__ constexpr uint32_t ps_weight_bytes(int n, int c8p) { return 9u * (uint32_t)c8p * 3u * n * 16u; }
 __host__ __device__ constexpr uint32_t ps_smem_bytes(int n, int c8p, int ring) {
     return (uint32_t)ring * (uint32_t)(c8p / 2) * PS_GROUP_BYTES + ps_weight_bytes(n, c8p) + 256;   // 256: alignment
@@ -1448,12 +1452,13 @@ __global__ void __launch_bounds__(ps_threads(NO), NO == 16 && G == 1 && C8P <= 8
         // after a failure, the tile loads still in flight land before the CTA ends
         if (tiles && *fail)
             for (uint32_t p = L > R ? L - R : 0; p < L; ++p) mbar_wait(&full[p % R], (p / R) & 1u);
-    } else if (warp < (G == 1 ? PS_ISSUERS : 1)) {
+    } else if (warp < ps_issuers(G)) {
         // ---- MMA issuer: per input plane one chain of 9 x c8p / 2 MMAs; the chains of a
         // group of planes are issued tap by tap in turn.  With G = 1 two warps
         // take alternate planes: the tensor core's queue is short, so one
         // warp's waits and commits between two planes would leave it idle
-        // where a CTA has the SM to itself ----
+        // where a CTA has the SM to itself; each waits for its own planes
+        // only, which bounds the rings they may run on (ps_ring_allowed) ----
         constexpr uint32_t STEP = G == 1 ? PS_ISSUERS : G;
         const uint64_t a0 = smem_desc_sw(sbase, 16, HALO_X * 32, swizzle_layout(32));   // 8 x-neighbours, then the next y row
         const uint64_t b0 = smem_desc(swt, NP * 16, 128);
@@ -2905,8 +2910,9 @@ int launch_conv_pair_g(const ConvP& P, int n_out, int co_lo, cudaStream_t st) {
     LaunchPlan plan;
     rc = device_plan(&caches[b16], plan, [&](int dev, LaunchPlan& p) {
         CU_CHECK(cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev));
-        p.ring = 2;
-        while (p.ring < WS_RING_MAX && pair_smem_bytes(a16, b16, p.ring + 1) <= PS_SMEM_MAX) ++p.ring;
+        p.ring = 2;                              // deepest that fits, as in launch_conv_ps_pass
+        for (int r = 3; r <= WS_RING_MAX && pair_smem_bytes(a16, b16, r) <= PS_SMEM_MAX; ++r)
+            if (ps_ring_allowed(r, 1)) p.ring = r;
         const int r_c = tc_launch_smem(kernel, pair_smem_bytes(a16, b16, p.ring), ps_tmem_cols(32, 1), p.smem, ps_threads(32));
         // one kernel serves several splits into a and b, each with its own ring: allow it the largest
         CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS_SMEM_MAX));
@@ -2954,9 +2960,11 @@ int launch_conv_ps_pass(const CUtensorMap& amap, const ConvP& P, const PsPass& Q
     int rc = device_plan(C8P > 0 ? &cache : nullptr, plan, [&](int dev, LaunchPlan& p) {
         const uint32_t cols = ps_tmem_cols(NO, G);
         CU_CHECK(cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev));
-        // deepest ring (group + 1 .. WS_RING_MAX planes) that keeps the CTAs per SM the tensor memory allows
+        // deepest ring (group + 1 .. WS_RING_MAX planes) that keeps the CTAs per SM the tensor memory
+        // allows, of the depths that the issuing warps may run on
         int best = 0, r_c = CCU_OK;
         for (int r = G + 1; r <= WS_RING_MAX && ps_smem_bytes(NO, c8p, r) <= PS_SMEM_MAX; ++r) {
+            if (!ps_ring_allowed(r, G)) continue;
             int res = 1;
             r_c = resident_ctas(kernel, (size_t)ps_smem_bytes(NO, c8p, r) + 1024, cols, res, ps_threads(NO));
             if (r_c != CCU_OK) return r_c;

@@ -179,3 +179,17 @@ def test_bias_gradient_beside_the_weight_gradient(U, ca, cb, cout, dims, slices,
     ref, mag = 1.0 + dz.double().sum(0), 1.0 + dz.double().abs().sum(0)
     assert bool(((db.double() - ref).abs() <= (n + 1) * 2.0 ** -24 * mag).all())
     assert bool((dw.abs().sum((0, 2)) > 0).all())
+
+
+@pytest.mark.parametrize("cin,cout,split,dims", [
+    (80, 16, 16, (2, 300, 17, 9)),          # 16 planes per CTA: the ring turns several times
+    (80, 48, 16, (1, 310, 18, 21)),
+    (112, 128, 128, (1, 150, 33, 7)),
+    (144, 16, 16, (1, 300, 20, 10)),        # two passes of 80 and 64 input channels
+    (112, 48, 40, (1, 3, 5, 6)),
+])
+@pytest.mark.parametrize("masked", [False, True])
+def test_convolution_on_rings_that_five_planes_would_fit(U, cin, cout, split, dims, masked):
+    """Passes of 80 and 112 input channels, whose deepest ring (5 or 3 planes)
+    two issuing warps may not use."""
+    test_convolution_output_slices(U, cin, cout, split, dims, masked)

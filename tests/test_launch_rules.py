@@ -1,0 +1,92 @@
+"""The launch rules of csrc/launch_rules.h, compiled for the host, over their
+whole range."""
+from __future__ import annotations
+
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "chatcarlo_b200" / "csrc"
+SHIM = """
+#include "launch_rules.h"
+extern "C" int ring_allowed(int ring, int issuers, int regions) { return cc::issue_ring_allowed(ring, issuers, regions); }
+"""
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    d = tmp_path_factory.mktemp("rules")
+    (d / "shim.cpp").write_text(SHIM)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", f"-I{CSRC}", str(d / "shim.cpp"), "-o", str(d / "shim.so")],
+                   check=True)
+    return C.CDLL(str(d / "shim.so"))
+
+
+class _Bar:
+    """An mbarrier of one arrival: a wait by parity passes when the phase in
+    progress has the other one."""
+
+    def __init__(self):
+        self.done = 0
+
+    def passes(self, parity):
+        return self.done & 1 != parity
+
+
+def _reads_stale_slot(ring, issuers, regions, late, planes=40):
+    """The plane-stationary convolution's hand-offs with the loads into the slot
+    of plane `late`, from that plane on, landing only when nothing else can
+    move: whether an issuer's instructions of some plane read a slot that does
+    not hold it."""
+    full, empty = [_Bar() for _ in range(ring)], [_Bar() for _ in range(ring)]
+    rfull, rfree = [_Bar() for _ in range(regions)], [_Bar() for _ in range(regions)]
+    holds = [None] * ring
+    load, pending, epi = 0, [], 0
+    nxt, seen = list(range(issuers)), [False] * issuers      # an issuer's next plane, and whether its "full" wait is over
+    while min(nxt) < planes:
+        moved = False
+        if load < planes and (load < ring or empty[load % ring].passes((load // ring - 1) & 1)):
+            if load >= late and (load - late) % ring == 0:
+                pending.append(load)
+            else:
+                holds[load % ring] = load
+                full[load % ring].done += 1
+            load += 1
+            moved = True
+        for w in range(issuers):
+            p = nxt[w]
+            if p < planes and not seen[w] and full[p % ring].passes((p // ring) & 1):
+                seen[w] = moved = True
+            if seen[w] and (p < regions or rfree[p % regions].passes((p // regions - 1) & 1)):
+                if holds[p % ring] != p:
+                    return True
+                seen[w] = False
+                rfull[p % regions].done += 1
+                empty[p % ring].done += 1
+                nxt[w] += issuers
+                moved = True
+        # the epilogue waits for the planes in order; an output is read, and plane epi - 2 released, with plane epi
+        if epi < planes and rfull[epi % regions].passes((epi // regions) & 1):
+            if epi >= 2:
+                rfree[(epi - 2) % regions].done += 1
+            epi += 1
+            moved = True
+        if not moved:
+            assert pending, (ring, issuers, regions, late)      # else the hand-offs themselves are stuck
+            holds[late % ring] = pending.pop(0)
+            full[late % ring].done += 1
+    return False
+
+
+def test_rings_of_alternate_issuers(rules):
+    """Two issuing warps on five regions, and one on any: no late load is read
+    before it lands on a ring that the rule allows; it is on 3 and 5 planes."""
+    for issuers, regions in ((2, 5), (1, 5), (1, 6), (1, 8)):
+        for ring in range(2, 13):
+            stale = any(_reads_stale_slot(ring, issuers, regions, late) for late in range(30))
+            allowed = bool(rules.ring_allowed(ring, issuers, regions))
+            assert not (allowed and stale), (ring, issuers, regions)
+            assert allowed != (issuers == 2 and ring in (3, 5)), (ring, issuers, regions)
+    assert _reads_stale_slot(3, 2, 5, 1) and _reads_stale_slot(5, 2, 5, 1)
