@@ -33,6 +33,7 @@
 #include <string>
 #include <vector>
 
+#include "launch_rules.h"
 #include "philox.cuh"
 #include "../../include/chatcarlo_b200.h"
 
@@ -182,7 +183,7 @@ struct KSource {
 struct KRun {
     long long n;              // histories in this launch
     long long first;          // global index of the first history
-    long long batch_size;     // histories per scratch buffer
+    long long batch_size;     // histories per scratch buffer, at most n (unit_batch)
     int n_scratch;
     int group;                // batches whose units alternate (see HIST_UNIT)
     int copy_shift;           // log2 of the scratch copies of a batch's slot
@@ -880,7 +881,6 @@ __device__ __forceinline__ void sample_source(const KSource& S, RNG& rng, real p
 // fold of small runs more); chunks of 256 consecutive histories per warp, the
 // order before, 1.26 / 2.26 / 6.8, with most warps idle in small runs.
 // Where the beam is wide and the slots are large, fewer at once (SlotOrder).
-constexpr int HIST_UNIT = 32;
 constexpr int SPREAD_SLOTS = 16;
 constexpr size_t SLOT_BYTES_COMPACT = (size_t)32 << 20;     // slots above this are large (SlotOrder)
 // Voxel visits per piece when a warp splits its track segments.  The split
@@ -1048,22 +1048,10 @@ constexpr int LOCKSTEP_PER_LANE = 4;
 // voxel walk, which keeps the loop's code small.
 constexpr int TV_DEFER = 3;
 
-// The next unit of the launch's counter: histories [first, end) of one batch
-// (empty beyond a short last batch) and their scratch slot; first < 0: none left.
+// The next unit of the launch's counter (unit_at); first < 0: none left.
 __device__ __forceinline__ void take_unit(const KRun& R, long long& first, long long& end, int& slot) {
-    const long long per = (R.batch_size + HIST_UNIT - 1) / HIST_UNIT;
-    const long long k = (long long)atomicAdd(R.work, 1ull);
     first = end = -1;
-    if (k >= per * R.n_scratch) return;
-    const long long in_group = per * R.group;
-    const int g = (int)(k / in_group) * R.group;                       // the group's first batch
-    const long long r = k % in_group;
-    const int members = min(R.group, R.n_scratch - g);
-    const long long unit = r / members;
-    const int batch = g + (int)(r - unit * members);
-    first = (long long)batch * R.batch_size + unit * HIST_UNIT;
-    end = max(first, min(first + HIST_UNIT, min((long long)(batch + 1) * R.batch_size, R.n)));
-    slot = (batch << R.copy_shift) | ((int)unit & ((1 << R.copy_shift) - 1));
+    unit_at((long long)atomicAdd(R.work, 1ull), R.n, R.batch_size, R.n_scratch, R.group, R.copy_shift, first, end, slot);
 }
 
 template <bool FROM_SOURCE, bool TALLY, bool HEEL = false, int TV = CELL_FP64>
@@ -3038,7 +3026,7 @@ static int enqueue_launch(cc_ctx* c, const cc_scene* scene, const cc_tables* tab
                           int cell32, cc_ctx::LaunchRec& rec, int copy_shift = 0) {
     const KTables& T = tables->k;
     R.n_scratch = n_slots;
-    R.batch_size = batch_size;
+    R.batch_size = unit_batch(batch_size, R.n);
     const SlotOrder order = slot_order(src, grid, batch_size);
     R.group = order.group;
     R.copy_shift = copy_shift;
@@ -3430,7 +3418,7 @@ int cc_run(cc_ctx* c, const cc_scene* scene, const cc_tables* tables, const cc_s
     while (done < n_hist) {
         int ns = slots;
         long long n_launch = std::min<long long>(n_hist - done, (long long)ns * batch_size);
-        ns = (int)((n_launch + batch_size - 1) / batch_size);
+        ns = (int)batches_of(n_launch, batch_size);
         int copy_shift = 0;
         if (order.copies)
             while ((ns << (copy_shift + 1)) <= std::min(+SPREAD_SLOTS, grid->n_scratch) &&
@@ -3480,7 +3468,7 @@ int cc_run(cc_ctx* c, const cc_scene* scene, const cc_tables* tables, const cc_s
         out->n_escaped = (int64_t)tot[1];
         out->scatter_sum = (int64_t)tot[2];
         out->n_fluorescence = (int64_t)tot[3];
-        out->n_batches = (n_hist + batch_size - 1) / batch_size;
+        out->n_batches = n_hist > 0 ? batches_of(n_hist, batch_size) : 0;
         out->gpu_launches = launches;
         out->elapsed_ms = ms_total;
         out->n_steps = (int64_t)tot[4];

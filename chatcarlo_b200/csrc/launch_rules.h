@@ -2,6 +2,12 @@
 // the tests can check them on the host over their whole range.
 #pragma once
 
+#ifdef __CUDACC__
+#define CC_RULE __host__ __device__ __forceinline__
+#else
+#define CC_RULE inline
+#endif
+
 namespace cc {
 
 // Whether `issuers` warps that take the planes of a plane-stationary
@@ -18,5 +24,40 @@ namespace cc {
 constexpr bool issue_ring_allowed(int ring, int issuers, int regions) {
     return ring % issuers == 0 || ring >= regions + issuers;
 }
+
+// A transport launch hands out its n histories in units of HIST_UNIT of one
+// batch, round-robin over groups of `group` batches (cc_engine.cu says why);
+// unit u of a batch goes to copy u mod 2^copy_shift of the batch's slot.
+constexpr int HIST_UNIT = 32;
+
+// Histories of a batch for counting units: units beyond the launch's histories
+// are handed out too, each an empty turn of the counter, so a batch size above
+// them ("never split") must not enter.  At most n / 16 + 2 n_batches units then.
+CC_RULE long long unit_batch(long long batch_size, long long n) { return batch_size < n ? batch_size : n; }
+
+CC_RULE long long units_per_batch(long long batch_size) { return (batch_size + HIST_UNIT - 1) / HIST_UNIT; }
+
+// Unit k: histories [first, end) (empty beyond a short last batch) and their
+// scratch slot; false where there are no more.
+CC_RULE bool unit_at(long long k, long long n, long long batch_size, int n_batches, int group, int copy_shift,
+                     long long& first, long long& end, int& slot) {
+    const long long per = units_per_batch(batch_size);
+    if (k >= per * n_batches) return false;
+    const long long in_group = per * group;
+    const int g = (int)(k / in_group) * group;                         // the group's first batch
+    const long long r = k % in_group;
+    const int members = group < n_batches - g ? group : n_batches - g;
+    const long long unit = r / members;
+    const int batch = g + (int)(r - unit * members);
+    first = (long long)batch * batch_size + unit * HIST_UNIT;
+    const long long batch_end = (long long)(batch + 1) * batch_size < n ? (long long)(batch + 1) * batch_size : n;
+    end = first + HIST_UNIT < batch_end ? first + HIST_UNIT : batch_end;
+    if (end < first) end = first;
+    slot = (batch << copy_shift) | ((int)unit & ((1 << copy_shift) - 1));
+    return true;
+}
+
+// Batches of n > 0 histories (no overflow at the largest batch sizes).
+CC_RULE long long batches_of(long long n, long long batch_size) { return (n - 1) / batch_size + 1; }
 
 }  // namespace cc

@@ -115,3 +115,26 @@ def test_batch_groups_of_warps(block):
     for a, b in zip(got[0][1], got[1][1]):
         # additions of positive FP64 numbers, fewer than 2^20 per voxel
         np.testing.assert_allclose(b, a, rtol=2.0 ** -33, atol=0)
+
+
+@pytest.mark.parametrize("dose_grid", [True, False])
+def test_batch_size_above_the_histories_is_one_batch(dose_grid):
+    """"Never split" values: one batch of all histories, whatever the size."""
+    from chatcarlo_b200 import workloads as W
+    from chatcarlo_b200.transport import run_transport
+    n, res = 10_000, []
+    for b in (10_000, 1_000_000, 10 ** 9):
+        g = W.make_grid(W.ROOM_GRID) if dose_grid else None
+        res.append((run_transport(W.room(), n_histories=n, seed=4, batch_size=b, dose_grid=dose_grid, grid=g), g))
+    r0, g0 = res[0]
+    for r, g in res:
+        assert (r.n_batches, r.fraction_absorbed, r.n_voxel_visits) == (1, r0.fraction_absorbed, r0.n_voxel_visits)
+        assert r.energy_deposited_MeV.keys() == r0.energy_deposited_MeV.keys()
+        for k, v in r0.energy_deposited_MeV.items():
+            # FP64 sums of at most 2^17 positive deposits each
+            np.testing.assert_allclose(r.energy_deposited_MeV[k], v, rtol=2.0 ** -36, atol=0)
+        if g is not None:
+            assert (g.n_batches, g.n_histories) == (1, n) and np.array_equal(g.n_batches_hit, g0.n_batches_hit)
+            for a, a0 in ((g.kerma_keV, g0.kerma_keV), (g.h10_track_pSv_cm3, g0.h10_track_pSv_cm3)):
+                np.testing.assert_allclose(a, a0, rtol=2.0 ** -36, atol=0)
+            np.testing.assert_allclose(g.kerma_sum2, g0.kerma_sum2, rtol=2.0 ** -34, atol=0)

@@ -12,6 +12,15 @@ CSRC = Path(__file__).resolve().parent.parent / "chatcarlo_b200" / "csrc"
 SHIM = """
 #include "launch_rules.h"
 extern "C" int ring_allowed(int ring, int issuers, int regions) { return cc::issue_ring_allowed(ring, issuers, regions); }
+extern "C" long long unit_batch(long long batch_size, long long n) { return cc::unit_batch(batch_size, n); }
+extern "C" long long batches_of(long long n, long long batch_size) { return cc::batches_of(n, batch_size); }
+extern "C" long long units_per_batch(long long batch_size) { return cc::units_per_batch(batch_size); }
+extern "C" int unit_at(long long k, long long n, long long batch_size, int n_batches, int group, int shift, long long* out) {
+    int slot = -1;
+    const int ok = cc::unit_at(k, n, batch_size, n_batches, group, shift, out[0], out[1], slot);
+    out[2] = slot;
+    return ok;
+}
 """
 
 
@@ -21,7 +30,11 @@ def rules(tmp_path_factory):
     (d / "shim.cpp").write_text(SHIM)
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", f"-I{CSRC}", str(d / "shim.cpp"), "-o", str(d / "shim.so")],
                    check=True)
-    return C.CDLL(str(d / "shim.so"))
+    lib = C.CDLL(str(d / "shim.so"))
+    for f in (lib.unit_batch, lib.batches_of, lib.units_per_batch):
+        f.restype, f.argtypes = C.c_longlong, [C.c_longlong] * (1 if f is lib.units_per_batch else 2)
+    lib.unit_at.argtypes = [C.c_longlong] * 3 + [C.c_int] * 3 + [C.c_void_p]
+    return lib
 
 
 class _Bar:
@@ -90,3 +103,30 @@ def test_rings_of_alternate_issuers(rules):
             assert not (allowed and stale), (ring, issuers, regions)
             assert allowed != (issuers == 2 and ring in (3, 5)), (ring, issuers, regions)
     assert _reads_stale_slot(3, 2, 5, 1) and _reads_stale_slot(5, 2, 5, 1)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 1000, 10_007, 4_000_000, 2 ** 40])
+def test_units_are_bounded_by_the_histories(rules, n):
+    """Whatever the batch size, a launch's counter runs over at most
+    n / 16 + 2 batches + 1 units."""
+    for size in (1, 2, 31, 32, 33, 1000, 200_000, 10 ** 9, 2 ** 62, 2 ** 63 - 1):
+        nb = rules.batches_of(n, size)
+        assert nb == -(-n // size)
+        units = rules.units_per_batch(rules.unit_batch(size, n)) * nb
+        assert n <= 32 * units and 16 * units <= n + 32 * nb + 16, (n, size)
+
+
+@pytest.mark.parametrize("n,size", [(1, 2 ** 62), (33, 10 ** 9), (5_003, 5_003), (5_003, 700), (640, 20), (2_000, 999), (64, 1)])
+@pytest.mark.parametrize("group,shift", [(1, 0), (3, 0), (16, 0), (16, 2)])
+def test_units_cover_every_history_once(rules, n, size, group, shift):
+    """Every history in one unit of its own batch, in that batch's slots."""
+    nb, b = rules.batches_of(n, size), rules.unit_batch(size, n)
+    out, seen, k = (C.c_longlong * 3)(), [], 0
+    while rules.unit_at(k, n, b, nb, group, shift, out):
+        first, end, slot = out
+        assert 0 <= end - first <= 32
+        if end > first:
+            assert first // b == (end - 1) // b == slot >> shift
+            seen += range(first, end)
+        k += 1
+    assert k == rules.units_per_batch(b) * nb and sorted(seen) == list(range(n))
