@@ -1962,15 +1962,20 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const WgradP P) {
 // the three planes of a window are one slot apart wherever it starts.
 // Warp 0 loads; warps 1 and 2 issue (dy = 0 and 1; dy = 2: separate
 // accumulators); every warp then adds the accumulators into dw.
-// Voxels outside the volume read zeros in both operands (an infinite X next
-// to a zero gradient row of the padding gives NaN, as it does next to a
-// zero inside the volume).
-// Warps 4 to 7 add the gradient planes up for the bias gradient meanwhile (in
-// the CTAs of the first input channel group): a launch of its own per layer
-// took 60 of the 1085 us of a gradient of 4 x 64^3 voxels, this nothing that
-// shows (16 -> 16 channels 36.9 us either way).
+// Voxels outside the volume read zeros in both operands, and a gradient row that
+// no voxel has meets X rows that exist: in the planes -1 and D, and in the rest of
+// a tile that the volume cuts. 0 x inf there would be the NaN of no voxel, and
+// the products of an infinite gradient with the padding's planes are left out.
+// So where such X rows or gradient planes hold a value that is not finite, the
+// CTA drops its accumulators and sums its share in plain FP32, voxel by voxel
+// (wgrad_plain).
+// Warps 4 to 7 look for those values, and add the gradient planes up for the
+// bias gradient (in the CTAs of the first input channel group): a launch of its
+// own per layer took 60 of the 1085 us of a gradient of 4 x 64^3 voxels, this
+// nothing that shows (16 -> 16 channels 36.9 us either way).
 struct WgradH {
-    Src vol;                     // sizes only
+    Src vol;                     // the operand X (a, ca channels) and the sizes
+    const __nv_bfloat16* dz;
     float* dw;                   // [27][cout][ld], accumulated at columns c_off ..
     float* db;                   // [cout], accumulated, or null
     int ld, c_off, cout;
@@ -1988,6 +1993,82 @@ __host__ __device__ constexpr uint32_t wh_smem_bytes(int ci, int co, int ring) {
 }
 __host__ __device__ constexpr uint32_t wh_tmem_cols(int co) { return co <= 16 ? 256u : 512u; }
 
+// A bit where any of the BF16 values of a buffer in shared memory is an infinity
+// or a NaN (an exponent of ones, to which one more carries into the sign's
+// place); thread t of 128 looks at every 128th 16-byte piece.
+template <int BYTES>
+__device__ __forceinline__ uint32_t not_finite(const uint8_t* p, int t) {
+    uint32_t bits = 0;
+#pragma unroll
+    for (int k = 0; k < (BYTES / 16 + 127) / 128; ++k)
+        if (k * 128 + t < BYTES / 16) {
+            const uint4 v = *reinterpret_cast<const uint4*>(p + (k * 128 + t) * 16);
+            bits |= ((v.x & 0x7f807f80u) + 0x00800080u) | ((v.y & 0x7f807f80u) + 0x00800080u) |
+                    ((v.z & 0x7f807f80u) + 0x00800080u) | ((v.w & 0x7f807f80u) + 0x00800080u);
+        }
+    return bits & 0x80008000u;
+}
+
+// The CTA's share of dw without the tensor core: every gradient voxel of the
+// volume with the X planes that the CTA owns, and at the volume's ends with the
+// padding's; the planes are PsWalk's (`left`: its position and end in the planes
+// left over after the whole columns). Rare (16 -> 16 on 4 x 64^3, every CTA: 14
+// ms), so it is kept out of the way of the rest: three sums per thread at a time,
+// and no 64-bit division (with those of a second PsWalk the finite ones took
+// 33.9 us instead of 32.8).
+template <int CI, int CO>
+__device__ __forceinline__ void wgrad_plain(const WgradH& P, const long long* left, int ci_lo, int co_lo) {
+    const Src& S = P.vol;
+    const int tiles_x = (S.W + 7) / 8, tiles_y = (S.H + 15) / 16, cols = S.B * tiles_y * tiles_x;
+    const int full = cols - cols % (int)gridDim.x;
+#pragma unroll 1
+    for (int e = threadIdx.x; e < 9 * CI * CO; e += THREADS) {
+        const int ci = ci_lo + e % CI, co = co_lo + e / CI % CO, t = e / (CI * CO), dz = t / 3 - 1, dy = t % 3 - 1;
+        float sum[3] = {0.0f, 0.0f, 0.0f};
+        long long a = left[0], end = left[1];                  // planes from the left-over columns' first on
+        int col = blockIdx.x;
+        bool whole = col < full;
+        if (!whole)
+            for (col = full; a >= S.D; a -= S.D, end -= S.D) ++col;
+#pragma unroll 1
+        while (whole || a < end) {
+            const int zs = whole ? 0 : (int)a, ze = whole || end > S.D ? S.D : (int)end;
+            const int n = col / (tiles_y * tiles_x), y0 = col / tiles_x % tiles_y * 16, x0 = col % tiles_x * 8;
+            const int z0 = zs == 0 ? -1 : zs, z1 = ze == S.D ? S.D + 1 : ze;      // X planes [z0, z1)
+            const int y1 = min(y0 + 16, S.H), x1 = min(x0 + 8, S.W);
+#pragma unroll 1
+            for (int gz = max(z0 - dz, 0); gz < min(z1 - dz, S.D); ++gz)
+#pragma unroll 1
+                for (int gy = y0; gy < y1; ++gy) {
+                    const int row = ((n * S.D + gz) * S.H + gy) * S.W;
+                    const bool inside = (unsigned)(gz + dz) < (unsigned)S.D && (unsigned)(gy + dy) < (unsigned)S.H;
+                    const __nv_bfloat16* g = P.dz + (long long)row * P.cout + co;
+                    const __nv_bfloat16* x = S.a + ((long long)row + (long long)dz * S.H * S.W + dy * S.W) * S.ca + ci;
+#pragma unroll 1
+                    for (int gx = x0; gx < x1; ++gx) {
+                        const float u = __bfloat162float(g[(long long)gx * P.cout]);
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            const bool in = inside && (unsigned)(gx + k - 1) < (unsigned)S.W;
+                            sum[k] = fmaf(in ? __bfloat162float(x[(long long)(gx + k - 1) * S.ca]) : 0.0f, u, sum[k]);
+                        }
+                    }
+                }
+            if (whole) {
+                col += gridDim.x;
+                whole = col < full;
+                if (!whole)
+                    for (col = full; a >= S.D; a -= S.D, end -= S.D) ++col;
+            } else {
+                a = 0, end -= S.D, ++col;
+            }
+        }
+        float* d = P.dw + ((size_t)(3 * t) * P.cout + co) * P.ld + P.c_off + ci;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) atomicAdd(d + (size_t)k * P.cout * P.ld, sum[k]);
+    }
+}
+
 template <int CI, int CO>
 __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_constant__ CUtensorMap xmap,
                                                              const __grid_constant__ CUtensorMap zmap,
@@ -1998,7 +2079,8 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t full[WH_RING_MAX], empty[WH_RING_MAX], done;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_fail;
+    __shared__ int s_fail, s_plain;
+    __shared__ long long s_left[2];
     __shared__ float s_db[CO];
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const Src& S = P.vol;
@@ -2011,10 +2093,10 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
     if (tid == 0) {
         for (uint32_t i = 0; i < R; ++i) {
             mbar_init(&full[i], 1);
-            mbar_init(&empty[i], sums ? 2 + 4 : 2);            // one commit per issuing warp, one arrival per summing warp
+            mbar_init(&empty[i], 2 + 4);                       // one commit per issuing warp, one arrival per reading warp
         }
         mbar_init(&done, 2);
-        s_fail = 0;
+        s_fail = s_plain = 0;
         mbar_init_fence();
     }
     if (tid < CO) s_db[tid] = 0.0f;
@@ -2087,18 +2169,26 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
         }
         if (elect_one()) mma_commit(&done);                    // arrives once every MMA issued above has finished
         __syncwarp();
-    } else if (sums && warp >= 4) {
-        // ---- bias gradient: each plane [zs, ze) of the gradient once, 8 channels of every (128 / CH)-th row per thread ----
+    } else if (warp >= 4) {
+        // ---- bias gradient: each plane [zs, ze) of the gradient once, 8 channels of every (128 / CH)-th row per thread;
+        // values that are not finite beside the padding ----
         constexpr int CH = CO / 8;
         const int chunk = lane % CH, row0 = (tid - 128) / CH;
         float f[8] = {};
         bool ok = true;
+        uint32_t plain = 0;
+        if (tid == 128) s_left[0] = walk.g, s_left[1] = walk.g_end;
         for (WsSeg q; ok && walk.next(S, q);) {
+            const bool cut = q.x0 + 8 > S.W || q.y0 + 16 > S.H;
             for (int i = 0; i < q.ze - q.zs + 2; ++i, ++L, ring_next(slot, ph, R)) {
                 ok = warp_wait_or_fail(&full[slot], ph, fail);
                 if (!ok) break;
-                if (i >= 1 && i <= q.ze - q.zs) {
-                    const uint8_t* plane = smem + (zbase - smem_u32(smem)) + slot * ZB;
+                const uint8_t* plane = smem + (zbase - smem_u32(smem)) + slot * ZB;
+                const int gz = q.zs - 1 + i, z = gz - 1;       // the step's planes of the gradient and of X
+                if (gz == 0 || gz == S.D - 1) plain |= not_finite<(int)ZB>(plane, tid - 128);
+                if (i >= 2 && (cut || z == 0 || z == S.D - 1))
+                    plain |= not_finite<RING_V * (int)AR>(smem + (xbase - smem_u32(smem)) + slot * XB, tid - 128);
+                if (sums && i >= 1 && i <= q.ze - q.zs) {
 #pragma unroll
                     for (int k = 0; k < CH; ++k) {
                         const int row = row0 + k * (TILE_M / CH);
@@ -2117,12 +2207,15 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
                 if (elect_one()) mbar_arrive(&empty[slot]);
             }
         }
+        if (sums) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < 8; ++c) {
 #pragma unroll
-            for (int m = CH; m < 32; m <<= 1) f[c] += __shfl_xor_sync(0xffffffffu, f[c], m);
-            if (lane < CH) atomicAdd(&s_db[8 * lane + c], f[c]);
+                for (int m = CH; m < 32; m <<= 1) f[c] += __shfl_xor_sync(0xffffffffu, f[c], m);
+                if (lane < CH) atomicAdd(&s_db[8 * lane + c], f[c]);
+            }
         }
+        if (plain) s_plain = 1;
     }
     // ---- epilogue: the accumulators into dw; lane quarter q holds dx = q ----
     mbar_wait_or_fail(&done, 0u, fail);
@@ -2133,7 +2226,9 @@ __global__ void __launch_bounds__(THREADS) wgrad_halo_kernel(const __grid_consta
     if (!*fail && any.next(S, first)) {
         if (sums && tid < CO) atomicAdd(P.db + co_lo + tid, s_db[tid]);
         const int dx = warp & 3, half = warp >> 2;
-        if (dx < 3) {
+        if (s_plain) {
+            wgrad_plain<CI, CO>(P, s_left, ci_lo, co_lo);
+        } else if (dx < 3) {
             for (int g = half; g < WH_DY * NP / 8; g += 2) {
                 const int col = 8 * g, dy = col / NP, z = 2 - (col / CO) % 3, co = co_lo + col % CO;
                 float f[8];
@@ -3094,7 +3189,8 @@ int launch_wgrad_halo(const void* x, int cx, int batch, int d, int h, int w, con
     });
     if (rc != CCU_OK) return rc;
     WgradH P;
-    P.vol = Src{nullptr, nullptr, 0, 0, batch, d, h, w};
+    P.vol = Src{(const __nv_bfloat16*)x, nullptr, cx, 0, batch, d, h, w};
+    P.dz = (const __nv_bfloat16*)dz;
     P.dw = dw;
     P.db = db;
     P.ld = ld;

@@ -193,3 +193,49 @@ def test_convolution_on_rings_that_five_planes_would_fit(U, cin, cout, split, di
     """Passes of 80 and 112 input channels, whose deepest ring (5 or 3 planes)
     two issuing warps may not use."""
     test_convolution_output_slices(U, cin, cout, split, dims, masked)
+
+
+@pytest.mark.parametrize("ca,cb,cout,dims", [
+    (16, 0, 16, (2, 5, 17, 9)),             # a row and a column of a tile's padding beside real voxels
+    (32, 0, 64, (1, 33, 16, 8)),            # whole tiles: only the planes -1 and D are padding
+    (16, 0, 32, (1, 1, 3, 5)),
+    (32, 64, 16, (1, 4, 18, 16)),           # concatenated
+    (16, 0, 16, (1, 2, 160, 237)),          # 300 columns: whole ones per CTA, and some left over
+])
+@pytest.mark.parametrize("where", ["x", "dz", "both"])
+def test_weight_gradient_of_infinities_and_nan(U, ca, cb, cout, dims, where):
+    """An infinity reaches the taps and channels whose sums contain it, and no
+    others; what stays finite is within the bound of the finite test."""
+    g = torch.Generator(device="cuda").manual_seed(ca + cout + dims[1])
+    n = dims[0] * dims[1] * dims[2] * dims[3]
+    coarse = (dims[0], *(s // 2 for s in dims[1:]))
+    x = torch.rand(*dims, ca, generator=g, device="cuda").add(0.5).to(torch.bfloat16)
+    b = torch.rand(*(coarse if cb else (1, 1, 1, 1)), max(cb, 1), generator=g, device="cuda").add(0.5).to(torch.bfloat16)
+    dz = torch.rand(*dims, cout, generator=g, device="cuda").add(0.5).to(torch.bfloat16)      # no zeros: 0 x inf is a NaN
+    if where != "dz":
+        x[0, 0, 0, 0, 3], x[-1, -1, -1, -1, 5] = float("inf"), -float("inf")
+        x[0, dims[1] // 2, -1, 0, 7] = float("nan")
+        b[0, 0, 0, 0, 0] = float("inf")
+    if where != "x":
+        dz[0, 0, 0, 0, 1], dz[-1, -1, -1, -1, 2] = float("inf"), float("inf")
+    dw, db = torch.zeros(27, cout, ca + cb, device="cuda"), torch.zeros(cout, device="cuda")
+    U.check(U.lib().ccu_conv3d_wgrad_bias(x.data_ptr(), ca, b.data_ptr() if cb else None, cb, *dims, dz.data_ptr(), cout,
+                                          dw.data_ptr(), db.data_ptr(), 2, torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert U.status() == 0
+    full = x.double()
+    if cb:
+        up = b.double().repeat_interleave(2, 1).repeat_interleave(2, 2).repeat_interleave(2, 3)
+        full = torch.cat([full, up], -1)
+    z = dz.double().reshape(n, cout)
+    finite = lambda t: torch.nan_to_num(t, nan=0.0, posinf=0.0, neginf=0.0)  # noqa: E731
+    for t, v in _taps(full):
+        v = v.reshape(n, ca + cb)
+        ref = torch.stack([(z[:, c, None] * v).sum(0) for c in range(cout)])
+        assert torch.equal(torch.isnan(dw[t]), torch.isnan(ref)), t
+        inf = torch.isinf(ref)
+        assert torch.equal(torch.isinf(dw[t]), inf) and torch.equal(dw[t][inf].sign().double(), ref[inf].sign()), t
+        keep = torch.isfinite(ref)
+        bound = (n + 1) * 2.0 ** -23 * (finite(z).abs().T @ finite(v).abs())
+        assert bool(((dw[t].double() - ref).abs() <= bound)[keep].all()), t
+    assert torch.equal(torch.isinf(db), torch.isinf(z.sum(0)))
