@@ -2991,6 +2991,7 @@ static int grid_blocks_for(cc_ctx* c, size_t smem, bool fs, bool tl, bool one_bl
         else if (fs) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<true, false>, c->block, smem);
         else if (tl) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<false, true>, c->block, smem);
         else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<false, false>, c->block, smem);
+        if (e != cudaSuccess) cudaGetLastError();      // one block per SM will do; not the launch's error
         if (e != cudaSuccess || occ < 1) occ = 1;
         per_sm = one_block ? 1 : occ;
     }
@@ -3645,8 +3646,10 @@ int cc_transport_photons_device_noalloc(const cc_scene* scene, const cc_tables* 
     int sms = 0, occ = 0;
     CC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, transport_kernel<false, false>, BLOCK, smem) != cudaSuccess ||
-        occ < 1)
+        occ < 1) {
+        cudaGetLastError();
         occ = 1;
+    }
     transport_kernel<false, false><<<sms * occ, BLOCK, smem, st>>>(tables->k, scene->k, G, S, R);
     CC_CUDA(cudaGetLastError());
     unsigned long long words[8 + MAX_MATS];
@@ -3784,16 +3787,19 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
             sc[k] = hi - lo;
         }
     }
-    if (b->tally) {
-        const cudaError_t e = heel ? allow_smem(batch_kernel<true, true>, smem) : allow_smem(batch_kernel<true>, smem);
+    // the kernel that the graph will hold: its shared memory, its occupancy and its launch
+    const auto kernel = b->tally ? (heel ? batch_kernel<true, true> : batch_kernel<true, false>)
+                                 : (heel ? batch_kernel<false, true> : batch_kernel<false, false>);
+    {
+        const cudaError_t e = allow_smem(kernel, smem);
         if (e != cudaSuccess) { batch_free(b); return set_error(CC_E_DEVICE, std::string("batch launch: ") + cudaGetErrorString(e)); }
     }
     // launch shape: the context's block size and blocks per SM (the autotuner sets them)
     int per_sm = c->blocks_per_sm;
     if (per_sm == 0) {
         int occ = 0;
-        cudaError_t oe = b->tally ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<true>, c->block, smem)
-                                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<false>, c->block, smem);
+        const cudaError_t oe = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, c->block, smem);
+        if (oe != cudaSuccess) cudaGetLastError();     // one block per SM will do; not the launch's error
         per_sm = (oe == cudaSuccess && occ > 0) ? occ : 1;
     }
     b->blocks = c->sm_count * per_sm;
@@ -3866,10 +3872,7 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
     if (e == cudaSuccess) e = cudaMemsetAsync(b->d_mem + o_c8, 0, total - o_c8, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_mem + o_run, b->h_run, 2 * sizeof(unsigned long long), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
-        if (b->tally && heel) batch_kernel<true, true><<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
-        else if (b->tally) batch_kernel<true><<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
-        else if (heel) batch_kernel<false, true><<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
-        else batch_kernel<false><<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
+        kernel<<<b->blocks, c->block, smem, st>>>(tables->k, k, R);
         e = cudaGetLastError();
         b->launches = 1;
     }

@@ -91,3 +91,45 @@ def test_autotuner_picks_and_caches_a_shape(engine, tmp_path, monkeypatch):
     assert shape in cands
     assert (tmp_path / "autotune.json").exists()
     assert batched.autotune(scenes, specs, counts, engine=engine, candidates=[]) == shape
+
+
+HEEL_FIRST = """
+import sys
+import numpy as np
+sys.path.insert(0, {root!r})
+import chatcarlo_b200.source as S
+from chatcarlo_b200 import phantoms as PH
+from chatcarlo_b200.batched import BatchedRun
+from chatcarlo_b200.transport import Engine
+g = np.load({golden!r})
+bins = (g["rect_centers"], tuple(zip(g["rect_spec_e"], g["rect_spec_w"])), g["rect_rel"], g["rect_rel"] * 1e6)
+S.heel_spectra_for_source = lambda src, sid, span, n_bins=15: bins
+scenes, specs = PH.phantoms(2, 4, side=32, voxel_cm=1.0)
+heel = [dict(scenes[0], source={{"position": [0, -100, 0], "direction": [0, 1, 0], "heel_effect": True, "kvp": 80,
+                                "field": {{"shape": "rect", "size_cm": [35, 43], "sid_cm": 100}},
+                                "anode_direction": [1.0, 0.3, 0.0]}}), scenes[1]]
+eng = Engine(0, precision="fp64")
+ms, counts = [], []
+for sc in (heel, scenes, heel):
+    br = BatchedRun(sc, specs, [1_000_000] * 2, engine=eng)
+    runs = [br.run(seed=1) for _ in range(6)]
+    ms.append(min(o.elapsed_ms for _, o in runs[1:]))
+    counts.append(runs[0][0])
+    br.close()
+assert np.array_equal(counts[0], counts[2]) and counts[0].sum() > 0
+print(*ms)
+"""
+
+
+def test_a_heel_source_in_the_first_batch_of_a_process():
+    """The FP64 engine's tallying batch asks for more than 48 KB of shared
+    memory: the kernel with the heel effect gets the same launch (two blocks
+    per SM, not one: 1.4 times the time) whether or not another batch ran before."""
+    import subprocess
+    import sys
+    from conftest import GOLDEN, ROOT
+    code = HEEL_FIRST.format(root=str(ROOT), golden=str(GOLDEN / "heel.npz"))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    first, _, again = map(float, r.stdout.split())
+    assert first < 1.1 * again, r.stdout
