@@ -2103,8 +2103,14 @@ static int dev_upload(std::vector<void*>& allocs, const std::vector<T>& v, const
 // Shared memory beyond 48 KB has to be asked for (the FP64 build's records).
 template <typename K>
 static cudaError_t allow_smem(K kernel, size_t smem) {
+    static SmemLimits limits;
     if (smem <= (size_t)48 << 10) return cudaSuccess;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)limits.raise((const void*)kernel, dev, smem, [&](size_t bytes) {
+        return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    });
 }
 
 template <bool FS, bool TL, bool HEEL, int TV>

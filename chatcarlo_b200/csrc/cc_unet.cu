@@ -2755,7 +2755,10 @@ int tc_launch_smem(K kernel, size_t stages_bytes, uint32_t cols, size_t& smem, i
     const size_t floor_smem = (size_t)per_sm / (size_t)(max_ctas + 1) + 1024;
     if (smem < floor_smem) smem = floor_smem;
     if (smem > PS_SMEM_MAX) return set_error(CCU_E_INVALID, "stages too large for shared memory");
-    CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static cc::SmemLimits limits;              // per kernel type; the kernel and the device are its keys
+    CU_CHECK((cudaError_t)limits.raise((const void*)kernel, dev, smem, [&](size_t bytes) {
+        return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    }));
     CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   (int)cudaSharedmemCarveoutMaxShared));
     int occ = 0;
@@ -3009,8 +3012,6 @@ int launch_conv_pair_g(const ConvP& P, int n_out, int co_lo, cudaStream_t st) {
         for (int r = 3; r <= WS_RING_MAX && pair_smem_bytes(a16, b16, r) <= PS_SMEM_MAX; ++r)
             if (ps_ring_allowed(r, 1)) p.ring = r;
         const int r_c = tc_launch_smem(kernel, pair_smem_bytes(a16, b16, p.ring), ps_tmem_cols(32, 1), p.smem, ps_threads(32));
-        // one kernel serves several splits into a and b, each with its own ring: allow it the largest
-        CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS_SMEM_MAX));
         return r_c == CCU_OK ? resident_ctas(kernel, p.smem, ps_tmem_cols(32, 1), p.resident, ps_threads(32)) : r_c;
     });
     if (rc != CCU_OK) return rc;

@@ -2,6 +2,12 @@
 // the tests can check them on the host over their whole range.
 #pragma once
 
+#include <stddef.h>
+
+#include <map>
+#include <mutex>
+#include <utility>
+
 #ifdef __CUDACC__
 #define CC_RULE __host__ __device__ __forceinline__
 #else
@@ -59,5 +65,28 @@ CC_RULE bool unit_at(long long k, long long n, long long batch_size, int n_batch
 
 // Batches of n > 0 histories (no overflow at the largest batch sizes).
 CC_RULE long long batches_of(long long n, long long batch_size) { return (n - 1) / batch_size + 1; }
+
+// The dynamic shared memory that kernels are allowed. The limit belongs to a
+// kernel on a device, whichever context or thread launches it, and launches
+// differ in size: set to each launch's own, one thread's smaller size between
+// another's setting and its launch makes that launch fail. So it only rises.
+class SmemLimits {
+public:
+    // set(bytes): the limit of this kernel on this device to the most that any
+    // call asked for; returns what it returns (0: success).
+    template <typename Set>
+    int raise(const void* kernel, int device, size_t bytes, Set set) {
+        std::lock_guard<std::mutex> lock(mu_);
+        size_t& most = most_[std::make_pair(kernel, device)];
+        const size_t want = bytes > most ? bytes : most;
+        const int e = set(want);
+        if (e == 0) most = want;
+        return e;
+    }
+
+private:
+    std::mutex mu_;
+    std::map<std::pair<const void*, int>, size_t> most_;
+};
 
 }  // namespace cc

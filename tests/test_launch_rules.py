@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import ctypes as C
 import subprocess
+import threading
 from pathlib import Path
 
 import pytest
@@ -21,6 +22,15 @@ extern "C" int unit_at(long long k, long long n, long long batch_size, int n_bat
     out[2] = slot;
     return ok;
 }
+static cc::SmemLimits limits;
+static size_t allowed[4];           // what the device would hold, by kernel (a fake of it)
+extern "C" size_t allow(long kernel, int device, size_t bytes, int fail) {
+    const int e = limits.raise((const void*)kernel, device, bytes, [&](size_t most) {
+        if (!fail) allowed[kernel] = most;
+        return fail;
+    });
+    return e ? 0 : allowed[kernel];
+}
 """
 
 
@@ -33,6 +43,7 @@ def rules(tmp_path_factory):
     lib = C.CDLL(str(d / "shim.so"))
     for f in (lib.unit_batch, lib.batches_of, lib.units_per_batch):
         f.restype, f.argtypes = C.c_longlong, [C.c_longlong] * (1 if f is lib.units_per_batch else 2)
+    lib.allow.restype, lib.allow.argtypes = C.c_size_t, [C.c_long, C.c_int, C.c_size_t, C.c_int]
     lib.unit_at.argtypes = [C.c_longlong] * 3 + [C.c_int] * 3 + [C.c_void_p]
     return lib
 
@@ -130,3 +141,24 @@ def test_units_cover_every_history_once(rules, n, size, group, shift):
             seen += range(first, end)
         k += 1
     assert k == rules.units_per_batch(b) * nb and sorted(seen) == list(range(n))
+
+
+def test_shared_memory_limits_only_rise(rules):
+    """A launch's own size set between another thread's setting and its launch
+    would make that launch fail; a failed setting is not taken for a limit."""
+    assert rules.allow(0, 0, 60_000, 0) == 60_000
+    assert rules.allow(0, 0, 50_000, 0) == 60_000
+    assert rules.allow(0, 0, 90_000, 7) == 0 and rules.allow(0, 0, 70_000, 0) == 70_000
+    assert rules.allow(1, 0, 50_000, 0) == 50_000                  # another kernel
+    assert rules.allow(0, 1, 55_000, 0) == 55_000                  # another device
+    seen = []
+
+    def work(bytes_):
+        seen.append(all(rules.allow(2, 0, bytes_, 0) >= bytes_ for _ in range(20_000)))
+
+    threads = [threading.Thread(target=work, args=(b,)) for b in (50_000, 80_000, 60_000)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert seen == [True] * 3
