@@ -31,6 +31,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <unordered_set>
 #include <vector>
 
 #include "launch_rules.h"
@@ -1774,10 +1775,12 @@ __global__ void fold_plain_kernel(double2* __restrict__ total, double2* __restri
 }
 
 // fold_plain_kernel on every scene of a batch (blockIdx.y): 24 launches of 3 us
-// each in the graph of a 24-scene batch otherwise.
+// each in the graph of a 24-scene batch otherwise. A grid that several scenes
+// score into has its totals at the first of them only: one row folds it.
 __global__ void fold_plain_scenes_kernel(const KGrid* __restrict__ grids, double2* const* __restrict__ totals) {
     const KGrid& G = grids[blockIdx.y];
     double2* const total = totals[blockIdx.y];
+    if (!total) return;
     double2* const scratch = reinterpret_cast<double2*>(G.tally);
     const long long nvox = G.nvox;
     const int cell32 = G.tally32;
@@ -1796,6 +1799,7 @@ __global__ void fold_plain_scenes_kernel(const KGrid* __restrict__ grids, double
 // The totals of every scene of a batch to zero (blockIdx.y).
 __global__ void zero_scenes_kernel(const KGrid* __restrict__ grids, double2* const* __restrict__ totals) {
     double2* const total = totals[blockIdx.y];
+    if (!total) return;
     const long long nvox = grids[blockIdx.y].nvox;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvox; i += (long long)gridDim.x * blockDim.x)
         total[i] = make_double2(0.0, 0.0);
@@ -3694,7 +3698,7 @@ struct cc_batch {
     unsigned long long* h_run = nullptr;      // pinned: seed, fluorescence
     unsigned long long* d_counters = nullptr; // [8]: 4 steps, 5 voxel visits, 6 work
     unsigned* d_status = nullptr;
-    double2** d_totals = nullptr;             // [n_scenes] totals of the scenes' grids
+    double2** d_totals = nullptr;             // [n_scenes] totals of the scenes' grids, null where an earlier scene has the grid
     long long max_vox = 0;                    // largest grid
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -3843,8 +3847,9 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
     if (e == cudaSuccess && b->tally) e = cudaMemcpy(b->d_mem + o_g, hg.data(), sizeof(KGrid) * n_scenes, cudaMemcpyHostToDevice);
     b->d_totals = (double2**)(b->d_mem + o_tot);
     std::vector<double2*> totals(n_scenes, nullptr);
+    std::unordered_set<const cc_grid*> seen;
     for (size_t i = 0; i < b->grids.size(); ++i) {
-        totals[i] = (double2*)b->grids[i]->d_total;
+        if (seen.insert(b->grids[i]).second) totals[i] = (double2*)b->grids[i]->d_total;
         b->max_vox = std::max(b->max_vox, b->grids[i]->k.nvox);
     }
     if (e == cudaSuccess) e = cudaMemcpy(b->d_totals, totals.data(), sizeof(double2*) * n_scenes, cudaMemcpyHostToDevice);

@@ -335,7 +335,8 @@ int cc_transport_photons_device_noalloc(const cc_scene* scene, const cc_tables* 
  * histories that never span two scenes; history i of scene s draws the
  * Philox stream of history (s << 40) + i.  With slots > 1 (grids created
  * with CC_GRID_STATS) each scene's histories form `slots` batches for the
- * batch statistics.  cc_batch_create captures the whole sequence (counter
+ * batch statistics; a grid named for several scenes holds their sum.
+ * cc_batch_create captures the whole sequence (counter
  * reset, transport, batch folds) in a CUDA graph; cc_batch_run replays it.
  * The launch shape is the context's (cc_ctx_set_launch).  scene_counts gets
  * [n_scenes][4] absorbed, escaped, interactions, fluorescence emissions. */

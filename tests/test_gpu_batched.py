@@ -133,3 +133,30 @@ def test_a_heel_source_in_the_first_batch_of_a_process():
     assert r.returncode == 0, r.stderr
     first, _, again = map(float, r.stdout.split())
     assert first < 1.1 * again, r.stdout
+
+
+@pytest.mark.parametrize("scenes_n", [2, 9])
+def test_scenes_that_share_a_grid_are_summed_once(engine, scenes_n):
+    """One grid handle for several scenes holds the sum of their scores."""
+    from chatcarlo_b200 import phantoms as PH
+    from chatcarlo_b200.batched import BatchedRun
+    scenes, specs = PH.phantoms(1, 4, side=48, voxel_cm=0.7)
+    br = BatchedRun(scenes * scenes_n, specs * scenes_n, [30_000 + 1_000 * i for i in range(scenes_n)], engine=engine)
+    try:
+        br.run(seed=3)
+        each = [(g.kerma_keV.copy(), g.h10_track_pSv_cm3.copy()) for g in br.download()]
+        own = list(br.dgrids)
+        br.dgrids = [own[0]] * scenes_n
+        br._build()
+        br.reset()
+        for turns in (1, 2):
+            br.run(seed=3)
+            got = br.download()[0]
+            for k, a in enumerate((got.kerma_keV, got.h10_track_pSv_cm3)):
+                # FP64 additions of positive numbers, fewer than 2^17 per voxel
+                np.testing.assert_allclose(a, turns * sum(e[k] for e in each), rtol=2.0 ** -36, atol=0)
+        br.reset()
+        assert br.download()[0].kerma_keV.max() == 0.0
+        br.dgrids = own
+    finally:
+        br.close()
