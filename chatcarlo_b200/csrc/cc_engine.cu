@@ -2084,6 +2084,12 @@ struct cc_grid {
     // that cc_grid_reset clears the slots (33 of 246 MB on the CT grid, 1.25 ms)
     // only where something is left in them
     bool scratch_dirty = false;
+    // A batch's graph scores into the scratch it was captured with and leaves it
+    // cleared. Once one has, the blocks that larger ones replace are kept, and
+    // freed with the grid: a run that needs more slots must not free them under
+    // the graph.
+    bool captured = false;
+    std::vector<double*> old_scratch;
     char* d_out = nullptr;          // download staging: kerma, h10, kerma_sum2, h10_sum2 (f64), n_hit (i32)
     double* d_maps = nullptr;       // cc_grid_maps staging: 4 maps (f64), allocated on first use
     double origin64[3] = {0, 0, 0}; // the caller's FP64 origin and voxel edge (the kernels track in FP32)
@@ -2573,10 +2579,12 @@ static int grid_alloc_scratch(cc_grid* g, int n) {
     CC_CUDA(cudaMalloc(&p, bytes));
     CC_CUDA(cudaMemsetAsync(p, 0, bytes, g->ctx->stream));
     if (g->d_scratch) {
-        CC_CUDA(cudaMemcpyAsync(p, g->d_scratch, (size_t)g->n_scratch * 2 * g->k.nvox * sizeof(double),
-                                cudaMemcpyDeviceToDevice, g->ctx->stream));
+        const size_t old = (size_t)g->n_scratch * 2 * g->k.nvox * sizeof(double);
+        CC_CUDA(cudaMemcpyAsync(p, g->d_scratch, old, cudaMemcpyDeviceToDevice, g->ctx->stream));
+        if (g->captured) CC_CUDA(cudaMemsetAsync(g->d_scratch, 0, old, g->ctx->stream));      // its scores have moved
         CC_CUDA(cudaStreamSynchronize(g->ctx->stream));
-        cudaFree(g->d_scratch);
+        if (g->captured) g->old_scratch.push_back(g->d_scratch);
+        else cudaFree(g->d_scratch);
     }
     g->d_scratch = p;
     g->n_scratch = n;
@@ -2626,6 +2634,7 @@ int cc_grid_destroy(cc_grid* g) {
     cudaFree(g->d_q);
     cudaFree(g->d_nhit);
     cudaFree(g->d_scratch);
+    for (double* p : g->old_scratch) cudaFree(p);
     cudaFree(g->d_out);
     cudaFree(g->d_maps);
     cudaFreeHost(g->h_out);
@@ -3785,6 +3794,7 @@ int cc_batch_create(cc_ctx* c, const cc_tables* tables, int32_t n_scenes, const 
             if (slots > 1) { int rc = grid_alloc_scratch(g, slots); if (rc != CC_OK) { batch_free(b); return rc; } }
             hg[i] = g->k;
             hg[i].tally = g->d_scratch;
+            g->captured = true;
             hg[i].tally32 = cell32_for(c, (n_histories[i] + slots - 1) / slots);
             b->grids.push_back(g);
         }

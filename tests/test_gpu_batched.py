@@ -160,3 +160,41 @@ def test_scenes_that_share_a_grid_are_summed_once(engine, scenes_n):
         br.dgrids = own
     finally:
         br.close()
+
+
+@pytest.mark.parametrize("batch_size", [5_000_000, 1_000])
+def test_a_run_that_grows_a_grid_leaves_its_batch_usable(engine, batch_size):
+    """A run on a batch's grid takes more scratch slots than the batch was
+    captured with; both then add their scores to the grid."""
+    from chatcarlo_b200 import _native as N
+    from chatcarlo_b200 import phantoms as PH
+    from chatcarlo_b200.batched import BatchedRun
+    scenes, specs = PH.phantoms(2, 4, side=40, voxel_cm=0.8)
+    scenes[0] = dict(scenes[0], source=dict(scenes[0]["source"], field={"shape": "parallel", "size_cm": [2.0, 2.0]}))
+    br = BatchedRun(scenes, specs, [40_000, 50_000], engine=engine)
+    out, edep = N.RunOut(), np.zeros(len(br.ts.names))
+
+    def run_on_the_first_grid():
+        N.check(engine.lib.cc_run(engine.ctx, br.scene_h[0], br.th, br.source_h[0], br.dgrids[0].handle, 20_000, batch_size,
+                                  7, 0, 1, N.dptr(edep), None, out))
+
+    def totals():
+        return [g.kerma_keV.copy() for g in br.download()]
+
+    try:
+        br.run(seed=3)
+        batch = totals()
+        br.reset()
+        run_on_the_first_grid()
+        run = totals()
+        assert run[0].sum() > 0 and run[1].max() == 0.0
+        br.run(seed=3)
+        for got, a, b in zip(totals(), run, batch):
+            # FP64 additions of positive numbers, fewer than 2^17 per voxel
+            np.testing.assert_allclose(got, a + b, rtol=2.0 ** -36, atol=0)
+        br.reset()
+        br.run(seed=3)
+        for got, b in zip(totals(), batch):
+            np.testing.assert_allclose(got, b, rtol=2.0 ** -36, atol=0)
+    finally:
+        br.close()
