@@ -7,12 +7,14 @@ folds, captured once as a CUDA graph and replayed by ``run``.
 
 ``autotune`` times a few launch shapes (block size, blocks per SM, histories
 per chunk) on a scaled-down copy of the plan and keeps the fastest in a
-JSON cache keyed by the GPU and the workload, so later runs of the same
-workload start from it.
+JSON cache keyed by the GPU, the build of the kernels and the workload, so
+later runs of the same workload start from it.
 """
 from __future__ import annotations
 
 import ctypes as C
+import functools
+import hashlib
 import json
 import os
 import time
@@ -114,6 +116,18 @@ def _gpu_key(engine: Engine) -> str:
         return f"device{engine.device}"
 
 
+@functools.lru_cache(maxsize=8)
+def _file_digest(path: str, mtime_ns: int, size: int) -> str:
+    return hashlib.blake2b(Path(path).read_bytes(), digest_size=6).hexdigest()
+
+
+def _kernels_key(engine: Engine) -> str:
+    """The build of the engine's kernels: a shape that was the fastest for
+    others, with other registers and shared memory, is not taken over."""
+    st = os.stat(engine.lib._name)
+    return _file_digest(engine.lib._name, st.st_mtime_ns, st.st_size)
+
+
 def workload_key(n_histories: list[int], slots: int, tally: bool) -> str:
     n = len(n_histories)
     tot = int(sum(n_histories))
@@ -125,7 +139,7 @@ def autotune(scenes, grid_specs, n_histories, slots=1, engine=None, scale=0.02,
     """Fastest launch shape for this workload: times each candidate on a plan
     with the history counts scaled by `scale` (at least 20,000 per scene)."""
     eng = engine or default_engine()
-    key = f"{_gpu_key(eng)}|{workload_key(n_histories, slots, grid_specs is not None)}"
+    key = f"{_gpu_key(eng)}|{_kernels_key(eng)}|{workload_key(n_histories, slots, grid_specs is not None)}"
     cache = {}
     if use_cache and CACHE_PATH.exists():
         try:

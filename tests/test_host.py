@@ -380,3 +380,25 @@ def test_heel_descriptor_from_supplied_bins(monkeypatch):
     assert sum(h.bin_sizes[i] for i in range(15)) == sum(len(e) for e, _ in spectra)
     with pytest.raises(ValueError):
         S.SourceSpec(dict(src, field={"shape": "parallel", "size_cm": [10, 10]}))
+
+
+def test_autotuned_shapes_belong_to_a_build_of_the_kernels(tmp_path, monkeypatch):
+    """A launch shape that an earlier build cached is tuned again; one of this
+    build is returned."""
+    import json
+    from types import SimpleNamespace
+    from chatcarlo_b200 import batched
+    lib, cache = tmp_path / "lib.so", tmp_path / "autotune.json"
+    lib.write_bytes(b"first build")
+    eng = SimpleNamespace(device=0, lib=SimpleNamespace(_name=str(lib)))
+    monkeypatch.setattr(batched, "CACHE_PATH", cache)
+    shape, counts = {"block": 256, "blocks_per_sm": 4, "chunk": 256}, [100_000, 20_000]
+    gpu, work = batched._gpu_key(eng), batched.workload_key(counts, 1, True)
+    cache.write_text(json.dumps({f"{gpu}|{work}": {"shape": shape}}))
+    with pytest.raises(IndexError):                   # nothing cached, and no candidates to time
+        batched.autotune([], [{}, {}], counts, engine=eng, candidates=[])
+    cache.write_text(json.dumps({f"{gpu}|{batched._kernels_key(eng)}|{work}": {"shape": shape}}))
+    assert batched.autotune([], [{}, {}], counts, engine=eng, candidates=[]) == shape
+    lib.write_bytes(b"another build")
+    with pytest.raises(IndexError):
+        batched.autotune([], [{}, {}], counts, engine=eng, candidates=[])
