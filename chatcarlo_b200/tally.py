@@ -9,7 +9,7 @@ sigma^2 = (Q - T^2/N)/(M-1) with T = sum S_b, Q = sum S_b^2/n_b.
 """
 from __future__ import annotations
 
-from dataclasses import dataclass, field
+from dataclasses import InitVar, dataclass, field
 
 import numpy as np
 
@@ -40,7 +40,6 @@ class VoxelGrid:
     voxel_size_cm: float
     track_uncertainty: bool = False
     pinned: bool = False            # page-locked arrays: the device writes results straight into them
-    zeroed: bool = True             # False: the arrays start unfilled, for a caller that overwrites all of them
     kerma_keV: np.ndarray = field(init=False)
     h10_track_pSv_cm3: np.ndarray = field(init=False)
     kerma_sum2: np.ndarray = field(init=False, default=None)
@@ -48,16 +47,19 @@ class VoxelGrid:
     n_batches_hit: np.ndarray = field(init=False, default=None)
     n_batches: int = field(init=False, default=0)
     n_histories: int = field(init=False, default=0)
+    # False: the arrays start unfilled, for a caller that overwrites all of them.
+    # Not kept with the grid: one made from it (dataclasses.replace) is zeroed.
+    zeroed: InitVar[bool] = True
 
-    def __post_init__(self):
+    def __post_init__(self, zeroed):
         self.origin_cm = np.asarray(self.origin_cm, dtype=float)
         self.shape = tuple(int(s) for s in self.shape)
-        self.kerma_keV = host_zeros(self.shape, pinned=self.pinned, zeroed=self.zeroed)
-        self.h10_track_pSv_cm3 = host_zeros(self.shape, pinned=self.pinned, zeroed=self.zeroed)
+        self.kerma_keV = host_zeros(self.shape, pinned=self.pinned, zeroed=zeroed)
+        self.h10_track_pSv_cm3 = host_zeros(self.shape, pinned=self.pinned, zeroed=zeroed)
         if self.track_uncertainty:
-            self.kerma_sum2 = host_zeros(self.shape, pinned=self.pinned, zeroed=self.zeroed)
-            self.h10_sum2 = host_zeros(self.shape, pinned=self.pinned, zeroed=self.zeroed)
-            self.n_batches_hit = host_zeros(self.shape, np.int32, pinned=self.pinned, zeroed=self.zeroed)
+            self.kerma_sum2 = host_zeros(self.shape, pinned=self.pinned, zeroed=zeroed)
+            self.h10_sum2 = host_zeros(self.shape, pinned=self.pinned, zeroed=zeroed)
+            self.n_batches_hit = host_zeros(self.shape, np.int32, pinned=self.pinned, zeroed=zeroed)
 
     @classmethod
     def from_bbox(cls, bbox_min, bbox_max, resolution_cm: float, track_uncertainty: bool = False,

@@ -402,3 +402,21 @@ def test_autotuned_shapes_belong_to_a_build_of_the_kernels(tmp_path, monkeypatch
     lib.write_bytes(b"another build")
     with pytest.raises(IndexError):
         batched.autotune([], [{}, {}], counts, engine=eng, candidates=[])
+
+
+def test_grids_made_from_an_unfilled_grid_are_zeroed(monkeypatch):
+    """A grid whose arrays start unfilled is equal in kind to any other: what is
+    made from it starts at zero."""
+    import copy
+    import dataclasses
+    from chatcarlo_b200 import tally
+    # an allocation with something in it
+    monkeypatch.setattr(tally.np, "empty", lambda shape, dtype=np.float64: np.full(shape, 7, dtype))
+    g = tally.VoxelGrid(origin_cm=[0, 0, 0], shape=(2, 3, 4), voxel_size_cm=1.0, track_uncertainty=True, zeroed=False)
+    assert g.kerma_keV.min() == 7 and g.n_batches_hit.min() == 7
+    new = dataclasses.replace(g, voxel_size_cm=2.0)
+    for a in (new.kerma_keV, new.h10_track_pSv_cm3, new.kerma_sum2, new.h10_sum2, new.n_batches_hit):
+        assert a.shape == (2, 3, 4) and a.max() == 0
+    assert copy.deepcopy(g).kerma_keV.min() == 7
+    assert {f.name for f in dataclasses.fields(g)} == {f.name for f in dataclasses.fields(new)} and "zeroed" not in repr(g)
+    assert tally.VoxelGrid.from_bbox([0, 0, 0], [2, 2, 2], 1.0, zeroed=False).kerma_keV.min() == 7
