@@ -2955,7 +2955,7 @@ static double beam_faces(const KSource& S, const cc_grid* g) {
 // Beams of fewer voxel faces than NARROW_FACES score SPREAD_SLOTS slots at a
 // time whatever their size, the others as many as GROUP_BYTES hold, and with
 // slots above SLOT_BYTES_COMPACT one block per SM once those that the
-// histories of four (FULL_HISTORIES) reach exceed LIVE_BYTES.  Device time of
+// histories of four (FULL_BLOCKS) reach exceed LIVE_BYTES.  Device time of
 // 1.4e6 histories in batches of 200,000 (ms; 1, 2, 4, 8 slots at a time with
 // four blocks per SM, and 1 slot with one block):
 //   room, source in the grid, slot  47 MB  9.4  7.8  6.4  5.5 | 10.0
@@ -2977,9 +2977,9 @@ static double beam_faces(const KSource& S, const cc_grid* g) {
 constexpr double NARROW_FACES = 32;
 constexpr size_t GROUP_BYTES = (size_t)64 << 20, LIVE_BYTES = (size_t)96 << 20;
 constexpr double COPY_BYTES_PER_HISTORY = 16384;
-constexpr double FULL_HISTORIES = 4 * 148 * BLOCK;
+constexpr double FULL_BLOCKS = 4;
 
-static SlotOrder slot_order(const KSource* src, const cc_grid* grid, long long batch_size) {
+static SlotOrder slot_order(const cc_ctx* c, const KSource* src, const cc_grid* grid, long long batch_size) {
     SlotOrder O;
     if (!grid) return O;
     const size_t per = (size_t)grid->k.nvox * 16;
@@ -2991,7 +2991,8 @@ static SlotOrder slot_order(const KSource* src, const cc_grid* grid, long long b
         O.copies = O.lockstep = true;
     } else {
         O.group = (int)std::max<size_t>(1, std::min<size_t>(SPREAD_SLOTS, GROUP_BYTES / per));
-        O.one_block = large && (double)per * (1.0 + FULL_HISTORIES / (double)batch_size) > (double)LIVE_BYTES;
+        const double in_flight = FULL_BLOCKS * c->sm_count * BLOCK;
+        O.one_block = large && (double)per * (1.0 + in_flight / (double)batch_size) > (double)LIVE_BYTES;
         O.lockstep = !large;
     }
     return O;
@@ -3047,7 +3048,7 @@ static int enqueue_launch(cc_ctx* c, const cc_scene* scene, const cc_tables* tab
     const KTables& T = tables->k;
     R.n_scratch = n_slots;
     R.batch_size = unit_batch(batch_size, R.n);
-    const SlotOrder order = slot_order(src, grid, batch_size);
+    const SlotOrder order = slot_order(c, src, grid, batch_size);
     R.group = order.group;
     R.copy_shift = copy_shift;
     R.max_steps = c->max_steps;
@@ -3380,7 +3381,7 @@ int cc_run(cc_ctx* c, const cc_scene* scene, const cc_tables* tables, const cc_s
     // statistics need that, and FP32 cells must not sum more than a batch)
     const bool slotted = grid != nullptr;
     const int cell32 = slotted ? cell32_for(c, batch_size) : 0;
-    const SlotOrder order = slot_order(&src->k, grid, batch_size);
+    const SlotOrder order = slot_order(c, &src->k, grid, batch_size);
     if (grid) {
         size_t per = (size_t)grid->k.nvox * 2 * sizeof(double);
         size_t budget = (size_t)8 << 30;
