@@ -3339,11 +3339,17 @@ int ccu_conv3d_wgrad_bias(const void* a, int ca, const void* b, int cb, int batc
     // per-device buffer: only for the shapes documented to use that buffer
     auto box_channels = [](int c) { return c == 16 || c == 32 || c % 64 == 0; };
     if (g_wgrad_path == 0 && (cb == 0 || (w % 8 == 0 && box_channels(ca) && box_channels(cb)))) {
+        // Groups of 16 output channels for 16, and where the planes times those groups are fewer than the SMs: a CTA
+        // then has a plane or so, and adding its accumulators into dw is most of its time (32 -> 32 on 8^3 voxels,
+        // cleared before, 10.4 us with a group of 32, 8.5 with two of 16; 32 -> 64 on 2 x 8^3 10.3 and 8.8). With
+        // more planes the gradient's second reading costs more (32 -> 32 on 4 x 16^3 12.35 and 13.25).
+        const long long planes = (long long)batch * ((h + 15) / 16) * ((w + 7) / 8) * d;
+        auto narrow = [&](int ci_groups) { return cout == 16 || ci_groups * (cout / 16) * planes <= sm_count(); };
         auto run = [&](const void* x, int cx, int c_off, float* sums) {
             if (cx % 32 == 0)
-                return cout == 16 ? launch_wgrad_halo<32, 16>(x, cx, batch, d, h, w, dz, cout, dw, sums, ca + cb, c_off, slices, st)
+                return narrow(cx / 32) ? launch_wgrad_halo<32, 16>(x, cx, batch, d, h, w, dz, cout, dw, sums, ca + cb, c_off, slices, st)
                                   : launch_wgrad_halo<32, 32>(x, cx, batch, d, h, w, dz, cout, dw, sums, ca + cb, c_off, slices, st);
-            return cout == 16 ? launch_wgrad_halo<16, 16>(x, cx, batch, d, h, w, dz, cout, dw, sums, ca + cb, c_off, slices, st)
+            return narrow(cx / 16) ? launch_wgrad_halo<16, 16>(x, cx, batch, d, h, w, dz, cout, dw, sums, ca + cb, c_off, slices, st)
                               : launch_wgrad_halo<16, 32>(x, cx, batch, d, h, w, dz, cout, dw, sums, ca + cb, c_off, slices, st);
         };
         if (cb == 0) return run(a, ca, 0, db);

@@ -239,3 +239,15 @@ def test_weight_gradient_of_infinities_and_nan(U, ca, cb, cout, dims, where):
         bound = (n + 1) * 2.0 ** -23 * (finite(z).abs().T @ finite(v).abs())
         assert bool(((dw[t].double() - ref).abs() <= bound)[keep].all()), t
     assert torch.equal(torch.isinf(db), torch.isinf(z.sum(0)))
+
+
+@pytest.mark.parametrize("ca,cout,planes", [
+    (16, 32, 74), (16, 32, 75),             # 2 groups of 16 output channels x planes: 148 SMs, and beyond
+    (32, 128, 18), (32, 128, 19),           # 8 groups
+    (64, 64, 18), (64, 64, 300),            # 2 groups of input channels x 4
+])
+def test_weight_gradient_on_both_sides_of_the_group_rule(U, ca, cout, planes):
+    """Groups of 16 and of 32 output channels, at the line between them."""
+    test_weight_gradient_halo_planes(U, ca, cout, (1, planes, 13, 7), 1)
+    test_bias_gradient_beside_the_weight_gradient(U, ca, 0, cout, (1, planes, 13, 7), 1, 0)
+    test_weight_gradient_of_infinities_and_nan(U, ca, 0, cout, (1, planes, 13, 7), "both")
