@@ -251,3 +251,29 @@ def test_weight_gradient_on_both_sides_of_the_group_rule(U, ca, cout, planes):
     test_weight_gradient_halo_planes(U, ca, cout, (1, planes, 13, 7), 1)
     test_bias_gradient_beside_the_weight_gradient(U, ca, 0, cout, (1, planes, 13, 7), 1, 0)
     test_weight_gradient_of_infinities_and_nan(U, ca, 0, cout, (1, planes, 13, 7), "both")
+
+
+def _on_pairs(cin, dims):
+    """Whether a slice of 16 output channels runs on pairs of voxels: an even
+    width, 32 or 48 input channels, little padding and enough planes per SM."""
+    b, d, h, w = dims
+    planes = b * d * -(-h // 16) * -(-w // 16)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return w % 2 == 0 and cin in (32, 48) and -(-w // 16) * 16 * 5 <= -(-w // 8) * 8 * 6 and planes >= sms * (10 if cin == 48 else 20)
+
+
+@pytest.mark.parametrize("cin,cout,split,dims,pairs", [
+    (32, 16, 16, (2, 250, 33, 30), True),   # ragged in y and x
+    (48, 16, 8, (1, 380, 31, 32), True),    # the split between the two halves of a voxel
+    (32, 48, 16, (2, 250, 33, 30), True),   # the last 16 of 48 channels, all of them in the second output
+    (48, 48, 40, (1, 380, 31, 32), True),   # the split inside that slice
+    (48, 48, 16, (1, 600, 33, 24), False),  # 24 voxels would pad to 32
+    (32, 48, 40, (2, 250, 33, 31), False),  # an odd width
+    (32, 16, 16, (1, 900, 17, 16), False),  # 1800 planes: too few
+])
+@pytest.mark.parametrize("masked", [False, True])
+def test_pairs_of_voxels_against_fp64(U, cin, cout, split, dims, pairs, masked):
+    """The slices on pairs of voxels, and their neighbours that run without,
+    against the sums in FP64."""
+    assert _on_pairs(cin, dims) == pairs
+    test_convolution_output_slices(U, cin, cout, split, dims, masked)
