@@ -2779,11 +2779,10 @@ int launch_conv(const ConvP& P, cudaStream_t st) {
     return CCU_OK;
 }
 
-// 0: the plane-stationary kernel where it applies, else the streaming halo
-// kernel where it applies, else the gathering kernel; 1: always the
-// gathering kernel; 2: the one-tile halo kernel where it applies; 3: the
-// warp-role streaming kernel where the streaming kernel applies; 4: path 0
-// without the plane-stationary kernel
+// 0: the plane-stationary kernel where it applies, else the gathering kernel;
+// 1: always the gathering kernel; for comparisons, where they apply, 2: the
+// one-tile halo kernel, 3: the streaming kernel with warp roles, 4: the
+// streaming kernel
 int g_conv_path = 0;
 
 bool halo_applies(const ConvP& P, int n_out) {
@@ -2794,7 +2793,7 @@ bool halo_applies(const ConvP& P, int n_out) {
 
 bool stream_applies(const ConvP& P, int n_out) {
     const int cin = P.src.ca + P.src.cb;
-    return (g_conv_path == 0 || g_conv_path == 3 || g_conv_path == 4) && cin <= 48 && n_out <= 48 &&
+    return (g_conv_path == 3 || g_conv_path == 4) && cin <= 48 && n_out <= 48 &&
            stream_smem_bytes(n_out, cin) <= 200 * 1024;
 }
 
@@ -3486,10 +3485,9 @@ int ccu_pack_weights(const float* w32, int cout, int cin, void* w, void* wt, voi
 
 int ccu_set_conv_path(int path) {
     if (path < 0 || path > 4)
-        return set_error(CCU_E_INVALID, "path must be 0 (plane-stationary, else streaming, else gathering kernel), "
-                                        "1 (gathering kernel), 2 (one-tile halo kernel where it applies), 3 (the "
-                                        "streaming kernel with warp roles) or 4 (path 0 without the "
-                                        "plane-stationary kernel)");
+        return set_error(CCU_E_INVALID, "path must be 0 (plane-stationary, else gathering kernel), 1 (gathering kernel), "
+                                        "2 (one-tile halo kernel where it applies), 3 (the streaming kernel with warp "
+                                        "roles where it applies) or 4 (the streaming kernel where it applies)");
     g_conv_path = path;
     return CCU_OK;
 }

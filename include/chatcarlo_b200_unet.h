@@ -56,7 +56,10 @@ int ccu_conv3d_head(const void* a, int ca, int batch, int d, int h, int w, const
 
 /* Weight gradient of ccu_conv3d: dw[27][cout][ca + cb] (FP32) +=
  * sum over voxels of dz[v][co] * input[v + tap][ci].  The voxels are split
- * into `slices` ranges reduced with atomics.  cout in {16, 32, 64, 128}.
+ * into `slices` ranges at least, reduced with atomics.  cout in {16, 32, 64,
+ * 128}.  The padding's input is zero: infinities and NaN of a voxel reach the
+ * taps and channels whose sums contain it (a kernel that finds some beside the
+ * padding takes hundreds of times as long).
  * The inputs are read by tensor-memory-accelerator tile loads of whole halo
  * planes.  A second input is first upsampled into a per-device buffer that
  * the first such call allocates (synchronously) and the process keeps; that
@@ -133,14 +136,13 @@ int ccu_pack_weights(const float* w32, int cout, int cin, void* w, void* wt, voi
  * passes with an FP32 partial sum when the weights do not fit shared memory
  * at once; the partial lives in a per-device workspace of n_vox x cout x 4
  * bytes that the first such call allocates and the process keeps) and for
- * 48, 96, 128 or 192 where one pass holds the weights, else the
- * persistent halo kernel that streams z-planes through a shared-memory ring
- * where it applies (input and output channels <= 48), else the gathering
- * kernel; 1 always the gathering kernel; 2 the one-tile halo kernel where
- * it applies (channels <= 48, h % 16 == 0, w % 8 == 0; for comparisons);
- * 3 the streaming kernel with warp roles (loader, MMA and epilogue warps
- * handing off through mbarriers) where the streaming kernel applies; 4
- * path 0 without the plane-stationary kernel.  Process-wide. */
+ * 48, 96, 128 or 192 where one pass holds the weights, else the gathering
+ * kernel; 1 always the gathering kernel.  The others are for comparisons,
+ * where they apply, else the gathering kernel: 2 the one-tile halo kernel
+ * (channels <= 48, h % 16 == 0, w % 8 == 0); 3 and 4 the persistent kernel
+ * that streams z-planes through a shared-memory ring (input and output
+ * channels <= 48), 3 with warp roles (loader, MMA and epilogue warps handing
+ * off through mbarriers).  Process-wide. */
 int ccu_set_conv_path(int path);
 
 /* Kernel of ccu_conv3d_wgrad: 0 (default) tile loads where they apply, else
