@@ -78,7 +78,7 @@ class BatchedRun:
             N.check(self.eng.lib.cc_ctx_set_launch(self.eng.ctx, 256, 0))
 
     def reset(self):
-        if self.tally:
+        if self.tally and self.plan is not None:        # closed: no grids to reset
             N.check(self.eng.lib.cc_batch_reset(self.plan))
 
     def run(self, seed: int, fluorescence: bool = True):

@@ -420,3 +420,11 @@ def test_grids_made_from_an_unfilled_grid_are_zeroed(monkeypatch):
     assert copy.deepcopy(g).kerma_keV.min() == 7
     assert {f.name for f in dataclasses.fields(g)} == {f.name for f in dataclasses.fields(new)} and "zeroed" not in repr(g)
     assert tally.VoxelGrid.from_bbox([0, 0, 0], [2, 2, 2], 1.0, zeroed=False).kerma_keV.min() == 7
+
+
+def test_reset_of_a_closed_batch_does_nothing():
+    from chatcarlo_b200.batched import BatchedRun
+    br = BatchedRun.__new__(BatchedRun)
+    br.eng, br.plan, br.tally, br.dgrids, br.scene_h, br.source_h = None, None, True, [], [], []
+    br.close()
+    br.reset()
