@@ -124,8 +124,11 @@ def _file_digest(path: str, mtime_ns: int, size: int) -> str:
 def _kernels_key(engine: Engine) -> str:
     """The build of the engine's kernels: a shape that was the fastest for
     others, with other registers and shared memory, is not taken over."""
-    st = os.stat(engine.lib._name)
-    return _file_digest(engine.lib._name, st.st_mtime_ns, st.st_size)
+    try:
+        st = os.stat(engine.lib._name)
+        return _file_digest(engine.lib._name, st.st_mtime_ns, st.st_size)
+    except OSError:                                  # replaced or gone since it was loaded
+        return "unknown"
 
 
 def workload_key(n_histories: list[int], slots: int, tally: bool) -> str:

@@ -402,6 +402,9 @@ def test_autotuned_shapes_belong_to_a_build_of_the_kernels(tmp_path, monkeypatch
     lib.write_bytes(b"another build")
     with pytest.raises(IndexError):
         batched.autotune([], [{}, {}], counts, engine=eng, candidates=[])
+    lib.unlink()                                      # rebuilt while loaded
+    with pytest.raises(IndexError):
+        batched.autotune([], [{}, {}], counts, engine=eng, candidates=[])
 
 
 def test_grids_made_from_an_unfilled_grid_are_zeroed(monkeypatch):
